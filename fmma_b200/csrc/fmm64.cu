@@ -709,7 +709,7 @@ template void solve_exact<float>(fmma_ctx*, int, int64_t, const float*, int64_t,
 // ---------------------------------------------------------------------------
 // operator cache
 // ---------------------------------------------------------------------------
-double* cached_op(fmma_ctx* ctx, const std::string& key, size_t bytes, bool* fresh) {
+double* cached_op(fmma_ctx* ctx, const std::string& key, size_t bytes, bool* fresh, const std::string* keep) {
   auto it = ctx->ops.find(key);
   if (it != ctx->ops.end()) {
     *fresh = false;
@@ -719,8 +719,14 @@ double* cached_op(fmma_ctx* ctx, const std::string& key, size_t bytes, bool* fre
   for (auto& kv : ctx->ops) total += kv.second.bytes;
   if (total + bytes > (size_t)16 << 30) {  // keep the cache under 16 GiB
     FMMA_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
-    for (auto& kv : ctx->ops) dev_free(ctx, kv.second.p, kv.second.bytes);
-    ctx->ops.clear();
+    for (auto o = ctx->ops.begin(); o != ctx->ops.end();) {
+      if (keep && o->first == *keep) {  // the caller still reads this one
+        ++o;
+        continue;
+      }
+      dev_free(ctx, o->second.p, o->second.bytes);
+      o = ctx->ops.erase(o);
+    }
   }
   DevBuf b;
   b.p = dev_alloc(ctx, bytes);

@@ -1105,7 +1105,7 @@ static void m2l_level_tc_t(fmma_ctx* ctx, int pair_pref, int units_pref, const L
   // split operator blocks (cached with the FP64 table)
   bool fresh = false;
   const size_t tab_bytes = (size_t)ntab * noff * KCH * 2 * Npad * F::ROW;
-  char* tab = (char*)cached_op(ctx, tabkey + (BF16 ? "_bf16" : "_tf32"), tab_bytes, &fresh);
+  char* tab = (char*)cached_op(ctx, tabkey + (BF16 ? "_bf16" : "_tf32"), tab_bytes, &fresh, &tabkey);
   if (fresh) {  // the ntab tables are contiguous: one conversion over ntab * noff operators
     int64_t total = (int64_t)ntab * noff * KCH * Npad * F::CHUNK;
     FMMA_LAUNCH(ctx, k_tc_table<BF16>, grid_for(total, 256, (int64_t)ctx->sm_count * 32), 256, 0, tab64, P, Npad64,

@@ -67,7 +67,10 @@ void solve_nrnmm(fmma_ctx* ctx, const SolveArgs& a, int nrn, int64_t nt, const T
 // rounded to the caller's type first (src/nrnmm.cpp:21-23).
 int nrnmm_default_grid(int64_t ns, int dim, bool isf);
 
-double* cached_op(fmma_ctx* ctx, const std::string& key, size_t bytes, bool* fresh);
+// Cached operator of `bytes` bytes (*fresh: just allocated, the caller fills
+// it).  An allocation that would take the cache over its limit empties it
+// first, except for the operator `keep` that the caller is still reading.
+double* cached_op(fmma_ctx* ctx, const std::string& key, size_t bytes, bool* fresh, const std::string* keep = nullptr);
 std::string op_key(const char* kind, fmma_ctx* ctx, int d, int n, double len, int a, int b);
 std::vector<int4> m2l_tiles(const Level& Lv, int R, int TM);
 
