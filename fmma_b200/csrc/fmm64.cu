@@ -1145,10 +1145,16 @@ void solve_forest(fmma_ctx* ctx, const SolveArgs& a, const std::vector<int64_t>&
         const Cube& c = tr.h_cube[(size_t)p];
         lens[(size_t)t] = isf ? (double)(c.Lenf / (float)(1 << l)) : c.Len / (double)(1 << l);
       }
-      bool fresh = false;
-      const size_t bytes = sizeof(double) * (size_t)ntab * F.noff * Npad * Kp;
       const std::string tkey = op_key("m2l64", ctx, d, n, ntab == 1 ? lens[0] : (double)hash_doubles(lens), Npad, Kp) +
                                "_t" + std::to_string(ntab);
+      const int engine = (size_t)v < ctx->m2l_engine.size() ? ctx->m2l_engine[(size_t)v] : -1;
+      const bool tensor = a.precision != FMMA_PREC_FP64 && engine != 0;
+      if (!tensor && m2l_sym_ok(ctx, d, n, Lv.nbox * R)) {
+        m2l_level_sym(ctx, Lv, v, n, Kpad, R, lens, tkey, node_all, Wm[(size_t)v], Wl[(size_t)v]);
+        continue;
+      }
+      bool fresh = false;
+      const size_t bytes = sizeof(double) * (size_t)ntab * F.noff * Npad * Kp;
       double* tab = cached_op(ctx, tkey, bytes, &fresh);
       if (fresh) {
         if (user) {
@@ -1171,8 +1177,7 @@ void solve_forest(fmma_ctx* ctx, const SolveArgs& a, const std::vector<int64_t>&
                                        0, tab);
         }
       }
-      const int engine = (size_t)v < ctx->m2l_engine.size() ? ctx->m2l_engine[(size_t)v] : -1;
-      if (a.precision != FMMA_PREC_FP64 && engine != 0) {
+      if (tensor) {
         // engine 1 + 2 i + pair: the 1-SM (pair 0) or 2-SM tensor-core kernel
         // with kM2LUnitChoices[i] units per stage; -1: the context's options
         const int pair = engine > 0 ? (engine - 1) & 1 : -1;

@@ -1,0 +1,678 @@
+// m2l_sym.cu — FP64 M2L in three dimensions for radial kernels, on the
+// reflection symmetry of the Chebyshev grid.
+//
+// The sum is that of src/fmm_core.cpp:375-455: Wl[b] = sum over the far slots
+// of K(offset) Wm[source].  The node set is symmetric (node n-1-k = -node k),
+// so for f(x, y) = g(|x - y|) the operator of an offset with some components
+// negated is the operator of |offset| with rows and columns reversed along
+// those dimensions.  In the basis of even and odd parts along every dimension
+// (x_k + x_{n-1-k}, x_k - x_{n-1-k}) a reversal is a sign per parity block, so
+// the up to eight sources at the offsets (+-o_0, +-o_1, +-o_2) of one target
+// share the 8 x 8 parity blocks of one operator:
+//
+//   y_a += sum_b K_ab z_{a^b, b},   z_{c, b} = sum_g (-1)^{c.g} x_{g, b}
+//
+// (a, b: parity of the target and source block, one bit per dimension; g: the
+// signs of the offset): P^2 multiply-adds for eight sources instead of 8 P^2,
+// and the z by an 8-point Walsh-Hadamard butterfly of the gathered sources.
+// Along a dimension with o_q = 0 there is one source and K_ab = 0 unless
+// a_q = b_q, which halves the operator instead.  The 189 far slots of a target
+// fall into 56 orbits worth 39.5 P^2 multiply-adds (189 P^2 before).
+//
+// FP64 tensor (DMMA) bound.  A block owns 8 MB target rows (box x rhs) of one
+// child-parity class.  Warp w accumulates the rows' outputs of one parity a
+// (w and 7 - w share a scheduler, so with an odd node count, where an
+// even-parity block is larger, each scheduler has the same number of
+// columns).  A pipeline stage is two K steps of 4: the threads gather the 8
+// source values of a (row, k), run the butterfly in registers and store the z
+// for the next stage while the current one is multiplied; operator fragments
+// are read from L2 straight into registers (a warp shares them with no other
+// warp of the block), one stage ahead.  Row groups of 8 with no source in an
+// orbit are skipped.
+#include <algorithm>
+#include <cmath>
+
+#include "fmm_stages.cuh"
+#include "fmma_internal.cuh"
+#include "kernels.cuh"
+#include "solver.cuh"
+
+namespace fmma_b200 {
+
+namespace {
+
+constexpr int kOrbits = 56;       // |o| in {0..3}^3 without {0,1}^3
+constexpr int kSymThreads = 256;
+constexpr int kSymMaxStages = 64; // stages of one orbit: 8 blocks of up to 16 K steps, two per stage
+constexpr int kSymSlots = 189;
+
+// Constant geometry of one node count, uploaded in front of the operators.
+struct SymGeom {
+  int n, he, ho;         // nodes per dimension, even and odd parts per dimension
+  int KB, NB, MB;        // padded block length, column groups of 8 per warp, row groups of 8 per block
+  int P, total;          // coefficients, pipeline stages of one operator set
+  int size[8], off[8];   // coefficients of a parity block and its offset in a folded row of P
+  int nst[8];            // stages of an orbit by its zero mask
+  int zmask[kOrbits];    // bit q: o_q = 0
+  int stage0[kOrbits];   // first stage of the orbit's operator
+  int desc[8][kSymMaxStages][2];  // K step: b0 | k4 << 3, or -1 (no step)
+  int slot[8][kOrbits][8];        // far slot of (class, orbit, signs), -1 where there is none
+  int rep[kOrbits][3];            // |o|
+};
+
+int block_size(int he, int ho, int b) {
+  int s = 1;
+  for (int q = 0; q < 3; ++q) s *= ((b >> q) & 1) ? ho : he;
+  return s;
+}
+
+SymGeom make_geom(int n) {
+  SymGeom g;
+  g.n = n;
+  g.he = (n + 1) / 2;
+  g.ho = n / 2;
+  g.P = n * n * n;
+  const int full = g.he * g.he * g.he;
+  g.KB = (full + 3) / 4 * 4;
+  g.NB = full <= 8 ? 1 : (full <= 32 ? 4 : 8);
+  g.MB = g.NB == 8 ? 4 : 8;
+  int o = 0;
+  for (int b = 0; b < 8; ++b) {
+    g.size[b] = block_size(g.he, g.ho, b);
+    g.off[b] = o;
+    o += g.size[b];
+  }
+  // K steps by zero mask: the blocks b0 over the nonzero dimensions; along
+  // the zero ones the step spans the blocks of both parities (the even one
+  // is the longer)
+  for (int z = 0; z < 8; ++z) {
+    int steps = 0;
+    for (int s = 0; s < kSymMaxStages; ++s) g.desc[z][s][0] = g.desc[z][s][1] = -1;
+    if (z != 7)
+      for (int b0 = 0; b0 < 8; ++b0) {
+        if (b0 & z) continue;
+        const int k4s = (g.size[b0] + 3) / 4;
+        for (int k4 = 0; k4 < k4s; ++k4, ++steps) g.desc[z][steps / 2][steps % 2] = b0 | (k4 << 3);
+      }
+    g.nst[z] = (steps + 1) / 2;
+  }
+  int w = 0;
+  g.total = 0;
+  int orbit_of[64];
+  for (int i = 0; i < 64; ++i) {
+    const int r[3] = {i / 16, (i / 4) % 4, i % 4};
+    orbit_of[i] = -1;
+    if (r[0] <= 1 && r[1] <= 1 && r[2] <= 1) continue;
+    orbit_of[i] = w;
+    int z = 0;
+    for (int q = 0; q < 3; ++q) {
+      g.rep[w][q] = r[q];
+      if (r[q] == 0) z |= 1 << q;
+    }
+    g.zmask[w] = z;
+    g.stage0[w] = g.total;
+    g.total += g.nst[z];
+    ++w;
+  }
+  const FarTables& F = far_tables(3);
+  for (int c = 0; c < 8; ++c) {
+    for (int i = 0; i < kOrbits; ++i)
+      for (int s = 0; s < 8; ++s) g.slot[c][i][s] = -1;
+    for (int q = 0; q < F.nfar; ++q) {
+      const int* v = F.off_vec[F.slot_off[c][q]];
+      int sg = 0;
+      for (int e = 0; e < 3; ++e) sg |= v[e] < 0 ? 1 << e : 0;
+      g.slot[c][orbit_of[std::abs(v[0]) * 16 + std::abs(v[1]) * 4 + std::abs(v[2])]][sg] = q;
+    }
+  }
+  return g;
+}
+
+const SymGeom& sym_geom(int n) {
+  static const SymGeom g[6] = {make_geom(3), make_geom(4), make_geom(5), make_geom(6), make_geom(7), make_geom(8)};
+  return g[n - 3];
+}
+
+// Half-index h of a node triple, its parity block offsets and node numbers.
+struct Half {
+  int j[3], mid;  // mid bit q: j_q is the centre node (odd n), which has no odd part
+  __device__ __forceinline__ Half(int h, int he, int ho) {
+    j[2] = h % he;
+    j[1] = (h / he) % he;
+    j[0] = h / (he * he);
+    mid = 0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) mid |= j[q] >= ho ? 1 << q : 0;
+  }
+  __device__ __forceinline__ int in_block(int b, int he, int ho) const {
+    const int s1 = (b & 2) ? ho : he, s2 = (b & 4) ? ho : he;
+    return (j[0] * s1 + j[1]) * s2 + j[2];
+  }
+  __device__ __forceinline__ int node(int sg, int n) const {
+    int k = 0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) k = k * n + (((sg >> q) & 1) ? n - 1 - j[q] : j[q]);
+    return k;
+  }
+};
+
+__device__ __forceinline__ void butterfly8(double* v) {
+#pragma unroll
+  for (int q = 1; q < 8; q <<= 1)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (!(i & q)) {
+        const double u = v[i], t = v[i | q];
+        v[i] = u + t;
+        v[i | q] = u - t;
+      }
+}
+
+// Operators in the parity basis, one warp per (table, orbit, i, j) with i, j
+// half-indices: the 64 values of f over the reversals of i and j (two per
+// lane), transformed along both by shuffles, give the entry (i, j) of all 64
+// blocks.  The factor 1/64 holds the halves of the inverse transforms on both
+// sides (exact).
+template <int KID>
+__global__ void __launch_bounds__(256) k_sym_table(const double* __restrict__ lens, int ntab,
+                                                   const double* __restrict__ node_all,
+                                                   const SymGeom* __restrict__ gp, double p0,
+                                                   double* __restrict__ tab) {
+  const SymGeom& g = *gp;
+  const int n = g.n, he = g.he, ho = g.ho, NB = g.NB;
+  const int nh = he * he * he, lane = threadIdx.x & 31;
+  const int64_t total = (int64_t)ntab * kOrbits * nh * nh;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < total; e += nw) {
+    const int hj = (int)(e % nh), hi = (int)(e / nh % nh), w = (int)(e / ((int64_t)nh * nh) % kOrbits);
+    const int64_t t = e / ((int64_t)nh * nh * kOrbits);
+    const double len = lens[t];
+    const Half I(hi, he, ho), J(hj, he, ho);
+    double v[2];  // index = row reversal * 8 + column reversal = lane + 32 u
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int kl = I.node((lane >> 3) + 4 * u, n), km = J.node(lane & 7, n);
+      double x[3], y[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        x[q] = len * (node_all[kl * 3 + q] / 2);
+        y[q] = len * ((double)g.rep[w][q] + node_all[km * 3 + q] / 2);
+      }
+      v[u] = keval<KID, 3>(x, y, p0);
+    }
+    const double s = v[0] + v[1], d = v[0] - v[1];
+    v[0] = s;
+    v[1] = d;
+#pragma unroll
+    for (int q = 1; q < 32; q <<= 1)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const double o = __shfl_xor_sync(0xffffffffu, v[u], q);
+        v[u] = (lane & q) ? o - v[u] : v[u] + o;
+      }
+    const int z = g.zmask[w], b = lane & 7, b0 = b & ~z;
+    if (b & J.mid) continue;
+    const int k = J.in_block(b, he, ho);
+    int step = k >> 2;  // K steps of the blocks before b0
+    for (int c = 0; c < b0; ++c)
+      if (!(c & z)) step += (g.size[c] + 3) / 4;
+    double* base = tab + (t * g.total + g.stage0[w] + (step >> 1)) * (int64_t)(8 * 2 * 32) * NB;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int a = (lane >> 3) + 4 * u;
+      if ((a & I.mid) || ((a ^ b) & z)) continue;
+      const int col = I.in_block(a, he, ho);
+      base[(((int64_t)a * 2 + (step & 1)) * 32 + (col & 7) * 4 + (k & 3)) * NB + (col >> 3)] = v[u] * (1.0 / 64);
+    }
+  }
+}
+
+// out[row][b][KB]: the even and odd parts of Wm's rows (box x rhs), zero padded,
+// and a row of zeros behind them (the source of an empty slot).
+__global__ void __launch_bounds__(256) k_sym_fold(const double* __restrict__ Wm, int64_t nrows, int Kpad,
+                                                  const SymGeom* __restrict__ gp, double* __restrict__ out) {
+  const int n = gp->n, he = gp->he, ho = gp->ho, KB = gp->KB;
+  const int nh = he * he * he, lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row <= nrows; row += nw) {
+    const double* w = Wm + row * Kpad;
+    double* o = out + row * 8 * KB;
+    if (row == nrows) {
+      for (int k = lane; k < 8 * KB; k += 32) o[k] = 0.0;
+      break;
+    }
+    for (int h = lane; h < nh; h += 32) {
+      const Half H(h, he, ho);
+      double v[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s) v[s] = (s & H.mid) ? 0.0 : w[H.node(s, n)];
+      butterfly8(v);
+#pragma unroll
+      for (int b = 0; b < 8; ++b)
+        if (!(b & H.mid)) o[b * KB + H.in_block(b, he, ho)] = v[b];
+    }
+#pragma unroll
+    for (int b = 0; b < 8; ++b)
+      for (int k = gp->size[b] + lane; k < KB; k += 32) o[b * KB + k] = 0.0;
+  }
+}
+
+// Wl rows from their parity blocks: the nparts partial sums in order, then the
+// inverse transform (its halves are in the operators).  With one part the
+// blocks lie in Wl itself and a warp turns a row in place.
+__global__ void __launch_bounds__(256) k_sym_unfold(const double* __restrict__ part, int nparts, int64_t nv, int R,
+                                                    const int* __restrict__ row_box, int Kpad,
+                                                    const SymGeom* __restrict__ gp, double* __restrict__ Wl) {
+  const int n = gp->n, he = gp->he, ho = gp->ho, P = gp->P;
+  const int nh = he * he * he, lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < nv; v += nw) {
+    const int64_t brow = v / R;
+    double* dst = Wl + ((int64_t)row_box[brow] * R + (v - brow * R)) * Kpad;
+    const double* src = nparts > 1 ? part + v * P : dst;
+    double y[2][8];  // at most 64 half-indices: two per lane
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int h = lane + 32 * u;
+      const Half H(h < nh ? h : 0, he, ho);
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        double s = 0.0;
+        if (h < nh && !(a & H.mid)) {
+          const int64_t k = gp->off[a] + H.in_block(a, he, ho);
+          s = src[k];
+          for (int p = 1; p < nparts; ++p) s += part[((int64_t)p * nv + v) * P + k];
+        }
+        y[u][a] = s;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int h = lane + 32 * u;
+      if (h >= nh) continue;
+      const Half H(h, he, ho);
+      butterfly8(y[u]);
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (!(s & H.mid)) dst[H.node(s, n)] = y[u][s];
+    }
+    __syncwarp();
+  }
+}
+
+struct SymParams {
+  const int4* tiles;
+  const int* il;
+  const int* row_box;
+  const SymGeom* geom;
+  const double* W;     // folded sources [box * R + r][8][KB]
+  const double* tab;   // [table][stage][a][step][lane][NB]
+  const int* part_lo;  // [gridDim.y + 1] first orbit of each part
+  double* Wl;          // parity blocks into Wl (one part) ...
+  double* part;        // ... or [part][virtual row][P]
+  int64_t nv;          // virtual rows (rows x rhs)
+  int R, Kpad;
+  int zero_row;        // the row of zeros of W
+};
+
+__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
+template <int NB, int MB>
+struct SymShape {
+  static constexpr int TM = 8 * MB;
+  static constexpr int TPR = kSymThreads / TM;       // threads gathering one row
+  static constexpr int EPT = 8 / TPR;                // values of a stage's 8 per thread
+  static constexpr int PLANE = 8 * TM * 4 + 8;       // doubles of one K step's z (padded by 64 B)
+  static constexpr int ILS = TM + 1;                 // stride of a slot's source list
+  static constexpr size_t kSmem =
+      sizeof(double) * 4 * PLANE + sizeof(int) * (kSymSlots * ILS + 8 * kSymMaxStages * 2 + kOrbits * 8 + kOrbits * 5);
+};
+
+template <int NB, int MB>
+__global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
+  using S = SymShape<NB, MB>;
+  constexpr int TM = S::TM, EPT = S::EPT;
+  constexpr int kTabStage = 8 * 2 * 32 * NB;  // doubles of a stage's operator
+  extern __shared__ __align__(16) double sym_smem[];
+  double* const sZ = sym_smem;                                   // [2][2][PLANE]
+  int4* const sAct = reinterpret_cast<int4*>(sZ + 4 * S::PLANE); // active orbits: (orbit | zero mask << 8, stages, row groups, first stage)
+  int* const sIl = reinterpret_cast<int*>(sAct + kOrbits);       // [slot][ILS] source row (box * R + r)
+  int* const sDesc = sIl + kSymSlots * S::ILS;                   // [zero mask][stage][2]
+  int* const sSlot = sDesc + 8 * kSymMaxStages * 2;              // [orbit][8]
+  int* const sMask = sSlot + kOrbits * 8;                        // [orbit] row groups with a source
+  __shared__ int s_nact;
+  const SymGeom& g = *p.geom;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int a = warp < 4 ? warp : 11 - warp;  // output parity of this warp
+  const int4 tile = p.tiles[blockIdx.x];
+  const int cls = tile.x, v0 = tile.y, vcnt = tile.z;
+  const int KB = g.KB, R = p.R, none = p.zero_row;
+  const int lo = p.part_lo[blockIdx.y], hi = p.part_lo[blockIdx.y + 1];
+
+  for (int i = tid; i < TM * kSymSlots; i += kSymThreads) {
+    const int r = i / kSymSlots, q = i - r * kSymSlots;
+    int s = none;
+    if (r < vcnt) {
+      const int v = v0 + r, brow = v / R;
+      const int sb = p.il[(int64_t)brow * kSymSlots + q];
+      if (sb >= 0) s = sb * R + (v - brow * R);
+    }
+    sIl[q * S::ILS + r] = s;
+  }
+  for (int i = tid; i < 8 * kSymMaxStages * 2; i += kSymThreads) sDesc[i] = (&g.desc[0][0][0])[i];
+  for (int i = tid; i < kOrbits * 8; i += kSymThreads) sSlot[i] = g.slot[cls][i >> 3][i & 7];
+  for (int i = tid; i < kOrbits; i += kSymThreads) sMask[i] = 0;
+  __syncthreads();
+  for (int i = tid; i < (hi - lo) * MB; i += kSymThreads) {
+    const int w = lo + i / MB, mb = i % MB;
+    bool any = false;
+    for (int s = 0; s < 8; ++s) {
+      const int q = sSlot[w * 8 + s];
+      if (q < 0) continue;
+      for (int r = 0; r < 8; ++r) any |= sIl[q * S::ILS + mb * 8 + r] != none;
+    }
+    if (any) atomicOr(&sMask[w], 1 << mb);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int base = 0;
+    for (int w0 = 0; w0 < kOrbits; w0 += 32) {
+      const int w = w0 + lane;
+      const bool on = w < kOrbits && sMask[w] != 0;
+      const unsigned m = __ballot_sync(0xffffffffu, on);
+      if (on) {
+        const int z = g.zmask[w];
+        sAct[base + __popc(m & ((1u << lane) - 1u))] = make_int4(w | (z << 8), g.nst[z], sMask[w], g.stage0[w]);
+      }
+      base += __popc(m);
+    }
+    if (lane == 0) s_nact = base;
+  }
+  __syncthreads();
+  const int nact = s_nact;
+
+  // gather role: one row, EPT consecutive k of one K step
+  const int grow = tid / S::TPR, gp = tid % S::TPR;
+  const int gks = EPT == 2 ? gp >> 1 : gp >> 2;
+  const int gk = EPT == 2 ? (gp & 1) * 2 : gp & 3;
+  const int ggrp = grow >> 3;
+  // a pipeline stage: zero mask and row groups of its orbit, K steps, operator stage
+  struct Stage {
+    int z, mask, step[2], tab;
+  };
+  Stage cur{}, nxt{}, fut{};          // multiplied, stored and gathered next
+  int oi = 0, st = -1, nst = 0;       // gather cursor over the active orbits' stages
+  unsigned off[8];                    // the cursor's sources, in units of 4 doubles
+  double raw[8][EPT];
+  // moves the cursor on and issues the stage's loads; false at the end
+  auto gather = [&]() -> bool {
+    if (++st >= nst) {
+      if (st > 0) ++oi;
+      if (oi >= nact) return false;
+      const int4 f = sAct[oi];
+      st = 0;
+      nst = f.y;
+      fut.z = f.x >> 8;
+      fut.mask = f.z;
+      fut.tab = f.w - 1;
+      const int* sl = sSlot + (f.x & 255) * 8;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int q = sl[j & ~fut.z];
+        const int s = q >= 0 ? sIl[q * S::ILS + grow] : none;
+        off[j] = (unsigned)s * (unsigned)(2 * KB) + (unsigned)((j & fut.z) * (KB / 4));
+      }
+    }
+    ++fut.tab;
+    const int* ds = sDesc + (fut.z * kSymMaxStages + st) * 2;
+    fut.step[0] = ds[0];
+    fut.step[1] = ds[1];
+    const int step = max(ds[gks], 0);  // no step: any data, not multiplied
+    if ((fut.mask >> ggrp) & 1) {      // warp-uniform
+      const char* src = reinterpret_cast<const char*>(p.W + (step & 7) * KB + (step >> 3) * 4 + gk);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const char* sj = src + (uint64_t)off[j] * 32u;
+        if constexpr (EPT == 2) {
+          const double2 t = __ldg(reinterpret_cast<const double2*>(sj));
+          raw[j][0] = t.x;
+          raw[j][EPT - 1] = t.y;
+        } else {
+          raw[j][0] = __ldg(reinterpret_cast<const double*>(sj));
+        }
+      }
+    }
+    return true;
+  };
+  // the butterfly over the signs of stage `nxt`, its z stored in buffer buf
+  auto put = [&](int buf) {
+    if (!((nxt.mask >> ggrp) & 1)) return;
+#pragma unroll
+    for (int q = 1; q < 8; q <<= 1)
+      if (!(nxt.z & q)) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (!(j & q)) {
+#pragma unroll
+            for (int e = 0; e < EPT; ++e) {
+              const double u = raw[j][e], t = raw[j | q][e];
+              raw[j][e] = u + t;
+              raw[j | q][e] = u - t;
+            }
+          }
+      }
+    double* dst = sZ + (buf * 2 + gks) * S::PLANE + grow * 4 + gk;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if constexpr (EPT == 2)
+        *reinterpret_cast<double2*>(dst + j * TM * 4) = make_double2(raw[j][0], raw[j][EPT - 1]);
+      else
+        dst[j * TM * 4] = raw[j][0];
+    }
+  };
+
+  double acc[MB][NB][2];
+#pragma unroll
+  for (int i = 0; i < MB; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int nba = (g.size[a] + 7) >> 3;  // column groups of this parity
+
+  const double* const tabw = p.tab + (int64_t)tile.w * g.total * kTabStage + (int64_t)a * (2 * 32 * NB) + lane * NB;
+  double bf[2][NB];
+  auto load_b = [&](int stage, int ks) {
+    const double* src = tabw + (int64_t)stage * kTabStage + ks * (32 * NB);
+    if constexpr (NB == 1) {
+      bf[ks][0] = __ldg(src);
+    } else {
+#pragma unroll
+      for (int j = 0; j < NB; j += 2) {
+        const double2 t = __ldg(reinterpret_cast<const double2*>(src + j));
+        bf[ks][j] = t.x;
+        bf[ks][j + (NB > 1 ? 1 : 0)] = t.y;
+      }
+    }
+  };
+
+  if (gather()) {
+    nxt = fut;
+    put(0);
+    bool hn = gather();  // a stage after the current one
+    cur = nxt;
+    nxt = fut;
+    load_b(cur.tab, 0);
+    load_b(cur.tab, 1);
+    int buf = 0;
+    // Of the two warps of a scheduler one stores the next stage's z before
+    // its multiplications and the other after them, so that one's butterfly
+    // and stores overlap the other's DMMAs.
+    const bool early = warp < 4;
+    bool hf = false;  // a stage after the next one
+    while (true) {
+      __syncthreads();  // this stage's z stored by all; the other buffer read by all
+      if (early && hn) {
+        put(buf ^ 1);
+        hf = gather();
+      }
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks) {
+        const int step = cur.step[ks];
+        if (step >= 0) {
+          const double* A = sZ + (buf * 2 + ks) * S::PLANE + (a ^ (step & 7)) * (TM * 4) + lane;
+          double av[MB];
+#pragma unroll
+          for (int mb = 0; mb < MB; ++mb) av[mb] = A[mb * 32];
+          if (cur.mask == (1 << MB) - 1) {
+#pragma unroll
+            for (int nb = 0; nb < NB; ++nb)
+              if (nb < nba) {
+#pragma unroll
+                for (int mb = 0; mb < MB; ++mb) dmma(acc[mb][nb][0], acc[mb][nb][1], av[mb], bf[ks][nb]);
+              }
+          } else {
+#pragma unroll
+            for (int mb = 0; mb < MB; ++mb)
+              if ((cur.mask >> mb) & 1) {
+#pragma unroll
+                for (int nb = 0; nb < NB; ++nb)
+                  if (nb < nba) dmma(acc[mb][nb][0], acc[mb][nb][1], av[mb], bf[ks][nb]);
+              }
+          }
+        }
+        if (hn) load_b(nxt.tab, ks);
+      }
+      if (!hn) break;
+      if (!early) {
+        put(buf ^ 1);
+        hf = gather();
+      }
+      cur = nxt;
+      nxt = fut;
+      hn = hf;
+      buf ^= 1;
+    }
+  }
+
+  const int size = g.size[a], first = g.off[a];
+#pragma unroll
+  for (int mb = 0; mb < MB; ++mb) {
+    const int i = mb * 8 + (lane >> 2);
+    if (i >= vcnt) continue;
+    const int64_t v = v0 + i;
+    double* dst;
+    if (gridDim.y > 1) {
+      dst = p.part + ((int64_t)blockIdx.y * p.nv + v) * g.P + first;
+    } else {
+      const int64_t brow = v / R;
+      dst = p.Wl + ((int64_t)p.row_box[brow] * R + (v - brow * R)) * p.Kpad + first;
+    }
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      const int col = nb * 8 + (lane & 3) * 2;
+      if (col < size) dst[col] = acc[mb][nb][0];
+      if (col + 1 < size) dst[col + 1] = acc[mb][nb][1];
+    }
+  }
+}
+
+template <int NB, int MB>
+void launch_sym(fmma_ctx* ctx, const SymParams& p, int ntiles, int nparts) {
+  constexpr size_t smem = SymShape<NB, MB>::kSmem;
+  static bool attr_set = false;
+  if (!attr_set) {
+    FMMA_CHECK_CUDA(cudaFuncSetAttribute(k_m2l_sym<NB, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr_set = true;
+  }
+  FMMA_LAUNCH(ctx, (k_m2l_sym<NB, MB>), dim3((unsigned)ntiles, (unsigned)nparts), kSymThreads, smem, p);
+}
+
+struct SymTableLaunch {
+  template <int KID, int D>
+  static void run(fmma_ctx* ctx, const double* lens, int ntab, const double* node_all, const SymGeom* g, int64_t total,
+                  double p0, double* tab) {
+    if constexpr (D == 3 && (KID == FMMA_KERNEL_INV_R || KID == FMMA_KERNEL_INV_R_SAFE || KID == FMMA_KERNEL_LOG_R ||
+                             KID == FMMA_KERNEL_GAUSSIAN || KID == FMMA_KERNEL_MULTIQUADRIC))
+      FMMA_LAUNCH(ctx, (k_sym_table<KID>), grid_for(total * 32, 256, (int64_t)ctx->sm_count * 16), 256, 0, lens, ntab,
+                  node_all, g, p0, tab);
+  }
+};
+
+// blocks aimed at per level: about four per SM, so that the last wave is a
+// small part of the level
+constexpr int kSymBlocksPerSm = 4;
+constexpr int kSymMaxParts = 16;
+
+}  // namespace
+
+bool m2l_sym_ok(const fmma_ctx* ctx, int d, int n, int64_t rows) {
+  // source rows are addressed in units of 4 doubles, in 32 bits
+  if (rows >= ((int64_t)1 << 25)) return false;
+  switch (ctx->kernel_id) {
+    case FMMA_KERNEL_INV_R:
+    case FMMA_KERNEL_INV_R_SAFE:
+    case FMMA_KERNEL_LOG_R:
+    case FMMA_KERNEL_GAUSSIAN:
+    case FMMA_KERNEL_MULTIQUADRIC: return d == 3 && n >= 3 && n <= 8;
+    default: return false;
+  }
+}
+
+void m2l_level_sym(fmma_ctx* ctx, const Level& Lv, int v, int n, int Kpad, int R, const std::vector<double>& lens,
+                   const std::string& tabkey, const double* node_all, const double* Wm, double* Wl) {
+  const SymGeom& g = sym_geom(n);
+  const int ntab = (int)lens.size();
+  // geometry and operators in one cached block
+  constexpr size_t kGeomBytes = (sizeof(SymGeom) + 255) / 256 * 256;
+  const size_t per_tab = (size_t)g.total * 8 * 2 * 32 * g.NB;
+  bool fresh = false;
+  char* blk = reinterpret_cast<char*>(cached_op(ctx, "sym_" + tabkey, kGeomBytes + sizeof(double) * per_tab * ntab,
+                                                &fresh));
+  const SymGeom* dg = reinterpret_cast<const SymGeom*>(blk);
+  double* tab = reinterpret_cast<double*>(blk + kGeomBytes);
+  if (fresh) {
+    upload(ctx, blk, &g, sizeof(SymGeom));
+    double* dl = ctx_buf_t<double>(ctx, "table_lens", (size_t)ntab);
+    upload(ctx, dl, lens.data(), sizeof(double) * (size_t)ntab);
+    FMMA_CHECK_CUDA(cudaMemsetAsync(tab, 0, sizeof(double) * per_tab * ntab, ctx->stream));
+    const int64_t nh = (int64_t)g.he * g.he * g.he;
+    dispatch_kernel<SymTableLaunch>(ctx->kernel_id, 3, ctx, dl, ntab, node_all, dg, (int64_t)ntab * kOrbits * nh * nh,
+                                    ctx->p0, tab);
+  }
+  const int TM = 8 * g.MB;
+  std::vector<int4> tiles = m2l_tiles(Lv, R, TM);
+  const int ntiles = (int)tiles.size();
+  int4* dt = ctx_buf_t<int4>(ctx, "m2l_tiles" + std::to_string(v), tiles.size());
+  upload(ctx, dt, tiles.data(), sizeof(int4) * tiles.size());
+
+  // orbits split over blocks on levels with few tiles, by equal stage counts
+  int nparts = (ctx->sm_count * kSymBlocksPerSm + ntiles - 1) / ntiles;
+  nparts = std::max(1, std::min(nparts, kSymMaxParts));
+  std::vector<int> lo((size_t)nparts + 1, 0);
+  for (int s = 1, w = 0; s < nparts; ++s) {
+    while (w < kOrbits && (int64_t)g.stage0[w] * nparts < (int64_t)s * g.total) ++w;
+    lo[(size_t)s] = w;
+  }
+  lo[(size_t)nparts] = kOrbits;
+  int* dlo = ctx_buf_t<int>(ctx, "sym_parts" + std::to_string(v), lo.size());
+  upload(ctx, dlo, lo.data(), sizeof(int) * lo.size());
+
+  const int64_t nv = Lv.nrow * R, nsrc = Lv.nbox * R;
+  double* W = ctx_buf_t<double>(ctx, "sym_src", (size_t)(nsrc + 1) * 8 * g.KB);
+  double* part = nparts > 1 ? ctx_buf_t<double>(ctx, "sym_part", (size_t)nparts * nv * g.P) : nullptr;
+  SymParams p{dt, Lv.il, Lv.row_box, dg, W, tab, dlo, Wl, part, nv, R, Kpad, (int)nsrc};
+  kernel_timer_begin(ctx);
+  const int64_t wcap = (int64_t)ctx->sm_count * 32;
+  FMMA_LAUNCH(ctx, k_sym_fold, grid_for((nsrc + 1) * 32, 256, wcap), 256, 0, Wm, nsrc, Kpad, dg, W);
+  if (g.NB == 1) launch_sym<1, 8>(ctx, p, ntiles, nparts);
+  else if (g.NB == 4) launch_sym<4, 8>(ctx, p, ntiles, nparts);
+  else launch_sym<8, 4>(ctx, p, ntiles, nparts);
+  FMMA_LAUNCH(ctx, k_sym_unfold, grid_for(nv * 32, 256, wcap), 256, 0, part, nparts, nv, R, Lv.row_box, Kpad, dg, Wl);
+  kernel_timer_end(ctx, 2.0 * g.P * g.P * R, v);
+}
+
+}  // namespace fmma_b200

@@ -33,6 +33,14 @@ void m2l_level_tc(fmma_ctx* ctx, bool bf16, int pair, int units, const Level& Lv
                   int Kpad64, int R, const double* Wm64, double* Wl64, const double* tab64, int Npad64,
                   const std::string& tabkey, int noff, int ntab);
 
+// FP64 M2L of one virtual level on the reflection symmetry of the Chebyshev
+// grid (m2l_sym.cu): radial built-in kernels in 3-D with 3 to 8 nodes per
+// dimension.  rows: boxes x rhs of the level; lens: box width of each of its
+// operator tables.
+bool m2l_sym_ok(const fmma_ctx* ctx, int d, int n, int64_t rows);
+void m2l_level_sym(fmma_ctx* ctx, const Level& Lv, int v, int n, int Kpad, int R, const std::vector<double>& lens,
+                   const std::string& tabkey, const double* node_all, const double* Wm, double* Wl);
+
 // Mixed-precision near field: FP32 box-local evaluations, compensated sums.
 // wst_ready: the FP32 weight rows were written by gather_weights_mixed.
 template <typename T>

@@ -1,0 +1,103 @@
+"""The FP64 M2L on the reflection symmetry of the grid (radial kernels in 3-D, 3 to 8 nodes per
+dimension) against the oracle.
+
+Tolerance: relative L2 <= 1e-12, that of the plain FP64 parity tests: the same sums in another order,
+P terms per far box and at most 189 boxes, in FP64 (2^-53 sqrt(189 * 512) ~ 3e-14).
+
+Sizes where it can go wrong: every node count of its range (odd ones have a centre node without an odd
+part), tiles of 64 (32 from 7 nodes) rows with a few rows only and with remainders, levels split over
+several blocks and levels that are not, orbits with no source for some row groups (clustered points),
+several right-hand sides sharing a tile, and several problems with operator tables of their own."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+KERNELS = [(0, 0.0), (1, 0.0), (3, 0.0), (4, 0.3), (5, 1e-2)]  # 1/r, 1/r (0 at r = 0), log r, Gaussian, multiquadric
+TOL = 1e-12
+
+
+def _points(r, n, clustered):
+    if not clustered:
+        return r.random((n, 3))
+    c = r.uniform(0.1, 0.9, (4, 3))
+    return np.clip(c[r.integers(0, 4, n)] + 0.03 * r.standard_normal((n, 3)), 0.0, 1.0)
+
+
+@pytest.mark.parametrize("poly_ord", [2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("clustered", [False, True])
+def test_every_node_count(ctx, oracle, poly_ord, clustered):
+    r = np.random.default_rng(poly_ord)
+    depth = 4 if poly_ord <= 4 else 3
+    n = 700 if poly_ord == 7 else (3000 if clustered else 2500)
+    t, s, w = _points(r, n, clustered), _points(r, n + 77, clustered), r.uniform(-1, 1, n + 77)
+    kid, p0 = KERNELS[poly_ord % len(KERNELS)]
+    ctx.set_kernel(kid, p0)
+    # 8 nodes: dense leaves need more shared memory in the target-lane L2P than there is
+    ctx.set_schedule_options(l2p_mode=2 if poly_ord == 7 else 0)
+    try:
+        got, _ = ctx.solve(t, s, w, poly_ord=poly_ord, depth=depth)
+    finally:
+        ctx.set_schedule_options()
+    want, _ = oracle.fmm(3, kid, p0, poly_ord, depth, 1, t, s, w)
+    assert rel_l2(got, want) <= TOL
+
+
+@pytest.mark.parametrize("kid,p0", KERNELS)
+def test_every_radial_kernel(ctx, oracle, kid, p0):
+    r = np.random.default_rng(17 + kid)
+    t, s, w = r.random((900, 3)), r.random((1100, 3)) * [1.0, 0.4, 0.7], r.standard_normal(1100)
+    ctx.set_kernel(kid, p0)
+    got, _ = ctx.solve(t, s, w, poly_ord=3, depth=4)
+    want, _ = oracle.fmm(3, kid, p0, 3, 4, 1, t, s, w)
+    assert rel_l2(got, want) <= TOL
+
+
+def test_right_hand_sides_and_unsplit_level(ctx, oracle):
+    # 4096 leaves x 7 rhs = 56 tiles per class, 448 in all: the leaf level in one or two parts, the others split
+    r = np.random.default_rng(5)
+    t, s, w = r.random((20000, 3)), r.random((20000, 3)), r.standard_normal((7, 20000))
+    ctx.set_kernel("inv_r_safe")
+    got, _ = ctx.solve(t, s, w, poly_ord=4, depth=5)
+    for k in (0, 6):
+        want, _ = oracle.fmm(3, 1, 0.0, 4, 5, 1, t, s, w[k])
+        assert rel_l2(got[k], want) <= TOL
+
+
+def test_few_points(ctx, oracle):
+    r = np.random.default_rng(8)
+    for n in (1, 2, 9, 40):
+        t, s, w = r.random((n, 3)), r.random((n, 3)), r.standard_normal(n)
+        ctx.set_kernel("inv_r_safe")
+        got, _ = ctx.solve(t, s, w, poly_ord=4, depth=4)
+        want, _ = oracle.fmm(3, 1, 0.0, 4, 4, 1, t, s, w)
+        assert np.linalg.norm(got - want) <= TOL * max(np.linalg.norm(want), 1e-300) + 1e-300
+
+
+def test_forest_of_different_boxes(ctx, oracle):
+    r = np.random.default_rng(9)
+    sizes = [300, 1500, 37]
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    side = np.repeat([0.5, 3.0, 1.0], sizes)[:, None]
+    t, s = (side * r.random((off[-1], 3)) for _ in range(2))
+    w = r.standard_normal((2, off[-1]))
+    ctx.set_kernel("multiquadric", 1e-2)
+    got = ctx.forest_solve(t, off, s, off, w, [3, 4, 3], poly_ord=4)
+    for p, depth in enumerate([3, 4, 3]):
+        a, b = off[p], off[p + 1]
+        for k in range(2):
+            want, _ = oracle.fmm(3, 5, 1e-2, 4, depth, 1, t[a:b], s[a:b], w[k, a:b])
+            assert rel_l2(got[k, a:b], want) <= TOL
+
+
+def test_plan_replay_is_the_solve(ctx):
+    r = np.random.default_rng(10)
+    t, s, w = r.random((5000, 3)), r.random((5000, 3)), r.standard_normal((2, 5000))
+    ctx.set_kernel("inv_r_safe")
+    plan = ctx.plan(t, [0, 5000], s, [0, 5000], 2, [4], poly_ord=5)
+    want, _ = ctx.solve(t, s, w, poly_ord=5, depth=4)
+    np.testing.assert_array_equal(plan.execute(w), want)
+    np.testing.assert_array_equal(plan.execute(w), want)
+    plan.close()
