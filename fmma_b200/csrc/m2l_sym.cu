@@ -16,19 +16,22 @@
 // signs of the offset): P^2 multiply-adds for eight sources instead of 8 P^2,
 // and the z by an 8-point Walsh-Hadamard butterfly of the gathered sources.
 // Along a dimension with o_q = 0 there is one source and K_ab = 0 unless
-// a_q = b_q, which halves the operator instead.  The 189 far slots of a target
+// a_q = b_q, which halves the operator instead; along one with |o_q| = 3 the
+// far list has one side only, so there is one source and nothing to combine
+// (on the negative side the operator's a_q != b_q blocks change sign).  The 189 far slots of a target
 // fall into 56 orbits worth 39.5 P^2 multiply-adds (189 P^2 before).
 //
 // FP64 tensor (DMMA) bound.  A block owns 8 MB target rows (box x rhs) of one
-// child-parity class.  Warp w accumulates the rows' outputs of one parity a
-// (w and 7 - w share a scheduler, so with an odd node count, where an
-// even-parity block is larger, each scheduler has the same number of
-// columns).  A pipeline stage is two K steps of 4: the threads gather the 8
-// source values of a (row, k), run the butterfly in registers and store the z
-// for the next stage while the current one is multiplied; operator fragments
-// are read from L2 straight into registers (a warp shares them with no other
-// warp of the block), one stage ahead.  Row groups of 8 with no source in an
-// orbit are skipped.
+// child-parity class.  Eight multiplying warps: warp w accumulates the rows'
+// outputs of one parity a (w and 7 - w share a scheduler, so with an odd node
+// count, where an even-parity block is larger, each scheduler has the same
+// number of columns).  Eight gathering warps read the 8 source values of a
+// (row, k), run the butterfly in registers and store the z of a stage (two K
+// steps of 4) into a ring of four in shared memory; a full and an empty
+// mbarrier per slot tie the two sides.  Operator fragments are read from L2
+// straight into registers (a warp shares them with no other warp of the
+// block), one stage ahead.  Orbits with no source for a tile are skipped, and
+// so are a tile's unused row groups of 8.
 #include <algorithm>
 #include <cmath>
 
@@ -42,7 +45,9 @@ namespace fmma_b200 {
 namespace {
 
 constexpr int kOrbits = 56;       // |o| in {0..3}^3 without {0,1}^3
-constexpr int kSymThreads = 256;
+constexpr int kSymThreads = 512;  // 8 multiplying warps, 8 gathering warps
+constexpr int kSymRing = 4;       // stages of z in shared memory
+constexpr long long kSymWaitCycles = 4000000000ll;  // bound of a pipeline wait (~2 s)
 constexpr int kSymMaxStages = 64; // stages of one orbit: 8 blocks of up to 16 K steps, two per stage
 constexpr int kSymSlots = 189;
 
@@ -54,6 +59,8 @@ struct SymGeom {
   int size[8], off[8];   // coefficients of a parity block and its offset in a folded row of P
   int nst[8];            // stages of an orbit by its zero mask
   int zmask[kOrbits];    // bit q: o_q = 0
+  int umask[kOrbits];    // bit q: |o_q| = 3, which a class has on one side only ...
+  int neg[8];            // ... the negative one where bit q is set (by class)
   int stage0[kOrbits];   // first stage of the orbit's operator
   int desc[8][kSymMaxStages][2];  // K step: b0 | k4 << 3, or -1 (no step)
   int slot[8][kOrbits][8];        // far slot of (class, orbit, signs), -1 where there is none
@@ -104,24 +111,30 @@ SymGeom make_geom(int n) {
     orbit_of[i] = -1;
     if (r[0] <= 1 && r[1] <= 1 && r[2] <= 1) continue;
     orbit_of[i] = w;
-    int z = 0;
+    int z = 0, u = 0;
     for (int q = 0; q < 3; ++q) {
       g.rep[w][q] = r[q];
       if (r[q] == 0) z |= 1 << q;
+      if (r[q] == 3) u |= 1 << q;
     }
     g.zmask[w] = z;
+    g.umask[w] = u;
     g.stage0[w] = g.total;
     g.total += g.nst[z];
     ++w;
   }
   const FarTables& F = far_tables(3);
   for (int c = 0; c < 8; ++c) {
+    g.neg[c] = 0;
     for (int i = 0; i < kOrbits; ++i)
       for (int s = 0; s < 8; ++s) g.slot[c][i][s] = -1;
     for (int q = 0; q < F.nfar; ++q) {
       const int* v = F.off_vec[F.slot_off[c][q]];
       int sg = 0;
-      for (int e = 0; e < 3; ++e) sg |= v[e] < 0 ? 1 << e : 0;
+      for (int e = 0; e < 3; ++e) {
+        sg |= v[e] < 0 ? 1 << e : 0;
+        if (v[e] == -3) g.neg[c] |= 1 << e;
+      }
       g.slot[c][orbit_of[std::abs(v[0]) * 16 + std::abs(v[1]) * 4 + std::abs(v[2])]][sg] = q;
     }
   }
@@ -314,7 +327,49 @@ struct SymParams {
   int64_t nv;          // virtual rows (rows x rhs)
   int R, Kpad;
   int zero_row;        // the row of zeros of W
+  int* err;            // set when a bounded wait gives up
 };
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
+  asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(smem_addr(bar)) : "memory");
+}
+__device__ __forceinline__ bool bar_try(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_addr(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Whether the phase is complete, without waiting.
+__device__ __forceinline__ bool bar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_addr(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Bounded wait: false when the bound passes or another warp has given up.
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
+  if (bar_try(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (true) {
+    for (int i = 0; i < 32; ++i)
+      if (bar_try(bar, parity)) return true;
+    if (*abort) return false;
+    if (clock64() - t0 > kSymWaitCycles) {
+      *abort = 1;
+      return false;
+    }
+  }
+}
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -325,33 +380,243 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
 template <int NB, int MB>
 struct SymShape {
   static constexpr int TM = 8 * MB;
-  static constexpr int TPR = kSymThreads / TM;       // threads gathering one row
+  static constexpr int TPR = 256 / TM;               // threads gathering one row
   static constexpr int EPT = 8 / TPR;                // values of a stage's 8 per thread
   static constexpr int PLANE = 8 * TM * 4 + 8;       // doubles of one K step's z (padded by 64 B)
+  // registers a thread after the split: 256 (kMulRegs + kGatherRegs) = 512 * 128, the launch's
+  static constexpr int kMulRegs = 176, kGatherRegs = 256 - kMulRegs;
+  static constexpr int KB = NB == 1 ? 8 : (NB == 4 ? 28 : 64);  // SymGeom::KB of its node counts
   static constexpr int ILS = TM + 1;                 // stride of a slot's source list
   static constexpr size_t kSmem =
-      sizeof(double) * 4 * PLANE + sizeof(int) * (kSymSlots * ILS + 8 * kSymMaxStages * 2 + kOrbits * 8 + kOrbits * 5);
+      sizeof(double) * 2 * kSymRing * PLANE + sizeof(int) * (kSymSlots * ILS + 8 * kSymMaxStages * 2 + kOrbits * 8 + kOrbits * 5);
 };
 
-template <int NB, int MB>
+// What the multiplying warps read of the block.
+struct SymBlock {
+  const double* z;     // ring of z
+  const int4* act;     // active orbits
+  const int2* desc;    // K steps by zero mask and stage
+  uint64_t *full, *empty;
+  int* abort;
+  const double* tab;   // operators of the tile's table
+  int nact, neg, v0, vcnt;
+};
+
+// One multiplying warp.  Its accumulators are two parts of MB / 2 row groups:
+// with an even node count (PAIR false) the two halves of the rows for one
+// parity a0, with an odd one half of the rows for the parities a0 and 7 - a0,
+// whose column groups N0 + N1 are the same for every warp.  A stage is four
+// units (K step, part) in a straight line: the next unit's source fragments
+// load under the DMMAs of one, the next stage's first ones too when that stage
+// is there already, and the operator fragments a stage ahead.
+template <int NB, int MB, bool PAIR, int N0, int N1>
+__device__ __forceinline__ bool sym_multiply(const SymParams& p, const SymBlock& sb, int warp, int lane) {
+  using S = SymShape<NB, MB>;
+  constexpr int TM = S::TM, H = MB / 2, NF = PAIR ? N0 + N1 : N0;
+  constexpr int kTabStage = 8 * 2 * 32 * NB;  // doubles of a stage's operator
+  const int a0 = PAIR ? warp & 3 : (warp < 4 ? warp : 11 - warp);
+  const int a1 = PAIR ? 7 - a0 : a0;
+  const int row1 = PAIR ? 0 : H * 32, row0 = PAIR ? (warp >> 2) * H * 32 : 0;
+  const int rows = ((1 << H) - 1) << (PAIR ? (warp >> 2) * H : 0);  // row groups of part 0
+  double acc0[H][N0][2], acc1[H][N1][2], bf[2][NF];
+#pragma unroll
+  for (int i = 0; i < H; ++i) {
+#pragma unroll
+    for (int j = 0; j < N0; ++j) acc0[i][j][0] = acc0[i][j][1] = 0.0;
+#pragma unroll
+    for (int j = 0; j < N1; ++j) acc1[i][j][0] = acc1[i][j][1] = 0.0;
+  }
+  auto load_b = [&](int stage, int ks) {
+    const double* src = sb.tab + (int64_t)stage * kTabStage + ks * (32 * NB) + lane * NB;
+#pragma unroll
+    for (int part = 0; part < (PAIR ? 2 : 1); ++part) {
+      const double* sp = src + (part ? a1 : a0) * (2 * 32 * NB);
+      const int n = part ? N1 : N0, f = part ? N0 : 0;
+#pragma unroll
+      for (int j = 0; j < n; j += 2) {
+        if (j + 1 < n) {
+          const double2 t = __ldg(reinterpret_cast<const double2*>(sp + j));
+          bf[ks][f + j] = t.x;
+          bf[ks][f + j + 1 < NF ? f + j + 1 : 0] = t.y;
+        } else {
+          bf[ks][f + j] = __ldg(sp + j);
+        }
+      }
+    }
+  };
+  struct Stage {
+    int s0, s1, u, mask, tab, slot;
+  };
+  int oi = 0, st = -1, nst = 0, slot = 0, phase = 0;
+  Stage cur, nxt{};
+  const int2* ds = nullptr;
+  // the next stage of the list; false at the end
+  auto advance = [&]() -> bool {
+    if (++st >= nst) {
+      if (nst > 0) ++oi;
+      if (oi >= sb.nact) return false;
+      const int4 f = sb.act[oi];
+      ds = sb.desc + ((f.x >> 8) & 7) * kSymMaxStages;
+      nxt.u = f.x >> 16;
+      nxt.mask = f.z;
+      nxt.tab = f.w - 1;
+      nst = f.y;
+      st = 0;
+    }
+    const int2 d = ds[st];
+    nxt.s0 = d.x;
+    nxt.s1 = d.y;
+    ++nxt.tab;
+    return true;
+  };
+  // z of (K step, part) of a stage, and the sign of its operator blocks
+  auto frag = [&](const Stage& s, int sl, int ks, int part) -> const double* {
+    const int c = (part ? a1 : a0) ^ ((ks ? s.s1 : s.s0) & 7);
+    return sb.z + (sl * 2 + ks) * S::PLANE + (c & ~s.u) * (TM * 4) + row0 + (part ? row1 : 0) + lane;
+  };
+  auto flip = [&](const Stage& s, int ks) {
+#pragma unroll
+    for (int part = 0; part < (PAIR ? 2 : 1); ++part) {
+      const int c = (part ? a1 : a0) ^ ((ks ? s.s1 : s.s0) & 7);
+      if (__popc(c & s.u & sb.neg) & 1) {
+#pragma unroll
+        for (int j = 0; j < (part ? N1 : N0); ++j) bf[ks][(part ? N0 : 0) + j] = -bf[ks][(part ? N0 : 0) + j];
+      }
+    }
+  };
+  constexpr int kAll = (1 << MB) - 1;
+  bool have = advance();
+  cur = nxt;
+  bool ready = false;  // av[0] holds the first unit of the stage
+  double av[2][H];
+  auto load_a = [&](double* v, const double* src) {
+#pragma unroll
+    for (int mb = 0; mb < H; ++mb) v[mb] = src[mb * 32];
+  };
+  auto mul = [&](const double* v, int ks, int part) {
+    if (part == 0) {
+#pragma unroll
+      for (int nb = 0; nb < N0; ++nb)
+#pragma unroll
+        for (int mb = 0; mb < H; ++mb) dmma(acc0[mb][nb][0], acc0[mb][nb][1], v[mb], bf[ks][nb]);
+    } else {
+#pragma unroll
+      for (int nb = 0; nb < N1; ++nb)
+#pragma unroll
+        for (int mb = 0; mb < H; ++mb) dmma(acc1[mb][nb][0], acc1[mb][nb][1], v[mb], bf[ks][(PAIR ? N0 : 0) + nb]);
+    }
+  };
+  if (have) {
+    load_b(cur.tab, 0);
+    load_b(cur.tab, 1);
+  }
+  while (have) {
+    const bool more = advance();  // nxt: the stage behind this one (at the end: this one's operator again)
+    if (!ready && !bar_wait(&sb.full[slot], phase, sb.abort)) return false;
+    const int nslot = slot + 1 == kSymRing ? 0 : slot + 1, nphase = slot + 1 == kSymRing ? phase ^ 1 : phase;
+    if (cur.mask == kAll && cur.s1 >= 0) {
+      if (!ready) load_a(av[0], frag(cur, slot, 0, 0));
+      flip(cur, 0);
+      load_a(av[1], frag(cur, slot, 0, 1));
+      mul(av[0], 0, 0);
+      load_a(av[0], frag(cur, slot, 1, 0));
+      mul(av[1], 0, 1);
+      load_b(nxt.tab, 0);
+      flip(cur, 1);
+      load_a(av[1], frag(cur, slot, 1, 1));
+      mul(av[0], 1, 0);
+      ready = more && nxt.mask == kAll && nxt.s1 >= 0 &&
+              __all_sync(0xffffffffu, bar_test(&sb.full[nslot], nphase));
+      if (ready) load_a(av[0], frag(nxt, nslot, 0, 0));
+      mul(av[1], 1, 1);
+      load_b(nxt.tab, 1);
+    } else {
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks) {
+        flip(cur, ks);
+        if (ks == 0 || cur.s1 >= 0) {  // the last stage of an orbit may have one K step
+#pragma unroll
+          for (int part = 0; part < 2; ++part) {
+            const double* A = frag(cur, slot, ks, part);
+            const int m = PAIR ? (cur.mask & rows) >> ((warp >> 2) * H) : cur.mask >> (part * H);
+#pragma unroll
+            for (int mb = 0; mb < H; ++mb)
+              if ((m >> mb) & 1) {
+                const double v = A[mb * 32];
+                if (part == 0) {
+#pragma unroll
+                  for (int nb = 0; nb < N0; ++nb) dmma(acc0[mb][nb][0], acc0[mb][nb][1], v, bf[ks][nb]);
+                } else {
+#pragma unroll
+                  for (int nb = 0; nb < N1; ++nb)
+                    dmma(acc1[mb][nb][0], acc1[mb][nb][1], v, bf[ks][(PAIR ? N0 : 0) + nb]);
+                }
+              }
+          }
+        }
+        load_b(nxt.tab, ks);
+      }
+      ready = false;
+    }
+    __syncwarp();
+    if (lane == 0) bar_arrive(&sb.empty[slot]);  // the z values are in registers
+    slot = nslot;
+    phase = nphase;
+    cur = nxt;
+    have = more;
+  }
+
+  const SymGeom& g = *p.geom;
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    const int a = part ? a1 : a0;
+    const int size = g.size[a], first = g.off[a];
+#pragma unroll
+    for (int mb = 0; mb < H; ++mb) {
+      const int i = (row0 + (part ? row1 : 0)) / 4 + mb * 8 + (lane >> 2);
+      if (i >= sb.vcnt) continue;
+      const int64_t v = sb.v0 + i;
+      double* dst;
+      if (gridDim.y > 1) {
+        dst = p.part + ((int64_t)blockIdx.y * p.nv + v) * g.P + first;
+      } else {
+        const int64_t brow = v / p.R;
+        dst = p.Wl + ((int64_t)p.row_box[brow] * p.R + (v - brow * p.R)) * p.Kpad + first;
+      }
+#pragma unroll
+      for (int nb = 0; nb < (part ? N1 : N0); ++nb) {
+        const int col = nb * 8 + (lane & 3) * 2;
+        const double x = part ? acc1[mb][part ? nb : 0][0] : acc0[mb][part ? 0 : nb][0];
+        const double y = part ? acc1[mb][part ? nb : 0][1] : acc0[mb][part ? 0 : nb][1];
+        if (col < size) dst[col] = x;
+        if (col + 1 < size) dst[col + 1] = y;
+      }
+    }
+  }
+  return true;
+}
+
+// N nodes per dimension.
+template <int N, int NB, int MB>
 __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
   using S = SymShape<NB, MB>;
-  constexpr int TM = S::TM, EPT = S::EPT;
+  constexpr int TM = S::TM, EPT = S::EPT, KB = S::KB;
   constexpr int kTabStage = 8 * 2 * 32 * NB;  // doubles of a stage's operator
   extern __shared__ __align__(16) double sym_smem[];
-  double* const sZ = sym_smem;                                   // [2][2][PLANE]
-  int4* const sAct = reinterpret_cast<int4*>(sZ + 4 * S::PLANE); // active orbits: (orbit | zero mask << 8, stages, row groups, first stage)
-  int* const sIl = reinterpret_cast<int*>(sAct + kOrbits);       // [slot][ILS] source row (box * R + r)
-  int* const sDesc = sIl + kSymSlots * S::ILS;                   // [zero mask][stage][2]
-  int* const sSlot = sDesc + 8 * kSymMaxStages * 2;              // [orbit][8]
+  double* const sZ = sym_smem;                                              // [ring][2][PLANE]
+  // active orbits: (orbit | zero mask << 8 | one-sided mask << 16, stages, row groups, first stage)
+  int4* const sAct = reinterpret_cast<int4*>(sZ + 2 * kSymRing * S::PLANE);
+  int2* const sDesc = reinterpret_cast<int2*>(sAct + kOrbits);   // [zero mask][stage] K steps
+  int* const sSlot = reinterpret_cast<int*>(sDesc + 8 * kSymMaxStages);  // [orbit][8]
   int* const sMask = sSlot + kOrbits * 8;                        // [orbit] row groups with a source
-  __shared__ int s_nact;
+  int* const sIl = sMask + kOrbits;                              // [slot][ILS] source row (box * R + r)
+  __shared__ uint64_t s_full[kSymRing], s_empty[kSymRing];
+  __shared__ int s_nact, s_abort;
   const SymGeom& g = *p.geom;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int a = warp < 4 ? warp : 11 - warp;  // output parity of this warp
   const int4 tile = p.tiles[blockIdx.x];
   const int cls = tile.x, v0 = tile.y, vcnt = tile.z;
-  const int KB = g.KB, R = p.R, none = p.zero_row;
+  const int R = p.R, none = p.zero_row;
   const int lo = p.part_lo[blockIdx.y], hi = p.part_lo[blockIdx.y + 1];
 
   for (int i = tid; i < TM * kSymSlots; i += kSymThreads) {
@@ -364,9 +629,17 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
     }
     sIl[q * S::ILS + r] = s;
   }
-  for (int i = tid; i < 8 * kSymMaxStages * 2; i += kSymThreads) sDesc[i] = (&g.desc[0][0][0])[i];
+  for (int i = tid; i < 8 * kSymMaxStages; i += kSymThreads)
+    sDesc[i] = make_int2((&g.desc[0][0][0])[2 * i], (&g.desc[0][0][0])[2 * i + 1]);
   for (int i = tid; i < kOrbits * 8; i += kSymThreads) sSlot[i] = g.slot[cls][i >> 3][i & 7];
   for (int i = tid; i < kOrbits; i += kSymThreads) sMask[i] = 0;
+  if (tid == 0) {
+    for (int s = 0; s < kSymRing; ++s) {
+      bar_init(&s_full[s], 8);   // a lane of each gathering warp
+      bar_init(&s_empty[s], 8);  // a lane of each multiplying warp
+    }
+    s_abort = 0;
+  }
   __syncthreads();
   for (int i = tid; i < (hi - lo) * MB; i += kSymThreads) {
     const int w = lo + i / MB, mb = i % MB;
@@ -387,7 +660,11 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
       const unsigned m = __ballot_sync(0xffffffffu, on);
       if (on) {
         const int z = g.zmask[w];
-        sAct[base + __popc(m & ((1u << lane) - 1u))] = make_int4(w | (z << 8), g.nst[z], sMask[w], g.stage0[w]);
+        // a full tile's empty row groups (about 2 %) are multiplied as zeros:
+        // skipping them costs the straight-line stages more
+        const int mask = vcnt > TM - 8 ? (1 << MB) - 1 : sMask[w];
+        sAct[base + __popc(m & ((1u << lane) - 1u))] = 
+            make_int4(w | (z << 8) | (g.umask[w] << 16), g.nst[z], mask, g.stage0[w]);
       }
       base += __popc(m);
     }
@@ -396,199 +673,117 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
   __syncthreads();
   const int nact = s_nact;
 
-  // gather role: one row, EPT consecutive k of one K step
-  const int grow = tid / S::TPR, gp = tid % S::TPR;
-  const int gks = EPT == 2 ? gp >> 1 : gp >> 2;
-  const int gk = EPT == 2 ? (gp & 1) * 2 : gp & 3;
-  const int ggrp = grow >> 3;
-  // a pipeline stage: zero mask and row groups of its orbit, K steps, operator stage
-  struct Stage {
-    int z, mask, step[2], tab;
-  };
-  Stage cur{}, nxt{}, fut{};          // multiplied, stored and gathered next
-  int oi = 0, st = -1, nst = 0;       // gather cursor over the active orbits' stages
-  unsigned off[8];                    // the cursor's sources, in units of 4 doubles
-  double raw[8][EPT];
-  // moves the cursor on and issues the stage's loads; false at the end
-  auto gather = [&]() -> bool {
-    if (++st >= nst) {
-      if (st > 0) ++oi;
-      if (oi >= nact) return false;
+  if (warp >= 8) {
+    // ---- gathering warps: one row, EPT consecutive k of one K step a thread ----
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(S::kGatherRegs));
+    const int gt = tid - 256;
+    const int grow = gt / S::TPR, gp = gt % S::TPR;
+    const int gks = EPT == 2 ? gp >> 1 : gp >> 2;
+    const int gk = EPT == 2 ? (gp & 1) * 2 : gp & 3;
+    const int ggrp = grow >> 3;
+    double* const zdst = sZ + gks * S::PLANE + grow * 4 + gk;
+    const int neg = g.neg[cls];
+    int it = 0;
+    for (int oi = 0; oi < nact; ++oi) {
       const int4 f = sAct[oi];
-      st = 0;
-      nst = f.y;
-      fut.z = f.x >> 8;
-      fut.mask = f.z;
-      fut.tab = f.w - 1;
+      // u: the one-sided dimensions; only the planes j with no bit of u are made
+      const int z = (f.x >> 8) & 7, u = f.x >> 16, nst = f.y;
+      const bool mine = (f.z >> ggrp) & 1;  // warp-uniform, as every test of u and z
       const int* sl = sSlot + (f.x & 255) * 8;
+      const int* ds = reinterpret_cast<const int*>(sDesc + z * kSymMaxStages) + gks;
+      unsigned off[8];  // the orbit's sources, in units of 4 doubles
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const int q = sl[j & ~fut.z];
+        const int q = sl[(j & ~z & ~u) | (neg & u)];
         const int s = q >= 0 ? sIl[q * S::ILS + grow] : none;
-        off[j] = (unsigned)s * (unsigned)(2 * KB) + (unsigned)((j & fut.z) * (KB / 4));
+        off[j] = (unsigned)s * (2u * KB) + (unsigned)((j & z) * (KB / 4));
       }
-    }
-    ++fut.tab;
-    const int* ds = sDesc + (fut.z * kSymMaxStages + st) * 2;
-    fut.step[0] = ds[0];
-    fut.step[1] = ds[1];
-    const int step = max(ds[gks], 0);  // no step: any data, not multiplied
-    if ((fut.mask >> ggrp) & 1) {      // warp-uniform
-      const char* src = reinterpret_cast<const char*>(p.W + (step & 7) * KB + (step >> 3) * 4 + gk);
+      for (int st = 0; st < nst; ++st, ++it) {
+        double raw[8][EPT];
+        if (mine) {
+          const int step = max(ds[st * 2], 0);  // no step: any data, not multiplied
+          const char* src = reinterpret_cast<const char*>(p.W + (step & 7) * KB + (step >> 3) * 4 + gk);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const char* sj = src + (uint64_t)off[j] * 32u;
-        if constexpr (EPT == 2) {
-          const double2 t = __ldg(reinterpret_cast<const double2*>(sj));
-          raw[j][0] = t.x;
-          raw[j][EPT - 1] = t.y;
-        } else {
-          raw[j][0] = __ldg(reinterpret_cast<const double*>(sj));
-        }
-      }
-    }
-    return true;
-  };
-  // the butterfly over the signs of stage `nxt`, its z stored in buffer buf
-  auto put = [&](int buf) {
-    if (!((nxt.mask >> ggrp) & 1)) return;
-#pragma unroll
-    for (int q = 1; q < 8; q <<= 1)
-      if (!(nxt.z & q)) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (!(j & q)) {
-#pragma unroll
-            for (int e = 0; e < EPT; ++e) {
-              const double u = raw[j][e], t = raw[j | q][e];
-              raw[j][e] = u + t;
-              raw[j | q][e] = u - t;
+          for (int j = 0; j < 8; ++j)
+            if (!(j & u)) {
+              const char* sj = src + (uint64_t)off[j] * 32u;
+              if constexpr (EPT == 2) {
+                const double2 t = __ldg(reinterpret_cast<const double2*>(sj));
+                raw[j][0] = t.x;
+                raw[j][EPT - 1] = t.y;
+              } else {
+                raw[j][0] = __ldg(reinterpret_cast<const double*>(sj));
+              }
             }
-          }
-      }
-    double* dst = sZ + (buf * 2 + gks) * S::PLANE + grow * 4 + gk;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if constexpr (EPT == 2)
-        *reinterpret_cast<double2*>(dst + j * TM * 4) = make_double2(raw[j][0], raw[j][EPT - 1]);
-      else
-        dst[j * TM * 4] = raw[j][0];
-    }
-  };
-
-  double acc[MB][NB][2];
-#pragma unroll
-  for (int i = 0; i < MB; ++i)
-#pragma unroll
-    for (int j = 0; j < NB; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  const int nba = (g.size[a] + 7) >> 3;  // column groups of this parity
-
-  const double* const tabw = p.tab + (int64_t)tile.w * g.total * kTabStage + (int64_t)a * (2 * 32 * NB) + lane * NB;
-  double bf[2][NB];
-  auto load_b = [&](int stage, int ks) {
-    const double* src = tabw + (int64_t)stage * kTabStage + ks * (32 * NB);
-    if constexpr (NB == 1) {
-      bf[ks][0] = __ldg(src);
-    } else {
-#pragma unroll
-      for (int j = 0; j < NB; j += 2) {
-        const double2 t = __ldg(reinterpret_cast<const double2*>(src + j));
-        bf[ks][j] = t.x;
-        bf[ks][j + (NB > 1 ? 1 : 0)] = t.y;
-      }
-    }
-  };
-
-  if (gather()) {
-    nxt = fut;
-    put(0);
-    bool hn = gather();  // a stage after the current one
-    cur = nxt;
-    nxt = fut;
-    load_b(cur.tab, 0);
-    load_b(cur.tab, 1);
-    int buf = 0;
-    // Of the two warps of a scheduler one stores the next stage's z before
-    // its multiplications and the other after them, so that one's butterfly
-    // and stores overlap the other's DMMAs.
-    const bool early = warp < 4;
-    bool hf = false;  // a stage after the next one
-    while (true) {
-      __syncthreads();  // this stage's z stored by all; the other buffer read by all
-      if (early && hn) {
-        put(buf ^ 1);
-        hf = gather();
-      }
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
-        const int step = cur.step[ks];
-        if (step >= 0) {
-          const double* A = sZ + (buf * 2 + ks) * S::PLANE + (a ^ (step & 7)) * (TM * 4) + lane;
-          double av[MB];
-#pragma unroll
-          for (int mb = 0; mb < MB; ++mb) av[mb] = A[mb * 32];
-          if (cur.mask == (1 << MB) - 1) {
-#pragma unroll
-            for (int nb = 0; nb < NB; ++nb)
-              if (nb < nba) {
-#pragma unroll
-                for (int mb = 0; mb < MB; ++mb) dmma(acc[mb][nb][0], acc[mb][nb][1], av[mb], bf[ks][nb]);
-              }
-          } else {
-#pragma unroll
-            for (int mb = 0; mb < MB; ++mb)
-              if ((cur.mask >> mb) & 1) {
-#pragma unroll
-                for (int nb = 0; nb < NB; ++nb)
-                  if (nb < nba) dmma(acc[mb][nb][0], acc[mb][nb][1], av[mb], bf[ks][nb]);
-              }
-          }
         }
-        if (hn) load_b(nxt.tab, ks);
+        const int slot = it & (kSymRing - 1);
+        if (!bar_wait(&s_empty[slot], ((it / kSymRing) & 1) ^ 1, &s_abort)) {
+          *p.err = 1;
+          return;
+        }
+        if (mine) {
+#pragma unroll
+          for (int q = 1; q < 8; q <<= 1)
+            if (!((z | u) & q)) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (!(j & q)) {
+                  if (j & u) continue;
+#pragma unroll
+                  for (int e = 0; e < EPT; ++e) {
+                    const double x = raw[j][e], y = raw[j | q][e];
+                    raw[j][e] = x + y;
+                    raw[j | q][e] = x - y;
+                  }
+                }
+            }
+          double* dst = zdst + slot * 2 * S::PLANE;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (!(j & u)) {
+              if constexpr (EPT == 2)
+                *reinterpret_cast<double2*>(dst + j * TM * 4) = make_double2(raw[j][0], raw[j][EPT - 1]);
+              else
+                dst[j * TM * 4] = raw[j][0];
+            }
+        }
+        __syncwarp();
+        if (lane == 0) bar_arrive(&s_full[slot]);
       }
-      if (!hn) break;
-      if (!early) {
-        put(buf ^ 1);
-        hf = gather();
-      }
-      cur = nxt;
-      nxt = fut;
-      hn = hf;
-      buf ^= 1;
     }
+    return;
   }
 
-  const int size = g.size[a], first = g.off[a];
-#pragma unroll
-  for (int mb = 0; mb < MB; ++mb) {
-    const int i = mb * 8 + (lane >> 2);
-    if (i >= vcnt) continue;
-    const int64_t v = v0 + i;
-    double* dst;
-    if (gridDim.y > 1) {
-      dst = p.part + ((int64_t)blockIdx.y * p.nv + v) * g.P + first;
-    } else {
-      const int64_t brow = v / R;
-      dst = p.Wl + ((int64_t)p.row_box[brow] * R + (v - brow * R)) * p.Kpad + first;
-    }
-#pragma unroll
-    for (int nb = 0; nb < NB; ++nb) {
-      const int col = nb * 8 + (lane & 3) * 2;
-      if (col < size) dst[col] = acc[mb][nb][0];
-      if (col + 1 < size) dst[col + 1] = acc[mb][nb][1];
-    }
+  // ---- multiplying warps ----
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(S::kMulRegs));
+  const SymBlock sb{sZ, sAct, sDesc, s_full, s_empty, &s_abort, p.tab + (int64_t)tile.w * g.total * kTabStage, nact,
+                    g.neg[cls], v0, vcnt};
+  bool ok;
+  if constexpr (N % 2 == 0) {
+    constexpr int C = (N / 2 * (N / 2) * (N / 2) + 7) / 8;  // column groups of every parity
+    ok = sym_multiply<NB, MB, false, C, C>(p, sb, warp, lane);
+  } else {
+    // column groups by the number of odd dimensions of the parity; warp & 3
+    // has 0, 1, 1 and 2 of them, its partner 3, 2, 2 and 1
+    constexpr int E = (N + 1) / 2, O = N / 2;
+    constexpr int C0 = (E * E * E + 7) / 8, C1 = (E * E * O + 7) / 8, C2 = (E * O * O + 7) / 8,
+                  C3 = (O * O * O + 7) / 8;
+    if ((warp & 3) == 0) ok = sym_multiply<NB, MB, true, C0, C3>(p, sb, warp, lane);
+    else if ((warp & 3) == 3) ok = sym_multiply<NB, MB, true, C2, C1>(p, sb, warp, lane);
+    else ok = sym_multiply<NB, MB, true, C1, C2>(p, sb, warp, lane);
   }
+  if (!ok) *p.err = 1;
 }
 
-template <int NB, int MB>
+template <int N, int NB, int MB>
 void launch_sym(fmma_ctx* ctx, const SymParams& p, int ntiles, int nparts) {
   constexpr size_t smem = SymShape<NB, MB>::kSmem;
   static bool attr_set = false;
   if (!attr_set) {
-    FMMA_CHECK_CUDA(cudaFuncSetAttribute(k_m2l_sym<NB, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    FMMA_CHECK_CUDA(cudaFuncSetAttribute(k_m2l_sym<N, NB, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set = true;
   }
-  FMMA_LAUNCH(ctx, (k_m2l_sym<NB, MB>), dim3((unsigned)ntiles, (unsigned)nparts), kSymThreads, smem, p);
+  FMMA_LAUNCH(ctx, (k_m2l_sym<N, NB, MB>), dim3((unsigned)ntiles, (unsigned)nparts), kSymThreads, smem, p);
 }
 
 struct SymTableLaunch {
@@ -602,9 +797,6 @@ struct SymTableLaunch {
   }
 };
 
-// blocks aimed at per level: about four per SM, so that the last wave is a
-// small part of the level
-constexpr int kSymBlocksPerSm = 4;
 constexpr int kSymMaxParts = 16;
 
 }  // namespace
@@ -649,9 +841,19 @@ void m2l_level_sym(fmma_ctx* ctx, const Level& Lv, int v, int n, int Kpad, int R
   int4* dt = ctx_buf_t<int4>(ctx, "m2l_tiles" + std::to_string(v), tiles.size());
   upload(ctx, dt, tiles.data(), sizeof(int4) * tiles.size());
 
-  // orbits split over blocks on levels with few tiles, by equal stage counts
-  int nparts = (ctx->sm_count * kSymBlocksPerSm + ntiles - 1) / ntiles;
-  nparts = std::max(1, std::min(nparts, kSymMaxParts));
+  // The orbits of a tile are split over blocks where that fills the last wave
+  // of a level: a block costs its share of a tile plus about 2 % of one (the
+  // prologue and the partial sums), and one block runs on an SM at a time.
+  int nparts = 1;
+  double best = 0.0;
+  for (int s = 1; s <= kSymMaxParts; ++s) {
+    const int64_t waves = ((int64_t)ntiles * s + ctx->sm_count - 1) / ctx->sm_count;
+    const double t = (double)waves * (1.0 / s + 0.02);
+    if (s == 1 || t < best) {
+      best = t;
+      nparts = s;
+    }
+  }
   std::vector<int> lo((size_t)nparts + 1, 0);
   for (int s = 1, w = 0; s < nparts; ++s) {
     while (w < kOrbits && (int64_t)g.stage0[w] * nparts < (int64_t)s * g.total) ++w;
@@ -664,15 +866,23 @@ void m2l_level_sym(fmma_ctx* ctx, const Level& Lv, int v, int n, int Kpad, int R
   const int64_t nv = Lv.nrow * R, nsrc = Lv.nbox * R;
   double* W = ctx_buf_t<double>(ctx, "sym_src", (size_t)(nsrc + 1) * 8 * g.KB);
   double* part = nparts > 1 ? ctx_buf_t<double>(ctx, "sym_part", (size_t)nparts * nv * g.P) : nullptr;
-  SymParams p{dt, Lv.il, Lv.row_box, dg, W, tab, dlo, Wl, part, nv, R, Kpad, (int)nsrc};
+  int* err = m2l_err_slot(ctx, v);
+  FMMA_CHECK_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
+  SymParams p{dt, Lv.il, Lv.row_box, dg, W, tab, dlo, Wl, part, nv, R, Kpad, (int)nsrc, err};
   kernel_timer_begin(ctx);
   const int64_t wcap = (int64_t)ctx->sm_count * 32;
   FMMA_LAUNCH(ctx, k_sym_fold, grid_for((nsrc + 1) * 32, 256, wcap), 256, 0, Wm, nsrc, Kpad, dg, W);
-  if (g.NB == 1) launch_sym<1, 8>(ctx, p, ntiles, nparts);
-  else if (g.NB == 4) launch_sym<4, 8>(ctx, p, ntiles, nparts);
-  else launch_sym<8, 4>(ctx, p, ntiles, nparts);
+  switch (n) {
+    case 3: launch_sym<3, 1, 8>(ctx, p, ntiles, nparts); break;
+    case 4: launch_sym<4, 1, 8>(ctx, p, ntiles, nparts); break;
+    case 5: launch_sym<5, 4, 8>(ctx, p, ntiles, nparts); break;
+    case 6: launch_sym<6, 4, 8>(ctx, p, ntiles, nparts); break;
+    case 7: launch_sym<7, 8, 4>(ctx, p, ntiles, nparts); break;
+    default: launch_sym<8, 8, 4>(ctx, p, ntiles, nparts); break;
+  }
   FMMA_LAUNCH(ctx, k_sym_unfold, grid_for(nv * 32, 256, wcap), 256, 0, part, nparts, nv, R, Lv.row_box, Kpad, dg, Wl);
   kernel_timer_end(ctx, 2.0 * g.P * g.P * R, v);
+  ctx->m2l_err_flags.push_back(err);
 }
 
 }  // namespace fmma_b200
