@@ -408,164 +408,7 @@ __global__ void __launch_bounds__(kL2PThreads) k_l2p_grad_f64(
   }
 }
 
-// ---------------------------------------------------------------------------
-// P2P (src/fmm.cpp:121-141): one warp per leaf row; lanes split as
-// (target, source subset) and reduce over the subsets with shuffles.
-// ---------------------------------------------------------------------------
-template <int KID, int D, int RB, typename T>
-__global__ void __launch_bounds__(256) k_p2p_f64(
-    const int* __restrict__ row_box, int64_t nrow, const int* __restrict__ near, int nnear,
-    const int* __restrict__ tb, const int* __restrict__ te, const int* __restrict__ sb, const int* __restrict__ se,
-    const double* __restrict__ tx, int64_t nt, const double* __restrict__ sx, int64_t ns,
-    const double* __restrict__ ws, int R, double p0, const double* __restrict__ pot,
-    const int* __restrict__ perm_t, T* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t row = wid; row < nrow; row += nw) {
-    const int b = row_box[row];
-    const int t0 = tb[b], t1 = te[b];
-    for (int tc = t0; tc < t1; tc += 32) {
-      const int cnt = min(32, t1 - tc);
-      int tp2 = 1;
-      while (tp2 < cnt) tp2 <<= 1;
-      const int G = 32 / tp2;
-      const int ti = lane & (tp2 - 1), g = lane / tp2;
-      const bool tv = ti < cnt;
-      double x[D];
-#pragma unroll
-      for (int q = 0; q < D; ++q) x[q] = tv ? tx[(int64_t)q * nt + tc + ti] : 0.0;
-      for (int r0 = 0; r0 < R; r0 += RB) {
-        double acc[RB];
-#pragma unroll
-        for (int r = 0; r < RB; ++r) acc[r] = 0.0;
-        if (tv) {
-          for (int qn = 0; qn < nnear; ++qn) {
-            const int s = near[row * nnear + qn];
-            if (s < 0) continue;
-            const int j1 = se[s];
-            for (int j = sb[s] + g; j < j1; j += G) {
-              double y[D];
-#pragma unroll
-              for (int q = 0; q < D; ++q) y[q] = sx[(int64_t)q * ns + j];
-              const double f = keval<KID, D>(x, y, p0);
-#pragma unroll
-              for (int r = 0; r < RB; ++r)
-                if (r0 + r < R) acc[r] += ws[(int64_t)(r0 + r) * ns + j] * f;
-            }
-          }
-        }
-#pragma unroll
-        for (int r = 0; r < RB; ++r)
-          for (int o = tp2; o < 32; o <<= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
-        if (g == 0 && tv) {
-          const int t = tc + ti;
-          const int64_t ot = perm_t[t];
-#pragma unroll
-          for (int r = 0; r < RB; ++r)
-            if (r0 + r < R) {
-              double v = acc[r] + (pot ? pot[(int64_t)(r0 + r) * nt + t] : 0.0);
-              out[(int64_t)(r0 + r) * nt + ot] = (T)v;
-            }
-        }
-      }
-    }
-  }
-}
-
-template <typename T>
-struct P2PLaunch {
-  template <int KID, int D>
-  static void run(fmma_ctx* ctx, const Tree& tr, const double* tx, const double* sx, const double* ws, int R,
-                  double p0, const double* pot, T* out) {
-    const Level& Lf = tr.lev[0];
-    const int nnear = D == 1 ? 3 : (D == 2 ? 9 : 27);
-    unsigned g = grid_for(tr.nnear_rows * 32, 256, (int64_t)ctx->sm_count * 16);
-    if (R == 1)
-      FMMA_LAUNCH(ctx, (k_p2p_f64<KID, D, 1, T>), g, 256, 0, tr.near_row_box, tr.nnear_rows, tr.near, nnear, Lf.tb,
-                  Lf.te, Lf.sb, Lf.se, tx, tr.nt, sx, tr.ns, ws, R, p0, pot, tr.perm_t, out);
-    else
-      FMMA_LAUNCH(ctx, (k_p2p_f64<KID, D, 8, T>), g, 256, 0, tr.near_row_box, tr.nnear_rows, tr.near, nnear, Lf.tb,
-                  Lf.te, Lf.sb, Lf.se, tx, tr.nt, sx, tr.ns, ws, R, p0, pot, tr.perm_t, out);
-  }
-};
-
 constexpr int kExactThreads = 256;
-
-// Near field with gradients: out[r][t] = pot + sum w f, grad[r][t][q] =
-// potg + sum w d f/d x_q (FP64, warp per leaf row like k_p2p_f64).
-template <int KID, int D>
-__global__ void __launch_bounds__(256) k_p2p_grad_f64(
-    const int* __restrict__ row_box, int64_t nrow, const int* __restrict__ near, int nnear,
-    const int* __restrict__ tb, const int* __restrict__ te, const int* __restrict__ sb, const int* __restrict__ se,
-    const double* __restrict__ tx, int64_t nt, const double* __restrict__ sx, int64_t ns,
-    const double* __restrict__ ws, int R, double p0, const double* __restrict__ pot, const double* __restrict__ potg,
-    const int* __restrict__ perm_t, double* __restrict__ out, double* __restrict__ grad) {
-  const int lane = threadIdx.x & 31;
-  const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t row = wid; row < nrow; row += nw) {
-    const int b = row_box[row];
-    const int t0 = tb[b], t1 = te[b];
-    for (int tc = t0; tc < t1; tc += 32) {
-      const int cnt = min(32, t1 - tc);
-      int tp2 = 1;
-      while (tp2 < cnt) tp2 <<= 1;
-      const int G = 32 / tp2;
-      const int ti = lane & (tp2 - 1), g = lane / tp2;
-      const bool tv = ti < cnt;
-      double x[D];
-#pragma unroll
-      for (int q = 0; q < D; ++q) x[q] = tv ? tx[(int64_t)q * nt + tc + ti] : 0.0;
-      for (int r = 0; r < R; ++r) {
-        double acc = 0.0, ga[D];
-#pragma unroll
-        for (int q = 0; q < D; ++q) ga[q] = 0.0;
-        if (tv) {
-          for (int qn = 0; qn < nnear; ++qn) {
-            const int s = near[row * nnear + qn];
-            if (s < 0) continue;
-            for (int j = sb[s] + g; j < se[s]; j += G) {
-              double y[D], gr[D];
-#pragma unroll
-              for (int q = 0; q < D; ++q) y[q] = sx[(int64_t)q * ns + j];
-              const double wj = ws[(int64_t)r * ns + j];
-              acc += wj * keval<KID, D>(x, y, p0);
-              kgrad_x<KID, D>(x, y, p0, gr);
-#pragma unroll
-              for (int q = 0; q < D; ++q) ga[q] += wj * gr[q];
-            }
-          }
-        }
-        for (int o = tp2; o < 32; o <<= 1) {
-          acc += __shfl_xor_sync(0xffffffffu, acc, o);
-#pragma unroll
-          for (int q = 0; q < D; ++q) ga[q] += __shfl_xor_sync(0xffffffffu, ga[q], o);
-        }
-        if (g == 0 && tv) {
-          const int t = tc + ti;
-          const int64_t ot = perm_t[t];
-          if (out) out[(int64_t)r * nt + ot] = acc + (pot ? pot[(int64_t)r * nt + t] : 0.0);
-#pragma unroll
-          for (int q = 0; q < D; ++q)
-            grad[((int64_t)r * nt + ot) * D + q] = ga[q] + (potg ? potg[((int64_t)r * nt + t) * D + q] : 0.0);
-        }
-      }
-    }
-  }
-}
-
-struct P2PGradLaunch {
-  template <int KID, int D>
-  static void run(fmma_ctx* ctx, const Tree& tr, const double* tx, const double* sx, const double* ws, int R,
-                  double p0, const double* pot, const double* potg, double* out, double* grad) {
-    const Level& Lf = tr.lev[0];
-    const int nnear = D == 1 ? 3 : (D == 2 ? 9 : 27);
-    unsigned g = grid_for(tr.nnear_rows * 32, 256, (int64_t)ctx->sm_count * 16);
-    FMMA_LAUNCH(ctx, (k_p2p_grad_f64<KID, D>), g, 256, 0, tr.near_row_box, tr.nnear_rows, tr.near, nnear, Lf.tb, Lf.te,
-                Lf.sb, Lf.se, tx, tr.nt, sx, tr.ns, ws, R, p0, pot, potg, tr.perm_t, out, grad);
-  }
-};
 
 // Exact gradient: grad[r][i][q] = sum_j w[r][j] d f(x_i, y_j) / d x_q.
 template <int KID, int D>
@@ -628,83 +471,6 @@ void solve_exact_grad(fmma_ctx* ctx, int dim, int64_t nt, const double* tgt, int
   FMMA_REQUIRE(ctx->kernel_id != kUserKernel, "gradients need a built-in kernel");
   dispatch_kernel<ExactGradLaunch>(ctx->kernel_id, dim, ctx, tgt, nt, rows, src, ns, w, R, ctx->p0, grad);
 }
-
-// ---------------------------------------------------------------------------
-// exact (src/fmma.cpp:80-101): all pairs, sources staged through shared memory.
-// `rows` (optional) restricts the targets to a subset (sampled FP64 oracle).
-// ---------------------------------------------------------------------------
-template <int KID, int D, typename T>
-__global__ void __launch_bounds__(kExactThreads) k_exact(const T* __restrict__ tgt, int64_t nt,
-                                                         const int64_t* __restrict__ rows, const T* __restrict__ src,
-                                                         int64_t ns, const T* __restrict__ w, int R, double p0,
-                                                         T* __restrict__ ans) {
-  __shared__ double sy[kExactThreads][D];
-  __shared__ double sw[kExactThreads];
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool ok = i < nt;
-  const int64_t ti = ok ? (rows ? rows[i] : i) : 0;
-  double x[D];
-#pragma unroll
-  for (int q = 0; q < D; ++q) x[q] = ok ? (double)tgt[ti * D + q] : 0.0;
-  for (int r = 0; r < R; ++r) {
-    double acc = 0.0;
-    for (int64_t j0 = 0; j0 < ns; j0 += kExactThreads) {
-      const int cnt = (int)min((int64_t)kExactThreads, ns - j0);
-      __syncthreads();
-      if ((int)threadIdx.x < cnt) {
-#pragma unroll
-        for (int q = 0; q < D; ++q) sy[threadIdx.x][q] = (double)src[(j0 + threadIdx.x) * D + q];
-        sw[threadIdx.x] = w ? (double)w[(int64_t)r * ns + j0 + threadIdx.x] : 1.0;
-      }
-      __syncthreads();
-      if (ok)
-        for (int j = 0; j < cnt; ++j) acc += sw[j] * keval<KID, D>(x, sy[j], p0);
-    }
-    if (ok) ans[(int64_t)r * nt + i] = (T)acc;
-  }
-}
-
-template <typename T>
-struct ExactLaunch {
-  template <int KID, int D>
-  static void run(fmma_ctx* ctx, const T* tgt, int64_t nt, const int64_t* rows, const T* src, int64_t ns, const T* w,
-                  int R, double p0, T* ans) {
-    FMMA_LAUNCH(ctx, (k_exact<KID, D, T>), (unsigned)((nt + kExactThreads - 1) / kExactThreads), kExactThreads, 0,
-                tgt, nt, rows, src, ns, w, R, p0, ans);
-  }
-};
-
-template <typename T>
-void solve_exact(fmma_ctx* ctx, int dim, int64_t nt, const T* tgt, int64_t ns, const T* src, int R, const T* w,
-                 T* ans, const int64_t* rows) {
-  if (nt == 0) return;
-  if (ns == 0) {
-    FMMA_CHECK_CUDA(cudaMemsetAsync(ans, 0, sizeof(T) * (size_t)(nt * R), ctx->stream));
-    return;
-  }
-  if (ctx->kernel_id == kUserKernel) {
-    fmma_user_launch a{};
-    a.what = FMMA_USER_EXACT;
-    a.dim = dim;
-    a.nrhs = R;
-    a.nt = nt;
-    a.ns = ns;
-    a.tgt = tgt;
-    a.src = src;
-    a.w = w;
-    a.rows = rows;
-    a.out = ans;
-    a.out_f32 = sizeof(T) == 4;
-    call_user_hook(ctx, a);
-    return;
-  }
-  dispatch_kernel<ExactLaunch<T>>(ctx->kernel_id, dim, ctx, tgt, nt, rows, src, ns, w, R, ctx->p0, ans);
-}
-
-template void solve_exact<double>(fmma_ctx*, int, int64_t, const double*, int64_t, const double*, int, const double*,
-                                  double*, const int64_t*);
-template void solve_exact<float>(fmma_ctx*, int, int64_t, const float*, int64_t, const float*, int, const float*,
-                                 float*, const int64_t*);
 
 // ---------------------------------------------------------------------------
 // operator cache
@@ -926,43 +692,6 @@ struct M2PLaunch {
   }
 };
 
-// ---------------------------------------------------------------------------
-// FP64 near field over the leaves' near lists (src/fmm.cpp:121-141), by the
-// built-in kernel or the user hook: out[r][perm_t[t]] = pot[r][t] + sum w f.
-// ---------------------------------------------------------------------------
-template <typename T>
-void near_field_f64(fmma_ctx* ctx, int d, int R, const Tree& tr, const double* tx, const double* sx, const double* ws,
-                    const double* pot, T* ans) {
-  if (tr.nnear_rows == 0) return;
-  if (ctx->kernel_id == kUserKernel) {
-    const Level& Lf = tr.lev[0];
-    fmma_user_launch ua{};
-    ua.what = FMMA_USER_P2P;
-    ua.dim = d;
-    ua.nrhs = R;
-    ua.nrow = tr.nnear_rows;
-    ua.row_box = tr.near_row_box;
-    ua.near = tr.near;
-    ua.nnear = d == 1 ? 3 : (d == 2 ? 9 : 27);
-    ua.tb = Lf.tb;
-    ua.te = Lf.te;
-    ua.sb = Lf.sb;
-    ua.se = Lf.se;
-    ua.tx = tx;
-    ua.nt = tr.nt;
-    ua.sx = sx;
-    ua.ns = tr.ns;
-    ua.ws = ws;
-    ua.pot = pot;
-    ua.perm_t = tr.perm_t;
-    ua.out = ans;
-    ua.out_f32 = sizeof(T) == 4;
-    call_user_hook(ctx, ua);
-  } else {
-    dispatch_kernel<P2PLaunch<T>>(ctx->kernel_id, d, ctx, tr, tx, sx, ws, R, ctx->p0, pot, ans);
-  }
-}
-
 template <typename T>
 void launch_gather_points(fmma_ctx* ctx, const T* p, const int* perm, int64_t n, int d, double* out) {
   if (n > 0) FMMA_LAUNCH(ctx, k_gather_points<T>, grid_for(n, 256), 256, 0, p, perm, n, d, out);
@@ -973,10 +702,6 @@ void launch_gather_weights(fmma_ctx* ctx, const T* w, const int* perm, int64_t n
   if (ns > 0) FMMA_LAUNCH(ctx, k_gather_weights<T>, grid_for(ns * R, 256), 256, 0, w, perm, ns, R, out);
 }
 
-template void near_field_f64<double>(fmma_ctx*, int, int, const Tree&, const double*, const double*, const double*,
-                                     const double*, double*);
-template void near_field_f64<float>(fmma_ctx*, int, int, const Tree&, const double*, const double*, const double*,
-                                    const double*, float*);
 template void launch_gather_points<double>(fmma_ctx*, const double*, const int*, int64_t, int, double*);
 template void launch_gather_points<float>(fmma_ctx*, const float*, const int*, int64_t, int, double*);
 template void launch_gather_weights<double>(fmma_ctx*, const double*, const int*, int64_t, int, double*);
@@ -1238,8 +963,7 @@ void solve_forest(fmma_ctx* ctx, const SolveArgs& a, const std::vector<int64_t>&
   stage_begin(ctx, ST_P2P);
   if (tr.nnear_rows > 0) {
     if (grad) {
-      FMMA_REQUIRE(ctx->kernel_id != kUserKernel, "gradients need a built-in kernel");
-      dispatch_kernel<P2PGradLaunch>(ctx->kernel_id, d, ctx, tr, tx, sx, ws, R, ctx->p0, pot, potg, (double*)ans, grad);
+      near_field_grad_f64(ctx, d, R, tr, tx, sx, ws, pot, potg, (double*)ans, grad);
     } else if (mixed_near) {
       p2p_mixed<T>(ctx, d, tx, sx, ws, R, pot, ans, true);
     } else {

@@ -61,6 +61,11 @@ template <typename T>
 void near_field_f64(fmma_ctx* ctx, int d, int R, const Tree& tr, const double* tx, const double* sx, const double* ws,
                     const double* pot, T* ans);
 
+// The same with gradients: grad[r][perm_t[t]][q] = potg[r][t][q] + sum w d f/d x_q
+// (potg may be NULL; ans may be NULL).
+void near_field_grad_f64(fmma_ctx* ctx, int d, int R, const Tree& tr, const double* tx, const double* sx,
+                         const double* ws, const double* pot, const double* potg, double* ans, double* grad);
+
 // out[q][i] = p[perm[i]][q] (FP64); out[r][i] = w[r][perm[i]] (1 when w is NULL).
 template <typename T>
 void launch_gather_points(fmma_ctx* ctx, const T* p, const int* perm, int64_t n, int d, double* out);
