@@ -565,16 +565,17 @@ constexpr int kM2PMaxFar = 192;
 // TPB threads per block: 256, or 64 on levels whose boxes hold few targets
 // (most of a wide block would idle there).
 template <int KID, int D, int RB, int TPB>
-__global__ void __launch_bounds__(TPB, (RB == 1 ? 768 : 512) / TPB) k_m2p_f64(
+__global__ void __launch_bounds__(TPB, (RB == 1 ? 640 : 512) / TPB) k_m2p_f64(
     const int* __restrict__ row_box, int64_t nrow, const int* __restrict__ il, int nfar,
     const uint64_t* __restrict__ key, const int* __restrict__ tb, const int* __restrict__ te, int v,
     const int* __restrict__ depth, const Cube* __restrict__ cubes, const double* __restrict__ tx, int64_t nt,
     const double* __restrict__ node_all, int n, int P, int Kpad, int R, int r0, int NB, double p0,
     const double* __restrict__ Wm, double* __restrict__ pot) {
-  extern __shared__ double m2p_sm[];
+  extern __shared__ __align__(16) double m2p_sm[];
   double* sW = m2p_sm;                        // [NB][RB][P]
   double* sX = sW + (size_t)NB * RB * P;      // [NB][D][n]
   constexpr int kWarps = TPB / 32;
+  const double ip = kinv<KID>(p0);
   __shared__ int sList[kM2PMaxFar];
   __shared__ int sWarp[kM2PMaxFar / 32 + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -639,7 +640,7 @@ __global__ void __launch_bounds__(TPB, (RB == 1 ? 768 : 512) / TPB) k_m2p_f64(
           sX[i] = (node_all[k * D + q] + 1.0) / 2.0 * len + corner;
         }
         __syncthreads();
-        if (tv)
+        if (tv && !far_batch<KID, D, RB>(x, sX, sW, nb, n, P, p0, ip, acc, [](int) { return false; }))
           for (int j = 0; j < nb; ++j) far_box_sum<KID, D, RB>(x, sX + j * D * n, sW + j * RB * P, n, P, p0, acc);
       }
       if (tv) {

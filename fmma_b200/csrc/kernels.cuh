@@ -96,10 +96,14 @@ __device__ __forceinline__ void kparts(const double* x, const double* y, double&
     if (KID == FMMA_KERNEL_SUM2_OVER_R2) { const double u = x[q] + y[q]; s += u * u; }
   }
 }
-template <int KID, int U>
+// MID: every r2 is known to lie within 2^+-500.
+template <int KID, int U, bool MID = false>
 __device__ __forceinline__ void kvals(const double (&r2)[U], const double (&s)[U], double p0, double ip,
                                       double (&f)[U]) {
-  if constexpr (KID == FMMA_KERNEL_INV_R || KID == FMMA_KERNEL_INV_R_SAFE) {
+  if constexpr (MID && (KID == FMMA_KERNEL_INV_R || KID == FMMA_KERNEL_INV_R_SAFE)) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) f[u] = inv_sqrt_normal(r2[u]);
+  } else if constexpr (KID == FMMA_KERNEL_INV_R || KID == FMMA_KERNEL_INV_R_SAFE) {
     bool odd = false;
 #pragma unroll
     for (int u = 0; u < U; ++u) {

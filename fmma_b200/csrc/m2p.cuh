@@ -16,22 +16,90 @@
 
 namespace fmma_b200 {
 
-// Kernel value for the far sums: 1/r through rsqrt (one rounding instead of
-// the square root and divide of keval, which keeps the near field and exact
-// sums bit-comparable with the reference); every other kernel as keval.
-template <int KID, int D>
-__device__ __forceinline__ double kfar(const double* x, const double* y, double p0) {
-  if constexpr (KID == FMMA_KERNEL_INV_R || KID == FMMA_KERNEL_INV_R_SAFE) {
-    double r2 = 0.0;
+// For the radial kernels the node grid saves work: the squares of the outer
+// dimensions are formed once per row of nodes, the innermost differences once
+// per box, so a pair costs one multiply-add for r^2, f (5 operations for 1/r)
+// and one multiply-add per right-hand side: 7 FP64 operations for 1/r instead
+// of 16 with rsqrt() and all differences per pair.  N nodes per dimension, at
+// compile time: a row's N evaluations are independent.
+template <int KID, int D, int RB, int N>
+__device__ __forceinline__ void far_box_row(const double* x, const double* __restrict__ X,
+                                            const double* __restrict__ W, int P, double p0, double ip, double* acc) {
+  double t[N];  // innermost differences
 #pragma unroll
-    for (int q = 0; q < D; ++q) {
-      const double t = x[q] - y[q];
-      r2 += t * t;
+  for (int o = 0; o < N; ++o) t[o] = x[D - 1] - X[(D - 1) * N + o];
+  // exponents of the outer part a and of the smallest and largest |t| that
+  // keep every r^2 = a + t^2 of a row within 2^+-500
+  constexpr int kLo = (1023 - 500) << 20, kHi = (1023 + 498) << 20;
+  int tlo = 0x7fffffff, thi = 0;
+#pragma unroll
+  for (int o = 0; o < N; ++o) {
+    const int h = __double2hiint(t[o]) & 0x7fffffff;
+    tlo = min(tlo, h);
+    thi = max(thi, h);
+  }
+  const bool top = thi < ((1023 + 248) << 20), bottom = tlo >= ((1023 - 249) << 20);
+  const double none[N] = {};
+  auto row = [&](double a, const double* Wk) {
+    double r2[N], f[N];
+#pragma unroll
+    for (int o = 0; o < N; ++o) r2[o] = fma(t[o], t[o], a);
+    const int h = __double2hiint(a);
+    if (top && h < kHi && (bottom || h >= kLo)) kvals<KID, N, true>(r2, none, p0, ip, f);
+    else kvals<KID, N>(r2, none, p0, ip, f);
+#pragma unroll
+    for (int rr = 0; rr < RB; ++rr) {
+      if constexpr (N % 2 == 0) {  // rows of weights on 16 bytes
+#pragma unroll
+        for (int o = 0; o < N; o += 2) {
+          const double2 w = *reinterpret_cast<const double2*>(Wk + rr * P + o);
+          acc[rr] = fma(f[o], w.x, acc[rr]);
+          acc[rr] = fma(f[o + 1], w.y, acc[rr]);
+        }
+      } else {
+#pragma unroll
+        for (int o = 0; o < N; ++o) acc[rr] = fma(f[o], Wk[rr * P + o], acc[rr]);
+      }
     }
-    if constexpr (KID == FMMA_KERNEL_INV_R_SAFE) return r2 > 0.0 ? rsqrt(r2) : 0.0;
-    return rsqrt(r2);
+  };
+  if constexpr (D == 1) {
+    row(0.0, W);
   } else {
-    return keval<KID, D>(x, y, p0);
+#pragma unroll 1
+    for (int o0 = 0; o0 < N; ++o0) {
+      const double d0 = x[0] - X[o0], a0 = d0 * d0;
+      if constexpr (D == 2) {
+        row(a0, W + o0 * N);
+      } else {
+#pragma unroll 1
+        for (int o1 = 0; o1 < N; ++o1) {
+          const double d1 = x[1] - X[N + o1];
+          row(fma(d1, d1, a0), W + (o0 * N + o1) * N);
+        }
+      }
+    }
+  }
+}
+
+// far_box_row for the boxes j < nb of a staged batch that `skip(j)` lets
+// through; false when the kernel or the node count is not covered.
+template <int KID, int D, int RB, typename Skip>
+__device__ __forceinline__ bool far_batch(const double* x, const double* X, const double* W, int nb, int n, int P,
+                                          double p0, double ip, double* acc, const Skip& skip) {
+  if constexpr (RB != 1 || (KID != FMMA_KERNEL_INV_R && KID != FMMA_KERNEL_INV_R_SAFE && KID != FMMA_KERNEL_LOG_R &&
+                            KID != FMMA_KERNEL_GAUSSIAN && KID != FMMA_KERNEL_MULTIQUADRIC)) {
+    return false;
+  } else {
+#define FMMA_FAR_N(N_)                                                                                         \
+  case N_:                                                                                                     \
+    for (int j = 0; j < nb; ++j)                                                                               \
+      if (!skip(j)) far_box_row<KID, D, RB, N_>(x, X + j * D * N_, W + (size_t)j * RB * P, P, p0, ip, acc);    \
+    return true;
+    switch (n) {
+      FMMA_FAR_N(2) FMMA_FAR_N(3) FMMA_FAR_N(4) FMMA_FAR_N(5) FMMA_FAR_N(6) FMMA_FAR_N(7) FMMA_FAR_N(8)
+      default: return false;
+    }
+#undef FMMA_FAR_N
   }
 }
 
@@ -43,7 +111,7 @@ __device__ __forceinline__ void far_box_sum(const double* x, const double* __res
 #pragma unroll 4
     for (int o0 = 0; o0 < n; ++o0) {
       y[0] = X[o0];
-      const double f = kfar<KID, D>(x, y, p0);
+      const double f = keval<KID, D>(x, y, p0);
 #pragma unroll
       for (int rr = 0; rr < RB; ++rr) acc[rr] += f * W[rr * P + o0];
     }
@@ -54,7 +122,7 @@ __device__ __forceinline__ void far_box_sum(const double* x, const double* __res
 #pragma unroll 4
       for (int o1 = 0; o1 < n; ++o1) {
         y[1] = X[n + o1];
-        const double f = kfar<KID, D>(x, y, p0);
+        const double f = keval<KID, D>(x, y, p0);
 #pragma unroll
         for (int rr = 0; rr < RB; ++rr) acc[rr] += f * Wk[rr * P + o1];
       }
@@ -68,7 +136,7 @@ __device__ __forceinline__ void far_box_sum(const double* x, const double* __res
 #pragma unroll 4
         for (int o2 = 0; o2 < n; ++o2) {
           y[2] = X[2 * n + o2];
-          const double f = kfar<KID, D>(x, y, p0);
+          const double f = keval<KID, D>(x, y, p0);
 #pragma unroll
           for (int rr = 0; rr < RB; ++rr) acc[rr] += f * Wk[rr * P + o2];
         }

@@ -119,14 +119,15 @@ __host__ __device__ inline int far_box_bytes(int D, int RB, int P, int n) {
 // part[y][r][t] for r in [r0, r0 + RB): the far sum of sorted target t over
 // the y-th slice of the source-box list.
 template <int KID, int D, int RB>
-__global__ void __launch_bounds__(kFarThreads, RB == 1 ? 3 : 2) k_nrn_far(
+__global__ void __launch_bounds__(kFarThreads, 2) k_nrn_far(
     const double* __restrict__ tx, int64_t nt, const uint64_t* __restrict__ tkey, const int* __restrict__ sbox,
     const int* __restrict__ nsbox, int N, int n, int P, int Kpad, int R, int r0, int NB,
     const double* __restrict__ gx, const double* __restrict__ Wm, double p0, double* __restrict__ part) {
-  extern __shared__ double far_sm[];
+  extern __shared__ __align__(16) double far_sm[];
   double* sW = far_sm;                                        // [NB][RB][P]
   double* sX = sW + (size_t)NB * RB * P;                      // [NB][D][n]
   int* sB = reinterpret_cast<int*>(sX + (size_t)NB * D * n);  // [NB][D] box coordinates
+  const double ip = kinv<KID>(p0);
   const int nsb = *nsbox;
   const int per = (nsb + (int)gridDim.y - 1) / (int)gridDim.y;
   const int b0 = (int)blockIdx.y * per, b1 = min(nsb, b0 + per);
@@ -164,13 +165,15 @@ __global__ void __launch_bounds__(kFarThreads, RB == 1 ? 3 : 2) k_nrn_far(
     }
     __syncthreads();
     if (!tv) continue;
-    for (int j = 0; j < nb; ++j) {
-      bool near = true;
+    auto near = [&](int j) {
+      bool in = true;
 #pragma unroll
-      for (int q = 0; q < D; ++q) near = near && abs(sB[j * D + q] - bi[q]) <= 1;
-      if (near) continue;
-      far_box_sum<KID, D, RB>(x, sX + j * D * n, sW + j * RB * P, n, P, p0, acc);
-    }
+      for (int q = 0; q < D; ++q) in = in && abs(sB[j * D + q] - bi[q]) <= 1;
+      return in;
+    };
+    if (far_batch<KID, D, RB>(x, sX, sW, nb, n, P, p0, ip, acc, near)) continue;
+    for (int j = 0; j < nb; ++j)
+      if (!near(j)) far_box_sum<KID, D, RB>(x, sX + j * D * n, sW + j * RB * P, n, P, p0, acc);
   }
   if (tv) {
 #pragma unroll
