@@ -882,77 +882,101 @@ __global__ void __launch_bounds__(kWarpThreads, 4) k_l2lp_coef(
 // leaves only boxes holding targets are listed (the near-field rows).  nbr,
 // il and slot_mask must be pre-filled (-1, -1, 0).
 // ---------------------------------------------------------------------------
-__global__ void k_lists_topdown(const uint64_t* __restrict__ key, const int* __restrict__ parent, int64_t nbox,
-                                const int* __restrict__ tb, const int* __restrict__ te, bool leaf,
-                                const int* __restrict__ sb, const int* __restrict__ se,
-                                const int* __restrict__ pnbr, const int* __restrict__ pcb,
-                                const int* __restrict__ pce, int d, const int* __restrict__ row_of_box, int nfar,
-                                const int* __restrict__ jslot, int* __restrict__ nbr, int* __restrict__ il,
-                                unsigned* __restrict__ slot_mask, unsigned long long* __restrict__ pairs) {
+// Boxes of level v from entry `first`, `step` entries apart.
+__device__ __forceinline__ void lists_of_level(const ListLevels& g, int v, int64_t first, int64_t step,
+                                               unsigned long long& mine) {
+  const int d = g.d;
   const int nnb = d == 1 ? 3 : (d == 2 ? 9 : 27);
   const int center = (nnb - 1) / 2;
-  const int64_t total = nbox * nnb;
   const uint64_t cmask = (1ull << d) - 1ull;
-  unsigned long long mine = 0;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
+  const int64_t o = g.box0[v], po = v + 1 < g.V ? g.box0[v + 1] : 0;
+  const uint64_t* key = g.key + o;
+  const int *sb = g.sb + o, *se = g.se + o;
+  int* nbr = g.nbr + o * nnb;
+  int* il = g.il + g.row0[v] * g.nfar;
+  unsigned* slot_mask = g.slot_mask + g.row0[v] * kSlotWords;
+  const int64_t total = g.nbox[v] * nnb;
+  for (int64_t e = first; e < total; e += step) {
     const int64_t b = e / nnb;
     const int s = (int)(e - b * nnb);
-    if (leaf && te[b] <= tb[b]) continue;  // no level below reads a leaf's neighbours: targets only
-    const int p = parent[b];
+    if (v == 0 && g.te[b] <= g.tb[b]) continue;  // no level below reads a leaf's neighbours: targets only
+    const int p = g.parent[o + b];
     if (p < 0) {  // a root: its only neighbour is itself
       if (s == center) nbr[b * nnb + center] = (int)b;
       continue;
     }
-    const int pn = pnbr[(int64_t)p * nnb + s];
+    const int pn = g.nbr[(po + p) * nnb + s];
     if (pn < 0) continue;
     const int cls = (int)(key[b] & cmask);
-    const int row = row_of_box ? row_of_box[b] : -1;
+    const int row = g.rows[v] ? g.row_of[o + b] : -1;
     int dig[kMaxDim] = {0, 0, 0};
     int sc = s;
     for (int q = d - 1; q >= 0; --q) {
       dig[q] = sc % 3;  // the parent's neighbour at offset dig - 1
       sc /= 3;
     }
-    for (int ch = pce[pn] - 1; ch >= pcb[pn]; --ch) {
+    for (int ch = g.ce[po + pn] - 1; ch >= g.cb[po + pn]; --ch) {
       const uint64_t ck = key[ch];
       bool near = true;
       int js = 0, jw = 0;
       for (int q = 0; q < d; ++q) {
         const int w = 2 * dig[q] + (int)((ck >> (d - 1 - q)) & 1ull);         // position in the 6^d window
-        const int o = w - 2 - (int)((cls >> (d - 1 - q)) & 1);                  // offset from the box
-        near = near && o >= -1 && o <= 1;
-        js = js * 3 + (o + 1);
+        const int oo = w - 2 - (int)((cls >> (d - 1 - q)) & 1);                 // offset from the box
+        near = near && oo >= -1 && oo <= 1;
+        js = js * 3 + (oo + 1);
         jw = jw * 6 + w;
       }
       if (near) {
         nbr[b * nnb + js] = ch;
       } else if (row >= 0 && se[ch] > sb[ch]) {
-        const int slot = jslot[cls * 216 + jw];
-        il[(int64_t)row * nfar + slot] = ch;
+        const int slot = g.jslot[cls * 216 + jw];
+        il[(int64_t)row * g.nfar + slot] = ch;
         atomicOr(slot_mask + (int64_t)row * kSlotWords + (slot >> 5), 1u << (slot & 31));
         ++mine;
       }
     }
   }
+}
+
+__device__ __forceinline__ void add_pairs(unsigned long long mine, unsigned long long* pairs) {
   for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
   if ((threadIdx.x & 31) == 0 && mine) atomicAdd(pairs, mine);
 }
 
-__global__ void k_rows_of_boxes(const int* __restrict__ row_box, int64_t nrow, int* __restrict__ row_of_box) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrow; r += (int64_t)gridDim.x * blockDim.x)
-    row_of_box[row_box[r]] = (int)r;
+__global__ void k_lists_topdown(const __grid_constant__ ListLevels g, int v) {
+  unsigned long long mine = 0;
+  lists_of_level(g, v, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x, mine);
+  add_pairs(mine, g.pairs + v);
 }
 
-// near[row][s] = the leaf neighbour at slot s when it holds sources, else -1
+// The levels V-1 .. vlast, each of at most a few thousand list entries, in one
+// block with a barrier between levels (a launch each otherwise).
+__global__ void __launch_bounds__(1024) k_lists_coarse(const __grid_constant__ ListLevels g, int vlast) {
+  for (int v = g.V - 1; v >= vlast; --v) {
+    unsigned long long mine = 0;
+    lists_of_level(g, v, threadIdx.x, blockDim.x, mine);
+    add_pairs(mine, g.pairs + v);
+    __syncthreads();  // this level's neighbours are read by the next
+  }
+}
+
+// near[row][s] = the leaf neighbour at slot s when it holds sources, else -1;
+// *pairs += targets x sources over the lists.
 __global__ void k_near_rows(const int* __restrict__ nbr, const int* __restrict__ row_box, int64_t nrow, int nnb,
-                            const int* __restrict__ sb, const int* __restrict__ se, int* __restrict__ near) {
+                            const int* __restrict__ tb, const int* __restrict__ te, const int* __restrict__ sb,
+                            const int* __restrict__ se, int* __restrict__ near, unsigned long long* pairs) {
+  unsigned long long mine = 0;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nrow * nnb;
        e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = e / nnb;
     const int s = (int)(e - r * nnb);
-    const int nb = nbr[(int64_t)row_box[r] * nnb + s];
-    near[e] = (nb >= 0 && se[nb] > sb[nb]) ? nb : -1;
+    const int b = row_box[r];
+    const int nb = nbr[(int64_t)b * nnb + s];
+    const int cnt = nb >= 0 ? se[nb] - sb[nb] : 0;
+    near[e] = cnt > 0 ? nb : -1;
+    if (cnt > 0) mine += (unsigned long long)cnt * (unsigned long long)(te[b] - tb[b]);
   }
+  add_pairs(mine, pairs);
 }
 
 // ---------------------------------------------------------------------------
@@ -1155,31 +1179,24 @@ bool launch_l2lp_leaf(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t 
   return false;
 }
 
-void launch_lists_topdown(fmma_ctx* ctx, const Level& Lv, const Level* Pl, const int* pnbr, int d, int nfar,
-                          const int* jslot, int* nbr, int* row_of_box, unsigned long long* pairs) {
-  const int nnb = d == 1 ? 3 : (d == 2 ? 9 : 27);
-  const int64_t nb = Lv.nbox;
-  if (nb == 0) return;
-  FMMA_CHECK_CUDA(cudaMemsetAsync(nbr, 0xff, sizeof(int) * (size_t)nb * nnb, ctx->stream));
-  const int* rob = nullptr;
-  if (Lv.nrow > 0) {
-    FMMA_CHECK_CUDA(cudaMemsetAsync(row_of_box, 0xff, sizeof(int) * (size_t)nb, ctx->stream));
-    FMMA_LAUNCH(ctx, k_rows_of_boxes, grid_for(Lv.nrow, 256), 256, 0, Lv.row_box, Lv.nrow, row_of_box);
-    FMMA_CHECK_CUDA(cudaMemsetAsync(Lv.il, 0xff, sizeof(int) * (size_t)Lv.nrow * nfar, ctx->stream));
-    FMMA_CHECK_CUDA(cudaMemsetAsync(Lv.slot_mask, 0, sizeof(unsigned) * (size_t)Lv.nrow * kSlotWords, ctx->stream));
-    rob = row_of_box;
-  }
-  FMMA_LAUNCH(ctx, k_lists_topdown, grid_for(nb * nnb, 256, (int64_t)ctx->sm_count * 64), 256, 0, Lv.key, Lv.parent,
-              nb, Lv.tb, Lv.te, Lv.v == 0, Lv.sb, Lv.se, pnbr, Pl ? Pl->cb : nullptr, Pl ? Pl->ce : nullptr, d, rob, nfar, jslot, nbr,
-              Lv.il, Lv.slot_mask, pairs);
+void launch_lists_topdown(fmma_ctx* ctx, const ListLevels& ll) {
+  const int nnb = ll.d == 1 ? 3 : (ll.d == 2 ? 9 : 27);
+  // a block of 1024 takes 4096 entries in the time of a launch
+  constexpr int64_t kCoarse = 4096;
+  int v = ll.V - 1;
+  while (v >= 0 && ll.nbox[v] * nnb <= kCoarse) --v;
+  if (v + 1 < ll.V) FMMA_LAUNCH(ctx, k_lists_coarse, 1, 1024, 0, ll, v + 1);
+  for (; v >= 0; --v)
+    if (ll.nbox[v] > 0)
+      FMMA_LAUNCH(ctx, k_lists_topdown, grid_for(ll.nbox[v] * nnb, 256, (int64_t)ctx->sm_count * 64), 256, 0, ll, v);
 }
 
-void launch_near_rows(fmma_ctx* ctx, const int* nbr, const int* row_box, int64_t nrow, int d, const int* sb,
-                      const int* se, int* near) {
+void launch_near_rows(fmma_ctx* ctx, const int* nbr, const int* row_box, int64_t nrow, int d, const int* tb,
+                      const int* te, const int* sb, const int* se, int* near, unsigned long long* pairs) {
   const int nnb = d == 1 ? 3 : (d == 2 ? 9 : 27);
   if (nrow > 0)
     FMMA_LAUNCH(ctx, k_near_rows, grid_for(nrow * nnb, 256, (int64_t)ctx->sm_count * 64), 256, 0, nbr, row_box, nrow,
-                nnb, sb, se, near);
+                nnb, tb, te, sb, se, near, pairs);
 }
 
 }  // namespace fmma_b200

@@ -115,14 +115,7 @@ struct Tree {
   int* near_row_box = nullptr;
   int* near = nullptr;
   int64_t p2p_pairs = 0;
-  // counted from the sorted keys before the levels are emitted: M2L rows of
-  // every virtual level and near-field rows; a nonzero *d_err means a level
-  // emitted more boxes than counted (checked at the last read-back)
-  std::vector<int> row_count;
-  int64_t near_count = 0;
-  int* d_err = nullptr;
-  // the pair counts (il_pairs per level, p2p_pairs) and d_err stay on the
-  // device until the host needs them (tree_read_pairs), so the build itself
+  // the pair counts (il_pairs per level, p2p_pairs) stay on the device until the host needs them (tree_read_pairs), so the build itself
   // ends without a wait
   unsigned long long* d_pairs = nullptr;
   bool pairs_read = true;
@@ -288,8 +281,11 @@ void kernel_timer_begin(fmma_ctx* ctx);
 // M2L launch timer; flops_per_pair x the level's (target box, source box)
 // pairs (read when the timers are collected) gives the launch's flops
 void kernel_timer_end(fmma_ctx* ctx, double flops_per_pair, int tag);
-// brings the tree's pair counts to the host (one wait, once per build) and
-// checks the build's overflow flag
+// brings the tree's pair counts to the host: the copy into pinned memory (at
+// most 33 values), enqueued on the stream (false: nothing to read), and taking
+// them after a wait; or both with a wait of its own
+bool tree_fetch_pairs(fmma_ctx* ctx, void* pinned);
+void tree_take_pairs(fmma_ctx* ctx, const void* pinned);
 void tree_read_pairs(fmma_ctx* ctx);
 
 // Stage timing with CUDA events on the context stream.
@@ -306,12 +302,22 @@ void scan_exclusive(fmma_ctx* ctx, const int* in, int* out, int64_t n, int* tota
 // Stable LSD radix sort of (key, val) pairs on bits [bit0, bit1) of the key.
 // Results end in keys/vals (tmp buffers from the context).
 void radix_sort_pairs(fmma_ctx* ctx, uint64_t* keys, int* vals, int64_t n, int bit0, int bit1);
+// The same, leaving the result wherever the passes end: *keys and *vals are
+// swapped with the second pair of buffers after each pass.
+void radix_sort_swap(fmma_ctx* ctx, uint64_t** keys, int** vals, uint64_t** keys2, int** vals2, int64_t n, int bit0,
+                     int bit1);
+// Exclusive scans of nrow rows of n values in one launch (out may not be in);
+// totals_dev[row] = the row's sum.
+void scan_rows(fmma_ctx* ctx, const int* in, int* out, int64_t n, int nrow, int* totals_dev);
 // Copy n ints device -> host (synchronous on the context stream).
 void read_ints(fmma_ctx* ctx, const int* dev, int* host, int n);
-// error flag of the tensor-core M2L at virtual level v (one buffer for all
-// levels), and the check of a solve's flags with one read (FMMA_ERR_TIMEOUT)
+// error flag of the M2L at virtual level v (one buffer for all levels); the
+// copy of a solve's flags to pinned memory (kErrSlots ints), enqueued on the
+// stream, and their check after a wait (FMMA_ERR_TIMEOUT)
+constexpr int kErrSlots = 64;
 int* m2l_err_slot(fmma_ctx* ctx, int v);
-void check_m2l_errs(fmma_ctx* ctx, const std::vector<int*>& flags);
+void fetch_m2l_errs(fmma_ctx* ctx, const std::vector<int*>& flags, int* host);
+void check_m2l_errs(fmma_ctx* ctx, const std::vector<int*>& flags, const int* host);
 
 // ---------------------------------------------------------------------------
 // tree (tree.cu)
@@ -446,14 +452,25 @@ bool l2lp_leaf_ok(const Level& Lf, int64_t nt, int d, int n, int mode);
 bool launch_l2lp_leaf(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t nt, const Cube* cubes,
                       const int* depth, int d, bool isf, int n, int Kpad, const double* Tn, const double* A,
                       const double* Wp, const double* Wc, double* pot);
-// Neighbour lists of every box of level Lv (nbr, [nbox][3^d]) from the
-// parent level's (pnbr; Pl == nullptr at the top level), and the far lists
-// (il, slot_mask) of Lv's rows; row_of_box is scratch of Lv.nbox ints.
-void launch_lists_topdown(fmma_ctx* ctx, const Level& Lv, const Level* Pl, const int* pnbr, int d, int nfar,
-                          const int* jslot, int* nbr, int* row_of_box, unsigned long long* pairs);
-// P2P near lists of the leaf rows from the leaf neighbour lists.
-void launch_near_rows(fmma_ctx* ctx, const int* nbr, const int* row_box, int64_t nrow, int d, const int* sb,
-                      const int* se, int* near);
+// Neighbour lists of every box of every level (nbr, [box][3^d]), top-down, and
+// the far lists (il, slot_mask) of the rows.  The arrays hold all levels: box b
+// of level v at box0[v] + b, row r at row0[v] + r; row_of[box] is the row
+// within the level or -1.  nbr, il and slot_mask are pre-filled (-1, -1, 0).
+struct ListLevels {
+  int V, d, nfar;
+  int64_t box0[32], row0[32], nbox[32];
+  bool rows[32];  // the level has rows
+  const uint64_t* key;
+  const int *parent, *tb, *te, *sb, *se, *cb, *ce, *row_of, *jslot;
+  int *nbr, *il;
+  unsigned* slot_mask;
+  unsigned long long* pairs;  // per level
+};
+void launch_lists_topdown(fmma_ctx* ctx, const ListLevels& ll);
+// P2P near lists of the leaf rows from the leaf neighbour lists; *pairs += the
+// point pairs.
+void launch_near_rows(fmma_ctx* ctx, const int* nbr, const int* row_box, int64_t nrow, int d, const int* tb,
+                      const int* te, const int* sb, const int* se, int* near, unsigned long long* pairs);
 
 // ---------------------------------------------------------------------------
 // FMM stages

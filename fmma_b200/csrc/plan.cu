@@ -299,11 +299,13 @@ fmma_status fmma_plan_execute_d(fmma_plan* p, const double* w, double* ans, int 
                                     mem_kind == FMMA_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice,
                                     c->stream));
     FMMA_CHECK_CUDA(cudaEventRecord(p->ev[1], c->stream));
-    FMMA_CHECK_CUDA(cudaEventSynchronize(p->ev[1]));
+    int* errs = static_cast<int*>(ctx_pinned(c, sizeof(int) * kErrSlots));
+    fetch_m2l_errs(c, p->err_flags, errs);
+    FMMA_CHECK_CUDA(cudaStreamSynchronize(c->stream));
     float ms = 0.f;
     FMMA_CHECK_CUDA(cudaEventElapsedTime(&ms, p->ev[0], p->ev[1]));
     p->last_ms = ms;
-    check_m2l_errs(c, p->err_flags);
+    check_m2l_errs(c, p->err_flags, errs);
   });
 }
 

@@ -99,20 +99,23 @@ void upload(fmma_ctx* ctx, void* dst, const void* src, size_t bytes) {
 
 // The bounded-wait error flags of the tensor-core M2L, one slot per virtual
 // level in one small buffer, so the host reads all of them with one copy.
-constexpr int kErrSlots = 64;
 
 int* m2l_err_slot(fmma_ctx* ctx, int v) {
   FMMA_REQUIRE(v >= 0 && v < kErrSlots, "too many levels");
   return ctx_buf_t<int>(ctx, "tc_err_all", kErrSlots) + v;
 }
 
-void check_m2l_errs(fmma_ctx* ctx, const std::vector<int*>& flags) {
+void fetch_m2l_errs(fmma_ctx* ctx, const std::vector<int*>& flags, int* host) {
   if (flags.empty()) return;
   const int* base = ctx_buf_t<int>(ctx, "tc_err_all", kErrSlots);
-  int h[kErrSlots];
-  FMMA_CHECK_CUDA(cudaMemcpy(h, base, sizeof(h), cudaMemcpyDeviceToHost));
+  FMMA_CHECK_CUDA(cudaMemcpyAsync(host, base, sizeof(int) * kErrSlots, cudaMemcpyDeviceToHost, ctx->stream));
+}
+
+void check_m2l_errs(fmma_ctx* ctx, const std::vector<int*>& flags, const int* host) {
+  if (flags.empty()) return;
+  const int* base = ctx_buf_t<int>(ctx, "tc_err_all", kErrSlots);
   for (const int* f : flags)
-    if (h[f - base]) throw Error(FMMA_ERR_TIMEOUT, "tensor-core M2L: a bounded pipeline wait gave up");
+    if (host[f - base]) throw Error(FMMA_ERR_TIMEOUT, "M2L: a bounded pipeline wait gave up");
 }
 
 void read_ints(fmma_ctx* ctx, const int* dev, int* host, int n) {
@@ -169,8 +172,14 @@ void stage_end(fmma_ctx* ctx, Stage s) {
 }
 
 void stages_collect(fmma_ctx* ctx) {
+  // the pair counts and the M2L error flags come with the solve's one final wait
+  char* pin = static_cast<char*>(ctx_pinned(ctx, 1024));
+  int* errs = reinterpret_cast<int*>(pin + 512);
+  static_assert(sizeof(int) * kErrSlots <= 512, "the flags' half of the buffer");
+  const bool pairs = tree_fetch_pairs(ctx, pin);
+  fetch_m2l_errs(ctx, ctx->m2l_err_flags, errs);
   FMMA_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
-  tree_read_pairs(ctx);  // no wait of its own once the stream is idle
+  if (pairs) tree_take_pairs(ctx, pin);
   for (int i = 0; i < ctx->ktimed; ++i) {
     float ms = 0.f;
     FMMA_CHECK_CUDA(cudaEventElapsedTime(&ms, ctx->kev[2 * i], ctx->kev[2 * i + 1]));
@@ -182,8 +191,9 @@ void stages_collect(fmma_ctx* ctx) {
       ctx->m2l_flops += ctx->kflops[i];
     }
   }
-  check_m2l_errs(ctx, ctx->m2l_err_flags);
+  const std::vector<int*> flags = std::move(ctx->m2l_err_flags);
   ctx->m2l_err_flags.clear();
+  check_m2l_errs(ctx, flags, errs);
   for (int i = 0; i < FMMA_NUM_STAGES; ++i) {
     if (!ctx->ev_used[i]) continue;
     float ms = 0.f;
@@ -305,6 +315,40 @@ static void scan_rec(fmma_ctx* ctx, const int* in, int* out, int64_t n, int* tot
   FMMA_LAUNCH(ctx, k_scan_add, (unsigned)nb, kScanThreads, 0, out, n, bo);
 }
 
+// Exclusive scans of nrow rows of n values each, one block a row, in one
+// launch; the rows' totals go to totals[row].
+__global__ void __launch_bounds__(kScanSmallThreads) k_scan_rows(const int* __restrict__ in, int* __restrict__ out,
+                                                                 int64_t n, int* __restrict__ totals) {
+  __shared__ int s_warp[32];
+  in += (int64_t)blockIdx.x * n;
+  out += (int64_t)blockIdx.x * n;
+  int carry = 0;
+  for (int64_t base = 0; base < n; base += (int64_t)kScanSmallThreads * kScanIpt) {
+    const int64_t b = base + (int64_t)threadIdx.x * kScanIpt;
+    int v[kScanIpt];
+    int tsum = 0;
+#pragma unroll
+    for (int i = 0; i < kScanIpt; ++i) {
+      v[i] = b + i < n ? in[b + i] : 0;
+      tsum += v[i];
+    }
+    int total;
+    int ex = carry + block_exclusive_scan(tsum, s_warp, &total);
+#pragma unroll
+    for (int i = 0; i < kScanIpt; ++i) {
+      if (b + i < n) out[b + i] = ex;
+      ex += v[i];
+    }
+    carry += total;
+    __syncthreads();  // s_warp is rewritten by the next tile
+  }
+  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
+
+void scan_rows(fmma_ctx* ctx, const int* in, int* out, int64_t n, int nrow, int* totals_dev) {
+  FMMA_LAUNCH(ctx, k_scan_rows, (unsigned)nrow, kScanSmallThreads, 0, in, out, n, totals_dev);
+}
+
 void scan_exclusive(fmma_ctx* ctx, const int* in, int* out, int64_t n, int* total_dev) {
   scan_rec(ctx, in, out, n, total_dev, 0);
 }
@@ -376,31 +420,30 @@ __global__ void k_rs_scatter(const uint64_t* __restrict__ kin, const int* __rest
   }
 }
 
-void radix_sort_pairs(fmma_ctx* ctx, uint64_t* keys, int* vals, int64_t n, int bit0, int bit1) {
+void radix_sort_swap(fmma_ctx* ctx, uint64_t** keys, int** vals, uint64_t** keys2, int** vals2, int64_t n, int bit0,
+                     int bit1) {
   if (n <= 1 || bit1 <= bit0) return;
-  int64_t nb64 = (n + kRsTile - 1) / kRsTile;
-  int nb = (int)nb64;
-  uint64_t* k2 = ctx_buf_t<uint64_t>(ctx, "rs_k2", (size_t)n);
-  int* v2 = ctx_buf_t<int>(ctx, "rs_v2", (size_t)n);
+  const int nb = (int)((n + kRsTile - 1) / kRsTile);
   int* gh = ctx_buf_t<int>(ctx, "rs_hist", (size_t)256 * nb);
   int* go = ctx_buf_t<int>(ctx, "rs_off", (size_t)256 * nb);
   int* tot = ctx_buf_t<int>(ctx, "rs_tot", 1);
-  uint64_t* ka = keys;
-  int* va = vals;
-  uint64_t* kb = k2;
-  int* vb = v2;
-  int passes = 0;
   for (int shift = bit0; shift < bit1; shift += 8) {
-    FMMA_LAUNCH(ctx, k_rs_hist, nb, kRsThreads, 0, ka, n, shift, gh, nb);
+    FMMA_LAUNCH(ctx, k_rs_hist, nb, kRsThreads, 0, *keys, n, shift, gh, nb);
     scan_exclusive(ctx, gh, go, (int64_t)256 * nb, tot);
-    FMMA_LAUNCH(ctx, k_rs_scatter, nb, kRsThreads, 0, ka, va, kb, vb, n, shift, go, nb);
-    std::swap(ka, kb);
-    std::swap(va, vb);
-    ++passes;
+    FMMA_LAUNCH(ctx, k_rs_scatter, nb, kRsThreads, 0, *keys, *vals, *keys2, *vals2, n, shift, go, nb);
+    std::swap(*keys, *keys2);
+    std::swap(*vals, *vals2);
   }
-  if (passes & 1) {
-    FMMA_CHECK_CUDA(cudaMemcpyAsync(keys, ka, sizeof(uint64_t) * (size_t)n, cudaMemcpyDeviceToDevice, ctx->stream));
-    FMMA_CHECK_CUDA(cudaMemcpyAsync(vals, va, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, ctx->stream));
+}
+
+void radix_sort_pairs(fmma_ctx* ctx, uint64_t* keys, int* vals, int64_t n, int bit0, int bit1) {
+  if (n <= 1 || bit1 <= bit0) return;
+  uint64_t *k = keys, *k2 = ctx_buf_t<uint64_t>(ctx, "rs_k2", (size_t)n);
+  int *v = vals, *v2 = ctx_buf_t<int>(ctx, "rs_v2", (size_t)n);
+  radix_sort_swap(ctx, &k, &v, &k2, &v2, n, bit0, bit1);
+  if (k != keys) {
+    FMMA_CHECK_CUDA(cudaMemcpyAsync(keys, k, sizeof(uint64_t) * (size_t)n, cudaMemcpyDeviceToDevice, ctx->stream));
+    FMMA_CHECK_CUDA(cudaMemcpyAsync(vals, v, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, ctx->stream));
   }
 }
 

@@ -88,12 +88,13 @@ __device__ __forceinline__ int find_seg(const int64_t* __restrict__ off, int np,
   return lo;
 }
 
-// problem id of each element of [targets | sources]
+// problem id of each element of [targets | sources] (a single problem needs none:
+// the kernels below take a null pid for 0)
 __global__ void k_point_pid(const int64_t* __restrict__ toff, const int64_t* __restrict__ soff, int np, int64_t nt,
                             int64_t ns, int* __restrict__ pid) {
   const int64_t n = nt + ns;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    pid[i] = np == 1 ? 0 : (i < nt ? find_seg(toff, np, i) : find_seg(soff, np, i - nt));
+    pid[i] = i < nt ? find_seg(toff, np, i) : find_seg(soff, np, i - nt);
 }
 
 __global__ void k_bbox_init(unsigned long long* mm, int np, int* flag) {
@@ -133,7 +134,7 @@ __global__ void k_bbox(const T* __restrict__ tgt, int64_t nt, const T* __restric
   unsigned long long lo[kMaxDim], hi[kMaxDim];
   for (int q = 0; q < kMaxDim; ++q) { lo[q] = ~0ull; hi[q] = 0ull; }
   for (int64_t i = b0 + lane; i < b1; i += 32) {
-    const int p = pid[i];
+    const int p = pid ? pid[i] : 0;
     if (p != cur) {
       if (cur >= 0) bbox_flush(mm, cur, d, lo, hi);
       for (int q = 0; q < kMaxDim; ++q) { lo[q] = ~0ull; hi[q] = 0ull; }
@@ -198,7 +199,7 @@ __global__ void k_leaf_keys(const T* __restrict__ tgt, int64_t nt, const T* __re
                             const Cube* __restrict__ cubes, uint64_t* __restrict__ keys, int* __restrict__ idx) {
   const int64_t n = nt + ns;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int p = pid[i];
+    const int p = pid ? pid[i] : 0;
     const Cube& c = cubes[p];
     const int bits = depth[p] - 1;
     const int N = 1 << bits;
@@ -211,218 +212,192 @@ __global__ void k_leaf_keys(const T* __restrict__ tgt, int64_t nt, const T* __re
 }
 
 // ---------------------------------------------------------------------------
-// leaves and levels
-// ---------------------------------------------------------------------------
-__global__ void k_leaf_flags(const uint64_t* __restrict__ keys, const int* __restrict__ idx, int64_t n,
-                             int64_t nt, int* __restrict__ fbox, int* __restrict__ ft) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    fbox[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1 : 0;
-    ft[i] = idx[i] < nt ? 1 : 0;
-  }
-}
-
-__global__ void k_leaf_emit(const uint64_t* __restrict__ keys, const int* __restrict__ idx, int64_t n,
-                            int64_t nt, const int* __restrict__ fbox, const int* __restrict__ boxex,
-                            const int* __restrict__ tex, int* __restrict__ perm_t,
-                            int* __restrict__ perm_s, uint64_t* __restrict__ lkey,
-                            int* __restrict__ ltb, int* __restrict__ lsb) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int id = idx[i];
-    int tpos = tex[i];
-    int spos = (int)i - tpos;
-    if (id < nt) perm_t[tpos] = id;
-    else perm_s[spos] = id - (int)nt;
-    if (fbox[i]) {
-      int b = boxex[i];
-      lkey[b] = keys[i];
-      ltb[b] = tpos;
-      lsb[b] = spos;
-    }
-  }
-}
-
-__global__ void k_leaf_ends(int64_t nb, const int* __restrict__ tb, const int* __restrict__ sb,
-                            int nt, int ns, int* __restrict__ te, int* __restrict__ se) {
-  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
-       b += (int64_t)gridDim.x * blockDim.x) {
-    te[b] = b + 1 < nb ? tb[b + 1] : nt;
-    se[b] = b + 1 < nb ? sb[b + 1] : ns;
-  }
-}
-
-__device__ __forceinline__ uint64_t parent_key(uint64_t k, int d) {
-  return (k & ~kMortonMask) | ((k & kMortonMask) >> d);
-}
-__device__ __forceinline__ int real_level(uint64_t k, const int* depth, int v) {
-  return depth[key_pid(k)] - 1 - v;
-}
-
-// A box of virtual level v has a parent when its real level is >= 1.
-__global__ void k_parent_flags(const uint64_t* __restrict__ ckey, int64_t nc, int d, int v,
-                               const int* __restrict__ depth, int* __restrict__ f) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nc;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = ckey[i];
-    const bool valid = real_level(k, depth, v) >= 1;
-    bool first = valid;
-    if (valid && i > 0) {
-      const uint64_t kp = ckey[i - 1];
-      first = real_level(kp, depth, v) < 1 || parent_key(kp, d) != parent_key(k, d);
-    }
-    f[i] = first ? 1 : 0;
-  }
-}
-
-// Box counts of every virtual level from key-sorted keys in one pass.  Key i
-// opens a new box at virtual level v when its level-v ancestor differs from
+// leaves and levels: every level from the sorted keys in three launches
+//
+// Key i opens a box at virtual level v when its level-v ancestor differs from
 // key i-1's: at every level v <= hb / d, hb the highest bit in which the two
-// Morton codes differ, and at every level when the problem changes.  Levels
-// stop at the problem's real level `cut` (virtual level depth - 1 - cut).
-// hist[t] counts the keys whose highest new level is t, so level v holds
-// sum_{t >= v} hist[t] boxes.  Two cuts at once: the points' keys give the
-// boxes of every level (cut 0); the targets' keys give the boxes holding
-// targets (cut 0: near-field rows) and those at real level >= 2 (cut 2: M2L
-// rows).
-__global__ void k_level_counts(const uint64_t* __restrict__ keys, int64_t n, int d,
-                               const int* __restrict__ depth, int nlev, int cut_a, int* __restrict__ hist_a,
-                               int cut_b, int* __restrict__ hist_b) {
-  __shared__ int ha[32], hb[32];
-  if (threadIdx.x < 32) {
-    ha[threadIdx.x] = 0;
-    hb[threadIdx.x] = 0;
+// Morton codes differ, and at every level when the problem changes, up to its
+// problem's root (virtual level depth - 1).  With t_i the highest such level
+// (-1: none), the box of key i at level v is number #{j <= i: t_j >= v} - 1 of
+// that level, so all levels' boxes, parents, children and point ranges follow
+// from one counting pass (per block and level), a scan over the blocks and one
+// emitting pass.  The launches do not grow with the depth (12 per level
+// before), which is what small trees cost.
+// ---------------------------------------------------------------------------
+constexpr int kTreeThreads = 256;
+constexpr int kTreeWarps = kTreeThreads / 32;
+constexpr int kMaxLevels = 32;
+
+// Highest level at which key i's ancestor differs from key i-1's (63: another
+// problem, or the first key; -1: the same leaf).
+__device__ __forceinline__ int key_diff(const uint64_t* __restrict__ keys, int64_t i, int d) {
+  if (i == 0) return 63;
+  const uint64_t k = keys[i], kp = keys[i - 1];
+  if (key_pid(k) != key_pid(kp)) return 63;
+  const uint64_t x = (k ^ kp) & kMortonMask;
+  return x == 0 ? -1 : (63 - __clzll((long long)x)) / d;
+}
+
+// cnt[v * gridDim.x + block] = keys of the block's tile with t >= v (v < V);
+// row V: targets.
+__global__ void __launch_bounds__(kTreeThreads) k_tree_count(const uint64_t* __restrict__ keys,
+                                                             const int* __restrict__ idx, int64_t n, int64_t nt,
+                                                             int rounds, int d, const int* __restrict__ depth, int V,
+                                                             int* __restrict__ cnt) {
+  __shared__ int h[kMaxLevels + 1];
+  if (threadIdx.x <= kMaxLevels) h[threadIdx.x] = 0;
+  __syncthreads();
+  const int64_t base = (int64_t)blockIdx.x * rounds * kTreeThreads;
+  for (int r = 0; r < rounds; ++r) {
+    const int64_t i = base + (int64_t)r * kTreeThreads + threadIdx.x;
+    const int t = i < n ? min(key_diff(keys, i, d), depth[key_pid(keys[i])] - 1) : -1;
+    if (t >= 0) atomicAdd(&h[t], 1);
+    const unsigned m = __ballot_sync(0xffffffffu, i < n && idx[i] < nt);
+    if ((threadIdx.x & 31) == 0 && m) atomicAdd(&h[kMaxLevels], __popc(m));
   }
   __syncthreads();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = keys[i];
-    const int p = key_pid(k);
-    int diff = 63;  // highest level at which key i-1's ancestor differs
-    if (i > 0) {
-      const uint64_t kp = keys[i - 1];
-      if (key_pid(kp) == p) {
-        const uint64_t x = (k ^ kp) & kMortonMask;
-        diff = x == 0 ? -1 : (63 - __clzll((long long)x)) / d;
+  if (threadIdx.x < V) {
+    int s = 0;
+    for (int t = threadIdx.x; t < V; ++t) s += h[t];
+    cnt[(int64_t)threadIdx.x * gridDim.x + blockIdx.x] = s;
+  }
+  if (threadIdx.x == V) cnt[(int64_t)V * gridDim.x + blockIdx.x] = h[kMaxLevels];
+}
+
+// First box of each level in the arrays of all levels.
+struct LevelOff {
+  int64_t o[kMaxLevels + 1];
+};
+
+struct LevelArrays {
+  uint64_t* key;
+  int *tb, *te, *sb, *se, *cb, *ce, *parent;
+};
+
+// The boxes of every level and the point permutations.  off: the scanned
+// counts (exclusive over the blocks).  The key that opens a box writes its
+// key, begins and parent; the next key that leaves it (or the end) its ends.
+__global__ void __launch_bounds__(kTreeThreads) k_tree_emit(const uint64_t* __restrict__ keys,
+                                                            const int* __restrict__ idx, int64_t n, int64_t nt,
+                                                            int rounds, int d, const int* __restrict__ depth, int V,
+                                                            const int* __restrict__ off, const LevelOff lo,
+                                                            const LevelArrays L, int* __restrict__ perm_t,
+                                                            int* __restrict__ perm_s) {
+  __shared__ int s_run[kMaxLevels + 1];                      // boxes (row V: targets) before this round
+  __shared__ int s_pre[kTreeWarps][kMaxLevels + 1];          // ... of the round before this warp
+  __shared__ unsigned s_bal[kTreeWarps][kMaxLevels + 1];     // the warp's keys with t >= v
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  if (threadIdx.x <= V) s_run[threadIdx.x] = off[(int64_t)threadIdx.x * gridDim.x + blockIdx.x];
+  const int64_t base = (int64_t)blockIdx.x * rounds * kTreeThreads;
+  for (int r = 0; r < rounds; ++r) {
+    const int64_t i = base + (int64_t)r * kTreeThreads + threadIdx.x;
+    const bool ok = i < n;
+    const uint64_t k = ok ? keys[i] : 0;
+    const int id = ok ? idx[i] : 0;
+    const int diff = ok ? key_diff(keys, i, d) : -1;
+    const int dp = ok ? depth[key_pid(k)] - 1 : -1;
+    const int t = min(diff, dp);
+    for (int v = 0; v < V; ++v) {
+      const unsigned m = __ballot_sync(0xffffffffu, ok && t >= v);
+      if (lane == 0) s_bal[warp][v] = m;
+    }
+    const unsigned mt = __ballot_sync(0xffffffffu, ok && id < nt);
+    if (lane == 0) s_bal[warp][V] = mt;
+    __syncthreads();
+    if (threadIdx.x <= V) {
+      int a = s_run[threadIdx.x];
+      for (int w = 0; w < kTreeWarps; ++w) {
+        s_pre[w][threadIdx.x] = a;
+        a += __popc(s_bal[w][threadIdx.x]);
+      }
+      s_run[threadIdx.x] = a;
+    }
+    __syncthreads();
+    if (ok) {
+      auto before = [&](int v) { return s_pre[warp][v] + __popc(s_bal[warp][v] & lt); };  // exclusive
+      const int tpos = before(V), spos = (int)i - tpos;
+      if (id < nt) perm_t[tpos] = id;
+      else perm_s[spos] = id - (int)nt;
+      if (i > 0 && diff >= 0) {  // the boxes of key i-1 that end here
+        const int top = min(diff, depth[key_pid(keys[i - 1])] - 1);
+        for (int v = 0; v <= top; ++v) {
+          const int64_t b = lo.o[v] + before(v) - 1;
+          L.te[b] = tpos;
+          L.se[b] = spos;
+          L.ce[b] = v > 0 ? before(v - 1) : 0;
+        }
+      }
+      for (int v = 0; v <= t; ++v) {
+        const int64_t b = lo.o[v] + before(v);
+        L.key[b] = (k & ~kMortonMask) | ((k & kMortonMask) >> (d * v));
+        L.tb[b] = tpos;
+        L.sb[b] = spos;
+        L.cb[b] = v > 0 ? before(v - 1) : 0;
+        // the enclosing box one level up: opened here (v < t) or before
+        L.parent[b] = v < dp ? before(v + 1) - (v < t ? 0 : 1) : -1;
+      }
+      if (i == n - 1) {  // the last boxes
+        const int e = id < nt ? 1 : 0;
+        for (int v = 0; v <= dp; ++v) {
+          const int64_t b = lo.o[v] + before(v) - (t >= v ? 0 : 1);
+          L.te[b] = tpos + e;
+          L.se[b] = spos + 1 - e;
+          L.ce[b] = v > 0 ? before(v - 1) + (t >= v - 1 ? 1 : 0) : 0;
+        }
       }
     }
-    const int ta = min(diff, depth[p] - 1 - cut_a);
-    if (ta >= 0) atomicAdd(&ha[ta], 1);
-    if (hist_b) {
-      const int tb = min(diff, depth[p] - 1 - cut_b);
-      if (tb >= 0) atomicAdd(&hb[tb], 1);
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < nlev) {
-    if (ha[threadIdx.x]) atomicAdd(&hist_a[threadIdx.x], ha[threadIdx.x]);
-    if (hist_b && hb[threadIdx.x]) atomicAdd(&hist_b[threadIdx.x], hb[threadIdx.x]);
+    __syncthreads();  // s_bal and s_pre are rewritten
   }
 }
 
-// Keys of the targets in key order (position = exclusive target count).
-__global__ void k_target_keys(const uint64_t* __restrict__ keys, const int* __restrict__ idx, int64_t n,
-                              int64_t nt, const int* __restrict__ tex, uint64_t* __restrict__ tkey) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    if (idx[i] < nt) tkey[tex[i]] = keys[i];
-}
-
-// Parents of virtual level v.  pcap is the parent level's size, counted
-// beforehand by k_level_counts; a parent index past it (which the counts rule
-// out) raises *err instead of writing.
-__global__ void k_parent_emit(const uint64_t* __restrict__ ckey, const int* __restrict__ ctb,
-                              const int* __restrict__ cte, const int* __restrict__ csb,
-                              const int* __restrict__ cse, int64_t nc, int d, int v,
-                              const int* __restrict__ depth, const int* __restrict__ f,
-                              const int* __restrict__ fex, int* __restrict__ cparent, uint64_t* __restrict__ pkey,
-                              int* __restrict__ ptb, int* __restrict__ pte, int* __restrict__ psb,
-                              int* __restrict__ pse, int* __restrict__ pcb, int* __restrict__ pce,
-                              int64_t pcap, int* __restrict__ err) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nc;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = ckey[i];
-    if (real_level(k, depth, v) < 1) {
-      cparent[i] = -1;
-      continue;
-    }
-    const int p = fex[i] + f[i] - 1;
-    if (p < 0 || p >= pcap) {
-      cparent[i] = -1;
-      atomicExch(err, 1);
-      continue;
-    }
-    cparent[i] = p;
-    if (f[i]) {
-      pkey[p] = parent_key(k, d);
-      ptb[p] = ctb[i];
-      psb[p] = csb[i];
-      pcb[p] = (int)i;
-    }
-    const bool last = i == nc - 1 || f[i + 1] || real_level(ckey[i + 1], depth, v) < 1;
-    if (last) {
-      pte[p] = cte[i];
-      pse[p] = cse[i];
-      pce[p] = (int)i + 1;
-    }
-  }
-}
-
-// M2L rows: boxes with targets at real level >= 2, sort key (problem, class)
-__global__ void k_row_flags(const uint64_t* __restrict__ key, const int* __restrict__ tb, const int* __restrict__ te,
-                            int64_t nb, int v, int min_level, const int* __restrict__ depth, int* __restrict__ f) {
-  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
-       b += (int64_t)gridDim.x * blockDim.x)
-    f[b] = (te[b] > tb[b] && real_level(key[b], depth, v) >= min_level) ? 1 : 0;
-}
-
-__global__ void k_row_compact(const uint64_t* __restrict__ key, const int* __restrict__ f,
-                              const int* __restrict__ fex, int64_t nb, int d,
-                              uint64_t* __restrict__ ck, int* __restrict__ cv) {
+// Sort keys of the rows of every level in one array: M2L rows of level v
+// (boxes with targets at real level >= 2) by (v, problem, class), then the
+// near-field rows (leaves with targets) as level V; boxes of neither kind last.
+// Entry i < total is box i - lo.o[v] of its level v, entry total + b leaf b.
+__global__ void k_row_keys(const uint64_t* __restrict__ key, const int* __restrict__ tb, const int* __restrict__ te,
+                           const LevelOff lo, int V, int64_t total, int64_t nleaf, int d, int np,
+                           const int* __restrict__ depth, uint64_t* __restrict__ ck, int* __restrict__ cv) {
   const uint64_t mask = (1ull << d) - 1ull;
-  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
-       b += (int64_t)gridDim.x * blockDim.x) {
-    if (f[b]) {
-      int r = fex[b];
-      if (ck) ck[r] = ((uint64_t)key_pid(key[b]) << d) | (key[b] & mask);
-      cv[r] = (int)b;
+  const uint64_t none = (uint64_t)(V * (int64_t)np + 1) << d;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total + nleaf;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    if (i >= total) {
+      const int64_t b = i - total;
+      ck[i] = te[b] > tb[b] ? (uint64_t)V * np << d : none;
+      cv[i] = (int)b;
+      continue;
     }
+    int v = 0;
+    while (i >= lo.o[v + 1]) ++v;
+    const uint64_t k = key[i];
+    const int p = key_pid(k);
+    const bool row = te[i] > tb[i] && depth[p] - 1 - v >= 2;
+    ck[i] = row ? (((uint64_t)v * np + p) << d) | (k & mask) : none;
+    cv[i] = (int)(i - lo.o[v]);
   }
 }
 
-__global__ void k_seg_flags(const uint64_t* __restrict__ ck, int64_t n, int* __restrict__ f) {
+// begin[key] = first entry of the sorted row keys with that key (-1: none).
+__global__ void k_row_segs(const uint64_t* __restrict__ ck, int64_t n, int* __restrict__ begin) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    f[i] = (i == 0 || ck[i] != ck[i - 1]) ? 1 : 0;
+    if (i == 0 || ck[i] != ck[i - 1]) begin[ck[i]] = (int)i;
 }
 
-// Segment table of one level at its slot of the table of all levels; cap is
-// the slot's size (an upper bound of the level's segments; never exceeded).
-__global__ void k_seg_emit(const uint64_t* __restrict__ ck, const int* __restrict__ f, const int* __restrict__ fex,
-                           int64_t n, int cap, int* __restrict__ seg_key, int* __restrict__ seg_begin) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    if (f[i] && fex[i] < cap) {
-      seg_key[fex[i]] = (int)ck[i];
-      seg_begin[fex[i]] = (int)i;
-    }
-}
+// First row of each level in the sorted rows.
+struct RowOff {
+  int64_t o[kMaxLevels + 1];
+};
 
-__global__ void k_pairs_p2p(const int* __restrict__ near, int64_t nrow, int nnear,
-                            const int* __restrict__ row_box, const int* __restrict__ tb,
-                            const int* __restrict__ te, const int* __restrict__ sb,
-                            const int* __restrict__ se, unsigned long long* __restrict__ pairs) {
-  unsigned long long mine = 0;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrow;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    int b = row_box[r];
-    long long nsrc = 0;
-    for (int q = 0; q < nnear; ++q) {
-      int s = near[r * nnear + q];
-      if (s >= 0) nsrc += se[s] - sb[s];
-    }
-    mine += (unsigned long long)nsrc * (unsigned long long)(te[b] - tb[b]);
+// row_of[box of any level] = its row within the level (pre-filled with -1).
+__global__ void k_rows_of_boxes(const int* __restrict__ row_box, const RowOff ro, const LevelOff lo, int V,
+                                int* __restrict__ row_of) {
+  const int64_t n = ro.o[V];
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    int v = 0;
+    while (i >= ro.o[v + 1]) ++v;
+    row_of[lo.o[v] + row_box[i]] = (int)(i - ro.o[v]);
   }
-  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(pairs, mine);
 }
 
 // ---------------------------------------------------------------------------
@@ -441,11 +416,14 @@ static void forest_cubes(fmma_ctx* ctx, int d, const std::vector<int64_t>& toff,
                          const char* cube_buf = "cube") {
   const int np = (int)toff.size() - 1;
   const int64_t nt = toff[(size_t)np], ns = soff[(size_t)np];
-  int64_t* dto = ctx_buf_t<int64_t>(ctx, "forest_toff", (size_t)np + 1);
-  int64_t* dso = ctx_buf_t<int64_t>(ctx, "forest_soff", (size_t)np + 1);
-  upload(ctx, dto, toff.data(), sizeof(int64_t) * (size_t)(np + 1));
-  upload(ctx, dso, soff.data(), sizeof(int64_t) * (size_t)(np + 1));
-  FMMA_LAUNCH(ctx, k_point_pid, grid_for(nt + ns, 256, (int64_t)ctx->sm_count * 16), 256, 0, dto, dso, np, nt, ns, pid);
+  if (pid) {
+    int64_t* dto = ctx_buf_t<int64_t>(ctx, "forest_toff", (size_t)np + 1);
+    int64_t* dso = ctx_buf_t<int64_t>(ctx, "forest_soff", (size_t)np + 1);
+    upload(ctx, dto, toff.data(), sizeof(int64_t) * (size_t)(np + 1));
+    upload(ctx, dso, soff.data(), sizeof(int64_t) * (size_t)(np + 1));
+    FMMA_LAUNCH(ctx, k_point_pid, grid_for(nt + ns, 256, (int64_t)ctx->sm_count * 16), 256, 0, dto, dso, np, nt, ns,
+                pid);
+  }
   unsigned long long* mm = ctx_buf_t<unsigned long long>(ctx, "bbox_mm", (size_t)np * 2 * kMaxDim);
   int* flag = ctx_buf_t<int>(ctx, "bbox_flag", 1);
   FMMA_LAUNCH(ctx, k_bbox_init, grid_for((int64_t)np * kMaxDim, 256), 256, 0, mm, np, flag);
@@ -459,21 +437,6 @@ static void forest_cubes(fmma_ctx* ctx, int d, const std::vector<int64_t>& toff,
   FMMA_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
   std::memcpy(tr.h_cube.data(), hp, sizeof(Cube) * (size_t)np);
   if (tr.h_cube[0].nonfinite) throw Error(FMMA_ERR_INVALID_ARG, "a coordinate is NaN or Inf");
-}
-
-static void alloc_level(fmma_ctx* ctx, Level& L, int v, int64_t nb) {
-  std::string s = "lev" + std::to_string(v) + "_";
-  L.v = v;
-  L.nbox = nb;
-  const size_t n = (size_t)(nb > 0 ? nb : 1);
-  L.key = ctx_buf_t<uint64_t>(ctx, s + "key", n);
-  L.tb = ctx_buf_t<int>(ctx, s + "tb", n);
-  L.te = ctx_buf_t<int>(ctx, s + "te", n);
-  L.sb = ctx_buf_t<int>(ctx, s + "sb", n);
-  L.se = ctx_buf_t<int>(ctx, s + "se", n);
-  L.cb = ctx_buf_t<int>(ctx, s + "cb", n);
-  L.ce = ctx_buf_t<int>(ctx, s + "ce", n);
-  L.parent = ctx_buf_t<int>(ctx, s + "parent", n);
 }
 
 // Leaf keys, sorted; leaves; all virtual levels (no lists).
@@ -505,72 +468,63 @@ static void forest_levels(fmma_ctx* ctx, int d, const std::vector<int64_t>& toff
   const int blk = 256;
   const unsigned g = grid_for(n, blk, (int64_t)ctx->sm_count * 16);
 
-  int* pid = ctx_buf_t<int>(ctx, "pt_pid", (size_t)(n > 0 ? n : 1));
+  int* pid = np > 1 ? ctx_buf_t<int>(ctx, "pt_pid", (size_t)(n > 0 ? n : 1)) : nullptr;
   forest_cubes<T>(ctx, d, toff, tgt, soff, src, tr, pid);
 
   uint64_t* keys = ctx_buf_t<uint64_t>(ctx, "pt_keys", (size_t)n);
   int* idx = ctx_buf_t<int>(ctx, "pt_idx", (size_t)n);
+  uint64_t* keys2 = ctx_buf_t<uint64_t>(ctx, "pt_keys2", (size_t)n);
+  int* idx2 = ctx_buf_t<int>(ctx, "pt_idx2", (size_t)n);
   FMMA_LAUNCH(ctx, (k_leaf_keys<T>), g, blk, 0, tgt, nt, src, ns, pid, d, tr.d_depth, tr.d_cube, keys, idx);
-  radix_sort_pairs(ctx, keys, idx, n, 0, d * (tr.vmax - 1));
-  if (np > 1) radix_sort_pairs(ctx, keys, idx, n, kPidShift, kPidShift + bits_for(np));
+  radix_sort_swap(ctx, &keys, &idx, &keys2, &idx2, n, 0, d * (tr.vmax - 1));
+  if (np > 1) radix_sort_swap(ctx, &keys, &idx, &keys2, &idx2, n, kPidShift, kPidShift + bits_for(np));
 
-  int* fbox = ctx_buf_t<int>(ctx, "pt_fbox", (size_t)n);
-  int* ft = ctx_buf_t<int>(ctx, "pt_ft", (size_t)n);
-  int* boxex = ctx_buf_t<int>(ctx, "pt_boxex", (size_t)n);
-  int* tex = ctx_buf_t<int>(ctx, "pt_tex", (size_t)n);
-  int* tot = ctx_buf_t<int>(ctx, "tree_tot", 4);
-  FMMA_LAUNCH(ctx, k_leaf_flags, g, blk, 0, keys, idx, n, nt, fbox, ft);
-  scan_exclusive(ctx, fbox, boxex, n, tot);
-  scan_exclusive(ctx, ft, tex, n, tot + 1);
-  // Sizes of every level and of the row sets of the lists, counted from the
-  // sorted keys and read back in one wait: [0, V) boxes, [V, 2V) boxes with
-  // targets, [2V, 3V) M2L rows (boxes with targets at real level >= 2), then
-  // the leaf count of the scan as a check.
+  // Boxes of every level, counted per block of keys, scanned and read back in
+  // one wait (row V: the targets).
   const int V = tr.vmax;
-  FMMA_REQUIRE(V <= 32, "Depth out of range");
-  int* lvc = ctx_buf_t<int>(ctx, "tree_lvc", (size_t)3 * V + 1);
-  FMMA_CHECK_CUDA(cudaMemsetAsync(lvc, 0, sizeof(int) * (size_t)3 * V, ctx->stream));
-  FMMA_LAUNCH(ctx, k_level_counts, g, blk, 0, keys, n, d, tr.d_depth, V, 0, lvc, 0, (int*)nullptr);
-  uint64_t* tkey = ctx_buf_t<uint64_t>(ctx, "pt_tkey", (size_t)(nt > 0 ? nt : 1));
-  FMMA_LAUNCH(ctx, k_target_keys, g, blk, 0, keys, idx, n, nt, tex, tkey);
-  FMMA_LAUNCH(ctx, k_level_counts, grid_for(nt, blk, (int64_t)ctx->sm_count * 16), blk, 0, tkey, nt, d, tr.d_depth,
-              V, 0, lvc + V, 2, lvc + 2 * V);
-  FMMA_CHECK_CUDA(cudaMemcpyAsync(lvc + 3 * V, tot, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
-  std::vector<int> hl((size_t)3 * V + 1, 0);
-  read_ints(ctx, lvc, hl.data(), 3 * V + 1);
-  for (int c = 0; c < 3; ++c)  // histogram of highest new level -> boxes per level
-    for (int v = V - 2; v >= 0; --v) hl[(size_t)(c * V + v)] += hl[(size_t)(c * V + v + 1)];
-  const int64_t nleaf = hl[(size_t)3 * V];
-  if (hl[0] != nleaf) throw Error(FMMA_ERR_CUDA, "tree build: level counts disagree with the leaf scan");
-  tr.near_count = hl[(size_t)V];
-  tr.row_count.assign(hl.begin() + 2 * V, hl.begin() + 3 * V);
-  tr.d_err = ctx_buf_t<int>(ctx, "tree_err", 1);
-  FMMA_CHECK_CUDA(cudaMemsetAsync(tr.d_err, 0, sizeof(int), ctx->stream));
+  FMMA_REQUIRE(V < kMaxLevels, "Depth out of range");
+  // keys per block: enough blocks for small trees, fewer counts for large ones
+  const int rounds = (int)std::max<int64_t>(1, std::min<int64_t>(8, n / ((int64_t)kTreeThreads * ctx->sm_count * 4)));
+  const int64_t tile = (int64_t)rounds * kTreeThreads;
+  const int64_t nblk = std::max<int64_t>(1, (n + tile - 1) / tile);
+  int* cnt = ctx_buf_t<int>(ctx, "tree_cnt", (size_t)(V + 1) * nblk);
+  int* off = ctx_buf_t<int>(ctx, "tree_off", (size_t)(V + 1) * nblk);
+  int* tot = ctx_buf_t<int>(ctx, "tree_tot", (size_t)V + 1);
+  FMMA_LAUNCH(ctx, k_tree_count, (unsigned)nblk, kTreeThreads, 0, keys, idx, n, nt, rounds, d, tr.d_depth, V, cnt);
+  scan_rows(ctx, cnt, off, nblk, V + 1, tot);
+  std::vector<int> hl((size_t)V + 1, 0);
+  read_ints(ctx, tot, hl.data(), V + 1);
 
   tr.perm_t = ctx_buf_t<int>(ctx, "perm_t", (size_t)(nt > 0 ? nt : 1));
   tr.perm_s = ctx_buf_t<int>(ctx, "perm_s", (size_t)(ns > 0 ? ns : 1));
-  Level& leaf = tr.lev[0];
-  alloc_level(ctx, leaf, 0, nleaf);
-  FMMA_LAUNCH(ctx, k_leaf_emit, g, blk, 0, keys, idx, n, nt, fbox, boxex, tex, tr.perm_t, tr.perm_s, leaf.key,
-              leaf.tb, leaf.sb);
-  FMMA_LAUNCH(ctx, k_leaf_ends, grid_for(nleaf, blk), blk, 0, nleaf, leaf.tb, leaf.sb, (int)nt, (int)ns, leaf.te,
-              leaf.se);
-  FMMA_CHECK_CUDA(cudaMemsetAsync(leaf.cb, 0, sizeof(int) * (size_t)nleaf, ctx->stream));
-  FMMA_CHECK_CUDA(cudaMemsetAsync(leaf.ce, 0, sizeof(int) * (size_t)nleaf, ctx->stream));
-
-  for (int v = 0; v + 1 < tr.vmax; ++v) {
-    Level& C = tr.lev[(size_t)v];
-    int* f = ctx_buf_t<int>(ctx, "lv_f", (size_t)C.nbox + 1);
-    int* fex = ctx_buf_t<int>(ctx, "lv_fex", (size_t)C.nbox + 1);
-    FMMA_LAUNCH(ctx, k_parent_flags, grid_for(C.nbox, blk), blk, 0, C.key, C.nbox, d, v, tr.d_depth, f);
-    scan_exclusive(ctx, f, fex, C.nbox, tot);
-    Level& Pl = tr.lev[(size_t)(v + 1)];
-    alloc_level(ctx, Pl, v + 1, hl[(size_t)(v + 1)]);
-    FMMA_LAUNCH(ctx, k_parent_emit, grid_for(C.nbox, blk), blk, 0, C.key, C.tb, C.te, C.sb, C.se, C.nbox, d, v,
-                tr.d_depth, f, fex, C.parent, Pl.key, Pl.tb, Pl.te, Pl.sb, Pl.se, Pl.cb, Pl.ce, Pl.nbox, tr.d_err);
+  LevelOff lo{};
+  for (int v = 0; v < V; ++v) lo.o[v + 1] = lo.o[v] + hl[(size_t)v];
+  const size_t total = (size_t)std::max<int64_t>(1, lo.o[V]);
+  LevelArrays L;
+  L.key = ctx_buf_t<uint64_t>(ctx, "lev_key", total);
+  L.tb = ctx_buf_t<int>(ctx, "lev_tb", total);
+  L.te = ctx_buf_t<int>(ctx, "lev_te", total);
+  L.sb = ctx_buf_t<int>(ctx, "lev_sb", total);
+  L.se = ctx_buf_t<int>(ctx, "lev_se", total);
+  L.cb = ctx_buf_t<int>(ctx, "lev_cb", total);
+  L.ce = ctx_buf_t<int>(ctx, "lev_ce", total);
+  L.parent = ctx_buf_t<int>(ctx, "lev_parent", total);
+  for (int v = 0; v < V; ++v) {
+    Level& Lv = tr.lev[(size_t)v];
+    const int64_t o = lo.o[v];
+    Lv.v = v;
+    Lv.nbox = hl[(size_t)v];
+    Lv.key = L.key + o;
+    Lv.tb = L.tb + o;
+    Lv.te = L.te + o;
+    Lv.sb = L.sb + o;
+    Lv.se = L.se + o;
+    Lv.cb = L.cb + o;
+    Lv.ce = L.ce + o;
+    Lv.parent = L.parent + o;
   }
-  Level& top = tr.lev[(size_t)(tr.vmax - 1)];
-  FMMA_CHECK_CUDA(cudaMemsetAsync(top.parent, 0xff, sizeof(int) * (size_t)(top.nbox > 0 ? top.nbox : 1), ctx->stream));
+  FMMA_LAUNCH(ctx, k_tree_emit, (unsigned)nblk, kTreeThreads, 0, keys, idx, n, nt, rounds, d, tr.d_depth, V, off, lo,
+              L, tr.perm_t, tr.perm_s);
 }
 
 template <typename T>
@@ -586,13 +540,34 @@ void build_forest(fmma_ctx* ctx, int d, const std::vector<int64_t>& toff, const 
     upload(ctx, jslot, F.jslot, sizeof(int) * 8 * 216);
     unsigned long long* pairs = ctx_buf_t<unsigned long long>(ctx, "il_pairs", (size_t)tr.vmax + 2);
     FMMA_CHECK_CUDA(cudaMemsetAsync(pairs, 0, sizeof(unsigned long long) * (size_t)(tr.vmax + 2), ctx->stream));
-    const int pbits = bits_for(np);
     const int V = tr.vmax;
-    // The row counts come from the level counts; the host waits on the device
-    // once for the segment tables of all levels and once for the pair counts.
-    // cnt receives the row scans' totals (unused: the counts are known).
-    int* cnt = ctx_buf_t<int>(ctx, "tree_cnt", (size_t)V + 1);
-    std::vector<int*> fv((size_t)V, nullptr), fexv((size_t)V, nullptr);
+    LevelOff lo{};
+    for (int v = 0; v < V; ++v) lo.o[v + 1] = lo.o[v] + tr.lev[(size_t)v].nbox;
+    const int64_t total = lo.o[V], nleaf = tr.lev[0].nbox, nkey = total + nleaf;
+    const Level& first = tr.lev[0];  // the arrays of all levels start at the leaves
+    // Rows of all levels and the near-field rows in one sort; the table of
+    // segment begins by (level, problem, class) is read back in one wait.
+    const int64_t ntable = ((int64_t)V * np + 2) << d;
+    uint64_t* ck = ctx_buf_t<uint64_t>(ctx, "row_ck", (size_t)nkey);
+    int* cv = ctx_buf_t<int>(ctx, "row_cv", (size_t)nkey);
+    uint64_t* ck2 = ctx_buf_t<uint64_t>(ctx, "row_ck2", (size_t)nkey);
+    int* cv2 = ctx_buf_t<int>(ctx, "row_cv2", (size_t)nkey);
+    int* begin = ctx_buf_t<int>(ctx, "row_begin", (size_t)ntable);
+    FMMA_CHECK_CUDA(cudaMemsetAsync(begin, 0xff, sizeof(int) * (size_t)ntable, ctx->stream));
+    FMMA_LAUNCH(ctx, k_row_keys, grid_for(nkey, blk), blk, 0, first.key, first.tb, first.te, lo, V, total, nleaf, d, np,
+                tr.d_depth, ck, cv);
+    radix_sort_swap(ctx, &ck, &cv, &ck2, &cv2, nkey, 0, d + bits_for(V * np + 2));
+    FMMA_LAUNCH(ctx, k_row_segs, grid_for(nkey, blk), blk, 0, ck, nkey, begin);
+    std::vector<int> hb((size_t)ntable);
+    read_ints(ctx, begin, hb.data(), (int)ntable);
+    // segment ends: the next begin present, in key order
+    int64_t end = nkey;
+    std::vector<int64_t> ends((size_t)ntable);
+    for (int64_t k = ntable - 1; k >= 0; --k) {
+      ends[(size_t)k] = end;
+      if (hb[(size_t)k] >= 0) end = hb[(size_t)k];
+    }
+    RowOff ro{};
     for (int v = 0; v < V; ++v) {
       Level& Lv = tr.lev[(size_t)v];
       // operator tables: problems with a real level >= 2 at this virtual level
@@ -603,121 +578,94 @@ void build_forest(fmma_ctx* ctx, int d, const std::vector<int64_t>& toff, const 
           Lv.pid_table[(size_t)p] = (int)Lv.table_pid.size();
           Lv.table_pid.push_back(p);
         }
-      Lv.nrow = 0;
       Lv.segs.clear();
-      if (Lv.table_pid.empty()) continue;
-      fv[(size_t)v] = ctx_buf_t<int>(ctx, "lv_f" + std::to_string(v), (size_t)Lv.nbox + 1);
-      fexv[(size_t)v] = ctx_buf_t<int>(ctx, "lv_fex" + std::to_string(v), (size_t)Lv.nbox + 1);
-      FMMA_LAUNCH(ctx, k_row_flags, grid_for(Lv.nbox, blk), blk, 0, Lv.key, Lv.tb, Lv.te, Lv.nbox, v, 2, tr.d_depth,
-                  fv[(size_t)v]);
-      scan_exclusive(ctx, fv[(size_t)v], fexv[(size_t)v], Lv.nbox, cnt + v);
+      const int64_t r0 = ro.o[v];
+      int64_t r1 = r0;
+      for (int64_t k = ((int64_t)v * np) << d; k < ((int64_t)(v + 1) * np) << d; ++k) {
+        if (hb[(size_t)k] < 0) continue;
+        r1 = ends[(size_t)k];
+        Lv.segs.push_back(make_int4((int)(k >> d) - v * np, (int)(k & ((1 << d) - 1)), (int)(hb[(size_t)k] - r0),
+                                    (int)(r1 - r0)));
+      }
+      ro.o[v + 1] = r1;
+      Lv.nrow = r1 - r0;
     }
-    int* fnear = ctx_buf_t<int>(ctx, "near_f", (size_t)tr.lev[0].nbox + 1);
-    int* fexnear = ctx_buf_t<int>(ctx, "near_fex", (size_t)tr.lev[0].nbox + 1);
-    FMMA_LAUNCH(ctx, k_row_flags, grid_for(tr.lev[0].nbox, blk), blk, 0, tr.lev[0].key, tr.lev[0].tb, tr.lev[0].te,
-                tr.lev[0].nbox, 0, 0, tr.d_depth, fnear);
-    scan_exclusive(ctx, fnear, fexnear, tr.lev[0].nbox, cnt + V);
-    // rows per level and near rows were counted with the levels
-    std::vector<int> hc((size_t)2 * V + 2, 0);
-    for (int v = 0; v < V; ++v) hc[(size_t)v] = tr.lev[(size_t)v].table_pid.empty() ? 0 : tr.row_count[(size_t)v];
-    hc[(size_t)V] = (int)tr.near_count;
-    // Rows sorted by (problem, class) and each level's segment table, all read
-    // back in one wait: seg_all = [segments per level (V) | keys | begins],
-    // level v's table at sbo[v] with room for min(rows, problems x classes).
-    std::vector<int> sbo((size_t)V + 1, 0);
-    for (int v = 0; v < V; ++v)
-      sbo[(size_t)v + 1] = sbo[(size_t)v] + (int)std::min<int64_t>(hc[(size_t)v], (int64_t)np << d);
-    const int TB = sbo[(size_t)V];
-    int* seg_all = ctx_buf_t<int>(ctx, "seg_all", (size_t)V + 2 * (size_t)TB);
-    FMMA_CHECK_CUDA(cudaMemsetAsync(seg_all, 0, sizeof(int) * (size_t)V, ctx->stream));
-    std::vector<uint64_t*> ckv((size_t)V, nullptr);
-    std::vector<int*> sfv((size_t)V, nullptr), sfxv((size_t)V, nullptr);
-    for (int v = 0; v < V; ++v) {
-      Level& Lv = tr.lev[(size_t)v];
-      if (Lv.table_pid.empty()) continue;
-      const int nr = hc[(size_t)v];
-      Lv.nrow = nr;
-      std::string s = "lev" + std::to_string(v) + "_";
-      ckv[(size_t)v] = ctx_buf_t<uint64_t>(ctx, s + "row_ck", (size_t)(nr > 0 ? nr : 1));
-      Lv.row_box = ctx_buf_t<int>(ctx, s + "row_box", (size_t)(nr > 0 ? nr : 1));
-      Lv.il = ctx_buf_t<int>(ctx, s + "il", (size_t)nr * F.nfar + 1);
-      Lv.slot_mask = ctx_buf_t<unsigned>(ctx, s + "smask", (size_t)nr * kSlotWords + 1);
-      if (nr == 0) continue;
-      uint64_t* ck = ckv[(size_t)v];
-      FMMA_LAUNCH(ctx, k_row_compact, grid_for(Lv.nbox, blk), blk, 0, Lv.key, fv[(size_t)v], fexv[(size_t)v], Lv.nbox,
-                  d, ck, Lv.row_box);
-      radix_sort_pairs(ctx, ck, Lv.row_box, nr, 0, d + pbits);
-      sfv[(size_t)v] = ctx_buf_t<int>(ctx, s + "seg_f", (size_t)nr);
-      sfxv[(size_t)v] = ctx_buf_t<int>(ctx, s + "seg_fex", (size_t)nr);
-      FMMA_LAUNCH(ctx, k_seg_flags, grid_for(nr, blk), blk, 0, ck, (int64_t)nr, sfv[(size_t)v]);
-      scan_exclusive(ctx, sfv[(size_t)v], sfxv[(size_t)v], nr, seg_all + v);
-      const int cap = sbo[(size_t)v + 1] - sbo[(size_t)v];
-      FMMA_LAUNCH(ctx, k_seg_emit, grid_for(nr, blk), blk, 0, ck, sfv[(size_t)v], sfxv[(size_t)v], (int64_t)nr, cap,
-                  seg_all + V + sbo[(size_t)v], seg_all + V + TB + sbo[(size_t)v]);
-    }
-    std::vector<int> hseg((size_t)V + 2 * (size_t)TB);
-    read_ints(ctx, seg_all, hseg.data(), V + 2 * TB);
-    for (int v = 0; v < V; ++v) {
-      Level& Lv = tr.lev[(size_t)v];
-      const int nseg = hseg[(size_t)v];
-      if (nseg > sbo[(size_t)v + 1] - sbo[(size_t)v])
-        throw Error(FMMA_ERR_CUDA, "tree build: more row segments than (problem, class) pairs");
-      const int* sk = hseg.data() + V + sbo[(size_t)v];
-      const int* sb = hseg.data() + V + TB + sbo[(size_t)v];
-      for (int i = 0; i < nseg; ++i)
-        Lv.segs.push_back(make_int4(sk[i] >> d, sk[i] & ((1 << d) - 1), sb[i], i + 1 < nseg ? sb[i + 1] : (int)Lv.nrow));
-    }
+    const int64_t nrow = ro.o[V], knear = ((int64_t)V * np) << d;
+    tr.nnear_rows = hb[(size_t)knear] >= 0 ? ends[(size_t)knear] - hb[(size_t)knear] : 0;
+    tr.near_row_box = cv + nrow;
     // neighbour lists of every level top-down, far lists of the rows on the way
     const int nnb = d == 1 ? 3 : (d == 2 ? 9 : 27);
-    int64_t maxbox = 1;
-    for (const Level& L : tr.lev) maxbox = std::max<int64_t>(maxbox, L.nbox);
-    int* nbr[2] = {ctx_buf_t<int>(ctx, "nbr_even", (size_t)maxbox * nnb),
-                   ctx_buf_t<int>(ctx, "nbr_odd", (size_t)maxbox * nnb)};
-    int* row_of = ctx_buf_t<int>(ctx, "row_of_box", (size_t)maxbox);
-    for (int v = tr.vmax - 1; v >= 0; --v) {
-      const bool top = v + 1 >= tr.vmax;
-      launch_lists_topdown(ctx, tr.lev[(size_t)v], top ? nullptr : &tr.lev[(size_t)(v + 1)],
-                           top ? nullptr : nbr[(v + 1) & 1], d, F.nfar, jslot, nbr[v & 1], row_of, pairs + v);
+    int* nbr = ctx_buf_t<int>(ctx, "nbr", (size_t)total * nnb);
+    int* row_of = ctx_buf_t<int>(ctx, "row_of_box", (size_t)total);
+    int* il = ctx_buf_t<int>(ctx, "il", (size_t)nrow * F.nfar + 1);
+    unsigned* smask = ctx_buf_t<unsigned>(ctx, "slot_mask", (size_t)nrow * kSlotWords + 1);
+    FMMA_CHECK_CUDA(cudaMemsetAsync(nbr, 0xff, sizeof(int) * (size_t)total * nnb, ctx->stream));
+    if (nrow > 0) {
+      FMMA_CHECK_CUDA(cudaMemsetAsync(row_of, 0xff, sizeof(int) * (size_t)total, ctx->stream));
+      FMMA_CHECK_CUDA(cudaMemsetAsync(il, 0xff, sizeof(int) * (size_t)nrow * F.nfar, ctx->stream));
+      FMMA_CHECK_CUDA(cudaMemsetAsync(smask, 0, sizeof(unsigned) * (size_t)nrow * kSlotWords, ctx->stream));
+      FMMA_LAUNCH(ctx, k_rows_of_boxes, grid_for(nrow, blk), blk, 0, cv, ro, lo, V, row_of);
     }
+    ListLevels ll{};
+    for (int v = 0; v < V; ++v) {
+      Level& Lv = tr.lev[(size_t)v];
+      Lv.row_box = cv + ro.o[v];
+      Lv.il = il + ro.o[v] * F.nfar;
+      Lv.slot_mask = smask + ro.o[v] * kSlotWords;
+      ll.box0[v] = lo.o[v];
+      ll.row0[v] = ro.o[v];
+      ll.nbox[v] = Lv.nbox;
+      ll.rows[v] = Lv.nrow > 0;
+    }
+    ll.V = V;
+    ll.d = d;
+    ll.nfar = F.nfar;
+    ll.key = first.key;
+    ll.parent = first.parent;
+    ll.tb = first.tb;
+    ll.te = first.te;
+    ll.sb = first.sb;
+    ll.se = first.se;
+    ll.cb = first.cb;
+    ll.ce = first.ce;
+    ll.row_of = row_of;
+    ll.jslot = jslot;
+    ll.nbr = nbr;
+    ll.il = il;
+    ll.slot_mask = smask;
+    ll.pairs = pairs;
+    launch_lists_topdown(ctx, ll);
     // near lists at the leaves (rows = leaves with targets, key order)
-    {
-      Level& Lv = tr.lev[0];
-      const int nr = hc[(size_t)V];
-      tr.nnear_rows = nr;
-      const int nnear = d == 1 ? 3 : (d == 2 ? 9 : 27);
-      tr.near_row_box = ctx_buf_t<int>(ctx, "near_row_box", (size_t)(nr > 0 ? nr : 1));
-      tr.near = ctx_buf_t<int>(ctx, "near", (size_t)nr * nnear + 1);
-      if (nr > 0) {
-        FMMA_LAUNCH(ctx, k_row_compact, grid_for(Lv.nbox, blk), blk, 0, Lv.key, fnear, fexnear, Lv.nbox, d,
-                    (uint64_t*)nullptr, tr.near_row_box);
-        launch_near_rows(ctx, nbr[0], tr.near_row_box, (int64_t)nr, d, Lv.sb, Lv.se, tr.near);
-        FMMA_LAUNCH(ctx, k_pairs_p2p, grid_for(nr, blk), blk, 0, tr.near, (int64_t)nr, nnear, tr.near_row_box, Lv.tb,
-                    Lv.te, Lv.sb, Lv.se, pairs + tr.vmax);
-      }
-    }
+    tr.near = ctx_buf_t<int>(ctx, "near", (size_t)tr.nnear_rows * nnb + 1);
+    launch_near_rows(ctx, nbr, tr.near_row_box, tr.nnear_rows, d, first.tb, first.te, first.sb, first.se, tr.near,
+                     pairs + V);
     tr.d_pairs = pairs;  // read when needed (tree_read_pairs)
     tr.pairs_read = false;
   }
   tr.valid = true;
 }
 
-void tree_read_pairs(fmma_ctx* ctx) {
+bool tree_fetch_pairs(fmma_ctx* ctx, void* pinned) {
+  const Tree& tr = ctx->tree;
+  if (tr.pairs_read || !tr.d_pairs) return false;
+  FMMA_CHECK_CUDA(cudaMemcpyAsync(pinned, tr.d_pairs, sizeof(unsigned long long) * (size_t)(tr.vmax + 1),
+                                  cudaMemcpyDeviceToHost, ctx->stream));
+  return true;
+}
+
+void tree_take_pairs(fmma_ctx* ctx, const void* pinned) {
   Tree& tr = ctx->tree;
-  if (tr.pairs_read || !tr.d_pairs) return;
-  std::vector<unsigned long long> hp((size_t)tr.vmax + 1);
-  unsigned long long* pp =
-      static_cast<unsigned long long*>(ctx_pinned(ctx, sizeof(unsigned long long) * (hp.size() + 1)));
-  FMMA_CHECK_CUDA(cudaMemcpyAsync(pp, tr.d_pairs, sizeof(unsigned long long) * hp.size(), cudaMemcpyDeviceToHost,
-                                  ctx->stream));
-  FMMA_CHECK_CUDA(cudaMemcpyAsync(pp + hp.size(), tr.d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  FMMA_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
-  std::memcpy(hp.data(), pp, sizeof(unsigned long long) * hp.size());
-  int herr = 0;
-  std::memcpy(&herr, pp + hp.size(), sizeof(int));
+  const unsigned long long* hp = static_cast<const unsigned long long*>(pinned);
   tr.pairs_read = true;
-  if (herr) throw Error(FMMA_ERR_CUDA, "tree build: a level holds more boxes than counted");
-  for (int v = 0; v < tr.vmax; ++v) tr.lev[(size_t)v].il_pairs = (int64_t)hp[(size_t)v];
-  tr.p2p_pairs = (int64_t)hp[(size_t)tr.vmax];
+  for (int v = 0; v < tr.vmax; ++v) tr.lev[(size_t)v].il_pairs = (int64_t)hp[v];
+  tr.p2p_pairs = (int64_t)hp[tr.vmax];
+}
+
+void tree_read_pairs(fmma_ctx* ctx) {
+  void* pp = ctx_pinned(ctx, 512);
+  if (!tree_fetch_pairs(ctx, pp)) return;
+  FMMA_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
+  tree_take_pairs(ctx, pp);
 }
 
 template void build_forest<double>(fmma_ctx*, int, const std::vector<int64_t>&, const double*,
@@ -792,7 +740,7 @@ void export_bins(fmma_ctx* ctx, int d, int depth, int64_t nt, const T* tgt, int6
                  int64_t* tbox, int64_t* sbox, Cube* cube_out) {
   Tree tmp;
   const int64_t n = nt + ns;
-  int* pid = ctx_buf_t<int>(ctx, "pt_pid", (size_t)(n > 0 ? n : 1));
+  int* pid = nullptr;
   forest_cubes<T>(ctx, d, {0, nt}, tgt, {0, ns}, src, tmp, pid);
   *cube_out = tmp.h_cube[0];
   int* dd = ctx_buf_t<int>(ctx, "export_depth", 1);
@@ -809,9 +757,7 @@ template <typename T>
 const Cube* problem_cube(fmma_ctx* ctx, int d, int64_t nt, const T* tgt, int64_t ns, const T* src,
                          const char* cube_buf, Cube* host) {
   Tree tmp;
-  const int64_t n = nt + ns;
-  int* pid = ctx_buf_t<int>(ctx, "pt_pid", (size_t)(n > 0 ? n : 1));
-  forest_cubes<T>(ctx, d, {0, nt}, tgt, {0, ns}, src, tmp, pid, cube_buf);
+  forest_cubes<T>(ctx, d, {0, nt}, tgt, {0, ns}, src, tmp, nullptr, cube_buf);
   *host = tmp.h_cube[0];
   return tmp.d_cube;
 }
