@@ -22,6 +22,8 @@
 // compensation at ~1 extra operation per term and right-hand side.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "fmm_stages.cuh"
 #include "fmma_internal.cuh"
 #include "kernels.cuh"
@@ -36,10 +38,54 @@ __device__ __forceinline__ void box_center(uint64_t key, int d, int bits, const 
 }
 
 // Double-float local coordinates of sorted points relative to their leaf
-// centre: xl[q][j] = hi, xl[d + q][j] = lo with hi + lo = x - centre.
+// centre, x - centre = hi + lo, as one record per point that a thread reads or
+// copies in 16-byte pieces: {h0 h1 h2 0 | l0 l1 l2 0} in three dimensions,
+// {h0 h1 l0 l1} in two, {h l} in one.
+template <int D>
+struct LocalRec {
+  static constexpr int N = D == 1 ? 2 : (D == 2 ? 4 : 8);  // floats
+  static constexpr int LO = D == 3 ? 4 : D;                // first lo
+};
+
+template <int D>
+__device__ __forceinline__ void store_local(float* rec, const double* v) {
+  float h[D], l[D];
+#pragma unroll
+  for (int q = 0; q < D; ++q) {
+    h[q] = (float)v[q];
+    l[q] = (float)(v[q] - (double)h[q]);
+  }
+  if constexpr (D == 3) {
+    reinterpret_cast<float4*>(rec)[0] = make_float4(h[0], h[1], h[2], 0.f);
+    reinterpret_cast<float4*>(rec)[1] = make_float4(l[0], l[1], l[2], 0.f);
+  } else if constexpr (D == 2) {
+    reinterpret_cast<float4*>(rec)[0] = make_float4(h[0], h[1], l[0], l[1]);
+  } else {
+    reinterpret_cast<float2*>(rec)[0] = make_float2(h[0], l[0]);
+  }
+}
+
+template <int D>
+__device__ __forceinline__ void load_local(const float* rec, float* h, float* l) {
+  if constexpr (D == 3) {
+    const float4 a = reinterpret_cast<const float4*>(rec)[0], b = reinterpret_cast<const float4*>(rec)[1];
+    h[0] = a.x; h[1] = a.y; h[2] = a.z;
+    l[0] = b.x; l[1] = b.y; l[2] = b.z;
+  } else if constexpr (D == 2) {
+    const float4 a = reinterpret_cast<const float4*>(rec)[0];
+    h[0] = a.x; h[1] = a.y;
+    l[0] = a.z; l[1] = a.w;
+  } else {
+    const float2 a = reinterpret_cast<const float2*>(rec)[0];
+    h[0] = a.x;
+    l[0] = a.y;
+  }
+}
+
+template <int D>
 __global__ void k_local_coords(const uint64_t* __restrict__ key, const int* __restrict__ b0,
                                const int* __restrict__ b1, int64_t nbox, const double* __restrict__ x, int64_t n,
-                               int d, const int* __restrict__ depth, const Cube* __restrict__ cubes,
+                               const int* __restrict__ depth, const Cube* __restrict__ cubes,
                                float* __restrict__ xl) {
   for (int64_t b = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; b < nbox; b += (int64_t)gridDim.x * blockDim.y) {
     const int pid = key_pid(key[b]);
@@ -47,23 +93,23 @@ __global__ void k_local_coords(const uint64_t* __restrict__ key, const int* __re
     const int bits = depth[pid] - 1;
     const double len = c.Len / (double)(1 << bits);
     double ctr[kMaxDim];
-    box_center(key[b] & kMortonMask, d, bits, c, len, ctr);
-    for (int j = b0[b] + threadIdx.x; j < b1[b]; j += blockDim.x)
-      for (int q = 0; q < d; ++q) {
-        const double v = x[(int64_t)q * n + j] - ctr[q];
-        const float hi = (float)v;
-        xl[(int64_t)q * n + j] = hi;
-        xl[(int64_t)(d + q) * n + j] = (float)(v - (double)hi);
-      }
+    box_center(key[b] & kMortonMask, D, bits, c, len, ctr);
+    for (int j = b0[b] + threadIdx.x; j < b1[b]; j += blockDim.x) {
+      double v[D];
+#pragma unroll
+      for (int q = 0; q < D; ++q) v[q] = x[(int64_t)q * n + j] - ctr[q];
+      store_local<D>(xl + (int64_t)j * LocalRec<D>::N, v);
+    }
   }
 }
 
 // The same with one thread per leaf, for leaves holding a few points (the
 // warp-per-leaf form above leaves most lanes idle there): consecutive
 // threads take consecutive leaves, whose points are consecutive in memory.
+template <int D>
 __global__ void k_local_coords_tpl(const uint64_t* __restrict__ key, const int* __restrict__ b0,
                                    const int* __restrict__ b1, int64_t nbox, const double* __restrict__ x, int64_t n,
-                                   int d, const int* __restrict__ depth, const Cube* __restrict__ cubes,
+                                   const int* __restrict__ depth, const Cube* __restrict__ cubes,
                                    float* __restrict__ xl) {
   for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nbox; b += (int64_t)gridDim.x * blockDim.x) {
     const int j0 = b0[b], j1 = b1[b];
@@ -73,14 +119,13 @@ __global__ void k_local_coords_tpl(const uint64_t* __restrict__ key, const int* 
     const int bits = depth[pid] - 1;
     const double len = c.Len / (double)(1 << bits);
     double ctr[kMaxDim];
-    box_center(key[b] & kMortonMask, d, bits, c, len, ctr);
-    for (int j = j0; j < j1; ++j)
-      for (int q = 0; q < d; ++q) {
-        const double v = x[(int64_t)q * n + j] - ctr[q];
-        const float hi = (float)v;
-        xl[(int64_t)q * n + j] = hi;
-        xl[(int64_t)(d + q) * n + j] = (float)(v - (double)hi);
-      }
+    box_center(key[b] & kMortonMask, D, bits, c, len, ctr);
+    for (int j = j0; j < j1; ++j) {
+      double v[D];
+#pragma unroll
+      for (int q = 0; q < D; ++q) v[q] = x[(int64_t)q * n + j] - ctr[q];
+      store_local<D>(xl + (int64_t)j * LocalRec<D>::N, v);
+    }
   }
 }
 
@@ -89,7 +134,7 @@ __global__ void k_local_coords_tpl(const uint64_t* __restrict__ key, const int* 
 // coordinates.
 __host__ __device__ constexpr int p2p_chunk(int RB) { return RB >= 16 ? 32 : 64; }
 __host__ __device__ constexpr size_t p2p_stage_bytes(int D, int RB) {
-  return sizeof(float) * p2p_chunk(RB) * RB + sizeof(float) * 2 * D * p2p_chunk(RB);
+  return sizeof(float) * p2p_chunk(RB) * RB + sizeof(float) * (D == 1 ? 2 : (D == 2 ? 4 : 8)) * p2p_chunk(RB);
 }
 __host__ __device__ constexpr size_t p2p_warp_bytes(int D, int RB) {
   return (RB >= 8 ? sizeof(double) * RB * 32 : 0) + 2 * p2p_stage_bytes(D, RB);
@@ -119,8 +164,21 @@ __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem));
 }
 
+// FP32 issue bound, with the staged sources read from shared memory second:
+// a record is one or two 16-byte loads for all lanes, and with one lane group
+// the terms go four at a time between folds.  With one rhs two consecutive
+// chunks of 32 targets (the second at least 17, so that both have one lane
+// group) share the sources.  Every (target, lane group) sums its terms in the
+// same order and folds them at the same places whatever the chunk's company.
+// Before (scalar coordinates, a fold test per term, one target a lane): 3-D
+// 250k targets, 81 sources a leaf: 1.38 -> 0.85 ms; 2-D log r 1M: 0.44 ->
+// 0.35 ms; 2-D forest, 16 rhs: 15.9 -> 15.0 ms.  Three blocks an SM, but two
+// in 3-D with one rhs (the pair's sums; 0.85 against 0.92 ms) and with 16.
+template <int RB>
+constexpr int p2p_targets() { return RB == 1 ? 2 : 1; }
+
 template <int KID, int D, int RB, typename T>
-__global__ void __launch_bounds__(256, (D == 3 && RB == 16) ? 2 : 3) k_p2p_f32(
+__global__ void __launch_bounds__(256, (D == 3 && (RB == 16 || RB == 1)) ? 2 : 3) k_p2p_f32(
     const int* __restrict__ row_box, int64_t nrow, const int* __restrict__ near, int nnear,
     const uint64_t* __restrict__ key, const int* __restrict__ tb, const int* __restrict__ te,
     const int* __restrict__ sb, const int* __restrict__ se, const float* __restrict__ txl, int64_t nt,
@@ -130,20 +188,20 @@ __global__ void __launch_bounds__(256, (D == 3 && RB == 16) ? 2 : 3) k_p2p_f32(
   // Per warp, in dynamic shared memory: the per-lane compensated FP32 sums
   // (sum, error) when the rhs block is wide (registers for up to 4 rhs;
   // keeps the kernel at 3 blocks per SM) and two staging buffers, each a
-  // chunk's weights and coordinates (hi[D], lo[D]).
-  constexpr int SC = p2p_chunk(RB);
+  // chunk's weights and coordinate records.
+  constexpr int SC = p2p_chunk(RB), REC = LocalRec<D>::N, BLK = p2p_block<RB>();
   constexpr bool kSmemAcc = RB >= 8;
   extern __shared__ __align__(16) unsigned char p2p_smem[];
   const int lane = threadIdx.x & 31;
   unsigned char* wb = p2p_smem + (size_t)(threadIdx.x >> 5) * p2p_warp_bytes(D, RB);
   float2 (*scs)[32] = reinterpret_cast<float2 (*)[32]>(wb);
-  // staging buffer b: weights sw[i][r] then coordinates sy[c][i]
+  // staging buffer b: weights sw[i][r] then records sy[i]
   unsigned char* const stage0 = wb + (kSmemAcc ? sizeof(double) * RB * 32 : 0);
   auto sw_of = [&](int b) {
     return reinterpret_cast<float (*)[RB]>(stage0 + (size_t)b * p2p_stage_bytes(D, RB));
   };
   auto sy_of = [&](int b) {
-    return reinterpret_cast<float (*)[SC]>(stage0 + (size_t)b * p2p_stage_bytes(D, RB) + sizeof(float) * SC * RB);
+    return reinterpret_cast<float (*)[REC]>(stage0 + (size_t)b * p2p_stage_bytes(D, RB) + sizeof(float) * SC * RB);
   };
   const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -152,23 +210,31 @@ __global__ void __launch_bounds__(256, (D == 3 && RB == 16) ? 2 : 3) k_p2p_f32(
     const int pid = key_pid(key[b]);
     const double len = cubes[pid].Len / (double)(1 << (depth[pid] - 1));
     const int t0 = tb[b], t1 = te[b];
-    for (int tc = t0; tc < t1; tc += 32) {
-      // cnt targets on the low lanes, G source groups on the high ones
-      const int cnt = min(32, t1 - tc);
+    // TT chunks of targets from tc: cnt targets on the low lanes of the last,
+    // G source groups on the high ones (one group when TT is 2)
+    auto chunks = [&](const int tc, const int cnt, auto tt_c) {
+      constexpr int TT = decltype(tt_c)::value;
       int tp2 = 1;
       while (tp2 < cnt) tp2 <<= 1;
       const int G = 32 / tp2;
       const int ti = lane & (tp2 - 1), g = lane / tp2;
-      const bool tv = ti < cnt;
-      double xd[D];
+      bool tv[TT];
+      double xd[TT][D];
 #pragma unroll
-      for (int q = 0; q < D; ++q)
-        xd[q] = tv ? (double)txl[(int64_t)q * nt + tc + ti] + (double)txl[(int64_t)(D + q) * nt + tc + ti] : 0.0;
+      for (int k = 0; k < TT; ++k) {
+        tv[k] = k + 1 < TT || ti < cnt;
+        float h[D], l[D];
+        if (tv[k]) load_local<D>(txl + (int64_t)(tc + 32 * k + ti) * REC, h, l);
+#pragma unroll
+        for (int q = 0; q < D; ++q) xd[k][q] = tv[k] ? (double)h[q] + (double)l[q] : 0.0;
+      }
       for (int r0 = 0; r0 < R; r0 += RB) {
         constexpr int RR = kSmemAcc ? 1 : RB;  // register pairs
-        float cs[RR], ce[RR];                  // compensated sum and its error (RB <= 4)
+        float cs[TT][RR], ce[TT][RR];          // compensated sum and its error (RB <= 4)
 #pragma unroll
-        for (int r = 0; r < RR; ++r) cs[r] = ce[r] = 0.f;
+        for (int k = 0; k < TT; ++k)
+#pragma unroll
+          for (int r = 0; r < RR; ++r) cs[k][r] = ce[k][r] = 0.f;
         if (kSmemAcc) {
 #pragma unroll
           for (int r = 0; r < RB; ++r) scs[r][lane] = make_float2(0.f, 0.f);
@@ -190,11 +256,14 @@ __global__ void __launch_bounds__(256, (D == 3 && RB == 16) ? 2 : 3) k_p2p_f32(
         };
         auto stage = [&](int b, int c0, int je) {
           const int m = min(SC, je - c0);
-          float (*syb)[SC] = sy_of(b);
+          float* syb = &sy_of(b)[0][0];
           float (*swb)[RB] = sw_of(b);
-#pragma unroll
-          for (int c = 0; c < 2 * D; ++c)
-            for (int i = lane; i < m; i += 32) cp_async4(&syb[c][i], sxl + (int64_t)c * ns + c0 + i);
+          if constexpr (REC >= 4) {
+            constexpr int PV = REC / 4;
+            for (int e = lane; e < m * PV; e += 32) cp_async16(syb + 4 * e, sxl + (int64_t)c0 * REC + 4 * e, true);
+          } else {
+            for (int e = lane; e < m * REC; e += 32) cp_async4(syb + e, sxl + (int64_t)c0 * REC + e);
+          }
           if constexpr (RB >= 4) {
             // rows of RB weights at 16-byte aligned offsets (Rp, r0: multiples of RB)
             constexpr int PV = RB / 4;
@@ -211,23 +280,27 @@ __global__ void __launch_bounds__(256, (D == 3 && RB == 16) ? 2 : 3) k_p2p_f32(
         if (have) stage(0, cc0, cje);
         cp_async_commit();
         int buf = 0, prevq = -1;
-        float ah[D], al[D];
-        float part[RB];  // plain FP32 partial of at most p2p_block<RB>() terms
+        float ah[TT][D], al[TT][D];
+        float part[TT][RB];  // plain FP32 partials of at most BLK terms
 #pragma unroll
-        for (int r = 0; r < RB; ++r) part[r] = 0.f;
+        for (int k = 0; k < TT; ++k)
+#pragma unroll
+          for (int r = 0; r < RB; ++r) part[k][r] = 0.f;
         int nterm = 0;
         auto fold = [&]() {
 #pragma unroll
-          for (int r = 0; r < RB; ++r) {
-            if (kSmemAcc) {
-              float2 sc = scs[r][lane];
-              two_sum_acc(sc.x, sc.y, part[r]);
-              scs[r][lane] = sc;
-            } else {
-              two_sum_acc(cs[kSmemAcc ? 0 : r], ce[kSmemAcc ? 0 : r], part[r]);
+          for (int k = 0; k < TT; ++k)
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+              if (kSmemAcc) {
+                float2 sc = scs[r][lane];
+                two_sum_acc(sc.x, sc.y, part[k][r]);
+                scs[r][lane] = sc;
+              } else {
+                two_sum_acc(cs[k][kSmemAcc ? 0 : r], ce[k][kSmemAcc ? 0 : r], part[k][r]);
+              }
+              part[k][r] = 0.f;
             }
-            part[r] = 0.f;
-          }
           nterm = 0;
         };
         while (have) {
@@ -245,34 +318,66 @@ __global__ void __launch_bounds__(256, (D == 3 && RB == 16) ? 2 : 3) k_p2p_f32(
             int qc = cq;
 #pragma unroll
             for (int q = D - 1; q >= 0; --q) {
-              const double av = xd[q] - len * (double)(qc % 3 - 1);
+              const double o = len * (double)(qc % 3 - 1);
               qc /= 3;
-              ah[q] = (float)av;
-              al[q] = (float)(av - (double)ah[q]);
+#pragma unroll
+              for (int k = 0; k < TT; ++k) {
+                const double av = xd[k][q] - o;
+                ah[k][q] = (float)av;
+                al[k][q] = (float)(av - (double)ah[k][q]);
+              }
             }
           }
           const int m = min(SC, cje - cc0);
-          const float (*sy)[SC] = sy_of(buf);
+          const float (*sy)[REC] = sy_of(buf);
           const float (*sw)[RB] = sw_of(buf);
-          if (tv) {
-            for (int i = g; i < m; i += G) {
+          // one source with the lane's targets
+          auto term = [&](int i) {
+            float h[D], l[D];
+            load_local<D>(sy[i], h, l);
+            float f[TT];
+#pragma unroll
+            for (int k = 0; k < TT; ++k) {
               float t[D];
 #pragma unroll
-              for (int q = 0; q < D; ++q) t[q] = (ah[q] - sy[q][i]) + (al[q] - sy[D + q][i]);
-              const float f = keval_diff_f32<KID, D>(t, p0);
-              if (RB == 1) {
-                part[0] = fmaf(sw[i][0], f, part[0]);
-              } else {
+              for (int q = 0; q < D; ++q) t[q] = (ah[k][q] - h[q]) + (al[k][q] - l[q]);
+              f[k] = keval_diff_f32<KID, D>(t, p0);
+            }
+            if constexpr (RB == 1) {
+              const float w = sw[i][0];
 #pragma unroll
-                for (int c4 = 0; c4 < RB / 4; ++c4) {
-                  const float4 w4 = reinterpret_cast<const float4*>(&sw[i][0])[c4];
-                  part[4 * c4 + 0] = fmaf(w4.x, f, part[4 * c4 + 0]);
-                  part[4 * c4 + 1] = fmaf(w4.y, f, part[4 * c4 + 1]);
-                  part[4 * c4 + 2] = fmaf(w4.z, f, part[4 * c4 + 2]);
-                  part[4 * c4 + 3] = fmaf(w4.w, f, part[4 * c4 + 3]);
+              for (int k = 0; k < TT; ++k) part[k][0] = fmaf(w, f[k], part[k][0]);
+            } else {
+#pragma unroll
+              for (int c4 = 0; c4 < RB / 4; ++c4) {
+                const float4 w4 = reinterpret_cast<const float4*>(&sw[i][0])[c4];
+#pragma unroll
+                for (int k = 0; k < TT; ++k) {
+                  part[k][4 * c4 + 0] = fmaf(w4.x, f[k], part[k][4 * c4 + 0]);
+                  part[k][4 * c4 + 1] = fmaf(w4.y, f[k], part[k][4 * c4 + 1]);
+                  part[k][4 * c4 + 2] = fmaf(w4.z, f[k], part[k][4 * c4 + 2]);
+                  part[k][4 * c4 + 3] = fmaf(w4.w, f[k], part[k][4 * c4 + 3]);
                 }
               }
-              if (++nterm == p2p_block<RB>()) fold();
+            }
+          };
+          if (TT > 1 || G == 1) {
+            // every lane takes every source: runs that end at a fold, four
+            // terms at a time (lanes without a target sum what nobody reads)
+            for (int i = 0; i < m;) {
+              const int e = min(m, i + BLK - nterm);
+              nterm += e - i;
+              for (; i + 4 <= e; i += 4) {
+#pragma unroll
+                for (int x = 0; x < 4; ++x) term(i + x);
+              }
+              for (; i < e; ++i) term(i);
+              if (nterm == BLK) fold();
+            }
+          } else if (tv[0]) {
+            for (int i = g; i < m; i += G) {
+              term(i);
+              if (++nterm == BLK) fold();
             }
           }
           __syncwarp();  // buffer buf is restaged two chunks on
@@ -284,20 +389,33 @@ __global__ void __launch_bounds__(256, (D == 3 && RB == 16) ? 2 : 3) k_p2p_f32(
         }
         fold();
 #pragma unroll
-        for (int r = 0; r < RB; ++r) {
-          double vr;
-          if (kSmemAcc) {
-            const float2 sc = scs[r][lane];
-            vr = (double)sc.x + (double)sc.y;
-          } else {
-            vr = (double)cs[kSmemAcc ? 0 : r] + (double)ce[kSmemAcc ? 0 : r];
+        for (int k = 0; k < TT; ++k)
+#pragma unroll
+          for (int r = 0; r < RB; ++r) {
+            double vr;
+            if (kSmemAcc) {
+              const float2 sc = scs[r][lane];
+              vr = (double)sc.x + (double)sc.y;
+            } else {
+              vr = (double)cs[k][kSmemAcc ? 0 : r] + (double)ce[k][kSmemAcc ? 0 : r];
+            }
+            for (int o = tp2; o < 32; o <<= 1) vr += __shfl_xor_sync(0xffffffffu, vr, o);
+            if (g == 0 && tv[k] && r0 + r < R) {
+              const int t = tc + 32 * k + ti;
+              out[(int64_t)(r0 + r) * nt + perm_t[t]] = (T)(vr + (pot ? pot[(int64_t)(r0 + r) * nt + t] : 0.0));
+            }
           }
-          for (int o = tp2; o < 32; o <<= 1) vr += __shfl_xor_sync(0xffffffffu, vr, o);
-          if (g == 0 && tv && r0 + r < R) {
-            const int t = tc + ti;
-            out[(int64_t)(r0 + r) * nt + perm_t[t]] = (T)(vr + (pot ? pot[(int64_t)(r0 + r) * nt + t] : 0.0));
-          }
-        }
+      }
+    };
+    for (int tc = t0; tc < t1;) {
+      const int rem = t1 - tc;
+      if (p2p_targets<RB>() == 2 && rem >= 32 + 17) {
+        const int c1 = min(32, rem - 32);
+        chunks(tc, c1, std::integral_constant<int, p2p_targets<RB>()>{});
+        tc += 32 + c1;
+      } else {
+        chunks(tc, min(32, rem), std::integral_constant<int, 1>{});
+        tc += 32;
       }
     }
   }
@@ -362,9 +480,14 @@ __global__ void __launch_bounds__(256, RB == 1 ? 4 : 2) k_p2p_f32_src(
     for (int tc = t0; tc < t1; tc += TB) {
       const int ntg = min(TB, t1 - tc);
       __syncwarp();
-      for (int e = lane; e < ntg * 2 * D; e += 32) {
-        const int i = e / (2 * D), c = e - i * 2 * D;  // c < D: hi of dim c, else lo of dim c - D
-        s_x[wib][i][c] = txl[(int64_t)c * nt + tc + i];
+      if (lane < ntg) {
+        float h[D], l[D];
+        load_local<D>(txl + (int64_t)(tc + lane) * LocalRec<D>::N, h, l);
+#pragma unroll
+        for (int q = 0; q < D; ++q) {
+          s_x[wib][lane][q] = h[q];
+          s_x[wib][lane][D + q] = l[q];
+        }
       }
       __syncwarp();
       // plain FP32 partials of at most kP2PBlock sources per lane (one source
@@ -404,13 +527,13 @@ __global__ void __launch_bounds__(256, RB == 1 ? 4 : 2) k_p2p_f32_src(
           const int sk = __shfl_sync(0xffffffffu, start, kq);
           if (e < total) {
             const int j = sb[bk] + (e - sk);
-            float yh[D], yl[D];
+            float yh[D], yl[D], h[D], l[D];
+            load_local<D>(sxl + (int64_t)j * LocalRec<D>::N, h, l);
             int qc = k;
 #pragma unroll
             for (int q = D - 1; q >= 0; --q) {
               // source relative to the target leaf's centre: own offset + len * (digit - 1)
-              const double yv = ((double)sxl[(int64_t)q * ns + j] + (double)sxl[(int64_t)(D + q) * ns + j]) +
-                                len * (double)(qc % 3 - 1);
+              const double yv = ((double)h[q] + (double)l[q]) + len * (double)(qc % 3 - 1);
               qc /= 3;
               yh[q] = (float)yv;
               yl[q] = (float)(yv - (double)yh[q]);
@@ -575,29 +698,38 @@ void gather_weights_mixed(fmma_ctx* ctx, const T* w, const int* perm, int64_t ns
 template void gather_weights_mixed<double>(fmma_ctx*, const double*, const int*, int64_t, int, double*);
 template void gather_weights_mixed<float>(fmma_ctx*, const float*, const int*, int64_t, int, double*);
 
+template <int D>
+static void local_coords(fmma_ctx* ctx, const Tree& tr, const double* tx, const double* sx, float* txl, float* sxl) {
+  const Level& Lf = tr.lev[0];
+  if (tr.nt + tr.ns < 16 * Lf.nbox) {  // a few points per leaf: one thread per leaf
+    const unsigned g = grid_for(Lf.nbox, 256, (int64_t)ctx->sm_count * 16);
+    FMMA_LAUNCH(ctx, k_local_coords_tpl<D>, g, 256, 0, Lf.key, Lf.tb, Lf.te, Lf.nbox, tx, tr.nt, tr.d_depth,
+                tr.d_cube, txl);
+    FMMA_LAUNCH(ctx, k_local_coords_tpl<D>, g, 256, 0, Lf.key, Lf.sb, Lf.se, Lf.nbox, sx, tr.ns, tr.d_depth,
+                tr.d_cube, sxl);
+  } else {
+    const dim3 blk(32, 8);
+    const unsigned g = grid_for(Lf.nbox, 8, (int64_t)ctx->sm_count * 32);
+    FMMA_LAUNCH(ctx, k_local_coords<D>, g, blk, 0, Lf.key, Lf.tb, Lf.te, Lf.nbox, tx, tr.nt, tr.d_depth, tr.d_cube,
+                txl);
+    FMMA_LAUNCH(ctx, k_local_coords<D>, g, blk, 0, Lf.key, Lf.sb, Lf.se, Lf.nbox, sx, tr.ns, tr.d_depth, tr.d_cube,
+                sxl);
+  }
+}
+
 template <typename T>
 void p2p_mixed(fmma_ctx* ctx, int d, const double* tx, const double* sx, const double* ws, int R, const double* pot,
                T* out, bool wst_ready) {
   Tree& tr = ctx->tree;
-  const Level& Lf = tr.lev[0];
-  float* txl = ctx_buf_t<float>(ctx, "txl", (size_t)(2 * d * tr.nt));
-  float* sxl = ctx_buf_t<float>(ctx, "sxl", (size_t)(2 * d * tr.ns));
+  const int rec = d == 1 ? 2 : (d == 2 ? 4 : 8);
+  float* txl = ctx_buf_t<float>(ctx, "txl", (size_t)rec * tr.nt);
+  float* sxl = ctx_buf_t<float>(ctx, "sxl", (size_t)rec * tr.ns);
   const int RB = p2p32_rhs_block(R);
   const int Rp = (R + RB - 1) / RB * RB;
   float* wst = ctx_buf_t<float>(ctx, "wsf", (size_t)Rp * tr.ns);
-  if (tr.nt + tr.ns < 16 * Lf.nbox) {  // a few points per leaf: one thread per leaf
-    const unsigned g = grid_for(Lf.nbox, 256, (int64_t)ctx->sm_count * 16);
-    FMMA_LAUNCH(ctx, k_local_coords_tpl, g, 256, 0, Lf.key, Lf.tb, Lf.te, Lf.nbox, tx, tr.nt, d, tr.d_depth, tr.d_cube,
-                txl);
-    FMMA_LAUNCH(ctx, k_local_coords_tpl, g, 256, 0, Lf.key, Lf.sb, Lf.se, Lf.nbox, sx, tr.ns, d, tr.d_depth, tr.d_cube,
-                sxl);
-  } else {
-    dim3 blk(32, 8);
-    FMMA_LAUNCH(ctx, k_local_coords, grid_for(Lf.nbox, 8, (int64_t)ctx->sm_count * 32), blk, 0, Lf.key, Lf.tb, Lf.te,
-                Lf.nbox, tx, tr.nt, d, tr.d_depth, tr.d_cube, txl);
-    FMMA_LAUNCH(ctx, k_local_coords, grid_for(Lf.nbox, 8, (int64_t)ctx->sm_count * 32), blk, 0, Lf.key, Lf.sb, Lf.se,
-                Lf.nbox, sx, tr.ns, d, tr.d_depth, tr.d_cube, sxl);
-  }
+  if (d == 1) local_coords<1>(ctx, tr, tx, sx, txl, sxl);
+  else if (d == 2) local_coords<2>(ctx, tr, tx, sx, txl, sxl);
+  else local_coords<3>(ctx, tr, tx, sx, txl, sxl);
   if (!wst_ready)  // else gather_weights_mixed wrote them with the sweep's weights
     FMMA_LAUNCH(ctx, k_weights_f32_t, grid_for((int64_t)Rp * tr.ns, 256), 256, 0, ws, R, Rp, tr.ns, wst);
   dispatch_kernel<P2P32Launch<T>>(ctx->kernel_id, d, ctx, tr, txl, sxl, wst, R, Rp, (float)ctx->p0, pot, out);
