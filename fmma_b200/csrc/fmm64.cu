@@ -785,7 +785,7 @@ void solve_forest(fmma_ctx* ctx, const SolveArgs& a, const std::vector<int64_t>&
     stage_begin(ctx, ST_P2M);
     {
       const Level& Lf = tr.lev[0];
-      launch_p2m_warp(ctx, Lf, sx, ns, ws, R, cubes, ddepth, d, isf, n, P, Kpad, dTn, Wm[0]);
+      launch_p2m_warp(ctx, Lf, sx, ns, ws, R, cubes, ddepth, d, isf, n, P, Kpad, dTn, Wm[0], tr.nprob);
     }
     stage_end(ctx, ST_P2M);
 

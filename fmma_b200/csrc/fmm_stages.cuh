@@ -28,10 +28,21 @@ __device__ __forceinline__ int bin_coord<float>(float x, const Cube& c, int q, i
 // and :595-596), in the caller's coordinate precision.  For float inputs the
 // reference computes (x-o)/len in float and the affine map in double, then
 // stores a float; the same steps are taken here.
-__device__ __forceinline__ double point_rel(double x, const Cube& c, int q, int N, bool isf) {
+// The leaf width is passed in (leaf_width): it is the same for all points of a
+// problem, a division each otherwise.
+struct LeafWidth {
+  double d;
+  float f;
+};
+__device__ __forceinline__ LeafWidth leaf_width(const Cube& c, int N, bool isf) {
+  LeafWidth w;
+  w.d = isf ? 0.0 : __ddiv_rn(c.Len, (double)N);
+  w.f = isf ? __fdiv_rn(c.Lenf, (float)N) : 0.f;
+  return w;
+}
+__device__ __forceinline__ double point_rel(double x, const Cube& c, const LeafWidth& w, int q, int N, bool isf) {
   if (!isf) {
-    double len = __ddiv_rn(c.Len, (double)N);
-    double qq = __ddiv_rn(__dsub_rn(x, c.origin[q]), len);
+    double qq = __ddiv_rn(__dsub_rn(x, c.origin[q]), w.d);
     int t = __double2int_rz(qq);
     t = t < N - 1 ? t : N - 1;
     double r = __dsub_rn(__dmul_rn(2.0, __dsub_rn(qq, (double)t)), 1.0);
@@ -40,14 +51,16 @@ __device__ __forceinline__ double point_rel(double x, const Cube& c, int q, int 
     return r;
   }
   float xf = (float)x;
-  float len = __fdiv_rn(c.Lenf, (float)N);
-  float qq = __fdiv_rn(__fsub_rn(xf, c.originf[q]), len);
+  float qq = __fdiv_rn(__fsub_rn(xf, c.originf[q]), w.f);
   int t = __float2int_rz(qq);
   t = t < N - 1 ? t : N - 1;
   double r = __dsub_rn(__dmul_rn(2.0, (double)__fsub_rn(qq, (float)t)), 1.0);
   r = r < 1.0 ? r : 1.0;
   r = r > -1.0 ? r : -1.0;
   return (double)(float)r;
+}
+__device__ __forceinline__ double point_rel(double x, const Cube& c, int q, int N, bool isf) {
+  return point_rel(x, c, leaf_width(c, N, isf), q, N, isf);
 }
 
 // S_n(node_k, y) for k = 0..n-1 (src/math.cpp:32-50):

@@ -1012,8 +1012,9 @@ static void p2m_warp_t(fmma_ctx* ctx, const Level& Lf, const double* sx, int64_t
 
 void launch_p2m_warp(fmma_ctx* ctx, const Level& Lf, const double* sx, int64_t ns, const double* ws, int R,
                      const Cube* cubes, const int* depth, int d, bool isf, int n, int P, int Kpad, const double* Tn,
-                     double* Wm, int grid_n) {
+                     double* Wm, int nprob, int grid_n) {
   FMMA_REQUIRE(d * n <= 32 && Kpad <= 512, "P2M: d * nodes must be <= 32 and P <= 512");
+  if (launch_p2m_tile(ctx, Lf, sx, ns, ws, R, cubes, depth, d, isf, n, P, Kpad, Wm, nprob, grid_n)) return;
   switch ((Kpad + 31) / 32) {
 #define FMMA_P2M_CASE(K_) \
   case K_: p2m_warp_t<K_>(ctx, Lf, sx, ns, ws, R, cubes, depth, d, isf, n, P, Kpad, Tn, Wm, grid_n); break;

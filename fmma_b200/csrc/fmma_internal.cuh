@@ -434,7 +434,11 @@ const FarTables& far_tables(int dim);
 // warp-per-box stage kernels (fmm_warp.cu)
 void launch_p2m_warp(fmma_ctx* ctx, const Level& Lf, const double* sx, int64_t ns, const double* ws, int R,
                      const Cube* cubes, const int* depth, int d, bool isf, int n, int P, int Kpad, const double* Tn,
-                     double* Wm, int grid_n = 0);
+                     double* Wm, int nprob, int grid_n = 0);
+// P2M of 2 to 8 nodes per dimension (p2m.cu); false for other node counts.
+bool launch_p2m_tile(fmma_ctx* ctx, const Level& Lf, const double* sx, int64_t ns, const double* ws, int R,
+                     const Cube* cubes, const int* depth, int d, bool isf, int n, int P, int Kpad, double* Wm,
+                     int nprob, int grid_n);
 void launch_l2p_warp(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t nt, const Cube* cubes,
                      const int* depth, int d, bool isf, int n, int P, int Kpad, int R, const double* Tn,
                      const double* Wl, double* pot, int ostride, int ooff);

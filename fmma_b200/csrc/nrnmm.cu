@@ -324,7 +324,7 @@ void solve_nrnmm(fmma_ctx* ctx, const SolveArgs& a, int nrn, int64_t nt, const T
   double* dTn = ctx_buf_t<double>(ctx, "nrn_Tn", kMaxNodes * kMaxNodes);
   upload(ctx, dTn, ct.Tn, sizeof(double) * n * n);
   double* Wm = ctx_buf_t<double>(ctx, "nrn_Wm", (size_t)nbox * R * Kpad);
-  launch_p2m_warp(ctx, L, sx, ns, ws, R, dc, nullptr, d, isf, n, P, Kpad, dTn, Wm, nrn);
+  launch_p2m_warp(ctx, L, sx, ns, ws, R, dc, nullptr, d, isf, n, P, Kpad, dTn, Wm, 1, nrn);
   stage_end(ctx, ST_P2M);
 
   // M2P from every box that is not adjacent (src/nrnmm.cpp:86-97)
