@@ -274,14 +274,17 @@ constexpr int kExThreads = 128;
 constexpr int kExTargets = 2;  // targets per thread
 constexpr int kExTile = 128;   // sources staged per step
 
-// part[(s * R + r) * nt + i] = sum over the sources of range s = blockIdx.y of
-// w[r][j] f(tgt[rows ? rows[i] : i], src[j]), RB right-hand sides per pass;
-// with one range the result itself.
-template <int KID, int D, int RB, typename T, typename O>
+// ans[r][i] = sum_j w[r][j] f(tgt[rows ? rows[i] : i], src[j]), RB right-hand
+// sides per pass.  Block (x, y) takes the targets of tile x and the sources of
+// range y.  With several ranges its sums go to part[(y * R + r) * nt + i], and
+// the tile's last block to finish (done[x], back to zero when it leaves) adds
+// the ranges in order: no second launch.
+template <int KID, int D, int RB, typename T>
 __global__ void __launch_bounds__(kExThreads) k_exact(const T* __restrict__ tgt, int64_t nt,
                                                       const int64_t* __restrict__ rows, const T* __restrict__ src,
                                                       int64_t ns, const T* __restrict__ w, int R, double p0,
-                                                      int64_t range, O* __restrict__ part) {
+                                                      int64_t range, double* part, unsigned* done,
+                                                      T* __restrict__ ans) {
   constexpr int U = 4 / kExTargets;
   __shared__ double sy[D][kExTile];
   __shared__ double sw[RB][kExTile];
@@ -344,18 +347,37 @@ __global__ void __launch_bounds__(kExThreads) k_exact(const T* __restrict__ tgt,
       if (ti[k] < nt)
 #pragma unroll
         for (int r = 0; r < RB; ++r)
-          if (r0 + r < R) part[((int64_t)blockIdx.y * R + r0 + r) * nt + ti[k]] = (O)acc[k][r];
+          if (r0 + r < R) {
+            if (gridDim.y == 1) ans[(int64_t)(r0 + r) * nt + ti[k]] = (T)acc[k][r];
+            else part[((int64_t)blockIdx.y * R + r0 + r) * nt + ti[k]] = acc[k][r];
+          }
   }
-}
-
-// ans[e] = sum over the ranges in order.
-template <typename T>
-__global__ void k_exact_sum(const double* __restrict__ part, int nranges, int64_t cnt, T* __restrict__ ans) {
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += (int64_t)gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int y = 0; y < nranges; ++y) s += part[(int64_t)y * cnt + e];
-    ans[e] = (T)s;
-  }
+  if (gridDim.y == 1) return;
+  __shared__ bool s_last;
+  __threadfence();  // this thread's sums before the count
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicInc(&done[blockIdx.x], gridDim.y - 1) == gridDim.y - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int k = 0; k < kExTargets; ++k)
+      if (ti[k] < nt) {
+        const double* p = part + (int64_t)r * nt + ti[k];
+        const int64_t step = (int64_t)R * nt;
+        double sum = 0.0;
+        int y = 0;
+        for (; y + 8 <= (int)gridDim.y; y += 8) {
+          double v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) v[u] = __ldcg(p + (y + u) * step);
+#pragma unroll
+          for (int u = 0; u < 8; ++u) sum += v[u];
+        }
+        for (; y < (int)gridDim.y; ++y) sum += __ldcg(p + y * step);
+        ans[(int64_t)r * nt + ti[k]] = (T)sum;
+      }
 }
 
 template <typename T>
@@ -381,21 +403,21 @@ struct ExactLaunch {
     const int64_t range = (ns + best - 1) / best;
     const int nranges = (int)((ns + range - 1) / range);
     const dim3 grid((unsigned)tiles, (unsigned)nranges);
-    if (nranges == 1) {
-      if (R == 1)
-        FMMA_LAUNCH(ctx, (k_exact<KID, D, 1, T, T>), grid, kExThreads, 0, tgt, nt, rows, src, ns, w, R, p0, range, ans);
-      else
-        FMMA_LAUNCH(ctx, (k_exact<KID, D, 4, T, T>), grid, kExThreads, 0, tgt, nt, rows, src, ns, w, R, p0, range, ans);
-      return;
+    double* part = nullptr;
+    unsigned* done = nullptr;
+    if (nranges > 1) {
+      part = ctx_buf_t<double>(ctx, "exact_part", (size_t)nranges * R * nt);
+      const size_t had = ctx->bufs["exact_done"].bytes;
+      done = ctx_buf_t<unsigned>(ctx, "exact_done", (size_t)tiles);
+      if (ctx->bufs["exact_done"].bytes != had)  // a new buffer: every launch leaves it at zero
+        FMMA_CHECK_CUDA(cudaMemsetAsync(done, 0, ctx->bufs["exact_done"].bytes, ctx->stream));
     }
-    double* part = ctx_buf_t<double>(ctx, "exact_part", (size_t)nranges * R * nt);
     if (R == 1)
-      FMMA_LAUNCH(ctx, (k_exact<KID, D, 1, T, double>), grid, kExThreads, 0, tgt, nt, rows, src, ns, w, R, p0, range,
-                  part);
+      FMMA_LAUNCH(ctx, (k_exact<KID, D, 1, T>), grid, kExThreads, 0, tgt, nt, rows, src, ns, w, R, p0, range, part,
+                  done, ans);
     else
-      FMMA_LAUNCH(ctx, (k_exact<KID, D, 4, T, double>), grid, kExThreads, 0, tgt, nt, rows, src, ns, w, R, p0, range,
-                  part);
-    FMMA_LAUNCH(ctx, k_exact_sum<T>, grid_for((int64_t)R * nt, 256), 256, 0, part, nranges, (int64_t)R * nt, ans);
+      FMMA_LAUNCH(ctx, (k_exact<KID, D, 4, T>), grid, kExThreads, 0, tgt, nt, rows, src, ns, w, R, p0, range, part,
+                  done, ans);
   }
 };
 
