@@ -35,12 +35,25 @@ SOLVERS = {"exact": _lib.SOLVER_EXACT, "fmm": _lib.SOLVER_FMM, "tree": _lib.SOLV
            "nrnmm": _lib.SOLVER_NRNMM}
 
 
+_torch = None  # the torch module, once a tensor has been seen
+
+
 def _is_torch(x) -> bool:
-    return type(x).__module__.startswith("torch")
+    global _torch
+    if _torch is not None and isinstance(x, _torch.Tensor):
+        return True
+    if type(x).__module__.startswith("torch"):
+        if _torch is None:
+            import torch
+            _torch = torch
+        return True
+    return False
 
 
 class _Arr:
     """A pointer view of a numpy array or torch tensor."""
+
+    __slots__ = ("obj", "ptr", "kind", "shape")
 
     def __init__(self, x, dtype, name):
         self.obj = x
@@ -48,16 +61,12 @@ class _Arr:
             self.ptr, self.kind, self.shape = None, None, None
             return
         if _is_torch(x):
-            import torch
-            want = torch.float64 if dtype == np.float64 else torch.float32
+            want = _torch.float64 if dtype == np.float64 else _torch.float32
             if x.dtype != want:
                 raise TypeError(f"{name}: expected {want}, got {x.dtype}")
             if not x.is_contiguous():
                 raise ValueError(f"{name}: tensor must be contiguous")
-            if x.is_cuda:
-                self.ptr, self.kind = x.data_ptr(), _lib.MEM_DEVICE
-            else:
-                self.ptr, self.kind = x.data_ptr(), _lib.MEM_HOST
+            self.ptr, self.kind = x.data_ptr(), _lib.MEM_DEVICE if x.is_cuda else _lib.MEM_HOST
             self.shape = tuple(x.shape)
             return
         if not isinstance(x, np.ndarray):
@@ -89,7 +98,6 @@ class Context:
         self.device = device
         self.lock = threading.RLock()
         self.kernel = ("inv_r", 0.0)
-        self._xstream = None
 
     def set_allocator(self, alloc=None, free=None):
         """Routes the context's device scratch and operator cache through
@@ -164,15 +172,7 @@ class Context:
         call returns (the library synchronises its stream)."""
         if kind != _lib.MEM_DEVICE:
             return
-        import torch
-        cur = torch.cuda.current_stream(self.device)
-        if cur.cuda_stream == self.stream_ptr():
-            return
-        if self._xstream is None:
-            self._xstream = torch.cuda.ExternalStream(self.stream_ptr(), device=f"cuda:{self.device}")
-        ev = torch.cuda.Event()
-        ev.record(cur)
-        self._xstream.wait_event(ev)
+        check(self._L.fmma_wait_stream(self._h, _torch.cuda.current_stream(self.device).cuda_stream))
 
     def close(self):
         if getattr(self, "_h", None) is not None and self._h.value:
@@ -210,8 +210,8 @@ class Context:
         ans has shape (N,) or (R, N) and the dtype of the inputs.  For
         solver "nrnmm", depth is nrn_N (boxes per dimension, <= 0: default)
         and the second result is the nrn_N used."""
-        t0 = tgt
-        dtype = np.float64 if (t0.dtype == np.float64 or str(t0.dtype) == "torch.float64") else np.float32
+        f64 = tgt.dtype == _torch.float64 if _is_torch(tgt) else tgt.dtype == np.float64
+        dtype = np.float64 if f64 else np.float32
         if tgt.ndim != 2 or src.ndim != 2 or tgt.shape[1] != src.shape[1]:
             raise ValueError("tgt and src must be (n, d) arrays of the same d")
         d = int(tgt.shape[1])
@@ -442,7 +442,7 @@ class Context:
     def stage_times(self) -> dict:
         ms = (C.c_double * _lib.NUM_STAGES)()
         check(self._L.fmma_stage_times(self._h, ms, _lib.NUM_STAGES))
-        return {self._L.fmma_stage_name(i).decode(): ms[i] for i in range(_lib.NUM_STAGES)}
+        return dict(zip(_lib.stage_names(), ms))
 
     def last_launch_count(self) -> int:
         return int(self._L.fmma_last_launch_count(self._h))

@@ -83,6 +83,7 @@ SIGNATURES = {
     "fmma_stage_name": (C.c_char_p, [_i]),
     "fmma_last_launch_count": (_i64, [_vp]),
     "fmma_ctx_stream": (_vp, [_vp]),
+    "fmma_wait_stream": (_i, [_vp, _vp]),
     "fmma_m2l_stats": (_i, [_vp, _pd, _pd, _pi64]),
     "fmma_tree_stats": (_i, [_vp, _pi64, _pi64, _pi64]),
     "fmma_set_user_kernel": (_i, [_vp, _vp, _vp, _i]),
@@ -129,6 +130,17 @@ def load() -> C.CDLL:
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+_names = None
+
+
+def stage_names() -> list:
+    """Names of the timed stages, in the order of fmma_stage_times."""
+    global _names
+    if _names is None:
+        _names = [load().fmma_stage_name(i).decode() for i in range(NUM_STAGES)]
+    return _names
 
 
 def check(status: int) -> None:

@@ -182,6 +182,7 @@ fmma_status fmma_ctx_destroy(fmma_ctx* ctx) {
     release_device_memory(ctx);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->up_host) cudaFreeHost(ctx->up_host);
+    if (ctx->ev_wait) cudaEventDestroy(ctx->ev_wait);
     for (int i = 0; i < 2 * FMMA_NUM_STAGES; ++i)
       if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     for (int i = 0; i < 2 * fmma_ctx::kMaxTimed; ++i)
@@ -655,6 +656,17 @@ const char* fmma_stage_name(int i) {
 int64_t fmma_last_launch_count(fmma_ctx* ctx) { return ctx ? ctx->launches : 0; }
 
 void* fmma_ctx_stream(fmma_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
+
+fmma_status fmma_wait_stream(fmma_ctx* ctx, void* stream) {
+  return guarded([&] {
+    use_device(ctx);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (st == ctx->stream) return;
+    if (!ctx->ev_wait) FMMA_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->ev_wait, cudaEventDisableTiming));
+    FMMA_CHECK_CUDA(cudaEventRecord(ctx->ev_wait, st));
+    FMMA_CHECK_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev_wait, 0));
+  });
+}
 
 fmma_status fmma_m2l_stats(fmma_ctx* ctx, double* kernel_ms, double* flops, int64_t* launches) {
   return guarded([&] {

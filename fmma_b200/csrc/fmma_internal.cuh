@@ -156,6 +156,7 @@ struct fmma_ctx {
   void* alloc_user = nullptr;
   cudaEvent_t ev[2 * FMMA_NUM_STAGES] = {};
   bool ev_used[FMMA_NUM_STAGES] = {};
+  cudaEvent_t ev_wait = nullptr;  // fmma_wait_stream
   double stage_ms[FMMA_NUM_STAGES] = {};
   int64_t launches = 0;
   fmma_b200::Tree tree;

@@ -298,6 +298,10 @@ const char* fmma_stage_name(int i);
 int64_t fmma_last_launch_count(fmma_ctx* ctx);
 /* The context's CUDA stream (a cudaStream_t), for event timing by callers. */
 void* fmma_ctx_stream(fmma_ctx* ctx);
+/* Makes the context's stream wait for the work queued so far on `stream` (a
+ * cudaStream_t of the same device; NULL = the legacy default stream), without
+ * blocking the host: for device buffers that another stream fills.         */
+fmma_status fmma_wait_stream(fmma_ctx* ctx, void* stream);
 /* M2L kernels of the last solve: summed CUDA-event time of the launches,
  * algorithmic flops (2 P^2 per target/source box pair and rhs), launches. */
 fmma_status fmma_m2l_stats(fmma_ctx* ctx, double* kernel_ms, double* flops,

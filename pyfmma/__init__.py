@@ -35,6 +35,7 @@ _SOLVER_ALIASES = {"exact": "exact", "exact_matvec": "exact", "fmm": "fmm", "tre
 
 class _FMMA:
     TYPE = np.float64
+    TORCH_TYPE = "torch.float64"
     DIM = 1
 
     def __init__(self):
@@ -153,38 +154,37 @@ class _FMMA:
         return fmma_b200.default_context(self._device).stage_times()
 
     def _check_shapes(self, target, source_weight, source, ans):
-        def nd(x):
-            return len(x.shape)
-        if nd(target) != 2:
-            raise RuntimeError(f"target shape must be 2 but {nd(target)}")
-        if source_weight is not None and nd(source_weight) not in (1, 2):
-            raise RuntimeError(f"source_weight shape must be 2 but {nd(source_weight)}")
-        if nd(source) != 2:
-            raise RuntimeError(f"source shape must be 2 but {nd(source)}")
-        want_ans = 1 if (source_weight is None or nd(source_weight) == 1) else 2
-        if nd(ans) != want_ans:
-            raise RuntimeError(f"ans shape must be {want_ans} but {nd(ans)}")
-        if target.shape[1] != self.DIM:
-            raise RuntimeError(f"target dimension must be {self.DIM} but {target.shape[1]}")
-        if source.shape[1] != self.DIM:
-            raise RuntimeError(f"source dimension must be {self.DIM} but {source.shape[1]}")
-        if ans.shape[-1] != target.shape[0]:
-            raise RuntimeError(f"ans num {ans.shape[-1]} is different from target num {target.shape[0]}")
-        if source_weight is not None and source.shape[0] != source_weight.shape[-1]:
-            raise RuntimeError(f"source num {source.shape[0]} is different from source_weight num "
-                               f"{source_weight.shape[-1]}")
+        ts, ss, as_ = target.shape, source.shape, ans.shape
+        ws = None if source_weight is None else source_weight.shape
+        if len(ts) != 2:
+            raise RuntimeError(f"target shape must be 2 but {len(ts)}")
+        if ws is not None and len(ws) not in (1, 2):
+            raise RuntimeError(f"source_weight shape must be 2 but {len(ws)}")
+        if len(ss) != 2:
+            raise RuntimeError(f"source shape must be 2 but {len(ss)}")
+        want_ans = 1 if (ws is None or len(ws) == 1) else 2
+        if len(as_) != want_ans:
+            raise RuntimeError(f"ans shape must be {want_ans} but {len(as_)}")
+        if ts[1] != self.DIM:
+            raise RuntimeError(f"target dimension must be {self.DIM} but {ts[1]}")
+        if ss[1] != self.DIM:
+            raise RuntimeError(f"source dimension must be {self.DIM} but {ss[1]}")
+        if as_[-1] != ts[0]:
+            raise RuntimeError(f"ans num {as_[-1]} is different from target num {ts[0]}")
+        if ws is not None and ss[0] != ws[-1]:
+            raise RuntimeError(f"source num {ss[0]} is different from source_weight num {ws[-1]}")
         for name, x in (("target", target), ("source", source), ("ans", ans), ("source_weight", source_weight)):
             if x is None:
                 continue
             dt = getattr(x, "dtype", None)
-            ok = (dt == self.TYPE) if isinstance(x, np.ndarray) else (str(dt) == f"torch.{np.dtype(self.TYPE).name}")
+            ok = (dt == self.TYPE) if isinstance(x, np.ndarray) else (str(dt) == self.TORCH_TYPE)
             if not ok:
                 raise TypeError(f"{name} must have dtype {np.dtype(self.TYPE).name}")
 
 
 def _make(type_char, dim):
     t = np.float64 if type_char == "d" else np.float32
-    return type(f"fmma{type_char}{dim}", (_FMMA,), {"TYPE": t, "DIM": dim,
+    return type(f"fmma{type_char}{dim}", (_FMMA,), {"TYPE": t, "TORCH_TYPE": f"torch.{np.dtype(t).name}", "DIM": dim,
                                                      "__doc__": f"FMMA<{np.dtype(t).name},{dim}> on the GPU."})
 
 
