@@ -22,16 +22,29 @@
 // fall into 56 orbits worth 39.5 P^2 multiply-adds (189 P^2 before).
 //
 // FP64 tensor (DMMA) bound.  A block owns 8 MB target rows (box x rhs) of one
-// child-parity class.  Eight multiplying warps: warp w accumulates the rows'
-// outputs of one parity a (w and 7 - w share a scheduler, so with an odd node
-// count, where an even-parity block is larger, each scheduler has the same
-// number of columns).  Eight gathering warps read the 8 source values of a
-// (row, k), run the butterfly in registers and store the z of a stage (two K
-// steps of 4) into a ring of four in shared memory; a full and an empty
-// mbarrier per slot tie the two sides.  Operator fragments are read from L2
-// straight into registers (a warp shares them with no other warp of the
-// block), one stage ahead.  Orbits with no source for a tile are skipped, and
-// so are a tile's unused row groups of 8.
+// child-parity class.  Eight multiplying warps hold the rows' sums, a warp the
+// outputs of one parity, or with an odd node count of the parities a and 7 - a
+// for half of the rows, so that every warp has the same number of columns
+// (an even-parity block is larger).  Eight gathering warps read the 8 source
+// values of a (row, k), run the butterfly in registers and store the z of a
+// stage (two K steps of 4) into a ring of four in shared memory; a full and an
+// empty mbarrier per slot tie the two sides.  Operator fragments are read from
+// L2 straight into registers (with an even node count a warp shares them with
+// no other warp of the block), a stage ahead.  Orbits with no source for a
+// tile are skipped, and so are a tile's unused row groups of 8, by kernels
+// compiled for 1, 2, half and all of them (a DMMA that is predicated off still
+// takes its turn on the pipe).
+// Measured on the 262k clustered level (6 nodes, 1945 tiles), on a million
+// points of the adjoint's two solves and on 4096 boxes x 2 rhs (5 nodes), ms of
+// all levels: gather, butterfly and multiply in the same warps 41.7, - and
+// 1.68; warps of their own 34.6, - and 1.40; straight-line multiplying,
+// one-sided dimensions and fragments loaded ahead 28.9, 10.2 and 0.98; row
+// groups at compile time and the prologue's loads all in flight 28.3, 9.4 and
+// 0.88.  A stage then takes 2750 cycles (6 nodes), of which the DMMAs need
+// 2048 and the butterfly's additions, which take turns on the same pipe, 390
+// (without them 2400).  Tried and slower: the operators in shared memory by
+// bulk copies (29.9, 10.0, 0.90), the butterfly ahead of the wait for a free
+// slot (31.1, 10.5, 0.94), a ring of three (28.5, 9.5, 0.88).
 #include <algorithm>
 #include <cmath>
 
@@ -235,7 +248,9 @@ __global__ void __launch_bounds__(256) k_sym_table(const double* __restrict__ le
       const int a = (lane >> 3) + 4 * u;
       if ((a & I.mid) || ((a ^ b) & z)) continue;
       const int col = I.in_block(a, he, ho);
-      base[(((int64_t)a * 2 + (step & 1)) * 32 + (col & 7) * 4 + (k & 3)) * NB + (col >> 3)] = v[u] * (1.0 / 64);
+      const int l = (col & 7) * 4 + (k & 3), nb = col >> 3;  // lane and column group of the fragment
+      const int64_t at = ((int64_t)a * 2 + (step & 1)) * (32 * NB) + (NB == 1 ? l : (nb >> 1) * 64 + l * 2 + (nb & 1));
+      base[at] = v[u] * (1.0 / 64);
     }
   }
 }
@@ -320,7 +335,7 @@ struct SymParams {
   const int* row_box;
   const SymGeom* geom;
   const double* W;     // folded sources [box * R + r][8][KB]
-  const double* tab;   // [table][stage][a][step][lane][NB]
+  const double* tab;   // [table][stage][a][step][column group pair][lane][2]
   const int* part_lo;  // [gridDim.y + 1] first orbit of each part
   double* Wl;          // parity blocks into Wl (one part) ...
   double* part;        // ... or [part][virtual row][P]
@@ -387,65 +402,67 @@ struct SymShape {
   static constexpr int kMulRegs = 176, kGatherRegs = 256 - kMulRegs;
   static constexpr int KB = NB == 1 ? 8 : (NB == 4 ? 28 : 64);  // SymGeom::KB of its node counts
   static constexpr int ILS = TM + 1;                 // stride of a slot's source list
-  static constexpr size_t kSmem =
-      sizeof(double) * 2 * kSymRing * PLANE + sizeof(int) * (kSymSlots * ILS + 8 * kSymMaxStages * 2 + kOrbits * 8 + kOrbits * 5);
+  static constexpr int kTabStage = 8 * 2 * 32 * NB;  // doubles of a stage's operator
+  static constexpr size_t kSmem = sizeof(double) * kSymRing * 2 * PLANE +
+                                  sizeof(int) * (kSymSlots * ILS + 8 * kSymMaxStages * 2 + kOrbits * 8 + kOrbits * 5);
 };
 
 // What the multiplying warps read of the block.
 struct SymBlock {
   const double* z;     // ring of z
+  const double* tab;   // operators of the tile's table
   const int4* act;     // active orbits
   const int2* desc;    // K steps by zero mask and stage
   uint64_t *full, *empty;
   int* abort;
-  const double* tab;   // operators of the tile's table
   int nact, neg, v0, vcnt;
 };
 
-// One multiplying warp.  Its accumulators are two parts of MB / 2 row groups:
-// with an even node count (PAIR false) the two halves of the rows for one
-// parity a0, with an odd one half of the rows for the parities a0 and 7 - a0,
-// whose column groups N0 + N1 are the same for every warp.  A stage is four
-// units (K step, part) in a straight line: the next unit's source fragments
-// load under the DMMAs of one, the next stage's first ones too when that stage
-// is there already, and the operator fragments a stage ahead.
-template <int NB, int MB, bool PAIR, int N0, int N1>
+// One multiplying warp.  Its accumulators are two parts of row groups: with an
+// even node count (PAIR false) the first G0 and the following G1 groups of the
+// tile for one parity a0, with an odd one G0 = G1 groups of one half of the
+// tile for the parities a0 and 7 - a0, whose column groups N0 + N1 are the
+// same for every warp.  A stage is four units (K step, part) in a straight
+// line: the source fragments of a unit load under the DMMAs of the one before,
+// the next stage's first ones too when that stage is there already, and the
+// operator fragments a stage ahead.
+template <int NB, int MB, bool PAIR, int N0, int N1, int G0, int G1>
 __device__ __forceinline__ bool sym_multiply(const SymParams& p, const SymBlock& sb, int warp, int lane) {
   using S = SymShape<NB, MB>;
-  constexpr int TM = S::TM, H = MB / 2, NF = PAIR ? N0 + N1 : N0;
-  constexpr int kTabStage = 8 * 2 * 32 * NB;  // doubles of a stage's operator
+  constexpr int TM = S::TM, H = MB / 2, NF = PAIR ? N0 + N1 : N0, GA = G0 > G1 ? G0 : G1, G1A = G1 > 0 ? G1 : 1;
   const int a0 = PAIR ? warp & 3 : (warp < 4 ? warp : 11 - warp);
   const int a1 = PAIR ? 7 - a0 : a0;
-  const int row1 = PAIR ? 0 : H * 32, row0 = PAIR ? (warp >> 2) * H * 32 : 0;
-  const int rows = ((1 << H) - 1) << (PAIR ? (warp >> 2) * H : 0);  // row groups of part 0
-  double acc0[H][N0][2], acc1[H][N1][2], bf[2][NF];
+  const int row1 = PAIR ? 0 : G0 * 32, row0 = PAIR ? (warp >> 2) * H * 32 : 0;
+  double acc0[G0][N0][2], acc1[G1A][N1][2], bf[2][NF], av[2][GA];
 #pragma unroll
-  for (int i = 0; i < H; ++i) {
+  for (int i = 0; i < G0; ++i)
 #pragma unroll
     for (int j = 0; j < N0; ++j) acc0[i][j][0] = acc0[i][j][1] = 0.0;
 #pragma unroll
+  for (int i = 0; i < G1A; ++i)
+#pragma unroll
     for (int j = 0; j < N1; ++j) acc1[i][j][0] = acc1[i][j][1] = 0.0;
-  }
+  const double* const b0 = sb.tab + a0 * (2 * 32 * NB) + lane * (NB == 1 ? 1 : 2);
+  const double* const b1 = sb.tab + a1 * (2 * 32 * NB) + lane * (NB == 1 ? 1 : 2);
   auto load_b = [&](int stage, int ks) {
-    const double* src = sb.tab + (int64_t)stage * kTabStage + ks * (32 * NB) + lane * NB;
 #pragma unroll
     for (int part = 0; part < (PAIR ? 2 : 1); ++part) {
-      const double* sp = src + (part ? a1 : a0) * (2 * 32 * NB);
+      const double* src = (part ? b1 : b0) + (int64_t)stage * S::kTabStage + ks * (32 * NB);
       const int n = part ? N1 : N0, f = part ? N0 : 0;
 #pragma unroll
       for (int j = 0; j < n; j += 2) {
-        if (j + 1 < n) {
-          const double2 t = __ldg(reinterpret_cast<const double2*>(sp + j));
+        if (NB > 1 && j + 1 < n) {
+          const double2 t = __ldg(reinterpret_cast<const double2*>(src + (j >> 1) * 64));
           bf[ks][f + j] = t.x;
           bf[ks][f + j + 1 < NF ? f + j + 1 : 0] = t.y;
         } else {
-          bf[ks][f + j] = __ldg(sp + j);
+          bf[ks][f + j] = __ldg(src + (j >> 1) * 64);
         }
       }
     }
   };
   struct Stage {
-    int s0, s1, u, mask, tab, slot;
+    int s0, s1, u, un, tab;  // un: the one-sided dimensions on the negative side
   };
   int oi = 0, st = -1, nst = 0, slot = 0, phase = 0;
   Stage cur, nxt{};
@@ -458,7 +475,7 @@ __device__ __forceinline__ bool sym_multiply(const SymParams& p, const SymBlock&
       const int4 f = sb.act[oi];
       ds = sb.desc + ((f.x >> 8) & 7) * kSymMaxStages;
       nxt.u = f.x >> 16;
-      nxt.mask = f.z;
+      nxt.un = nxt.u & sb.neg;
       nxt.tab = f.w - 1;
       nst = f.y;
       st = 0;
@@ -470,96 +487,68 @@ __device__ __forceinline__ bool sym_multiply(const SymParams& p, const SymBlock&
     return true;
   };
   // z of (K step, part) of a stage, and the sign of its operator blocks
-  auto frag = [&](const Stage& s, int sl, int ks, int part) -> const double* {
+  const double* const z0 = sb.z + row0 + lane;
+  auto load_a = [&](double* v, const Stage& s, int sl, int ks, int part) {
     const int c = (part ? a1 : a0) ^ ((ks ? s.s1 : s.s0) & 7);
-    return sb.z + (sl * 2 + ks) * S::PLANE + (c & ~s.u) * (TM * 4) + row0 + (part ? row1 : 0) + lane;
+    const double* src = z0 + (sl * 2 + ks) * S::PLANE + (c & ~s.u) * (TM * 4) + (part ? row1 : 0);
+#pragma unroll
+    for (int mb = 0; mb < (part ? G1 : G0); ++mb) v[mb] = src[mb * 32];
   };
   auto flip = [&](const Stage& s, int ks) {
+    if (s.un == 0) return;
 #pragma unroll
     for (int part = 0; part < (PAIR ? 2 : 1); ++part) {
       const int c = (part ? a1 : a0) ^ ((ks ? s.s1 : s.s0) & 7);
-      if (__popc(c & s.u & sb.neg) & 1) {
+      if (__popc(c & s.un) & 1) {
 #pragma unroll
         for (int j = 0; j < (part ? N1 : N0); ++j) bf[ks][(part ? N0 : 0) + j] = -bf[ks][(part ? N0 : 0) + j];
       }
     }
-  };
-  constexpr int kAll = (1 << MB) - 1;
-  bool have = advance();
-  cur = nxt;
-  bool ready = false;  // av[0] holds the first unit of the stage
-  double av[2][H];
-  auto load_a = [&](double* v, const double* src) {
-#pragma unroll
-    for (int mb = 0; mb < H; ++mb) v[mb] = src[mb * 32];
   };
   auto mul = [&](const double* v, int ks, int part) {
     if (part == 0) {
 #pragma unroll
       for (int nb = 0; nb < N0; ++nb)
 #pragma unroll
-        for (int mb = 0; mb < H; ++mb) dmma(acc0[mb][nb][0], acc0[mb][nb][1], v[mb], bf[ks][nb]);
+        for (int mb = 0; mb < G0; ++mb) dmma(acc0[mb][nb][0], acc0[mb][nb][1], v[mb], bf[ks][nb]);
     } else {
 #pragma unroll
       for (int nb = 0; nb < N1; ++nb)
 #pragma unroll
-        for (int mb = 0; mb < H; ++mb) dmma(acc1[mb][nb][0], acc1[mb][nb][1], v[mb], bf[ks][(PAIR ? N0 : 0) + nb]);
+        for (int mb = 0; mb < G1; ++mb) dmma(acc1[mb][nb][0], acc1[mb][nb][1], v[mb], bf[ks][(PAIR ? N0 : 0) + nb]);
     }
   };
+  bool have = advance(), ready = false;  // ready: the stage's first source fragments are in av[0]
+  cur = nxt;
   if (have) {
     load_b(cur.tab, 0);
     load_b(cur.tab, 1);
   }
   while (have) {
-    const bool more = advance();  // nxt: the stage behind this one (at the end: this one's operator again)
-    if (!ready && !bar_wait(&sb.full[slot], phase, sb.abort)) return false;
+    const bool more = advance();  // nxt: the stage behind this one
     const int nslot = slot + 1 == kSymRing ? 0 : slot + 1, nphase = slot + 1 == kSymRing ? phase ^ 1 : phase;
-    if (cur.mask == kAll && cur.s1 >= 0) {
-      if (!ready) load_a(av[0], frag(cur, slot, 0, 0));
-      flip(cur, 0);
-      load_a(av[1], frag(cur, slot, 0, 1));
-      mul(av[0], 0, 0);
-      load_a(av[0], frag(cur, slot, 1, 0));
-      mul(av[1], 0, 1);
-      load_b(nxt.tab, 0);
-      flip(cur, 1);
-      load_a(av[1], frag(cur, slot, 1, 1));
-      mul(av[0], 1, 0);
-      ready = more && nxt.mask == kAll && nxt.s1 >= 0 &&
-              __all_sync(0xffffffffu, bar_test(&sb.full[nslot], nphase));
-      if (ready) load_a(av[0], frag(nxt, nslot, 0, 0));
-      mul(av[1], 1, 1);
-      load_b(nxt.tab, 1);
-    } else {
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
-        flip(cur, ks);
-        if (ks == 0 || cur.s1 >= 0) {  // the last stage of an orbit may have one K step
-#pragma unroll
-          for (int part = 0; part < 2; ++part) {
-            const double* A = frag(cur, slot, ks, part);
-            const int m = PAIR ? (cur.mask & rows) >> ((warp >> 2) * H) : cur.mask >> (part * H);
-#pragma unroll
-            for (int mb = 0; mb < H; ++mb)
-              if ((m >> mb) & 1) {
-                const double v = A[mb * 32];
-                if (part == 0) {
-#pragma unroll
-                  for (int nb = 0; nb < N0; ++nb) dmma(acc0[mb][nb][0], acc0[mb][nb][1], v, bf[ks][nb]);
-                } else {
-#pragma unroll
-                  for (int nb = 0; nb < N1; ++nb)
-                    dmma(acc1[mb][nb][0], acc1[mb][nb][1], v, bf[ks][(PAIR ? N0 : 0) + nb]);
-                }
-              }
-          }
-        }
-        load_b(nxt.tab, ks);
-      }
-      ready = false;
+    if (!ready) {
+      if (!bar_wait(&sb.full[slot], phase, sb.abort)) return false;
+      load_a(av[0], cur, slot, 0, 0);
     }
+    const bool two = cur.s1 >= 0;  // the last stage of an orbit may have one K step
+    flip(cur, 0);
+    load_a(av[1], cur, slot, 0, 1);
+    mul(av[0], 0, 0);
+    if (two) load_a(av[0], cur, slot, 1, 0);
+    mul(av[1], 0, 1);
+    load_b(nxt.tab, 0);
+    if (two) {
+      flip(cur, 1);
+      load_a(av[1], cur, slot, 1, 1);
+      mul(av[0], 1, 0);
+    }
+    ready = more && __all_sync(0xffffffffu, bar_test(&sb.full[nslot], nphase));
+    if (ready) load_a(av[0], nxt, nslot, 0, 0);
+    if (two) mul(av[1], 1, 1);
+    load_b(nxt.tab, 1);
     __syncwarp();
-    if (lane == 0) bar_arrive(&sb.empty[slot]);  // the z values are in registers
+    if (lane == 0) bar_arrive(&sb.empty[slot]);  // the stage's values are in registers
     slot = nslot;
     phase = nphase;
     cur = nxt;
@@ -572,7 +561,7 @@ __device__ __forceinline__ bool sym_multiply(const SymParams& p, const SymBlock&
     const int a = part ? a1 : a0;
     const int size = g.size[a], first = g.off[a];
 #pragma unroll
-    for (int mb = 0; mb < H; ++mb) {
+    for (int mb = 0; mb < (part ? G1 : G0); ++mb) {
       const int i = (row0 + (part ? row1 : 0)) / 4 + mb * 8 + (lane >> 2);
       if (i >= sb.vcnt) continue;
       const int64_t v = sb.v0 + i;
@@ -586,8 +575,8 @@ __device__ __forceinline__ bool sym_multiply(const SymParams& p, const SymBlock&
 #pragma unroll
       for (int nb = 0; nb < (part ? N1 : N0); ++nb) {
         const int col = nb * 8 + (lane & 3) * 2;
-        const double x = part ? acc1[mb][part ? nb : 0][0] : acc0[mb][part ? 0 : nb][0];
-        const double y = part ? acc1[mb][part ? nb : 0][1] : acc0[mb][part ? 0 : nb][1];
+        const double x = part ? acc1[part ? mb : 0][part ? nb : 0][0] : acc0[part ? 0 : mb][part ? 0 : nb][0];
+        const double y = part ? acc1[part ? mb : 0][part ? nb : 0][1] : acc0[part ? 0 : mb][part ? 0 : nb][1];
         if (col < size) dst[col] = x;
         if (col + 1 < size) dst[col + 1] = y;
       }
@@ -596,49 +585,102 @@ __device__ __forceinline__ bool sym_multiply(const SymParams& p, const SymBlock&
   return true;
 }
 
+// A multiplying warp without rows (the upper half of a small tile): it frees
+// the stages as they come.
+__device__ __forceinline__ bool sym_pass(const SymBlock& sb, int nstages, int lane) {
+  for (int it = 0, slot = 0, phase = 0; it < nstages; ++it) {
+    if (!bar_wait(&sb.full[slot], phase, sb.abort)) return false;
+    __syncwarp();
+    if (lane == 0) bar_arrive(&sb.empty[slot]);
+    if (++slot == kSymRing) {
+      slot = 0;
+      phase ^= 1;
+    }
+  }
+  return true;
+}
+
+// The parity (pair) of a warp by its number, for G0 (and G1) row groups.
+template <int N, int NB, int MB, int G0, int G1>
+__device__ __forceinline__ bool sym_warp(const SymParams& p, const SymBlock& sb, int warp, int lane) {
+  if constexpr (N % 2 == 0) {
+    constexpr int C = (N / 2 * (N / 2) * (N / 2) + 7) / 8;  // column groups of every parity
+    return sym_multiply<NB, MB, false, C, C, G0, G1>(p, sb, warp, lane);
+  } else {
+    // column groups by the number of odd dimensions of the parity; warp & 3
+    // has 0, 1, 1 and 2 of them, its partner 3, 2, 2 and 1
+    constexpr int E = (N + 1) / 2, O = N / 2;
+    constexpr int C0 = (E * E * E + 7) / 8, C1 = (E * E * O + 7) / 8, C2 = (E * O * O + 7) / 8,
+                  C3 = (O * O * O + 7) / 8;
+    if ((warp & 3) == 0) return sym_multiply<NB, MB, true, C0, C3, G0, G0>(p, sb, warp, lane);
+    if ((warp & 3) == 3) return sym_multiply<NB, MB, true, C2, C1, G0, G0>(p, sb, warp, lane);
+    return sym_multiply<NB, MB, true, C1, C2, G0, G0>(p, sb, warp, lane);
+  }
+}
+
 // N nodes per dimension.
 template <int N, int NB, int MB>
 __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
   using S = SymShape<NB, MB>;
-  constexpr int TM = S::TM, EPT = S::EPT, KB = S::KB;
-  constexpr int kTabStage = 8 * 2 * 32 * NB;  // doubles of a stage's operator
-  extern __shared__ __align__(16) double sym_smem[];
+  constexpr int TM = S::TM, EPT = S::EPT, KB = S::KB, kTabStage = S::kTabStage;
+  extern __shared__ __align__(128) double sym_smem[];
   double* const sZ = sym_smem;                                              // [ring][2][PLANE]
-  // active orbits: (orbit | zero mask << 8 | one-sided mask << 16, stages, row groups, first stage)
+  // active orbits: (orbit | zero mask << 8 | one-sided mask << 16, stages, 0, first stage)
   int4* const sAct = reinterpret_cast<int4*>(sZ + 2 * kSymRing * S::PLANE);
   int2* const sDesc = reinterpret_cast<int2*>(sAct + kOrbits);   // [zero mask][stage] K steps
   int* const sSlot = reinterpret_cast<int*>(sDesc + 8 * kSymMaxStages);  // [orbit][8]
-  int* const sMask = sSlot + kOrbits * 8;                        // [orbit] row groups with a source
-  int* const sIl = sMask + kOrbits;                              // [slot][ILS] source row (box * R + r)
+  int* const sOn = sSlot + kOrbits * 8;                          // [orbit] it has a source
+  int* const sIl = sOn + kOrbits;                                // [slot][ILS] source row (box * R + r)
   __shared__ uint64_t s_full[kSymRing], s_empty[kSymRing];
-  __shared__ int s_nact, s_abort;
+  __shared__ int4 s_orb[kOrbits];  // sAct's entries of all orbits
+  __shared__ int s_nact, s_nst, s_abort;
   const SymGeom& g = *p.geom;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int4 tile = p.tiles[blockIdx.x];
   const int cls = tile.x, v0 = tile.y, vcnt = tile.z;
   const int R = p.R, none = p.zero_row;
   const int lo = p.part_lo[blockIdx.y], hi = p.part_lo[blockIdx.y + 1];
+  // row groups gathered (multiplied: rounded up to 1, 2, half or all)
+  const int used = (vcnt + 7) >> 3;
+  const int groups = used > MB / 2 ? MB : used;
 
-  for (int i = tid; i < TM * kSymSlots; i += kSymThreads) {
-    const int r = i / kSymSlots, q = i - r * kSymSlots;
-    int s = none;
-    if (r < vcnt) {
-      const int v = v0 + r, brow = v / R;
-      const int sb = p.il[(int64_t)brow * kSymSlots + q];
-      if (sb >= 0) s = sb * R + (v - brow * R);
+  // far slots of the rows (a warp takes TM / 16 rows, all loads in flight)
+  {
+    constexpr int RPW = TM / 16, LPR = (kSymSlots + 31) / 32;
+    int s[RPW][LPR];
+#pragma unroll
+    for (int k = 0; k < RPW; ++k) {
+      const int r = warp + 16 * k;
+      const int v = v0 + min(r, vcnt - 1), brow = v / R, rr = v - brow * R;
+      const int* row = p.il + (int64_t)brow * kSymSlots;
+#pragma unroll
+      for (int j = 0; j < LPR; ++j) {
+        const int q = lane + 32 * j;
+        const int sb = q < kSymSlots && r < vcnt ? row[q] : -1;
+        s[k][j] = sb >= 0 ? sb * R + rr : none;
+      }
     }
-    sIl[q * S::ILS + r] = s;
+    for (int i = tid; i < 8 * kSymMaxStages; i += kSymThreads)
+      sDesc[i] = make_int2((&g.desc[0][0][0])[2 * i], (&g.desc[0][0][0])[2 * i + 1]);
+    for (int i = tid; i < kOrbits * 8; i += kSymThreads) sSlot[i] = g.slot[cls][i >> 3][i & 7];
+    if (tid < kOrbits) {
+      const int z = g.zmask[tid];
+      s_orb[tid] = make_int4(tid | (z << 8) | (g.umask[tid] << 16), g.nst[z], 0, g.stage0[tid]);
+      sOn[tid] = 0;
+    }
+#pragma unroll
+    for (int k = 0; k < RPW; ++k)
+#pragma unroll
+      for (int j = 0; j < LPR; ++j)
+        if (lane + 32 * j < kSymSlots) sIl[(lane + 32 * j) * S::ILS + warp + 16 * k] = s[k][j];
   }
-  for (int i = tid; i < 8 * kSymMaxStages; i += kSymThreads)
-    sDesc[i] = make_int2((&g.desc[0][0][0])[2 * i], (&g.desc[0][0][0])[2 * i + 1]);
-  for (int i = tid; i < kOrbits * 8; i += kSymThreads) sSlot[i] = g.slot[cls][i >> 3][i & 7];
-  for (int i = tid; i < kOrbits; i += kSymThreads) sMask[i] = 0;
   if (tid == 0) {
     for (int s = 0; s < kSymRing; ++s) {
       bar_init(&s_full[s], 8);   // a lane of each gathering warp
       bar_init(&s_empty[s], 8);  // a lane of each multiplying warp
     }
     s_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
   for (int i = tid; i < (hi - lo) * MB; i += kSymThreads) {
@@ -647,28 +689,29 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
     for (int s = 0; s < 8; ++s) {
       const int q = sSlot[w * 8 + s];
       if (q < 0) continue;
+#pragma unroll
       for (int r = 0; r < 8; ++r) any |= sIl[q * S::ILS + mb * 8 + r] != none;
     }
-    if (any) atomicOr(&sMask[w], 1 << mb);
+    if (any) sOn[w] = 1;
   }
   __syncthreads();
   if (warp == 0) {
-    int base = 0;
+    int base = 0, stages = 0;
     for (int w0 = 0; w0 < kOrbits; w0 += 32) {
       const int w = w0 + lane;
-      const bool on = w < kOrbits && sMask[w] != 0;
+      const bool on = w < kOrbits && sOn[w] != 0;
       const unsigned m = __ballot_sync(0xffffffffu, on);
       if (on) {
-        const int z = g.zmask[w];
-        // a full tile's empty row groups (about 2 %) are multiplied as zeros:
-        // skipping them costs the straight-line stages more
-        const int mask = vcnt > TM - 8 ? (1 << MB) - 1 : sMask[w];
-        sAct[base + __popc(m & ((1u << lane) - 1u))] = 
-            make_int4(w | (z << 8) | (g.umask[w] << 16), g.nst[z], mask, g.stage0[w]);
+        sAct[base + __popc(m & ((1u << lane) - 1u))] = s_orb[w];
+        stages += s_orb[w].y;
       }
       base += __popc(m);
     }
-    if (lane == 0) s_nact = base;
+    stages = __reduce_add_sync(0xffffffffu, stages);
+    if (lane == 0) {
+      s_nact = base;
+      s_nst = stages;
+    }
   }
   __syncthreads();
   const int nact = s_nact;
@@ -680,15 +723,15 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
     const int grow = gt / S::TPR, gp = gt % S::TPR;
     const int gks = EPT == 2 ? gp >> 1 : gp >> 2;
     const int gk = EPT == 2 ? (gp & 1) * 2 : gp & 3;
-    const int ggrp = grow >> 3;
+    const bool mine = (grow >> 3) < groups;  // warp-uniform
     double* const zdst = sZ + gks * S::PLANE + grow * 4 + gk;
     const int neg = g.neg[cls];
-    int it = 0;
-    for (int oi = 0; oi < nact; ++oi) {
+    int slot = 0, phase = 1;
+    bool ok = true;
+    for (int oi = 0; oi < nact && ok; ++oi) {
       const int4 f = sAct[oi];
       // u: the one-sided dimensions; only the planes j with no bit of u are made
       const int z = (f.x >> 8) & 7, u = f.x >> 16, nst = f.y;
-      const bool mine = (f.z >> ggrp) & 1;  // warp-uniform, as every test of u and z
       const int* sl = sSlot + (f.x & 255) * 8;
       const int* ds = reinterpret_cast<const int*>(sDesc + z * kSymMaxStages) + gks;
       unsigned off[8];  // the orbit's sources, in units of 4 doubles
@@ -698,7 +741,7 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
         const int s = q >= 0 ? sIl[q * S::ILS + grow] : none;
         off[j] = (unsigned)s * (2u * KB) + (unsigned)((j & z) * (KB / 4));
       }
-      for (int st = 0; st < nst; ++st, ++it) {
+      for (int st = 0; st < nst; ++st) {
         double raw[8][EPT];
         if (mine) {
           const int step = max(ds[st * 2], 0);  // no step: any data, not multiplied
@@ -716,11 +759,8 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
               }
             }
         }
-        const int slot = it & (kSymRing - 1);
-        if (!bar_wait(&s_empty[slot], ((it / kSymRing) & 1) ^ 1, &s_abort)) {
-          *p.err = 1;
-          return;
-        }
+        ok = __all_sync(0xffffffffu, bar_wait(&s_empty[slot], phase, &s_abort));
+        if (!ok) break;
         if (mine) {
 #pragma unroll
           for (int q = 1; q < 8; q <<= 1)
@@ -749,29 +789,27 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
         }
         __syncwarp();
         if (lane == 0) bar_arrive(&s_full[slot]);
+        if (++slot == kSymRing) {
+          slot = 0;
+          phase ^= 1;
+        }
       }
     }
+    if (!ok) *p.err = 1;
     return;
   }
 
   // ---- multiplying warps ----
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(S::kMulRegs));
-  const SymBlock sb{sZ, sAct, sDesc, s_full, s_empty, &s_abort, p.tab + (int64_t)tile.w * g.total * kTabStage, nact,
-                    g.neg[cls], v0, vcnt};
+  const SymBlock sb{sZ,      p.tab + (int64_t)tile.w * g.total * kTabStage, sAct, sDesc, s_full, s_empty,
+                    &s_abort, nact, g.neg[cls], v0, vcnt};
+  constexpr int H = MB / 2;
   bool ok;
-  if constexpr (N % 2 == 0) {
-    constexpr int C = (N / 2 * (N / 2) * (N / 2) + 7) / 8;  // column groups of every parity
-    ok = sym_multiply<NB, MB, false, C, C>(p, sb, warp, lane);
-  } else {
-    // column groups by the number of odd dimensions of the parity; warp & 3
-    // has 0, 1, 1 and 2 of them, its partner 3, 2, 2 and 1
-    constexpr int E = (N + 1) / 2, O = N / 2;
-    constexpr int C0 = (E * E * E + 7) / 8, C1 = (E * E * O + 7) / 8, C2 = (E * O * O + 7) / 8,
-                  C3 = (O * O * O + 7) / 8;
-    if ((warp & 3) == 0) ok = sym_multiply<NB, MB, true, C0, C3>(p, sb, warp, lane);
-    else if ((warp & 3) == 3) ok = sym_multiply<NB, MB, true, C2, C1>(p, sb, warp, lane);
-    else ok = sym_multiply<NB, MB, true, C1, C2>(p, sb, warp, lane);
-  }
+  if (groups > H) ok = sym_warp<N, NB, MB, H, H>(p, sb, warp, lane);
+  else if (N % 2 == 1 && warp >= 4) ok = sym_pass(sb, s_nst, lane);
+  else if (groups > 2) ok = sym_warp<N, NB, MB, H, 0>(p, sb, warp, lane);
+  else if (groups == 2) ok = sym_warp<N, NB, MB, 2, 0>(p, sb, warp, lane);
+  else ok = sym_warp<N, NB, MB, 1, 0>(p, sb, warp, lane);
   if (!ok) *p.err = 1;
 }
 

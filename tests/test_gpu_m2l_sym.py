@@ -66,6 +66,20 @@ def test_right_hand_sides_and_unsplit_level(ctx, oracle):
         assert rel_l2(got[k], want) <= TOL
 
 
+@pytest.mark.parametrize("poly_ord", [3, 4, 6])
+@pytest.mark.parametrize("rhs", [1, 2, 3, 4, 5, 8, 9])
+def test_used_row_groups(ctx, oracle, poly_ord, rhs):
+    # all 64 boxes of level 2, 8 of every class: tiles of exactly rhs row groups of 8 (8 and 9: full and 1 more)
+    r = np.random.default_rng(20 + rhs)
+    t, s, w = r.random((900, 3)), r.random((1000, 3)), r.standard_normal((rhs, 1000))
+    ctx.set_kernel("inv_r_safe")
+    got, _ = ctx.solve(t, s, w, poly_ord=poly_ord, depth=3)
+    got = np.asarray(got).reshape(rhs, -1)
+    for k in (0, rhs - 1):
+        want, _ = oracle.fmm(3, 1, 0.0, poly_ord, 3, 1, t, s, w[k])
+        assert rel_l2(got[k], want) <= TOL
+
+
 def test_few_points(ctx, oracle):
     r = np.random.default_rng(8)
     for n in (1, 2, 9, 40):
