@@ -950,7 +950,7 @@ void solve_forest(fmma_ctx* ctx, const SolveArgs& a, const std::vector<int64_t>&
         } else if (fuse_leaf) {
           launch_l2lp_leaf(ctx, Lf, tx, nt, cubes, ddepth, d, isf, n, Kpad, dTn, dA, Wl[1], Wl[0], pt);
         } else {
-          launch_l2p_warp(ctx, Lf, tx, nt, cubes, ddepth, d, isf, n, P, Kpad, R, dTn, Wl[0], pt, 1, 0);
+          launch_l2p_warp(ctx, Lf, tx, nt, cubes, ddepth, d, isf, n, P, Kpad, R, dTn, Wl[0], pt, tr.nprob);
         }
       }
     }

@@ -111,4 +111,17 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
+// T_j(x_k) at k * N + j, passed to a kernel as constants.
+template <int N>
+struct NodeTable {
+  double T[N * N];
+};
+template <int N>
+inline NodeTable<N> node_table() {
+  const ChebTables ct = make_cheb_tables(N);
+  NodeTable<N> tn;
+  for (int i = 0; i < N * N; ++i) tn.T[i] = ct.Tn[i];
+  return tn;
+}
+
 }  // namespace fmma_b200

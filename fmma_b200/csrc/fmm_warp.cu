@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kWarpThreads, 2) k_p2m_warp(
 }
 
 // ---------------------------------------------------------------------------
-// L2P: pot[(r * nt + t) * ostride + ooff] = sum_k Wl[leaf][r][k] prod_q S_n(rel_tq, x_kq)
+// L2P: pot[r * nt + t] = sum_k Wl[leaf][r][k] prod_q S_n(rel_tq, x_kq)
 // ---------------------------------------------------------------------------
 // Staged row length of k_l2p_warp: every pass reads RB consecutive values
 // from r0 (a multiple of RB), so a row holds R rounded up to RB (and to an
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(kWarpThreads, 2) k_l2p_warp(
     const int* __restrict__ row_box, int64_t nrow, const uint64_t* __restrict__ key, const int* __restrict__ tb,
     const int* __restrict__ te, const double* __restrict__ tx, int64_t nt, const Cube* __restrict__ cubes,
     const int* __restrict__ depth, int d, int isf, int n, int P, int Kpad, int R, const double* __restrict__ Tn_g,
-    const double* __restrict__ Wl, double* __restrict__ pot, int ostride, int ooff, int wl_staged) {
+    const double* __restrict__ Wl, double* __restrict__ pot, int wl_staged) {
   __shared__ double sTn[kMaxNodes * kMaxNodes];
   // per warp: factors [q*n + j][lane], then (wl_staged) two buffers of a leaf's
   // Wl [Kpad][Rrow]: the next row's is copied (cp.async) while this one is used
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(kWarpThreads, 2) k_l2p_warp(
         if (ok) {
 #pragma unroll
           for (int j = 0; j < RB; ++j)
-            if (r0 + j < R) pot[((int64_t)(r0 + j) * nt + t) * ostride + ooff] = acc[j];
+            if (r0 + j < R) pot[(int64_t)(r0 + j) * nt + t] = acc[j];
         }
       }
     }
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kWarpThreads, (RB == 1 && KPL <= 8) ? 3 : 2) k
     const int* __restrict__ row_box, int64_t nrow, const uint64_t* __restrict__ key, const int* __restrict__ tb,
     const int* __restrict__ te, const double* __restrict__ tx, int64_t nt, const Cube* __restrict__ cubes,
     const int* __restrict__ depth, int d, int isf, int n, int P, int Kpad, int R, const double* __restrict__ Tn_g,
-    const double* __restrict__ Wl, double* __restrict__ pot, int ostride, int ooff) {
+    const double* __restrict__ Wl, double* __restrict__ pot) {
   __shared__ double sTn[kMaxNodes * kMaxNodes];
   for (int i = threadIdx.x; i < n * n; i += blockDim.x) sTn[i] = Tn_g[i];
   const double inv_n = 1.0 / n;
@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(kWarpThreads, (RB == 1 && KPL <= 8) ? 3 : 2) k
           for (int i = 0; i < KPL; ++i) part += wl[j][i] * prod[i];
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-          if (lane == j) pot[((int64_t)(r0 + j) * nt + t) * ostride + ooff] = part;
+          if (lane == j) pot[(int64_t)(r0 + j) * nt + t] = part;
         }
       }
     }
@@ -1028,22 +1028,19 @@ void launch_p2m_warp(fmma_ctx* ctx, const Level& Lf, const double* sx, int64_t n
 
 void launch_l2p_warp(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t nt, const Cube* cubes,
                      const int* depth, int d, bool isf, int n, int P, int Kpad, int R, const double* Tn,
-                     const double* Wl, double* pot, int ostride, int ooff) {
+                     const double* Wl, double* pot, int nprob) {
   FMMA_REQUIRE(d * n <= 32, "L2P: d * nodes must be <= 32");
-  // Sparse leaves (a few targets each, as in clustered sets at a uniform
-  // depth) leave most lanes of the target-per-lane kernel idle: lanes over
-  // coefficients then win.  Full leaves favour lanes over targets.
-  if (l2p_coef_lanes(Lf, nt, ctx->l2p_mode)) {
+  if (l2p_coef_lanes(Lf, nt, n, ctx->l2p_mode)) {
     switch ((Kpad + 31) / 32) {
 #define FMMA_L2P_CASE(K_)                                                                                          \
   case K_:                                                                                                        \
     if (R == 1 || K_ >= 16)                                                                                       \
       FMMA_LAUNCH(ctx, (k_l2p_coef<K_, 1>), warp_grid(ctx, Lf.nrow), kWarpThreads, 0, Lf.row_box, Lf.nrow, Lf.key, \
-                  Lf.tb, Lf.te, tx, nt, cubes, depth, d, isf ? 1 : 0, n, P, Kpad, R, Tn, Wl, pot, ostride, ooff);    \
+                  Lf.tb, Lf.te, tx, nt, cubes, depth, d, isf ? 1 : 0, n, P, Kpad, R, Tn, Wl, pot);    \
     else                                                                                                          \
       FMMA_LAUNCH(ctx, (k_l2p_coef<K_, (K_ >= 16 ? 1 : 16 / K_)>), warp_grid(ctx, Lf.nrow), kWarpThreads, 0,      \
                   Lf.row_box, Lf.nrow, Lf.key, Lf.tb, Lf.te, tx, nt, cubes, depth, d, isf ? 1 : 0, n, P, Kpad, R, Tn, \
-                  Wl, pot, ostride, ooff);                                                                        \
+                  Wl, pot);                                                                        \
     return;
       FMMA_L2P_CASE(1) FMMA_L2P_CASE(2) FMMA_L2P_CASE(3) FMMA_L2P_CASE(4) FMMA_L2P_CASE(5) FMMA_L2P_CASE(6)
       FMMA_L2P_CASE(7) FMMA_L2P_CASE(8) FMMA_L2P_CASE(9) FMMA_L2P_CASE(10) FMMA_L2P_CASE(11) FMMA_L2P_CASE(12)
@@ -1052,6 +1049,7 @@ void launch_l2p_warp(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t n
       default: break;
     }
   }
+  if (launch_l2p_mma(ctx, Lf, tx, nt, cubes, depth, d, isf, n, Kpad, R, Wl, pot, nprob)) return;
   const int staged = (int64_t)R * Kpad <= 512 ? 1 : 0;  // the leaf's Wl in shared memory
   const int rb = R >= 8 ? 8 : (R >= 4 ? 4 : (R >= 2 ? 2 : 1));
   const size_t rrow = (size_t)l2p_staged_row(R, rb);  // the kernel's staged row length
@@ -1062,7 +1060,7 @@ void launch_l2p_warp(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t n
     if (smem > 48 * 1024 && !ctx->capturing)                                                                         \
       FMMA_CHECK_CUDA(cudaFuncSetAttribute(k_l2p_warp<RB_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
     FMMA_LAUNCH(ctx, k_l2p_warp<RB_>, warp_grid(ctx, Lf.nrow), kWarpThreads, smem, Lf.row_box, Lf.nrow, Lf.key, Lf.tb,  \
-                Lf.te, tx, nt, cubes, depth, d, isf ? 1 : 0, n, P, Kpad, R, Tn, Wl, pot, ostride, ooff, staged);      \
+                Lf.te, tx, nt, cubes, depth, d, isf ? 1 : 0, n, P, Kpad, R, Tn, Wl, pot, staged);      \
     break;
     FMMA_L2P_RB(1) FMMA_L2P_RB(2) FMMA_L2P_RB(4) FMMA_L2P_RB(8)
 #undef FMMA_L2P_RB
@@ -1152,14 +1150,17 @@ void launch_l2l_warp(fmma_ctx* ctx, const Level& C, int vchild, const int* depth
   }
 }
 
-// Lanes over coefficients for the leaves: forced by mode 2, refused by mode 1,
-// else when the leaves hold fewer than 16 targets on average.
-bool l2p_coef_lanes(const Level& Lf, int64_t nt, int mode) {
-  return mode == 2 || (mode == 0 && nt < 16 * Lf.nrow);
+// Lanes over coefficients for the leaves: forced by mode 2, refused by mode 1.
+// By default not with 2 to 8 nodes, where the tensor-core L2P is as fast or
+// faster at every density measured (see l2p.cu; 1M targets in 2-D leaves of 15
+// 251 -> 108 us, 4M clustered the same), else below 16 targets a leaf, which
+// leave most lanes of the target-per-lane kernel idle.
+bool l2p_coef_lanes(const Level& Lf, int64_t nt, int n, int mode) {
+  return mode == 2 || (mode == 0 && (n < 2 || n > 8) && nt < 16 * Lf.nrow);
 }
 
 bool l2lp_leaf_ok(const Level& Lf, int64_t nt, int d, int n, int mode) {
-  if (Lf.nrow == 0 || !l2p_coef_lanes(Lf, nt, mode)) return false;  // dense leaves: the target-lane L2P
+  if (Lf.nrow == 0 || !l2p_coef_lanes(Lf, nt, n, mode)) return false;  // dense leaves: the target-lane L2P
   return (d == 3 && n >= 4 && n <= 7) || (d == 2 && n >= 4 && n <= 8);
 }
 

@@ -201,7 +201,7 @@ struct fmma_ctx {
   // 0 = tc_split) and for the context (fmma_set_schedule_options)
   std::vector<int> m2l_split;
   int tc_split = 0;
-  // leaf evaluation (L2P): 0 by the targets per leaf, 1 lanes over targets,
+  // leaf evaluation (L2P): 0 by default (l2p_coef_lanes), 1 lanes over targets,
   // 2 lanes over coefficients (with one rhs the leaf L2L fused in)
   int l2p_mode = 0;
   std::map<std::string, int> tuner;  // decisions by workload key
@@ -442,7 +442,11 @@ bool launch_p2m_tile(fmma_ctx* ctx, const Level& Lf, const double* sx, int64_t n
                      int nprob, int grid_n);
 void launch_l2p_warp(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t nt, const Cube* cubes,
                      const int* depth, int d, bool isf, int n, int P, int Kpad, int R, const double* Tn,
-                     const double* Wl, double* pot, int ostride, int ooff);
+                     const double* Wl, double* pot, int nprob);
+// L2P of 2 to 8 nodes per dimension on the FP64 tensor cores (l2p.cu); false
+// for other node counts.
+bool launch_l2p_mma(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t nt, const Cube* cubes, const int* depth,
+                    int d, bool isf, int n, int Kpad, int R, const double* Wl, double* pot, int nprob);
 void launch_m2m_warp(fmma_ctx* ctx, const Level& C, const Level& Pl, int vpar, const int* depth, int d, int n, int P,
                      int Kpad, int R, const double* A, const double* Wc, double* Wp);
 void launch_l2l_warp(fmma_ctx* ctx, const Level& C, int vchild, const int* depth, int d, int n, int P, int Kpad, int R,
@@ -450,9 +454,9 @@ void launch_l2l_warp(fmma_ctx* ctx, const Level& C, int vchild, const int* depth
 // Leaf L2L fused into L2P for one right-hand side on leaves with few targets
 // (pot[t] written for every target of the leaf rows); false when the case is
 // not covered (dense leaves, other node counts): run L2L and L2P instead.
-// mode: the context's l2p_mode (0 by the targets per leaf, 1 lanes over
+// mode: the context's l2p_mode (0 by default, 1 lanes over
 // targets, 2 lanes over coefficients)
-bool l2p_coef_lanes(const Level& Lf, int64_t nt, int mode);
+bool l2p_coef_lanes(const Level& Lf, int64_t nt, int n, int mode);
 bool l2lp_leaf_ok(const Level& Lf, int64_t nt, int d, int n, int mode);
 bool launch_l2lp_leaf(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t nt, const Cube* cubes,
                       const int* depth, int d, bool isf, int n, int Kpad, const double* Tn, const double* A,

@@ -24,11 +24,6 @@ constexpr int kTileWarps = 4;
 constexpr int kTileMaxLeaves = 32;  // leaves of a warp's run: their ranges sit in the lanes
 constexpr int kFRow = 33;           // doubles between factor rows: distinct banks for the rows of a source
 
-template <int N>
-struct NodeTable {
-  double T[N * N];  // T_j(x_k) at k * N + j
-};
-
 template <int D, int N>
 struct P2MShape {
   static constexpr int C = D == 1 ? N : N * N;        // node pairs (single nodes in 1-D)
@@ -195,16 +190,13 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_p2m_tile(
 template <int D, int N, int RB>
 void p2m_tile(fmma_ctx* ctx, const Level& Lf, const double* sx, int64_t ns, const double* ws, int R,
               const Cube* cubes, const int* depth, bool isf, int Kpad, double* Wm, int nprob, int grid_n) {
-  const ChebTables ct = make_cheb_tables(N);
-  NodeTable<N> tn;
-  for (int i = 0; i < N * N; ++i) tn.T[i] = ct.Tn[i];
   // Leaves per warp: sparse leaves share tiles of 32 sources, as long as the
   // runs fill the GPU four times (16 warps an SM)
   const int64_t want = Lf.nbox / ((int64_t)ctx->sm_count * 64);
   const int run = (int)(want < 1 ? 1 : (want > kTileMaxLeaves ? kTileMaxLeaves : want));
   const int64_t nrun = (Lf.nbox + run - 1) / run;
   FMMA_LAUNCH(ctx, (k_p2m_tile<D, N, RB>), grid_for(nrun, kTileWarps, (int64_t)ctx->sm_count * 64), 32 * kTileWarps, 0,
-              Lf.key, Lf.sb, Lf.se, Lf.nbox, run, sx, ns, ws, R, cubes, depth, isf, Kpad, tn, Wm,
+              Lf.key, Lf.sb, Lf.se, Lf.nbox, run, sx, ns, ws, R, cubes, depth, isf, Kpad, node_table<N>(), Wm,
               nprob > 1 && grid_n == 0, grid_n);
 }
 

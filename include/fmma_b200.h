@@ -269,10 +269,10 @@ fmma_status fmma_set_m2l_options(fmma_ctx* ctx, int pair, int stages,
  * splits the slot lists of levels with fewer 128-row tiles than SMs over
  * CTAs: 0 enough parts to fill the SMs (default), 1 none, 2 half as many,
  * 3 twice as many (at most 16); results move by FP32 rounding.  l2p_mode:
- * the leaf evaluation, 0 by the targets per leaf (default: lanes over
- * coefficients below 16 targets per leaf, with one rhs the leaf L2L fused
- * in), 1 lanes over targets, 2 lanes over coefficients; results move by
- * FP64 rounding.  Plans made afterwards inherit the options unless their
+ * the leaf evaluation, 0 by default lanes over targets (with 1 or more than
+ * 8 nodes per dimension lanes over coefficients below 16 targets per leaf),
+ * 1 lanes over targets, 2 lanes over coefficients (with one rhs the leaf L2L
+ * fused in); results move by FP64 rounding.  Plans made afterwards inherit the options unless their
  * autotuner (mixed precision) picks its own.                               */
 fmma_status fmma_set_schedule_options(fmma_ctx* ctx, int m2l_split, int l2p_mode);
 

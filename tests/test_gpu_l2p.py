@@ -1,0 +1,67 @@
+"""L2P on the FP64 tensor cores (l2p.cu) at the sizes where it can go wrong, through the fmm, against the oracle.
+
+Tolerance: relative L2 <= 1e-12, that of the plain FP64 parity tests: sums of at most 512 terms in another order.
+
+Every node count of the range; leaves from one target to several tiles of 32, most with remainders; right-hand sides
+around the choice between the split and the plain form and around a column group of 8; problems of different depths in
+one forest, one without expansions."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+def _solve(ctx, t, s, w, **kw):
+    ctx.set_schedule_options(l2p_mode=1)  # lanes over targets for every leaf
+    try:
+        return ctx.solve(t, s, w, **kw)[0]
+    finally:
+        ctx.set_schedule_options()
+
+
+@pytest.mark.parametrize("d,n,depth", [(1, 300, 5), (2, 900, 4), (3, 1500, 3)])
+@pytest.mark.parametrize("poly_ord", [1, 2, 3, 4, 5, 6, 7])
+def test_every_node_count(ctx, oracle, d, n, depth, poly_ord):
+    r = np.random.default_rng(10 * d + poly_ord)
+    t, s, w = r.random((n, d)) ** 2, r.random((n + 9, d)), r.standard_normal((9, n + 9))  # crowded towards the origin
+    kid = 1
+    ctx.set_kernel(kid, 0.0)
+    for nrhs in (1, 3, 9):
+        got = np.asarray(_solve(ctx, t, s, w[:nrhs], poly_ord=poly_ord, depth=depth)).reshape(nrhs, -1)
+        for k in (0, nrhs - 1):
+            want, _ = oracle.fmm(d, kid, 0.0, poly_ord, depth, 1, t, s, w[k].copy())
+            assert rel_l2(got[k], want) <= TOL
+
+
+@pytest.mark.parametrize("nrhs", [1, 2, 4, 5, 7, 8, 16, 17])
+def test_right_hand_sides(ctx, oracle, nrhs):
+    r = np.random.default_rng(nrhs)
+    t, s, w = r.random((1300, 3)), r.random((1200, 3)), r.standard_normal((nrhs, 1200))
+    ctx.set_kernel("inv_r_safe")
+    got = np.asarray(_solve(ctx, t, s, w, poly_ord=4, depth=3)).reshape(nrhs, -1)
+    for k in (0, nrhs - 1):
+        want, _ = oracle.fmm(3, 1, 0.0, 4, 3, 1, t, s, w[k].copy())
+        assert rel_l2(got[k], want) <= TOL
+
+
+@pytest.mark.parametrize("nrhs", [1, 16])
+def test_forest_with_a_problem_without_expansions(ctx, oracle, nrhs):
+    r = np.random.default_rng(3)
+    sizes, depths = [40, 1700, 3, 700], [2, 4, 3, 5]
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    t, s = r.random((off[-1], 2)), r.random((off[-1], 2))
+    w = r.standard_normal((nrhs, off[-1]))
+    ctx.set_kernel("multiquadric", 1e-2)
+    ctx.set_schedule_options(l2p_mode=1)
+    try:
+        got = np.asarray(ctx.forest_solve(t, off, s, off, w, depths, poly_ord=4)).reshape(nrhs, -1)
+    finally:
+        ctx.set_schedule_options()
+    for p, depth in enumerate(depths):
+        a, b = off[p], off[p + 1]
+        want, _ = oracle.fmm(2, 5, 1e-2, 4, depth, 1, t[a:b], s[a:b], w[nrhs - 1, a:b].copy())
+        assert rel_l2(got[nrhs - 1, a:b], want) <= TOL
