@@ -929,7 +929,7 @@ void solve_forest(fmma_ctx* ctx, const SolveArgs& a, const std::vector<int64_t>&
     for (int v = V - 2; v >= (fuse_leaf ? 1 : 0); --v) {
       const Level& C = tr.lev[(size_t)v];
       if (C.nrow == 0) continue;
-      launch_l2l_warp(ctx, C, v, ddepth, d, n, P, Kpad, R, dA, Wl[(size_t)(v + 1)], Wl[(size_t)v]);
+      launch_l2l_warp(ctx, C, tr.lev[(size_t)(v + 1)], v, ddepth, d, n, P, Kpad, R, dA, Wl[(size_t)(v + 1)], Wl[(size_t)v]);
     }
     stage_end(ctx, ST_L2L);
 

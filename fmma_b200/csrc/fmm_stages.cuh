@@ -107,6 +107,11 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool va
   int sz = valid ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(sz));
 }
+__device__ __forceinline__ void cp_async8_zfill(void* smem, const void* gmem, bool valid) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  const int sz = valid ? 8 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem), "r"(sz));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
@@ -117,10 +122,13 @@ struct NodeTable {
   double T[N * N];
 };
 template <int N>
-inline NodeTable<N> node_table() {
-  const ChebTables ct = make_cheb_tables(N);
-  NodeTable<N> tn;
-  for (int i = 0; i < N * N; ++i) tn.T[i] = ct.Tn[i];
+inline const NodeTable<N>& node_table() {
+  static const NodeTable<N> tn = [] {
+    const ChebTables ct = make_cheb_tables(N);
+    NodeTable<N> t;
+    for (int i = 0; i < N * N; ++i) t.T[i] = ct.Tn[i];
+    return t;
+  }();
   return tn;
 }
 

@@ -449,8 +449,14 @@ bool launch_l2p_mma(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t nt
                     int d, bool isf, int n, int Kpad, int R, const double* Wl, double* pot, int nprob);
 void launch_m2m_warp(fmma_ctx* ctx, const Level& C, const Level& Pl, int vpar, const int* depth, int d, int n, int P,
                      int Kpad, int R, const double* A, const double* Wc, double* Wp);
-void launch_l2l_warp(fmma_ctx* ctx, const Level& C, int vchild, const int* depth, int d, int n, int P, int Kpad, int R,
-                     const double* A, const double* Wp, double* Wc);
+void launch_l2l_warp(fmma_ctx* ctx, const Level& C, const Level& Pl, int vchild, const int* depth, int d, int n, int P,
+                     int Kpad, int R, const double* A, const double* Wp, double* Wc);
+// M2M and L2L between two levels by parent (translate.cu): 1 to 8 nodes per
+// dimension, 1 to 16 in 1-D; false for other node counts.
+bool launch_m2m_tree(fmma_ctx* ctx, const Level& C, const Level& Pl, int vpar, const int* depth, int d, int n, int Kpad,
+                     int R, const double* Wc, double* Wp);
+bool launch_l2l_tree(fmma_ctx* ctx, const Level& C, const Level& Pl, int vpar, const int* depth, int d, int n, int Kpad,
+                     int R, const double* Wp, double* Wc);
 // Leaf L2L fused into L2P for one right-hand side on leaves with few targets
 // (pot[t] written for every target of the leaf rows); false when the case is
 // not covered (dense leaves, other node counts): run L2L and L2P instead.
