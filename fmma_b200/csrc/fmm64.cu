@@ -941,12 +941,15 @@ void solve_forest(fmma_ctx* ctx, const SolveArgs& a, const std::vector<int64_t>&
       FMMA_REQUIRE(smem_l2p <= 200 * 1024, "nrhs * nodes per box too large for L2P");
       if (Lf.nrow > 0) {
         if (grad) {
-          if (smem_l2p > 48 * 1024 && !ctx->capturing)
-            FMMA_CHECK_CUDA(cudaFuncSetAttribute(k_l2p_grad_f64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem_l2p));
-          FMMA_LAUNCH(ctx, k_l2p_grad_f64, grid_for(Lf.nrow, 1, (int64_t)ctx->sm_count * 16), kL2PThreads,
-                      smem_l2p, Lf.row_box, Lf.nrow, Lf.key, Lf.tb, Lf.te, tx, nt, cubes, ddepth, d, n, P, Kpad, R,
-                      dTn, Wl[0], pt, pg);
+          // 1-D and the node counts the tensor cores' form does not take: a block a leaf
+          if (!launch_l2p_grad(ctx, Lf, tx, nt, cubes, ddepth, d, n, Kpad, R, Wl[0], pt, pg, tr.nprob)) {
+            if (smem_l2p > 48 * 1024 && !ctx->capturing)
+              FMMA_CHECK_CUDA(cudaFuncSetAttribute(k_l2p_grad_f64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)smem_l2p));
+            FMMA_LAUNCH(ctx, k_l2p_grad_f64, grid_for(Lf.nrow, 1, (int64_t)ctx->sm_count * 16), kL2PThreads,
+                        smem_l2p, Lf.row_box, Lf.nrow, Lf.key, Lf.tb, Lf.te, tx, nt, cubes, ddepth, d, n, P, Kpad, R,
+                        dTn, Wl[0], pt, pg);
+          }
         } else if (fuse_leaf) {
           launch_l2lp_leaf(ctx, Lf, tx, nt, cubes, ddepth, d, isf, n, Kpad, dTn, dA, Wl[1], Wl[0], pt);
         } else {

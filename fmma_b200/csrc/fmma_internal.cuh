@@ -447,6 +447,9 @@ void launch_l2p_warp(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t n
 // for other node counts.
 bool launch_l2p_mma(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t nt, const Cube* cubes, const int* depth,
                     int d, bool isf, int n, int Kpad, int R, const double* Wl, double* pot, int nprob);
+// Potential and gradient, 2-D and 3-D; false for other dimensions and node counts.
+bool launch_l2p_grad(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t nt, const Cube* cubes, const int* depth,
+                     int d, int n, int Kpad, int R, const double* Wl, double* pot, double* potg, int nprob);
 void launch_m2m_warp(fmma_ctx* ctx, const Level& C, const Level& Pl, int vpar, const int* depth, int d, int n, int P,
                      int Kpad, int R, const double* A, const double* Wc, double* Wp);
 void launch_l2l_warp(fmma_ctx* ctx, const Level& C, const Level& Pl, int vchild, const int* depth, int d, int n, int P,

@@ -4,7 +4,11 @@ Tolerance: relative L2 <= 1e-12, that of the plain FP64 parity tests: sums of at
 
 Every node count of the range; leaves from one target to several tiles of 32, most with remainders; right-hand sides
 around the choice between the split and the plain form and around a column group of 8; problems of different depths in
-one forest, one without expansions."""
+one forest, one without expansions.
+
+The gradient against differences of the potential, which within a leaf is a polynomial of degree below 8 plus a
+Gaussian's near field: (4 D(eps/2) - D(eps)) / 3 at eps = 1e-4 of a leaf width of 0.125 leaves (8e-4)^4 * 7^5 ~ 1e-8 of
+truncation at worst and 2^-53 / eps ~ 1e-12 of rounding: 1e-6 of the largest component."""
 import numpy as np
 import pytest
 
@@ -65,3 +69,29 @@ def test_forest_with_a_problem_without_expansions(ctx, oracle, nrhs):
         a, b = off[p], off[p + 1]
         want, _ = oracle.fmm(2, 5, 1e-2, 4, depth, 1, t[a:b], s[a:b], w[nrhs - 1, a:b].copy())
         assert rel_l2(got[nrhs - 1, a:b], want) <= TOL
+
+
+@pytest.mark.parametrize("d,depth", [(2, 4), (3, 4)])
+@pytest.mark.parametrize("poly_ord", [1, 2, 3, 4, 5, 6, 7])
+def test_gradient(ctx, d, depth, poly_ord):
+    r = np.random.default_rng(100 * d + poly_ord)
+    n = 250
+    leaf = 0.5 ** (depth - 1)
+    cells = r.integers(0, 1 << (depth - 1), (n, d)) // 2 * 2  # in every second leaf: some with several targets
+    t = (cells + r.uniform(0.2, 0.8, (n, d))) * leaf
+    s = np.concatenate([r.random((600, d)), np.zeros((1, d)), np.ones((1, d))])  # the corners hold the tree in place
+    w = r.standard_normal((2, len(s)))
+    ctx.set_kernel("gaussian", 0.3)
+    for nrhs in (1, 2):
+        kw = dict(poly_ord=poly_ord, depth=depth)
+        pot, grad = ctx.solve_grad(t, s, w[:nrhs], **kw)[:2]
+        pot, grad = np.asarray(pot).reshape(nrhs, n), np.asarray(grad).reshape(nrhs, n, d)
+
+        def at(shift):
+            return np.asarray(ctx.solve(t + shift, s, w[:nrhs], **kw)[0]).reshape(nrhs, n)
+
+        assert rel_l2(pot, at(0.0)) <= TOL
+        for q in range(d):
+            e = np.eye(d)[q]
+            d1, d2 = ((at(h * e) - at(-h * e)) / (2 * h) for h in (1e-4, 5e-5))
+            assert np.abs(grad[:, :, q] - (4 * d2 - d1) / 3).max() <= 1e-6 * np.abs(grad).max()
