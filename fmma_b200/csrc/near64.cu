@@ -10,6 +10,11 @@
 // that small problems fill the GPU too (the exact sum over source ranges, a
 // leaf's near field over the warps of a unit), with the partial sums added in
 // a fixed order.
+// Against a thread (exact) or warp (near) that walked its sources in global
+// memory with 1/r by square root and division: exact 2-D 131072^2 34.2 -> 12.9
+// ms (10 FP64 operations a pair are 9.7 ms at the pipe's 17.7e12 a second),
+// 2048^2 303 -> 57 us a call of which the kernel is 12; near field of 200k
+// points x 2 rhs in 3-D 2.08 -> 0.36 ms.
 #include <algorithm>
 #include <type_traits>
 
