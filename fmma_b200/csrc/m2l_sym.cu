@@ -816,11 +816,8 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
 template <int N, int NB, int MB>
 void launch_sym(fmma_ctx* ctx, const SymParams& p, int ntiles, int nparts) {
   constexpr size_t smem = SymShape<NB, MB>::kSmem;
-  static bool attr_set = false;
-  if (!attr_set) {
+  if (!ctx->capturing)  // the attribute is the current device's
     FMMA_CHECK_CUDA(cudaFuncSetAttribute(k_m2l_sym<N, NB, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set = true;
-  }
   FMMA_LAUNCH(ctx, (k_m2l_sym<N, NB, MB>), dim3((unsigned)ntiles, (unsigned)nparts), kSymThreads, smem, p);
 }
 
