@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kTreeThreads) k_tree_emit(const uint64_t* __re
                                                             const int* __restrict__ off, const LevelOff lo,
                                                             const LevelArrays L, int* __restrict__ perm_t,
                                                             int* __restrict__ perm_s) {
-  __shared__ int s_run[kMaxLevels + 1];                      // boxes (row V: targets) before this round
+  __shared__ int s_run[kMaxLevels + 1];                      // boxes (row V: targets) before these keys
   __shared__ int s_pre[kTreeWarps][kMaxLevels + 1];          // ... of the round before this warp
   __shared__ unsigned s_bal[kTreeWarps][kMaxLevels + 1];     // the warp's keys with t >= v
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
