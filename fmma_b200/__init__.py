@@ -169,7 +169,11 @@ class Context:
         """CUDA tensors are produced by work queued on torch's current stream;
         the context's own stream waits for that work (an event, no host
         block) before the library reads them.  Results are complete when a
-        call returns (the library synchronises its stream)."""
+        call returns (the library synchronises its stream).
+
+        The event is the context's one and the wait is for its last record,
+        so this runs under the lock that the call itself holds: between a
+        record and the call no other thread's stream may take its place."""
         if kind != _lib.MEM_DEVICE:
             return
         check(self._L.fmma_wait_stream(self._h, _torch.cuda.current_stream(self.device).cuda_stream))
@@ -229,7 +233,6 @@ class Context:
                 raise ValueError("w must be 1-D or 2-D")
         at, as_, aw = _Arr(tgt, dtype, "tgt"), _Arr(src, dtype, "src"), _Arr(w, dtype, "w")
         kind = _mem_kind(at, as_, aw)
-        self._order(kind)
         if out is None:
             shape = (nt,) if (w is None or w.ndim == 1) else (R, nt)
             if kind == _lib.MEM_DEVICE:
@@ -243,6 +246,7 @@ class Context:
         used = C.c_int(0)
         fn = self._L.fmma_solve_d if dtype == np.float64 else self._L.fmma_solve_f
         with self.lock:
+            self._order(kind)
             check(fn(self._h, d, SOLVERS[solver], int(poly_ord), int(depth), int(trans_sym),
                      PRECISIONS[precision] if isinstance(precision, str) else int(precision),
                      nt, at.ptr, ns, as_.ptr, R, aw.ptr, ao.ptr, kind, C.byref(used)))
@@ -258,7 +262,6 @@ class Context:
         R = 1 if (w is None or w.ndim == 1) else int(w.shape[0])
         at, as_, aw = _Arr(tgt, np.float64, "tgt"), _Arr(src, np.float64, "src"), _Arr(w, np.float64, "w")
         kind = _mem_kind(at, as_, aw)
-        self._order(kind)
         single = w is None or w.ndim == 1
         pshape = (nt,) if single else (R, nt)
         gshape = (nt, d) if single else (R, nt, d)
@@ -275,6 +278,7 @@ class Context:
             gp = grad.ctypes.data
         used = C.c_int(0)
         with self.lock:
+            self._order(kind)
             check(self._L.fmma_solve_grad_d(self._h, d, SOLVERS[solver], int(poly_ord), int(depth), int(trans_sym),
                                             PRECISIONS[precision] if isinstance(precision, str) else int(precision),
                                             nt, at.ptr, ns, as_.ptr, R, aw.ptr, pp, gp, kind, C.byref(used)))
@@ -287,10 +291,10 @@ class Context:
         soff = np.ascontiguousarray(soff, dtype=np.int64)
         at, as_ = _Arr(tgt, np.float64, "tgt"), _Arr(src, np.float64, "src")
         kind = _mem_kind(at, as_)
-        self._order(kind)
         nprob = len(toff) - 1
         out = np.zeros(nprob, dtype=np.int32)
         with self.lock:
+            self._order(kind)
             check(self._L.fmma_forest_depths_d(self._h, int(tgt.shape[1]), nprob, toff.ctypes.data_as(_lib._pi64),
                                                at.ptr, soff.ctypes.data_as(_lib._pi64), as_.ptr, int(leaf_cap), kind,
                                                out.ctypes.data_as(_lib._pi)))
@@ -308,7 +312,6 @@ class Context:
         R = 1 if w.ndim == 1 else int(w.shape[0])
         at, as_, aw = _Arr(tgt, np.float64, "tgt"), _Arr(src, np.float64, "src"), _Arr(w, np.float64, "w")
         kind = _mem_kind(at, as_, aw)
-        self._order(kind)
         nt = int(toff[-1])
         if out is None:
             shape = (nt,) if w.ndim == 1 else (R, nt)
@@ -319,6 +322,7 @@ class Context:
                 out = np.empty(shape)
         ao = _Arr(out, np.float64, "out")
         with self.lock:
+            self._order(kind)
             check(self._L.fmma_forest_solve_d(self._h, d, nprob, toff.ctypes.data_as(_lib._pi64), at.ptr,
                                               soff.ctypes.data_as(_lib._pi64), as_.ptr, R, aw.ptr, ao.ptr,
                                               int(poly_ord), depths.ctypes.data_as(_lib._pi), int(trans_sym),
@@ -339,7 +343,6 @@ class Context:
         d = int(tgt.shape[1])
         at, as_, aw = _Arr(tgt, np.float64, "tgt"), _Arr(src, np.float64, "src"), _Arr(w, np.float64, "w")
         kind = _mem_kind(at, as_, aw)
-        self._order(kind)
         if kind == _lib.MEM_DEVICE:
             import torch
             rows_t = torch.as_tensor(rows_a, dtype=torch.int64, device=tgt.device).contiguous()
@@ -350,6 +353,7 @@ class Context:
             out = np.empty((R, rows_t.shape[0]), dtype=np.float64)
             rp, op, nr = rows_t.ctypes.data, out.ctypes.data, int(rows_t.shape[0])
         with self.lock:
+            self._order(kind)
             check(self._L.fmma_exact_rows_d(self._h, d, nr, rp, int(tgt.shape[0]), at.ptr, int(src.shape[0]),
                                             as_.ptr, R, aw.ptr, op, kind))
         return out[0] if (w is None or w.ndim == 1) else out
@@ -365,7 +369,6 @@ class Context:
         nfunc = 1 if values.ndim == 1 else int(values.shape[0])
         av = _Arr(values, np.float64, "values")
         kind = _mem_kind(av)
-        self._order(kind)
         if kind == _lib.MEM_DEVICE:
             import torch
             out = torch.empty(tuple(values.shape), dtype=torch.float64, device=values.device)
@@ -373,6 +376,7 @@ class Context:
             out = np.empty(values.shape, dtype=np.float64)
         ao = _Arr(out, np.float64, "coef")
         with self.lock:
+            self._order(kind)
             check(self._L.fmma_cheb_fit_d(self._h, int(dim), int(nth), nfunc, av.ptr, ao.ptr, kind))
         return out
 
@@ -386,7 +390,6 @@ class Context:
         nfunc = 1 if coef.ndim == 1 else int(coef.shape[0])
         ac, ap = _Arr(coef, np.float64, "coef"), _Arr(pts, np.float64, "pts")
         kind = _mem_kind(ac, ap)
-        self._order(kind)
         npts = int(pts.shape[0])
         shape = (npts,) if coef.ndim == 1 else (nfunc, npts)
         if kind == _lib.MEM_DEVICE:
@@ -396,6 +399,7 @@ class Context:
             out = np.empty(shape, dtype=np.float64)
         ao = _Arr(out, np.float64, "out")
         with self.lock:
+            self._order(kind)
             check(self._L.fmma_cheb_eval_d(self._h, dim, int(nth), nfunc, ac.ptr, npts, ap.ptr, ao.ptr, kind))
         return out
 
@@ -431,9 +435,9 @@ class Context:
     def max_leaf_occupancy(self, tgt, src, depth):
         at, as_ = _Arr(tgt, np.float64, "tgt"), _Arr(src, np.float64, "src")
         kind = _mem_kind(at, as_)
-        self._order(kind)
         mt, ms = C.c_int64(0), C.c_int64(0)
         with self.lock:
+            self._order(kind)
             check(self._L.fmma_max_leaf_occupancy_d(self._h, int(tgt.shape[1]), depth, int(tgt.shape[0]), at.ptr,
                                                     int(src.shape[0]), as_.ptr, kind, C.byref(mt), C.byref(ms)))
         return mt.value, ms.value
@@ -484,11 +488,11 @@ class Plan:
         depths = np.ascontiguousarray(depths, dtype=np.int32)
         at, as_ = _Arr(tgt, np.float64, "tgt"), _Arr(src, np.float64, "src")
         kind = _mem_kind(at, as_)
-        ctx._order(kind)
         self._ctx = ctx
         self.nt, self.ns, self.nrhs, self.d = int(toff[-1]), int(soff[-1]), int(nrhs), int(tgt.shape[1])
         h = C.c_void_p()
         with ctx.lock:
+            ctx._order(kind)
             check(self._L.fmma_plan_create_d(ctx.handle, self.d, len(toff) - 1, toff.ctypes.data_as(_lib._pi64),
                                              at.ptr, soff.ctypes.data_as(_lib._pi64), as_.ptr, self.nrhs,
                                              int(poly_ord), depths.ctypes.data_as(_lib._pi), int(trans_sym),
@@ -506,7 +510,8 @@ class Plan:
             else:
                 out = np.empty(shape)
         ao = _Arr(out, np.float64, "out")
-        self._ctx._order(aw.kind)
+        with self._ctx.lock:
+            self._ctx._order(aw.kind)
         check(self._L.fmma_plan_execute_d(self._h, aw.ptr, ao.ptr, aw.kind))
         return out
 
