@@ -478,7 +478,9 @@ class Context:
 
 class Plan:
     """One geometry (a forest, or a single problem with toff = [0, n]), many
-    weight sets: the sweep is captured in a CUDA graph and replayed."""
+    weight sets: the sweep is captured in a CUDA graph and replayed on the
+    plan's own stream; one execute at a time (the weights' and the results'
+    buffers are the plan's)."""
 
     def __init__(self, ctx: "Context", tgt, toff, src, soff, nrhs, depths, *, poly_ord=4, trans_sym=0,
                  precision="fp64", autotune=True):
@@ -489,6 +491,7 @@ class Plan:
         at, as_ = _Arr(tgt, np.float64, "tgt"), _Arr(src, np.float64, "src")
         kind = _mem_kind(at, as_)
         self._ctx = ctx
+        self._lock = threading.RLock()
         self.nt, self.ns, self.nrhs, self.d = int(toff[-1]), int(soff[-1]), int(nrhs), int(tgt.shape[1])
         h = C.c_void_p()
         with ctx.lock:
@@ -510,9 +513,11 @@ class Plan:
             else:
                 out = np.empty(shape)
         ao = _Arr(out, np.float64, "out")
-        with self._ctx.lock:
-            self._ctx._order(aw.kind)
-        check(self._L.fmma_plan_execute_d(self._h, aw.ptr, ao.ptr, aw.kind))
+        with self._lock:
+            if aw.kind == _lib.MEM_DEVICE:
+                check(self._L.fmma_plan_wait_stream(self._h,
+                                                    _torch.cuda.current_stream(self._ctx.device).cuda_stream))
+            check(self._L.fmma_plan_execute_d(self._h, aw.ptr, ao.ptr, aw.kind))
         return out
 
     def stats(self) -> dict:

@@ -660,11 +660,7 @@ void* fmma_ctx_stream(fmma_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr
 fmma_status fmma_wait_stream(fmma_ctx* ctx, void* stream) {
   return guarded([&] {
     use_device(ctx);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (st == ctx->stream) return;
-    if (!ctx->ev_wait) FMMA_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->ev_wait, cudaEventDisableTiming));
-    FMMA_CHECK_CUDA(cudaEventRecord(ctx->ev_wait, st));
-    FMMA_CHECK_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev_wait, 0));
+    wait_for_stream(ctx, static_cast<cudaStream_t>(stream));
   });
 }
 

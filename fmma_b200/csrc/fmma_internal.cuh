@@ -156,7 +156,7 @@ struct fmma_ctx {
   void* alloc_user = nullptr;
   cudaEvent_t ev[2 * FMMA_NUM_STAGES] = {};
   bool ev_used[FMMA_NUM_STAGES] = {};
-  cudaEvent_t ev_wait = nullptr;  // fmma_wait_stream
+  cudaEvent_t ev_wait = nullptr;  // wait_for_stream
   double stage_ms[FMMA_NUM_STAGES] = {};
   int64_t launches = 0;
   fmma_b200::Tree tree;
@@ -288,6 +288,9 @@ void kernel_timer_end(fmma_ctx* ctx, double flops_per_pair, int tag);
 bool tree_fetch_pairs(fmma_ctx* ctx, void* pinned);
 void tree_take_pairs(fmma_ctx* ctx, const void* pinned);
 void tree_read_pairs(fmma_ctx* ctx);
+
+// The context's stream waits for the work queued so far on st (same device).
+void wait_for_stream(fmma_ctx* ctx, cudaStream_t st);
 
 // Stage timing with CUDA events on the context stream.
 void stage_begin(fmma_ctx* ctx, Stage s);

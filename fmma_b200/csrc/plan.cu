@@ -150,7 +150,9 @@ fmma_status fmma_plan_create_d(fmma_ctx* parent, int dim, int nprob, const int64
     FMMA_CHECK_CUDA(cudaEventCreate(&p->ev[0]));
     FMMA_CHECK_CUDA(cudaEventCreate(&p->ev[1]));
 
-    // points into the plan's memory; zero weights for the warm-up
+    // points into the plan's memory, once the work that the parent's stream
+    // waits for (fmma_wait_stream) has written them; zero weights for the warm-up
+    wait_for_stream(c, parent->stream);
     double* dt = ctx_buf_t<double>(c, "plan_tgt", (size_t)(p->nt * dim));
     double* ds = ctx_buf_t<double>(c, "plan_src", (size_t)(p->ns * dim));
     const cudaMemcpyKind kind = mem_kind == FMMA_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
@@ -280,6 +282,14 @@ fmma_status fmma_plan_create_d(fmma_ctx* parent, int dim, int nprob, const int64
     delete p;
   }
   return st;
+}
+
+fmma_status fmma_plan_wait_stream(fmma_plan* p, void* stream) {
+  return guarded_plan([&] {
+    FMMA_REQUIRE(p, "null plan");
+    FMMA_CHECK_CUDA(cudaSetDevice(p->ctx->device));
+    wait_for_stream(p->ctx, static_cast<cudaStream_t>(stream));
+  });
 }
 
 fmma_status fmma_plan_execute_d(fmma_plan* p, const double* w, double* ans, int mem_kind) {

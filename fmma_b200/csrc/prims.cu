@@ -76,6 +76,13 @@ void* ctx_pinned(fmma_ctx* ctx, size_t bytes) {
   return ctx->pinned;
 }
 
+void wait_for_stream(fmma_ctx* ctx, cudaStream_t st) {
+  if (st == ctx->stream) return;
+  if (!ctx->ev_wait) FMMA_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->ev_wait, cudaEventDisableTiming));
+  FMMA_CHECK_CUDA(cudaEventRecord(ctx->ev_wait, st));
+  FMMA_CHECK_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev_wait, 0));
+}
+
 void upload(fmma_ctx* ctx, void* dst, const void* src, size_t bytes) {
   if (ctx->capturing || bytes == 0) return;
   if (ctx->up_used + bytes > ctx->up_cap) {

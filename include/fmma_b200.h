@@ -186,6 +186,9 @@ fmma_status fmma_plan_create_d(fmma_ctx* parent, int dim, int nprob,
                                int nrhs, int poly_ord, const int* depths,
                                int trans_sym, int precision, int autotune,
                                int mem_kind, fmma_plan** out);
+/* fmma_wait_stream for the plan, which runs on a stream of its own: before an
+ * execute whose device buffers another stream fills.                       */
+fmma_status fmma_plan_wait_stream(fmma_plan* plan, void* stream);
 fmma_status fmma_plan_execute_d(fmma_plan* plan, const double* w, double* ans,
                                 int mem_kind);
 /* Build time, last execution time (ms, CUDA events), levels run on each M2L

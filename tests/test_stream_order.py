@@ -76,6 +76,59 @@ def test_wait_and_call_are_made_under_the_lock(fake, entry):
     assert all(held for name, _, held, _ in fake._L.calls if name in ("fmma_wait_stream", entry))
 
 
+def test_plan_waits_on_its_own_stream(fake, monkeypatch):
+    # a replay copies the weights on the plan's stream: the wait has to be that stream's, under the plan's lock
+    plan = fake.plan(T, OFF, S, OFF, 1, [3])
+    plan._h = ctypes.c_void_p(22)
+
+    class DeviceView(fmma_b200._Arr):
+        def __init__(self, *a):
+            super().__init__(*a)
+            self.kind = fmma_b200._lib.MEM_DEVICE
+    monkeypatch.setattr(fmma_b200, "_Arr", DeviceView)
+    fake._L.calls.clear()
+    held = []
+    fake._L.on_call = lambda name: held.append(plan._lock._is_owned())
+    plan.execute(W, torch.empty(6, dtype=torch.float64))
+    assert [(name, h.value) for name, h, _, _ in fake._L.calls] == [("fmma_plan_wait_stream", 22),
+                                                                   ("fmma_plan_execute_d", 22)]
+    assert held == [True, True]
+    plan._h = ctypes.c_void_p(0)
+
+
+@pytest.mark.gpu
+def test_device_buffers_written_late_are_waited_for():
+    # points, then weights, appear on torch's stream only after a pause in front of their copies
+    r = np.random.default_rng(1)
+    t, s = (torch.from_numpy(r.random((4000, 3))) for _ in range(2))
+    w1, w2 = (torch.from_numpy(r.standard_normal(4000)) for _ in range(2))
+    ctx = fmma_b200.Context()
+    ctx.set_kernel("inv_r_safe")
+    off = [0, 4000]
+    plan = ctx.plan(t.cuda(), off, s.cuda(), off, 1, [4])
+    want = [plan.execute(w.cuda()).cpu() for w in (w1, w2)]
+    plan.close()
+    td, sd, wd = (x.pin_memory().cuda() * 0 for x in (t, s, w1))
+    torch.cuda.synchronize()
+
+    def late(dst, src):
+        torch.cuda._sleep(40_000_000)  # about 20 ms of SM clocks
+        dst.copy_(src.pin_memory(), non_blocking=True)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        late(td, t)
+        sd.copy_(s.pin_memory(), non_blocking=True)
+        plan = ctx.plan(td, off, sd, off, 1, [4])
+        for w, ref in ((w1, want[0]), (w2, want[1])):
+            late(wd, w)
+            assert torch.equal(plan.execute(wd).cpu(), ref)
+        late(wd, w1)
+        a = ctx.solve(td, sd, wd, poly_ord=4, depth=4)[0].cpu()
+        late(wd, w2)
+        b = ctx.solve(td, sd, wd, poly_ord=4, depth=4)[0].cpu()
+    plan.close()
+    assert torch.equal(a, want[0]) and torch.equal(b, want[1])
+
+
 def test_other_threads_wait_stays_outside(fake):
     # the first thread stops inside its wait until the second one has had time to make its own
     inside, second = threading.Event(), threading.Event()
