@@ -145,9 +145,10 @@ class Context:
             check(self._L.fmma_set_schedule_options(self._h, int(m2l_split), int(l2p_mode)))
 
     def debug_m2l_wait(self, wait_cycles=0, hold_issuer=False):
-        """Test hook: the tensor-core M2L's wait bound in SM clocks (0: the
-        default, ~2 s) and a hold of its MMA issuer on a flag that nothing
-        sets, so the bound runs out and the solve raises status 5 (timeout)."""
+        """Test hook: the M2L kernels' wait bound in SM clocks (0: the default,
+        ~2 s) and a hold (of the MMA issuer on a flag that nothing sets; in
+        the FP64 kernel of the stages' reports), so the bound runs out and the
+        solve raises status 5 (timeout)."""
         with self.lock:
             check(self._L.fmma_debug_m2l_wait(self._h, int(wait_cycles), 1 if hold_issuer else 0))
 

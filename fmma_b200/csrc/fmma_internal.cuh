@@ -175,8 +175,8 @@ struct fmma_ctx {
   double m2l_kernel_ms = 0.0, m2l_flops = 0.0;
   int64_t m2l_launches = 0;
   std::vector<int*> m2l_err_flags;  // device flags of bounded waits, checked at the end
-  // bound of the tensor-core M2L's pipeline waits in SM clocks (0: ~2 s) and
-  // the test hook that makes its MMA issuer wait for a flag nothing sets
+  // bound of the M2L kernels' pipeline waits in SM clocks (0: ~2 s) and
+  // the test hook that makes them run out (fmma_debug_m2l_wait)
   long long tc_wait_cycles = 0;
   bool tc_hold = false;
   // tensor-core M2L options (fmma_set_m2l_options): the 2-SM kernel on levels

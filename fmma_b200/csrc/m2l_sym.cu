@@ -60,7 +60,7 @@ namespace {
 constexpr int kOrbits = 56;       // |o| in {0..3}^3 without {0,1}^3
 constexpr int kSymThreads = 512;  // 8 multiplying warps, 8 gathering warps
 constexpr int kSymRing = 4;       // stages of z in shared memory
-constexpr long long kSymWaitCycles = 4000000000ll;  // bound of a pipeline wait (~2 s)
+constexpr long long kSymWaitCycles = 4000000000ll;  // default bound of a pipeline wait (~2 s)
 constexpr int kSymMaxStages = 64; // stages of one orbit: 8 blocks of up to 16 K steps, two per stage
 constexpr int kSymSlots = 189;
 
@@ -352,6 +352,8 @@ struct SymParams {
   int R, Kpad;
   int zero_row;        // the row of zeros of W
   int* err;            // set when a bounded wait gives up
+  long long wait_cycles;  // the bound
+  int hold;            // test hook: the gathering warps never report a stage
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -380,19 +382,24 @@ __device__ __forceinline__ bool bar_test(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: false when the bound passes or another warp has given up.
-__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
-  if (bar_try(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (true) {
-    for (int i = 0; i < 32; ++i)
-      if (bar_try(bar, parity)) return true;
-    if (*abort) return false;
-    if (clock64() - t0 > kSymWaitCycles) {
-      *abort = 1;
-      return false;
+// Bounded wait of a whole warp: false, for all its lanes, when the bound passes
+// or another warp has given up.  The vote is what keeps the warp together: the
+// lanes poll on their own, and what follows (DMMAs, votes, shuffles) needs all
+// of them, or none where the wait failed.
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort, long long limit) {
+  bool ok = bar_try(bar, parity);
+  if (!ok) {
+    const long long t0 = clock64();
+    while (true) {
+      for (int i = 0; i < 32 && !ok; ++i) ok = bar_try(bar, parity);
+      if (ok || *abort) break;
+      if (clock64() - t0 > limit) {
+        *abort = 1;
+        break;
+      }
     }
   }
+  return __all_sync(0xffffffffu, ok);
 }
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
@@ -424,6 +431,7 @@ struct SymBlock {
   const int2* desc;    // K steps by zero mask and stage
   uint64_t *full, *empty;
   int* abort;
+  long long limit;     // bound of a wait
   int nact, neg, v0, vcnt;
 };
 
@@ -537,7 +545,7 @@ __device__ __forceinline__ bool sym_multiply(const SymParams& p, const SymBlock&
     const bool more = advance();  // nxt: the stage behind this one
     const int nslot = slot + 1 == kSymRing ? 0 : slot + 1, nphase = slot + 1 == kSymRing ? phase ^ 1 : phase;
     if (!ready) {
-      if (!bar_wait(&sb.full[slot], phase, sb.abort)) return false;
+      if (!bar_wait(&sb.full[slot], phase, sb.abort, sb.limit)) return false;
       load_a(av[0], cur, slot, 0, 0);
     }
     const bool two = cur.s1 >= 0;  // the last stage of an orbit may have one K step
@@ -598,7 +606,7 @@ __device__ __forceinline__ bool sym_multiply(const SymParams& p, const SymBlock&
 // the stages as they come.
 __device__ __forceinline__ bool sym_pass(const SymBlock& sb, int nstages, int lane) {
   for (int it = 0, slot = 0, phase = 0; it < nstages; ++it) {
-    if (!bar_wait(&sb.full[slot], phase, sb.abort)) return false;
+    if (!bar_wait(&sb.full[slot], phase, sb.abort, sb.limit)) return false;
     __syncwarp();
     if (lane == 0) bar_arrive(&sb.empty[slot]);
     if (++slot == kSymRing) {
@@ -768,7 +776,7 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
               }
             }
         }
-        ok = __all_sync(0xffffffffu, bar_wait(&s_empty[slot], phase, &s_abort));
+        ok = bar_wait(&s_empty[slot], phase, &s_abort, p.wait_cycles);
         if (!ok) break;
         if (mine) {
 #pragma unroll
@@ -797,7 +805,7 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
             }
         }
         __syncwarp();
-        if (lane == 0) bar_arrive(&s_full[slot]);
+        if (lane == 0 && !p.hold) bar_arrive(&s_full[slot]);
         if (++slot == kSymRing) {
           slot = 0;
           phase ^= 1;
@@ -811,7 +819,7 @@ __global__ void __launch_bounds__(kSymThreads, 1) k_m2l_sym(const SymParams p) {
   // ---- multiplying warps ----
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(S::kMulRegs));
   const SymBlock sb{sZ,      p.tab + (int64_t)tile.w * g.total * kTabStage, sAct, sDesc, s_full, s_empty,
-                    &s_abort, nact, g.neg[cls], v0, vcnt};
+                    &s_abort, p.wait_cycles, nact, g.neg[cls], v0, vcnt};
   constexpr int H = MB / 2;
   bool ok;
   if (groups > H) ok = sym_warp<N, NB, MB, H, H>(p, sb, warp, lane);
@@ -912,7 +920,8 @@ void m2l_level_sym(fmma_ctx* ctx, const Level& Lv, int v, int n, int Kpad, int R
   double* part = nparts > 1 ? ctx_buf_t<double>(ctx, "sym_part", (size_t)nparts * nv * g.P) : nullptr;
   int* err = m2l_err_slot(ctx, v);
   FMMA_CHECK_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
-  SymParams p{dt, Lv.il, Lv.row_box, dg, W, tab, dlo, Wl, part, nv, R, Kpad, (int)nsrc, err};
+  SymParams p{dt, Lv.il, Lv.row_box, dg, W, tab, dlo, Wl, part, nv, R, Kpad, (int)nsrc, err,
+              ctx->tc_wait_cycles > 0 ? ctx->tc_wait_cycles : kSymWaitCycles, ctx->tc_hold ? 1 : 0};
   kernel_timer_begin(ctx);
   const int64_t wcap = (int64_t)ctx->sm_count * 32;
   FMMA_LAUNCH(ctx, k_sym_fold, grid_for((nsrc + 1) * 32, 256, wcap), 256, 0, Wm, nsrc, Kpad, dg, W);

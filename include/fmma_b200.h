@@ -280,13 +280,15 @@ fmma_status fmma_set_m2l_options(fmma_ctx* ctx, int pair, int stages,
 fmma_status fmma_set_schedule_options(fmma_ctx* ctx, int m2l_split, int l2p_mode);
 
 /* ---- failure detection (tests) ------------------------------------------
- * Every pipeline wait of the tensor-core M2L is bounded; a wait that gives
- * up makes the solve return FMMA_ERR_TIMEOUT after the kernel has drained
- * (no copy or MMA left in flight, TMEM freed), and the context stays usable.
+ * Every pipeline wait of the tensor-core M2L and of the FP64 M2L on the
+ * reflection symmetry is bounded; a wait that gives up makes the solve return
+ * FMMA_ERR_TIMEOUT after the kernel has drained (no copy or MMA left in
+ * flight, TMEM freed), and the context stays usable.
  * No counterpart in the reference (no device code).  This hook sets the
  * bound to wait_cycles SM clocks (<= 0: the default, about 2 s) and, with
  * hold_issuer != 0, makes the MMA-issuing thread first wait for a device
- * flag that nothing sets, so that the bound runs out on purpose.           */
+ * flag that nothing sets (in the FP64 kernel: the gathering warps never report
+ * a stage), so that the bound runs out on purpose.                         */
 fmma_status fmma_debug_m2l_wait(fmma_ctx* ctx, long long wait_cycles,
                                 int hold_issuer);
 

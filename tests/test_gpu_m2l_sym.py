@@ -115,3 +115,27 @@ def test_plan_replay_is_the_solve(ctx):
     np.testing.assert_array_equal(plan.execute(w), want)
     np.testing.assert_array_equal(plan.execute(w), want)
     plan.close()
+
+
+@pytest.mark.parametrize("poly_ord,depth", [(3, 4), (4, 4), (4, 3), (6, 3)])
+def test_wait_that_gives_up_reports_and_context_recovers(poly_ord, depth):
+    """The gathering warps never report a stage and the waits are bounded at 2e6 SM clocks (~1 ms): the multiplying
+    warps' first wait gives up, both sides leave, the solve raises status 5 (timeout), and the same context then
+    solves bit for bit as before.  Even and odd node counts, full tiles and tiles whose upper half has no rows."""
+    import fmma_b200
+    r = np.random.default_rng(poly_ord)
+    t, s, w = r.random((2000, 3)), r.random((2100, 3)), r.standard_normal(2100)
+    c = fmma_b200.Context(0)
+    try:
+        c.set_kernel("inv_r_safe")
+        ref, _ = c.solve(t, s, w, poly_ord=poly_ord, depth=depth)
+        c.debug_m2l_wait(2_000_000, hold_issuer=True)
+        with pytest.raises(fmma_b200.FmmaError) as e:
+            c.solve(t, s, w, poly_ord=poly_ord, depth=depth)
+        assert e.value.status == 5, e.value
+        c.debug_m2l_wait(200_000_000)  # a bound that nothing runs into
+        out, _ = c.solve(t, s, w, poly_ord=poly_ord, depth=depth)
+        np.testing.assert_array_equal(out, ref)
+    finally:
+        c.debug_m2l_wait()
+        c.close()
