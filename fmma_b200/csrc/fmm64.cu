@@ -564,8 +564,9 @@ constexpr int kM2PMaxFar = 192;
 
 // TPB threads per block: 256, or 64 on levels whose boxes hold few targets
 // (most of a wide block would idle there).
-template <int KID, int D, int RB, int TPB>
-__global__ void __launch_bounds__(TPB, (RB == 1 ? 640 : 512) / TPB) k_m2p_f64(
+// ROW: far sums by rows of nodes (m2p.cuh).
+template <int KID, int D, int RB, int TPB, bool ROW>
+__global__ void __launch_bounds__(TPB, (RB > 1 ? 512 : ROW ? 640 : 768) / TPB) k_m2p_f64(
     const int* __restrict__ row_box, int64_t nrow, const int* __restrict__ il, int nfar,
     const uint64_t* __restrict__ key, const int* __restrict__ tb, const int* __restrict__ te, int v,
     const int* __restrict__ depth, const Cube* __restrict__ cubes, const double* __restrict__ tx, int64_t nt,
@@ -640,8 +641,11 @@ __global__ void __launch_bounds__(TPB, (RB == 1 ? 640 : 512) / TPB) k_m2p_f64(
           sX[i] = (node_all[k * D + q] + 1.0) / 2.0 * len + corner;
         }
         __syncthreads();
-        if (tv && !far_batch<KID, D, RB>(x, sX, sW, nb, n, P, p0, ip, acc, [](int) { return false; }))
+        if constexpr (ROW) {
+          if (tv) far_batch<KID, D, RB>(x, sX, sW, nb, n, P, p0, ip, acc, [](int) { return false; });
+        } else if (tv) {
           for (int j = 0; j < nb; ++j) far_box_sum<KID, D, RB>(x, sX + j * D * n, sW + j * RB * P, n, P, p0, acc);
+        }
       }
       if (tv) {
 #pragma unroll
@@ -652,7 +656,7 @@ __global__ void __launch_bounds__(TPB, (RB == 1 ? 640 : 512) / TPB) k_m2p_f64(
   }
 }
 
-template <int KID, int D, int RB, int TPB>
+template <int KID, int D, int RB, int TPB, bool ROW>
 static void m2p_launch(fmma_ctx* ctx, const Level& Lv, int v, int nfar, const int* depth, const Cube* cubes,
                        const double* tx, int64_t nt, const double* node_all, int n, int P, int Kpad, int R, double p0,
                        const double* Wm, double* pot) {
@@ -666,20 +670,31 @@ static void m2p_launch(fmma_ctx* ctx, const Level& Lv, int v, int nfar, const in
   int64_t gy = ((int64_t)ctx->sm_count * 4 + gx - 1) / gx;
   gy = std::max<int64_t>(1, std::min<int64_t>(gy, 64));
   for (int r0 = 0; r0 < R; r0 += RB)
-    FMMA_LAUNCH(ctx, (k_m2p_f64<KID, D, RB, TPB>), dim3((unsigned)gx, (unsigned)gy), TPB, smem, Lv.row_box,
+    FMMA_LAUNCH(ctx, (k_m2p_f64<KID, D, RB, TPB, ROW>), dim3((unsigned)gx, (unsigned)gy), TPB, smem, Lv.row_box,
                 Lv.nrow, Lv.il, nfar, Lv.key, Lv.tb, Lv.te, v, depth, cubes, tx, nt, node_all, n, P, Kpad, R, r0, NB,
                 p0, Wm, pot);
+}
+
+template <int KID, int D, int RB, bool ROW>
+static void m2p_tpb(fmma_ctx* ctx, const Level& Lv, int v, int nfar, const int* depth, const Cube* cubes,
+                   const double* tx, int64_t nt, const double* node_all, int n, int P, int Kpad, int R, double p0,
+                   const double* Wm, double* pot) {
+  // every target lies in one box of each level: nt / rows is the mean occupancy
+  if (nt < 128 * Lv.nrow)
+    m2p_launch<KID, D, RB, 64, ROW>(ctx, Lv, v, nfar, depth, cubes, tx, nt, node_all, n, P, Kpad, R, p0, Wm, pot);
+  else
+    m2p_launch<KID, D, RB, 256, ROW>(ctx, Lv, v, nfar, depth, cubes, tx, nt, node_all, n, P, Kpad, R, p0, Wm, pot);
 }
 
 template <int KID, int D, int RB>
 static void m2p_rb(fmma_ctx* ctx, const Level& Lv, int v, int nfar, const int* depth, const Cube* cubes,
                    const double* tx, int64_t nt, const double* node_all, int n, int P, int Kpad, int R, double p0,
                    const double* Wm, double* pot) {
-  // every target lies in one box of each level: nt / rows is the mean occupancy
-  if (nt < 128 * Lv.nrow)
-    m2p_launch<KID, D, RB, 64>(ctx, Lv, v, nfar, depth, cubes, tx, nt, node_all, n, P, Kpad, R, p0, Wm, pot);
-  else
-    m2p_launch<KID, D, RB, 256>(ctx, Lv, v, nfar, depth, cubes, tx, nt, node_all, n, P, Kpad, R, p0, Wm, pot);
+  if constexpr (far_row_kernel<KID, RB>()) {
+    if (far_row_nodes(n))
+      return m2p_tpb<KID, D, RB, true>(ctx, Lv, v, nfar, depth, cubes, tx, nt, node_all, n, P, Kpad, R, p0, Wm, pot);
+  }
+  m2p_tpb<KID, D, RB, false>(ctx, Lv, v, nfar, depth, cubes, tx, nt, node_all, n, P, Kpad, R, p0, Wm, pot);
 }
 
 struct M2PLaunch {

@@ -84,25 +84,53 @@ __device__ __forceinline__ void far_box_row(const double* x, const double* __res
   }
 }
 
+// Kernels and right-hand sides that far_box_row is made for, and the node
+// counts.  The kernels that hold it (ROW) are compiled apart from those of the
+// general loop, which needs fewer registers and more warps: in one kernel the
+// loop ran at the rows' 16 warps an SM (nrnmm, 2-D, 10 nodes, 100k points:
+// 1/r 12.87 ms against 11.41 at 24, Gaussian 31.99 against 30.75).
+template <int KID, int RB>
+constexpr bool far_row_kernel() {
+  return RB == 1 && (KID == FMMA_KERNEL_INV_R || KID == FMMA_KERNEL_INV_R_SAFE || KID == FMMA_KERNEL_LOG_R ||
+                     KID == FMMA_KERNEL_GAUSSIAN || KID == FMMA_KERNEL_MULTIQUADRIC);
+}
+inline bool far_row_nodes(int n) { return n >= 2 && n <= 8; }
+
 // far_box_row for the boxes j < nb of a staged batch that `skip(j)` lets
-// through; false when the kernel or the node count is not covered.
+// through, for n in far_row_nodes.
 template <int KID, int D, int RB, typename Skip>
-__device__ __forceinline__ bool far_batch(const double* x, const double* X, const double* W, int nb, int n, int P,
+__device__ __forceinline__ void far_batch(const double* x, const double* X, const double* W, int nb, int n, int P,
                                           double p0, double ip, double* acc, const Skip& skip) {
-  if constexpr (RB != 1 || (KID != FMMA_KERNEL_INV_R && KID != FMMA_KERNEL_INV_R_SAFE && KID != FMMA_KERNEL_LOG_R &&
-                            KID != FMMA_KERNEL_GAUSSIAN && KID != FMMA_KERNEL_MULTIQUADRIC)) {
-    return false;
-  } else {
 #define FMMA_FAR_N(N_)                                                                                         \
   case N_:                                                                                                     \
     for (int j = 0; j < nb; ++j)                                                                               \
       if (!skip(j)) far_box_row<KID, D, RB, N_>(x, X + j * D * N_, W + (size_t)j * RB * P, P, p0, ip, acc);    \
-    return true;
-    switch (n) {
-      FMMA_FAR_N(2) FMMA_FAR_N(3) FMMA_FAR_N(4) FMMA_FAR_N(5) FMMA_FAR_N(6) FMMA_FAR_N(7) FMMA_FAR_N(8)
-      default: return false;
-    }
+    break;
+  switch (n) {
+    FMMA_FAR_N(2) FMMA_FAR_N(3) FMMA_FAR_N(4) FMMA_FAR_N(5) FMMA_FAR_N(6) FMMA_FAR_N(7) FMMA_FAR_N(8)
+    default: break;
+  }
 #undef FMMA_FAR_N
+}
+
+// Kernel value of the general loop below: 1/r through rsqrt(), whose operands
+// outside the normal range cost no branch of their own; with one pair at a time
+// that beats inv_sqrt's fewer operations behind a check (nrnmm, 2-D, 10 nodes
+// 1.61 against 1.93 ms; 3-D, 6 nodes x 3 rhs 7.92 against 8.77; tree, 3-D, 6
+// nodes x 3 rhs 24.4 against 25.8).
+template <int KID, int D>
+__device__ __forceinline__ double kfar(const double* x, const double* y, double p0) {
+  if constexpr (KID == FMMA_KERNEL_INV_R || KID == FMMA_KERNEL_INV_R_SAFE) {
+    double r2 = 0.0;
+#pragma unroll
+    for (int q = 0; q < D; ++q) {
+      const double t = x[q] - y[q];
+      r2 += t * t;
+    }
+    if constexpr (KID == FMMA_KERNEL_INV_R_SAFE) return r2 > 0.0 ? rsqrt(r2) : 0.0;
+    return rsqrt(r2);
+  } else {
+    return keval<KID, D>(x, y, p0);
   }
 }
 
@@ -114,7 +142,7 @@ __device__ __forceinline__ void far_box_sum(const double* x, const double* __res
 #pragma unroll 4
     for (int o0 = 0; o0 < n; ++o0) {
       y[0] = X[o0];
-      const double f = keval<KID, D>(x, y, p0);
+      const double f = kfar<KID, D>(x, y, p0);
 #pragma unroll
       for (int rr = 0; rr < RB; ++rr) acc[rr] += f * W[rr * P + o0];
     }
@@ -125,7 +153,7 @@ __device__ __forceinline__ void far_box_sum(const double* x, const double* __res
 #pragma unroll 4
       for (int o1 = 0; o1 < n; ++o1) {
         y[1] = X[n + o1];
-        const double f = keval<KID, D>(x, y, p0);
+        const double f = kfar<KID, D>(x, y, p0);
 #pragma unroll
         for (int rr = 0; rr < RB; ++rr) acc[rr] += f * Wk[rr * P + o1];
       }
@@ -139,7 +167,7 @@ __device__ __forceinline__ void far_box_sum(const double* x, const double* __res
 #pragma unroll 4
         for (int o2 = 0; o2 < n; ++o2) {
           y[2] = X[2 * n + o2];
-          const double f = keval<KID, D>(x, y, p0);
+          const double f = kfar<KID, D>(x, y, p0);
 #pragma unroll
           for (int rr = 0; rr < RB; ++rr) acc[rr] += f * Wk[rr * P + o2];
         }

@@ -118,8 +118,9 @@ __host__ __device__ inline int far_box_bytes(int D, int RB, int P, int n) {
 
 // part[y][r][t] for r in [r0, r0 + RB): the far sum of sorted target t over
 // the y-th slice of the source-box list.
-template <int KID, int D, int RB>
-__global__ void __launch_bounds__(kFarThreads, 2) k_nrn_far(
+// ROW: far sums by rows of nodes (m2p.cuh).
+template <int KID, int D, int RB, bool ROW>
+__global__ void __launch_bounds__(kFarThreads, RB == 1 && !ROW ? 3 : 2) k_nrn_far(
     const double* __restrict__ tx, int64_t nt, const uint64_t* __restrict__ tkey, const int* __restrict__ sbox,
     const int* __restrict__ nsbox, int N, int n, int P, int Kpad, int R, int r0, int NB,
     const double* __restrict__ gx, const double* __restrict__ Wm, double p0, double* __restrict__ part) {
@@ -171,9 +172,12 @@ __global__ void __launch_bounds__(kFarThreads, 2) k_nrn_far(
       for (int q = 0; q < D; ++q) in = in && abs(sB[j * D + q] - bi[q]) <= 1;
       return in;
     };
-    if (far_batch<KID, D, RB>(x, sX, sW, nb, n, P, p0, ip, acc, near)) continue;
-    for (int j = 0; j < nb; ++j)
-      if (!near(j)) far_box_sum<KID, D, RB>(x, sX + j * D * n, sW + j * RB * P, n, P, p0, acc);
+    if constexpr (ROW) {
+      far_batch<KID, D, RB>(x, sX, sW, nb, n, P, p0, ip, acc, near);
+    } else {
+      for (int j = 0; j < nb; ++j)
+        if (!near(j)) far_box_sum<KID, D, RB>(x, sX + j * D * n, sW + j * RB * P, n, P, p0, acc);
+    }
   }
   if (tv) {
 #pragma unroll
@@ -194,16 +198,31 @@ struct FarArgs {
   double* part;
 };
 
-template <int KID, int D, int RB>
-void far_rb(fmma_ctx* ctx, const FarArgs& f, double p0) {
+template <int KID, int D, int RB, bool ROW>
+void far_launch(fmma_ctx* ctx, const FarArgs& f, double p0) {
   const int per_box = far_box_bytes(D, RB, f.P, f.n);
   int NB = kFarSmem / per_box;
   NB = NB < 1 ? 1 : (NB > kFarMaxBatch ? kFarMaxBatch : NB);
   const size_t smem = (size_t)NB * per_box + 16;
   const dim3 grid((unsigned)((f.nt + kFarThreads - 1) / kFarThreads), (unsigned)f.nsplit);
   for (int r0 = 0; r0 < f.R; r0 += RB)
-    FMMA_LAUNCH(ctx, (k_nrn_far<KID, D, RB>), grid, kFarThreads, smem, f.tx, f.nt, f.tkey, f.sbox, f.nsbox, f.N, f.n,
+    FMMA_LAUNCH(ctx, (k_nrn_far<KID, D, RB, ROW>), grid, kFarThreads, smem, f.tx, f.nt, f.tkey, f.sbox, f.nsbox, f.N, f.n,
                 f.P, f.Kpad, f.R, r0, NB, f.gx, f.Wm, p0, f.part);
+}
+
+// By rows of nodes, except log r and the multiquadric in 3-D: bound by the
+// latency of log and square root, they gain nothing from fewer operations and
+// lose by 16 warps an SM instead of 24 (20,000 and 60,000 points, 6 nodes: log r
+// 18.8 against 19.0 and 66.0 against 67.1 ms, multiquadric 7.4 against 7.9 and
+// 25.5 against 26.3; 1/r 6.0 -> 3.7 and 20.4 -> 12.4 by rows, the Gaussian 14.7
+// -> 8.8 and 51.3 -> 30.5).
+template <int KID, int D, int RB>
+void far_rb(fmma_ctx* ctx, const FarArgs& f, double p0) {
+  constexpr bool kSlow = D == 3 && (KID == FMMA_KERNEL_LOG_R || KID == FMMA_KERNEL_MULTIQUADRIC);
+  if constexpr (far_row_kernel<KID, RB>() && !kSlow) {
+    if (far_row_nodes(f.n)) return far_launch<KID, D, RB, true>(ctx, f, p0);
+  }
+  far_launch<KID, D, RB, false>(ctx, f, p0);
 }
 
 struct FarLaunch {

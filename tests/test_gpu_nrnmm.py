@@ -112,3 +112,20 @@ def test_nrnmm_large_linearity_and_error(ctx):
     rows = r.choice(n, 2000, replace=False)
     ex = ctx.exact_rows(rows, t, s, w1)
     assert rel_l2(a1[rows], ex) <= 1e-5
+
+
+# far sums by rows of nodes (radial kernels, one rhs, 2 to 8 nodes; in 3-D not log r and the multiquadric) and by the
+# general loop: every kernel on both sides of the rule's edges; the same sums in another order, so 1e-12 as above
+@pytest.mark.parametrize("kid,p0", [(0, 0.0), (1, 0.0), (3, 0.0), (4, 0.05), (5, 1e-2), (7, 0.0)])
+@pytest.mark.parametrize("d,po,rhs", [(3, 0, 1), (3, 1, 1), (3, 2, 1), (3, 5, 1), (3, 5, 2), (3, 7, 1), (2, 7, 1),
+                                      (2, 8, 1), (2, 9, 3), (1, 7, 1), (1, 8, 1)])
+@pytest.mark.parametrize("solver", ["nrnmm", "tree"])
+def test_far_sums_by_rows_and_by_the_general_loop(ctx, oracle, solver, kid, p0, d, po, rhs):
+    r = np.random.default_rng(31 * d + po)
+    n = 600 if d == 3 and po == 7 else 1500
+    t, s, w = r.random((n, d)), r.random((n - 100, d)), r.standard_normal((rhs, n - 100))
+    grid = {"nrnmm": {1: 32, 2: 8, 3: 4}, "tree": {1: 6, 2: 4, 3: 3}}[solver][d]
+    ctx.set_kernel(kid, p0)
+    got, _ = ctx.solve(t, s, w, solver=solver, poly_ord=po, depth=grid)
+    want, _ = (oracle.nrnmm if solver == "nrnmm" else oracle.tree)(d, kid, p0, po, grid, t, s, w[rhs - 1])
+    assert rel_l2(got[rhs - 1], want) <= 1e-12
