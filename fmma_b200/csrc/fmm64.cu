@@ -270,11 +270,8 @@ static void launch_m2l_f64_t(fmma_ctx* ctx, const int4* tiles, int ntiles, int n
                              int NpadT, int nfar, int R, int noff) {
   constexpr int NW = 32 * NBW;
   size_t smem = sizeof(double) * (size_t)kM2LST * (kM2LTM + NW) * kM2LLDS;
-  static bool attr_set = false;
-  if (!attr_set) {
+  if (!ctx->capturing)  // the attribute is the current device's
     FMMA_CHECK_CUDA(cudaFuncSetAttribute(k_m2l_f64<NBW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set = true;
-  }
   dim3 grid((unsigned)ntiles, (unsigned)ny);
   FMMA_LAUNCH(ctx, k_m2l_f64<NBW>, grid, 256, smem, tiles, il, row_box, slot_off, Wm, Wl, tab, P, Kpad, NpadT,
               nfar, R, noff);

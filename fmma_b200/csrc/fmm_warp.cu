@@ -854,11 +854,8 @@ static void p2m_warp_t(fmma_ctx* ctx, const Level& Lf, const double* sx, int64_t
                 ns, ws, R, cubes, depth, d, isf ? 1 : 0, n, P, Kpad, Tn, Wm, grid_n);
   } else if constexpr (RBM > 1) {
     const size_t smem = sizeof(double) * 2 * kP2MBuf<RBM> * kWarpsPerBlock;
-    static bool attr = false;
-    if (smem > 48 * 1024 && !attr && !ctx->capturing) {
+    if (smem > 48 * 1024 && !ctx->capturing)  // the attribute is the current device's
       FMMA_CHECK_CUDA(cudaFuncSetAttribute(k_p2m_warp<KPL, RBM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      attr = true;
-    }
     FMMA_LAUNCH(ctx, (k_p2m_warp<KPL, RBM>), warp_grid(ctx, Lf.nbox), kWarpThreads, smem, Lf.key, Lf.sb, Lf.se,
                 Lf.nbox, sx, ns, ws, R, cubes, depth, d, isf ? 1 : 0, n, P, Kpad, Tn, Wm, grid_n);
   }

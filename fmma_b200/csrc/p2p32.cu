@@ -627,12 +627,9 @@ struct P2P32Launch {
 #define FMMA_P2P32_RB(RB_)                                                                                         \
   case RB_: {                                                                                                     \
     const size_t smem = p2p_warp_bytes(D, RB_) * 8;                                                              \
-    static bool attr = false;                                                                                     \
-    if (smem > 48 * 1024 && !attr && !ctx->capturing) {                                                           \
+    if (smem > 48 * 1024 && !ctx->capturing)  /* the attribute is the current device's */                         \
       FMMA_CHECK_CUDA(cudaFuncSetAttribute(k_p2p_f32<KID, D, RB_, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
                                            (int)smem));                                                           \
-      attr = true;                                                                                                \
-    }                                                                                                             \
     FMMA_LAUNCH(ctx, (k_p2p_f32<KID, D, RB_, T>), g, 256, smem, tr.near_row_box, tr.nnear_rows, tr.near, nnear,    \
                 Lf.key, Lf.tb, Lf.te, Lf.sb, Lf.se, txl, tr.nt, sxl, tr.ns, wst, R, Rp, p0, tr.d_depth, tr.d_cube, \
                 pot, tr.perm_t, out);                                                                             \
