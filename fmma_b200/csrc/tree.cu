@@ -18,12 +18,8 @@ namespace fmma_b200 {
 // ---------------------------------------------------------------------------
 // far-slot tables
 // ---------------------------------------------------------------------------
-static FarTables g_far[kMaxDim + 1];
-static bool g_far_init[kMaxDim + 1] = {false, false, false, false};
-
-const FarTables& far_tables(int d) {
-  FarTables& F = g_far[d];
-  if (g_far_init[d]) return F;
+static FarTables make_far_tables(int d) {
+  FarTables F;
   std::memset(&F, 0, sizeof(F));
   int p7 = 1, p6 = 1, p3 = 1;
   for (int q = 0; q < d; ++q) { p7 *= 7; p6 *= 6; p3 *= 3; }
@@ -63,8 +59,12 @@ const FarTables& far_tables(int d) {
       ++k;
     }
   }
-  g_far_init[d] = true;
   return F;
+}
+
+const FarTables& far_tables(int d) {  // made once, by whichever thread comes first
+  static const FarTables F[kMaxDim] = {make_far_tables(1), make_far_tables(2), make_far_tables(3)};
+  return F[d - 1];
 }
 
 // ---------------------------------------------------------------------------
