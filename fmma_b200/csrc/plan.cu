@@ -53,12 +53,18 @@ fmma_status guarded_plan(F&& f) {
   }
 }
 
+// The number in front is that of the kernels the decisions were timed with; it
+// goes up when an engine or a leaf layout becomes another kernel, so that
+// decisions saved before are made again.  The kernel of interaction is in the
+// key because engine 0 is k_m2l_sym for radial ones in 3-D and k_m2l_f64, 4 to 5
+// times slower there, for the others.
 std::string tuner_key(const SolveArgs& a, int v, const Level& Lv) {
   // rows rounded to a power of two: one decision per size class
   int64_t b = 1;
   while (b < Lv.nrow) b <<= 1;
   char buf[160];
-  std::snprintf(buf, sizeof(buf), "m2l4_d%d_P%d_R%d_prec%d_rows%lld", a.dim, a.P, a.nrhs, a.precision, (long long)b);
+  std::snprintf(buf, sizeof(buf), "m2l5_k%d_d%d_P%d_R%d_prec%d_rows%lld", a.kernel_id, a.dim, a.P, a.nrhs, a.precision,
+                (long long)b);
   (void)v;
   return buf;
 }
@@ -69,7 +75,7 @@ std::string tuner_key_l2p(const SolveArgs& a, int64_t nt, const Level& leaf) {
   int64_t b = 1;
   while (b * (leaf.nrow > 0 ? leaf.nrow : 1) < nt) b <<= 1;
   char buf[160];
-  std::snprintf(buf, sizeof(buf), "l2p1_d%d_P%d_R%d_prec%d_tpr%lld", a.dim, a.P, a.nrhs, a.precision, (long long)b);
+  std::snprintf(buf, sizeof(buf), "l2p2_d%d_P%d_R%d_prec%d_tpr%lld", a.dim, a.P, a.nrhs, a.precision, (long long)b);
   return buf;
 }
 

@@ -67,3 +67,32 @@ def test_schedule_options_rejected_out_of_range(own_ctx):
         own_ctx.set_schedule_options(m2l_split=4)
     with pytest.raises(RuntimeError):
         own_ctx.set_schedule_options(l2p_mode=-1)
+
+
+def test_tuner_decisions_are_of_this_build_and_kernel(tmp_path):
+    """A plan takes no decision that was timed with other kernels: not those an older build saved (engine 0 and leaf
+    layout 1 were other kernels then), and not those of a radial kernel for one that is not (engine 0 is the symmetric
+    M2L for the one and the M2L by offsets for the other)."""
+    import fmma_b200
+    r = np.random.default_rng(3)
+    t, s = r.random((2000, 3)), r.random((2000, 3))
+    path = tmp_path / "tuner.txt"
+    sizes = [1 << k for k in range(1, 14)]
+    path.write_text("".join(f"{pre}m2l4_d3_P27_R1_prec2_rows{b} 3\n" for b in sizes for pre in ("", "split_")) +
+                    "".join(f"l2p1_d3_P27_R1_prec2_tpr{b} 2\n" for b in sizes))
+    old = set(path.read_text().split("\n")) - {""}
+    ctx = fmma_b200.Context(0)
+    try:
+        ctx.set_tuner_cache(str(path))
+        seen = old
+        for kernel in ("inv_r_safe", "sum_over_r2"):
+            ctx.set_kernel(kernel)
+            ctx.plan(t, [0, 2000], s, [0, 2000], 1, [4], poly_ord=2, precision="bf16x3").close()
+            now = set(path.read_text().split("\n")) - {""}
+            new = now - seen
+            assert seen <= now
+            assert sum(x.startswith("m2l") for x in new) == 2, (kernel, new)  # levels 2 and 3
+            seen = now
+        assert any(x.startswith("l2p") for x in seen - old)
+    finally:
+        ctx.close()
