@@ -197,8 +197,8 @@ __device__ __forceinline__ void butterfly8(double* v) {
 // Operators in the parity basis, one warp per (table, orbit, i, j) with i, j
 // half-indices: the 64 values of f over the reversals of i and j (two per
 // lane), transformed along both by shuffles, give the entry (i, j) of all 64
-// blocks.  The factor 1/64 holds the halves of the inverse transforms on both
-// sides (exact).
+// blocks.  The halves of the inverse transforms on both sides, 1/64 in all, are
+// in the folded sources.
 template <int KID>
 __global__ void __launch_bounds__(256) k_sym_table(const double* __restrict__ lens, int ntab,
                                                    const double* __restrict__ node_all,
@@ -250,13 +250,16 @@ __global__ void __launch_bounds__(256) k_sym_table(const double* __restrict__ le
       const int col = I.in_block(a, he, ho);
       const int l = (col & 7) * 4 + (k & 3), nb = col >> 3;  // lane and column group of the fragment
       const int64_t at = ((int64_t)a * 2 + (step & 1)) * (32 * NB) + (NB == 1 ? l : (nb >> 1) * 64 + l * 2 + (nb & 1));
-      base[at] = v[u] * (1.0 / 64);
+      base[at] = v[u];
     }
   }
 }
 
-// out[row][b][KB]: the even and odd parts of Wm's rows (box x rhs), zero padded,
-// and a row of zeros behind them (the source of an empty slot).
+// out[row][b][KB]: the even and odd parts of Wm's rows (box x rhs) by 1/64, zero
+// padded, and a row of zeros behind them (the source of an empty slot).  The
+// factor is exact, and taken here it keeps the sums of up to 64 coefficients,
+// in the fold and in the butterfly, within the largest of them: no weight
+// overflows that did not in the sum offset by offset.
 __global__ void __launch_bounds__(256) k_sym_fold(const double* __restrict__ Wm, int64_t nrows, int Kpad,
                                                   const SymGeom* __restrict__ gp, double* __restrict__ out) {
   const int n = gp->n, he = gp->he, ho = gp->ho, KB = gp->KB;
@@ -273,7 +276,7 @@ __global__ void __launch_bounds__(256) k_sym_fold(const double* __restrict__ Wm,
       const Half H(h, he, ho);
       double v[8];
 #pragma unroll
-      for (int s = 0; s < 8; ++s) v[s] = (s & H.mid) ? 0.0 : w[H.node(s, n)];
+      for (int s = 0; s < 8; ++s) v[s] = (s & H.mid) ? 0.0 : w[H.node(s, n)] * (1.0 / 64);
       butterfly8(v);
 #pragma unroll
       for (int b = 0; b < 8; ++b)
@@ -286,7 +289,7 @@ __global__ void __launch_bounds__(256) k_sym_fold(const double* __restrict__ Wm,
 }
 
 // Wl rows from their parity blocks: the nparts partial sums in order, then the
-// inverse transform (its halves are in the operators).  With one part the
+// inverse transform (its halves are in the folded sources).  With one part the
 // blocks lie in Wl itself and a warp turns a row in place.
 // Latency bound: a part's loads are all in flight before its sums (coefficient
 // by coefficient over the parts 437, 351 and 67 us in the three cases above,

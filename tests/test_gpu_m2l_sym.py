@@ -139,3 +139,20 @@ def test_wait_that_gives_up_reports_and_context_recovers(poly_ord, depth):
     finally:
         c.debug_m2l_wait()
         c.close()
+
+
+@pytest.mark.parametrize("poly_ord", [3, 4, 5, 7])
+@pytest.mark.parametrize("power", [1023, -900])
+def test_weights_of_any_size(ctx, poly_ord, power):
+    # A power of two in the weights is one in the result, bit for bit, up to where the sums offset by offset would
+    # overflow: one source near the centre of each of the 64 boxes, weights up to 2^1023 of one sign, 1/r below 2^-9.
+    r = np.random.default_rng(poly_ord)
+    grid = np.stack(np.meshgrid(*[np.arange(4.0)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    s = 1024.0 * (grid + 0.5 + r.uniform(-0.1, 0.1, (64, 3)))
+    s = np.concatenate([s, [[0.0] * 3, [4096.0] * 3]])  # the cube; weightless
+    w = np.concatenate([r.uniform(0.6, 1.0, 64), [0.0, 0.0]])
+    t = 4096.0 * r.random((900, 3))
+    ctx.set_kernel("inv_r_safe")
+    base, _ = ctx.solve(t, s, w, poly_ord=poly_ord, depth=3)
+    got, _ = ctx.solve(t, s, np.ldexp(w, power), poly_ord=poly_ord, depth=3)
+    np.testing.assert_array_equal(got, np.ldexp(base, power))
