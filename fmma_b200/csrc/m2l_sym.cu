@@ -194,11 +194,54 @@ __device__ __forceinline__ void butterfly8(double* v) {
       }
 }
 
+// s + e = a + b exactly (Knuth).
+__device__ __forceinline__ void two_sum(double a, double b, double& s, double& e) {
+  const double t = __dadd_rn(a, b), bb = __dsub_rn(t, a);
+  e = __dadd_rn(__dsub_rn(a, __dsub_rn(t, bb)), __dsub_rn(b, bb));
+  s = t;
+}
+
+// f + c = the kernel at |x - y|^2 = r2 + rl, c the rounding error of f and of r2.
+template <int KID>
+__device__ __forceinline__ void sym_value(double r2, double rl, double p0, double& f, double& c) {
+  switch (KID) {
+    case FMMA_KERNEL_LOG_R:
+      f = 0.5 * log(r2);
+      c = 0.5 * rl / r2;
+      break;
+    case FMMA_KERNEL_GAUSSIAN: {
+      const double a = r2 / p0;
+      f = exp(-a);
+      c = -f * ((fma(-a, p0, r2) + rl) / p0);
+      break;
+    }
+    case FMMA_KERNEL_MULTIQUADRIC: {
+      double h, e;
+      two_sum(r2, p0, h, e);
+      f = sqrt(h);
+      c = (fma(-f, f, h) + e + rl) / (2.0 * f);
+      break;
+    }
+    default: {  // 1/r: f (1 + (1 - f^2 r^2) / 2)
+      f = 1.0 / sqrt(r2);
+      const double p = f * f, pe = fma(f, f, -p);
+      c = 0.5 * f * (fma(-p, r2, 1.0) - pe * r2 - p * rl);
+      break;
+    }
+  }
+}
+
 // Operators in the parity basis, one warp per (table, orbit, i, j) with i, j
 // half-indices: the 64 values of f over the reversals of i and j (two per
 // lane), transformed along both by shuffles, give the entry (i, j) of all 64
 // blocks.  The halves of the inverse transforms on both sides, 1/64 in all, are
-// in the folded sources.
+// in the folded sources.  Value, argument and the sums of 64 carry their
+// rounding errors along, so that an entry is rounded once (34 -> 54 us a level
+// at 6 nodes, once a geometry).  What that is for is the narrow Gaussian, whose
+// value takes the argument's error r^2/p0 times over: error of the M2L against
+// long double, p0 = 0.01 in the unit cube, over that of k_m2l_f64, 4 nodes 1.13
+// -> 0.16, 6 nodes 0.58 -> 0.20; over 3 to 8 nodes, four kernels and all levels
+// the median is 0.29 -> 0.25 (the sums are 39.5/189 as long).
 template <int KID>
 __global__ void __launch_bounds__(256) k_sym_table(const double* __restrict__ lens, int ntab,
                                                    const double* __restrict__ node_all,
@@ -214,27 +257,40 @@ __global__ void __launch_bounds__(256) k_sym_table(const double* __restrict__ le
     const int64_t t = e / ((int64_t)nh * nh * kOrbits);
     const double len = lens[t];
     const Half I(hi, he, ho), J(hj, he, ho);
-    double v[2];  // index = row reversal * 8 + column reversal = lane + 32 u
+    double v[2], c[2];  // value and its error; index = row reversal * 8 + column reversal = lane + 32 u
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int kl = I.node((lane >> 3) + 4 * u, n), km = J.node(lane & 7, n);
-      double x[3], y[3];
+      double r2 = 0.0, rl = 0.0;
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        x[q] = len * (node_all[kl * 3 + q] / 2);
-        y[q] = len * ((double)g.rep[w][q] + node_all[km * 3 + q] / 2);
+      for (int q = 0; q < 3; ++q) {  // len (x_k / 2 - (o + x_m / 2))
+        double a, al, t, tl, e;
+        two_sum(node_all[kl * 3 + q] / 2, -node_all[km * 3 + q] / 2, a, al);
+        two_sum(a, -(double)g.rep[w][q], t, tl);
+        const double p = len * t, pl = fma(len, t, -p) + len * (tl + al);
+        const double s = p * p;
+        rl += fma(p, p, -s) + 2.0 * p * pl;
+        two_sum(r2, s, r2, e);
+        rl += e;
       }
-      v[u] = keval<KID, 3>(x, y, p0);
+      two_sum(r2, rl, r2, rl);
+      sym_value<KID>(r2, rl, p0, v[u], c[u]);
     }
-    const double s = v[0] + v[1], d = v[0] - v[1];
-    v[0] = s;
-    v[1] = d;
+    double s, d, es, ed;
+    two_sum(v[0], v[1], s, es);
+    two_sum(v[0], -v[1], d, ed);
+    es += c[0] + c[1];
+    ed += c[0] - c[1];
+    v[0] = s, c[0] = es;
+    v[1] = d, c[1] = ed;
 #pragma unroll
     for (int q = 1; q < 32; q <<= 1)
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const double o = __shfl_xor_sync(0xffffffffu, v[u], q);
-        v[u] = (lane & q) ? o - v[u] : v[u] + o;
+        const double o = __shfl_xor_sync(0xffffffffu, v[u], q), oc = __shfl_xor_sync(0xffffffffu, c[u], q);
+        const bool up = lane & q;
+        two_sum(up ? -v[u] : v[u], o, v[u], s);
+        c[u] = (up ? oc - c[u] : c[u] + oc) + s;
       }
     const int z = g.zmask[w], b = lane & 7, b0 = b & ~z;
     if (b & J.mid) continue;
@@ -250,7 +306,7 @@ __global__ void __launch_bounds__(256) k_sym_table(const double* __restrict__ le
       const int col = I.in_block(a, he, ho);
       const int l = (col & 7) * 4 + (k & 3), nb = col >> 3;  // lane and column group of the fragment
       const int64_t at = ((int64_t)a * 2 + (step & 1)) * (32 * NB) + (NB == 1 ? l : (nb >> 1) * 64 + l * 2 + (nb & 1));
-      base[at] = v[u];
+      base[at] = v[u] + c[u];
     }
   }
 }

@@ -156,3 +156,51 @@ def test_weights_of_any_size(ctx, poly_ord, power):
     base, _ = ctx.solve(t, s, w, poly_ord=poly_ord, depth=3)
     got, _ = ctx.solve(t, s, np.ldexp(w, power), poly_ord=poly_ord, depth=3)
     np.testing.assert_array_equal(got, np.ldexp(base, power))
+
+
+@pytest.mark.parametrize("poly_ord", [2, 3, 4, 7])
+def test_operators_of_a_narrow_gaussian(ctx, poly_ord):
+    """The far field of a Gaussian whose exponent is some hundreds at the far boxes, against the same sum in extended
+    precision: P2M, M2L and L2P with the double nodes, in long double.  Only far pairs count here (targets left,
+    sources right), positive weights.  Plain double arithmetic in the exponent alone is off by about 300 * 2^-53 =
+    3e-14 in every term; what is left otherwise is the rounding of P2M, L2P (4 (n - 1) + 4 steps a factor, three
+    factors) and of the M2L's sums, 64 * 2^-53 of the terms' absolute sum, which is kappa (2 to 3) times the result.
+    Node counts whose nodes nearest to the far box are exactly symmetric, as the symmetry assumes; the others carry
+    the nodes' own rounding."""
+    LD, n, p0 = np.longdouble, poly_ord + 1, 3e-4
+    r = np.random.default_rng(poly_ord)
+    t, s = r.random((60, 3)) * [0.2, 0.99, 0.99], r.random((70, 3)) * [0.2, 0.99, 0.99] + [0.55, 0.0, 0.0]
+    s = np.concatenate([s, [[0.0, 0.0, 0.0], [1.0, 1.0, 1.0]]])  # the unit cube; weightless
+    w = np.concatenate([r.uniform(0.5, 1.0, 70), [0.0, 0.0]])
+    ctx.set_kernel("gaussian", p0)
+    got, _ = ctx.solve(t, s, w, poly_ord=poly_ord, depth=3)
+
+    import math
+    node = np.array([math.cos((2.0 * k + 1.0) / (2 * n) * math.pi) for k in range(n)])
+
+    def factors(y):  # S_n(node, y), T_j by the recurrence
+        T = [np.ones_like(y), y]
+        X = [np.ones(n, LD), node.astype(LD)]
+        for _ in range(2, n):
+            T.append(2 * y * T[-1] - T[-2])
+            X.append(2 * node.astype(LD) * X[-1] - X[-2])
+        return LD(1) / n + LD(2) / n * sum(np.multiply.outer(T[j], X[j]) for j in range(1, n))
+
+    def boxes(p):
+        i = np.minimum((p * 4).astype(int), 3)
+        f = [factors(2 * (p[:, q].astype(LD) * 4 - i[:, q]) - 1) for q in range(3)]
+        return i, np.einsum("pi,pj,pk->pijk", *f).reshape(len(p), n ** 3)
+    ti, tf = boxes(t)
+    si, sf = boxes(s)
+    half = np.stack(np.meshgrid(*[node.astype(LD) / 2] * 3, indexing="ij"), -1).reshape(-1, 3)
+    want, terms = np.zeros(len(t), LD), np.zeros(len(t), LD)
+    for b in {tuple(x) for x in si[:70]}:
+        wb = (w * (si == b).all(1)).astype(LD)
+        for a in {tuple(x) for x in ti}:
+            d = (half[:, None] - (half[None] + np.subtract(b, a))) / 4
+            here = (ti == a).all(1)
+            K = np.exp(-(d * d).sum(-1) / LD(p0))
+            want[here] += tf[here] @ (K @ (wb @ sf))
+            terms[here] += abs(tf[here]) @ (K @ (wb @ abs(sf)))
+    err, scale = (np.linalg.norm(x.astype(float)) for x in (got - want, terms))
+    assert err <= 64 * 2.0 ** -53 * scale, err / scale
