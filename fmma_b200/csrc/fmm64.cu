@@ -841,7 +841,22 @@ void solve_forest(fmma_ctx* ctx, const SolveArgs& a, const std::vector<int64_t>&
       }
       stage_end(ctx, ST_M2L);
     } else {
-    // M2L on every level with rows (src/fmm_core.cpp:375-495)
+    // M2L on every level with rows (src/fmm_core.cpp:375-495).  Engine of a
+    // level (the plan autotuner's; -1: the context's options): the tensor
+    // cores' unless 0 or in plain precision; in FP64 on the grid's symmetry
+    // where that covers the case and its scratch can be had.
+    auto engine_of = [&](int v) { return (size_t)v < ctx->m2l_engine.size() ? ctx->m2l_engine[(size_t)v] : -1; };
+    auto tensor_level = [&](int v) { return a.precision != FMMA_PREC_FP64 && engine_of(v) != 0; };
+    std::vector<char> sym((size_t)V, 0);
+    std::vector<const Level*> sym_levels;
+    for (int v = 0; v < V; ++v) {
+      const Level& Lv = tr.lev[(size_t)v];
+      if (Lv.nrow == 0 || pairwise || tensor_level(v) || !m2l_sym_ok(ctx, d, n, Lv.nbox * R)) continue;
+      sym[(size_t)v] = 1;
+      sym_levels.push_back(&Lv);
+    }
+    int sym_parts = 1;
+    if (!sym_levels.empty() && !m2l_sym_scratch(ctx, sym_levels, n, R, &sym_parts)) sym.assign((size_t)V, 0);
     stage_begin(ctx, ST_M2L);
     for (int v = 0; v < V; ++v) {
       const Level& Lv = tr.lev[(size_t)v];
@@ -885,10 +900,10 @@ void solve_forest(fmma_ctx* ctx, const SolveArgs& a, const std::vector<int64_t>&
       }
       const std::string tkey = op_key("m2l64", ctx, d, n, ntab == 1 ? lens[0] : (double)hash_doubles(lens), Npad, Kp) +
                                "_t" + std::to_string(ntab);
-      const int engine = (size_t)v < ctx->m2l_engine.size() ? ctx->m2l_engine[(size_t)v] : -1;
-      const bool tensor = a.precision != FMMA_PREC_FP64 && engine != 0;
-      if (!tensor && m2l_sym_ok(ctx, d, n, Lv.nbox * R)) {
-        m2l_level_sym(ctx, Lv, v, n, Kpad, R, lens, tkey, node_all, Wm[(size_t)v], Wl[(size_t)v]);
+      const int engine = engine_of(v);
+      const bool tensor = tensor_level(v);
+      if (sym[(size_t)v]) {
+        m2l_level_sym(ctx, Lv, v, n, Kpad, R, lens, tkey, node_all, Wm[(size_t)v], Wl[(size_t)v], sym_parts);
         continue;
       }
       bool fresh = false;

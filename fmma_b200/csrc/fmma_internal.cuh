@@ -247,6 +247,9 @@ template <typename T>
 T* ctx_buf_t(fmma_ctx* ctx, const std::string& name, size_t count) {
   return static_cast<T*>(ctx_buf(ctx, name, count * sizeof(T) + 16));
 }
+// The same for scratch that a call can do without: null when the allocator
+// refuses, or where a captured sweep finds less than it needs.
+void* ctx_buf_try(fmma_ctx* ctx, const std::string& name, size_t bytes);
 // Pinned host scratch (readback of small results).
 void* ctx_pinned(fmma_ctx* ctx, size_t bytes);
 // Host -> device copy of constant data of a sweep; skipped while a sweep is

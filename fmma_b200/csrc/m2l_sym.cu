@@ -910,7 +910,44 @@ struct SymTableLaunch {
 
 constexpr int kSymMaxParts = 16;
 
+// The orbits of a tile are split over blocks where that fills the last wave
+// of a level: a block costs its share of a tile plus about 2 % of one (the
+// prologue and the partial sums), and one block runs on an SM at a time.
+int sym_parts(const fmma_ctx* ctx, int64_t ntiles, int most) {
+  int nparts = 1;
+  double best = 0.0;
+  for (int s = 1; s <= most; ++s) {
+    const int64_t waves = (ntiles * s + ctx->sm_count - 1) / ctx->sm_count;
+    const double t = (double)waves * (1.0 / s + 0.02);
+    if (s == 1 || t < best) {
+      best = t;
+      nparts = s;
+    }
+  }
+  return nparts;
+}
+
+size_t sym_src_bytes(const Level& Lv, const SymGeom& g, int R) {
+  return sizeof(double) * (size_t)(Lv.nbox * R + 1) * 8 * g.KB;
+}
+
 }  // namespace
+
+bool m2l_sym_scratch(fmma_ctx* ctx, const std::vector<const Level*>& levels, int n, int R, int* most_parts) {
+  const SymGeom& g = sym_geom(n);
+  const int TM = 8 * g.MB;
+  size_t src = 0, part = 0;
+  for (const Level* Lv : levels) {
+    int64_t ntiles = 0;  // as m2l_tiles cuts the segments
+    for (const int4& sg : Lv->segs) ntiles += ((int64_t)(sg.w - sg.z) * R + TM - 1) / TM;
+    const int nparts = sym_parts(ctx, ntiles, kSymMaxParts);
+    src = std::max(src, sym_src_bytes(*Lv, g, R));
+    if (nparts > 1) part = std::max(part, sizeof(double) * (size_t)(nparts * Lv->nrow * R) * g.P);
+  }
+  if (!ctx_buf_try(ctx, "sym_src", src)) return false;
+  *most_parts = part == 0 || ctx_buf_try(ctx, "sym_part", part) ? kSymMaxParts : 1;
+  return true;
+}
 
 bool m2l_sym_ok(const fmma_ctx* ctx, int d, int n, int64_t rows) {
   // source rows are addressed in units of 4 doubles, in 32 bits
@@ -926,7 +963,7 @@ bool m2l_sym_ok(const fmma_ctx* ctx, int d, int n, int64_t rows) {
 }
 
 void m2l_level_sym(fmma_ctx* ctx, const Level& Lv, int v, int n, int Kpad, int R, const std::vector<double>& lens,
-                   const std::string& tabkey, const double* node_all, const double* Wm, double* Wl) {
+                   const std::string& tabkey, const double* node_all, const double* Wm, double* Wl, int most_parts) {
   const SymGeom& g = sym_geom(n);
   const int ntab = (int)lens.size();
   // geometry and operators in one cached block
@@ -952,19 +989,7 @@ void m2l_level_sym(fmma_ctx* ctx, const Level& Lv, int v, int n, int Kpad, int R
   int4* dt = ctx_buf_t<int4>(ctx, "m2l_tiles" + std::to_string(v), tiles.size());
   upload(ctx, dt, tiles.data(), sizeof(int4) * tiles.size());
 
-  // The orbits of a tile are split over blocks where that fills the last wave
-  // of a level: a block costs its share of a tile plus about 2 % of one (the
-  // prologue and the partial sums), and one block runs on an SM at a time.
-  int nparts = 1;
-  double best = 0.0;
-  for (int s = 1; s <= kSymMaxParts; ++s) {
-    const int64_t waves = ((int64_t)ntiles * s + ctx->sm_count - 1) / ctx->sm_count;
-    const double t = (double)waves * (1.0 / s + 0.02);
-    if (s == 1 || t < best) {
-      best = t;
-      nparts = s;
-    }
-  }
+  const int nparts = sym_parts(ctx, ntiles, most_parts);
   std::vector<int> lo((size_t)nparts + 1, 0);
   for (int s = 1, w = 0; s < nparts; ++s) {
     while (w < kOrbits && (int64_t)g.stage0[w] * nparts < (int64_t)s * g.total) ++w;
@@ -975,8 +1000,9 @@ void m2l_level_sym(fmma_ctx* ctx, const Level& Lv, int v, int n, int Kpad, int R
   upload(ctx, dlo, lo.data(), sizeof(int) * lo.size());
 
   const int64_t nv = Lv.nrow * R, nsrc = Lv.nbox * R;
-  double* W = ctx_buf_t<double>(ctx, "sym_src", (size_t)(nsrc + 1) * 8 * g.KB);
-  double* part = nparts > 1 ? ctx_buf_t<double>(ctx, "sym_part", (size_t)nparts * nv * g.P) : nullptr;
+  double* W = static_cast<double*>(ctx_buf(ctx, "sym_src", sym_src_bytes(Lv, g, R)));
+  double* part = nullptr;
+  if (nparts > 1) part = static_cast<double*>(ctx_buf(ctx, "sym_part", sizeof(double) * (size_t)(nparts * nv) * g.P));
   int* err = m2l_err_slot(ctx, v);
   FMMA_CHECK_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
   SymParams p{dt, Lv.il, Lv.row_box, dg, W, tab, dlo, Wl, part, nv, R, Kpad, (int)nsrc, err,

@@ -405,18 +405,22 @@ struct ExactLaunch {
         best_t = t;
       }
     }
-    const int64_t range = (ns + best - 1) / best;
-    const int nranges = (int)((ns + range - 1) / range);
-    const dim3 grid((unsigned)tiles, (unsigned)nranges);
+    int64_t range = (ns + best - 1) / best;
+    int nranges = (int)((ns + range - 1) / range);
     double* part = nullptr;
     unsigned* done = nullptr;
     if (nranges > 1) {
-      part = ctx_buf_t<double>(ctx, "exact_part", (size_t)nranges * R * nt);
+      part = static_cast<double*>(ctx_buf_try(ctx, "exact_part", sizeof(double) * (size_t)nranges * R * nt));
       const size_t had = ctx->bufs["exact_done"].bytes;
-      done = ctx_buf_t<unsigned>(ctx, "exact_done", (size_t)tiles);
-      if (ctx->bufs["exact_done"].bytes != had)  // a new buffer: every launch leaves it at zero
+      if (part) done = static_cast<unsigned*>(ctx_buf_try(ctx, "exact_done", sizeof(unsigned) * (size_t)tiles));
+      if (done && ctx->bufs["exact_done"].bytes != had)  // a new buffer: every launch leaves it at zero
         FMMA_CHECK_CUDA(cudaMemsetAsync(done, 0, ctx->bufs["exact_done"].bytes, ctx->stream));
+      if (!done) {  // no scratch to be had: one range, which needs none
+        range = ns;
+        nranges = 1;
+      }
     }
+    const dim3 grid((unsigned)tiles, (unsigned)nranges);
     if (R == 1)
       FMMA_LAUNCH(ctx, (k_exact<KID, D, 1, T>), grid, kExThreads, 0, tgt, nt, rows, src, ns, w, R, p0, range, part,
                   done, ans);

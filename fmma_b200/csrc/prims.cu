@@ -44,23 +44,35 @@ void release_device_memory(fmma_ctx* ctx) {
   ctx->ops.clear();
 }
 
+static size_t buf_size(size_t bytes) { return bytes + bytes / 8 + 256; }
+
+// Grows a scratch buffer to `bytes`; false when the allocator refuses.
+static bool grow_buf(fmma_ctx* ctx, DevBuf& b, size_t bytes) {
+  if (b.bytes >= bytes) return true;
+  if (b.p) {
+    FMMA_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
+    dev_free(ctx, b.p, b.bytes);
+    b.p = nullptr;
+    b.bytes = 0;
+  }
+  b.p = dev_alloc(ctx, buf_size(bytes));
+  if (!b.p) return false;
+  b.bytes = buf_size(bytes);
+  return true;
+}
+
 void* ctx_buf(fmma_ctx* ctx, const std::string& name, size_t bytes) {
   DevBuf& b = ctx->bufs[name];
-  if (b.bytes < bytes) {
-    if (b.p) {
-      FMMA_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
-      dev_free(ctx, b.p, b.bytes);
-      b.p = nullptr;
-      b.bytes = 0;
-    }
-    size_t want = bytes + bytes / 8 + 256;
-    b.p = dev_alloc(ctx, want);
-    if (!b.p)
-      throw Error(FMMA_ERR_OOM, "device allocation of " + std::to_string(want) + " bytes for '" + name +
-                                    "' failed");
-    b.bytes = want;
-  }
+  if (!grow_buf(ctx, b, bytes))
+    throw Error(FMMA_ERR_OOM, "device allocation of " + std::to_string(buf_size(bytes)) + " bytes for '" + name +
+                                  "' failed");
   return b.p;
+}
+
+void* ctx_buf_try(fmma_ctx* ctx, const std::string& name, size_t bytes) {
+  DevBuf& b = ctx->bufs[name];
+  if (ctx->capturing && b.bytes < bytes) return nullptr;
+  return grow_buf(ctx, b, bytes) ? b.p : nullptr;
 }
 
 void* ctx_pinned(fmma_ctx* ctx, size_t bytes) {

@@ -36,10 +36,14 @@ void m2l_level_tc(fmma_ctx* ctx, bool bf16, int pair, int units, const Level& Lv
 // FP64 M2L of one virtual level on the reflection symmetry of the Chebyshev
 // grid (m2l_sym.cu): radial built-in kernels in 3-D with 3 to 8 nodes per
 // dimension.  rows: boxes x rhs of the level; lens: box width of each of its
-// operator tables.
+// operator tables.  m2l_sym_scratch gets the scratch of all the levels that a
+// sweep will run on it: false when the folded sources are refused (then none
+// of them runs on it: the kernel by offsets needs no scratch), and the most
+// parts that a level's orbits may be split into.
 bool m2l_sym_ok(const fmma_ctx* ctx, int d, int n, int64_t rows);
+bool m2l_sym_scratch(fmma_ctx* ctx, const std::vector<const Level*>& levels, int n, int R, int* most_parts);
 void m2l_level_sym(fmma_ctx* ctx, const Level& Lv, int v, int n, int Kpad, int R, const std::vector<double>& lens,
-                   const std::string& tabkey, const double* node_all, const double* Wm, double* Wl);
+                   const std::string& tabkey, const double* node_all, const double* Wm, double* Wl, int most_parts);
 
 // Mixed-precision near field: FP32 box-local evaluations, compensated sums.
 // wst_ready: the FP32 weight rows were written by gather_weights_mixed.

@@ -157,3 +157,73 @@ def test_m2l_wait_timeout_reports_and_context_recovers():
     finally:
         ctx.debug_m2l_wait()
         ctx.close()
+
+
+def _refusing(ctx, refuse):
+    """Routes the context through torch's allocator, which refuses the sizes that refuse(bytes) picks."""
+    import torch
+    asked = []
+
+    def alloc(n, stream):
+        asked.append(n)
+        return 0 if refuse(n) else torch.cuda.caching_allocator_alloc(n, 0, stream)
+
+    ctx.set_allocator(alloc, lambda p, n, stream: torch.cuda.caching_allocator_delete(p))
+    return asked
+
+
+def _buffer(nbytes):  # about what a context asks its allocator for when a buffer of nbytes grows
+    return nbytes + nbytes // 8 + 256
+
+
+@pytest.mark.parametrize("what", ["sources", "parts"])
+@pytest.mark.parametrize("as_plan", [False, True])
+def test_symmetric_m2l_without_its_scratch(what, as_plan):
+    """The FP64 M2L on the grid's symmetry keeps folded sources and partial sums that the M2L by offsets does not
+    need: where the allocator refuses them the call runs without (by offsets, or unsplit) instead of failing.  The sums
+    are then in another order: 1e-12, as for the plain FP64 parity tests; a plan replays what its sweeps ran."""
+    import fmma_b200
+    t, s, w = _case(5, 6000)
+    n, depth = 5, 4
+    ctx = fmma_b200.Context(0)
+    try:
+        ctx.set_kernel("inv_r_safe")
+        ref, _ = ctx.solve(t, s, w, poly_ord=n - 1, depth=depth)
+        lv = ctx.tree_levels()
+        boxes = max(b for b, r in zip(lv["boxes"], lv["rows"]) if r)
+        if what == "sources":  # 8 parity blocks of 27 coefficients, padded to 28, a box, and a row of zeros
+            sizes = {_buffer((boxes + 1) * 8 * 28 * 8)}
+        else:
+            sizes = {_buffer(k * r * n ** 3 * 8) for k in range(2, 17) for r in lv["rows"] if r}
+        hit = []
+        asked = _refusing(ctx, lambda b: any(0 <= b - x < 64 for x in sizes) and not hit.append(b))
+        if as_plan:
+            plan = ctx.plan(t, [0, len(t)], s, [0, len(s)], 1, [depth], poly_ord=n - 1)
+            out = plan.execute(w)
+            assert np.array_equal(plan.execute(w), out)
+            plan.close()
+        else:
+            out, _ = ctx.solve(t, s, w, poly_ord=n - 1, depth=depth)
+        assert hit and len(asked) > len(hit)
+        assert np.linalg.norm(out - ref) <= 1e-12 * np.linalg.norm(ref)
+    finally:
+        ctx.close()
+
+
+def test_exact_sum_without_scratch():
+    """The exact sum's source ranges need scratch for their partial sums; refused, it runs in one range."""
+    import torch
+
+    import fmma_b200
+    t, s, w = (torch.from_numpy(x).cuda() for x in _case(6, 3000))
+    ctx = fmma_b200.Context(0)
+    try:
+        ctx.set_kernel("inv_r_safe")
+        ref, _ = ctx.solve(t, s, w, solver="exact")
+        asked = _refusing(ctx, lambda b: True)
+        out, _ = ctx.solve(t, s, w, solver="exact")
+        assert asked
+        # 3000 terms in another order
+        assert float((out - ref).norm() / ref.norm()) <= 3000 * 2.0 ** -53
+    finally:
+        ctx.close()
