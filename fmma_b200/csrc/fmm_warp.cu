@@ -869,11 +869,11 @@ void launch_p2m_warp(fmma_ctx* ctx, const Level& Lf, const double* sx, int64_t n
   switch ((Kpad + 31) / 32) {
 #define FMMA_P2M_CASE(K_) \
   case K_: p2m_warp_t<K_>(ctx, Lf, sx, ns, ws, R, cubes, depth, d, isf, n, P, Kpad, Tn, Wm, grid_n); break;
-    FMMA_P2M_CASE(1) FMMA_P2M_CASE(2) FMMA_P2M_CASE(3) FMMA_P2M_CASE(4) FMMA_P2M_CASE(5) FMMA_P2M_CASE(6)
-    FMMA_P2M_CASE(7) FMMA_P2M_CASE(8) FMMA_P2M_CASE(9) FMMA_P2M_CASE(10) FMMA_P2M_CASE(11) FMMA_P2M_CASE(12)
-    FMMA_P2M_CASE(13) FMMA_P2M_CASE(14) FMMA_P2M_CASE(15) FMMA_P2M_CASE(16)
+    // one coefficient or 1-D (1), 2-D with 9 to 16 nodes (3 to 8)
+    FMMA_P2M_CASE(1) FMMA_P2M_CASE(3) FMMA_P2M_CASE(4) FMMA_P2M_CASE(5) FMMA_P2M_CASE(6) FMMA_P2M_CASE(7)
+    FMMA_P2M_CASE(8)
 #undef FMMA_P2M_CASE
-    default: break;
+    default: throw Error(FMMA_ERR_INVALID_ARG, "P2M: no kernel for this expansion size");
   }
 }
 
@@ -893,9 +893,9 @@ void launch_l2p_warp(fmma_ctx* ctx, const Level& Lf, const double* tx, int64_t n
                   Lf.row_box, Lf.nrow, Lf.key, Lf.tb, Lf.te, tx, nt, cubes, depth, d, isf ? 1 : 0, n, P, Kpad, R, Tn, \
                   Wl, pot);                                                                        \
     return;
+      // 1-D and 2-D (1 to 8), 3-D (up to 7 nodes 1, 2, 4, 7 and 11, 8 nodes 16)
       FMMA_L2P_CASE(1) FMMA_L2P_CASE(2) FMMA_L2P_CASE(3) FMMA_L2P_CASE(4) FMMA_L2P_CASE(5) FMMA_L2P_CASE(6)
-      FMMA_L2P_CASE(7) FMMA_L2P_CASE(8) FMMA_L2P_CASE(9) FMMA_L2P_CASE(10) FMMA_L2P_CASE(11) FMMA_L2P_CASE(12)
-      FMMA_L2P_CASE(13) FMMA_L2P_CASE(14) FMMA_L2P_CASE(15) FMMA_L2P_CASE(16)
+      FMMA_L2P_CASE(7) FMMA_L2P_CASE(8) FMMA_L2P_CASE(11) FMMA_L2P_CASE(16)
 #undef FMMA_L2P_CASE
       default: break;
     }

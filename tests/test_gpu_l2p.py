@@ -95,3 +95,23 @@ def test_gradient(ctx, d, depth, poly_ord):
             e = np.eye(d)[q]
             d1, d2 = ((at(h * e) - at(-h * e)) / (2 * h) for h in (1e-4, 5e-5))
             assert np.abs(grad[:, :, q] - (4 * d2 - d1) / 3).max() <= 1e-6 * np.abs(grad).max()
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("d,n", [(1, 1), (1, 8), (1, 9), (1, 16), (2, 1), (2, 5), (2, 6), (2, 8), (2, 9), (2, 10), (2, 11),
+                                 (2, 12), (2, 13), (2, 14), (2, 15), (2, 16), (3, 1), (3, 2), (3, 3), (3, 4), (3, 5),
+                                 (3, 6), (3, 7)])
+def test_every_expansion_size(ctx, oracle, d, n, mode):
+    # P2M and L2P have a kernel for every expansion size that is accepted, by default and with lanes over coefficients
+    r = np.random.default_rng(16 * d + n)
+    depth = {1: 6, 2: 4, 3: 3}[d]
+    t, s, w = r.random((300, d)), r.random((310, d)), r.standard_normal((3, 310))
+    ctx.set_kernel("inv_r_safe")
+    ctx.set_schedule_options(l2p_mode=mode)
+    try:
+        one, _ = ctx.solve(t, s, w[2].copy(), poly_ord=n - 1, depth=depth)
+        many, _ = ctx.solve(t, s, w, poly_ord=n - 1, depth=depth)
+    finally:
+        ctx.set_schedule_options()
+    want, _ = oracle.fmm(d, 1, 0.0, n - 1, depth, 1, t, s, w[2].copy())
+    assert rel_l2(one, want) <= TOL and rel_l2(many[2], want) <= TOL
