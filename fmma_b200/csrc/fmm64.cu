@@ -965,6 +965,8 @@ void solve_forest(fmma_ctx* ctx, const SolveArgs& a, const std::vector<int64_t>&
     {
       const Level& Lf = tr.lev[0];
       const size_t smem_l2p = sizeof(double) * (size_t)R * Kpad;
+      // the form with a block a leaf stages a leaf's expansions; the others do
+      // not, but the call's limit is the same for all
       FMMA_REQUIRE(smem_l2p <= 200 * 1024, "nrhs * nodes per box too large for L2P");
       if (Lf.nrow > 0) {
         if (grad) {

@@ -186,9 +186,8 @@ __global__ void __launch_bounds__(256, (D == 3 && (RB == 16 || RB == 1)) ? 2 : 3
     const int* __restrict__ depth, const Cube* __restrict__ cubes, const double* __restrict__ pot,
     const int* __restrict__ perm_t, T* __restrict__ out) {
   // Per warp, in dynamic shared memory: the per-lane compensated FP32 sums
-  // (sum, error) when the rhs block is wide (registers for up to 4 rhs;
-  // keeps the kernel at 3 blocks per SM) and two staging buffers, each a
-  // chunk's weights and coordinate records.
+  // (sum, error) when the rhs block is wide (registers for up to 4 rhs) and two
+  // staging buffers, each a chunk's weights and coordinate records.
   constexpr int SC = p2p_chunk(RB), REC = LocalRec<D>::N, BLK = p2p_block<RB>();
   constexpr bool kSmemAcc = RB >= 8;
   extern __shared__ __align__(16) unsigned char p2p_smem[];
@@ -421,12 +420,9 @@ __global__ void __launch_bounds__(256, (D == 3 && (RB == 16 || RB == 1)) ? 2 : 3
   }
 }
 
-// Right-hand sides per pass: 1, 4, 8 or 16 (one pass for 9-16 right-hand
-// sides, the kernel evaluated once per pair).  Every block width runs three
-// 256-thread blocks per SM (80 registers; 8 and 16 keep their FP64 sums in
-// shared memory), except 3-D with 16, whose sums and two staging buffers
-// leave room for two (and so up to 128 registers for the 16 compensated
-// FP32 sums).
+// Right-hand sides per pass of k_p2p_f32: 1, 4, 8 or 16 (one pass for 9-16
+// right-hand sides, the kernel evaluated once per pair).
+
 // Sparse leaves (a few targets each, as in clustered sets at a uniform
 // depth): lanes over the sources of the 3^d neighbour leaves taken as one
 // list, targets looped.  Lane e finds its neighbour slot k from the prefix

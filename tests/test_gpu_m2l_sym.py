@@ -204,3 +204,15 @@ def test_operators_of_a_narrow_gaussian(ctx, poly_ord):
             terms[here] += abs(tf[here]) @ (K @ (wb @ abs(sf)))
     err, scale = (np.linalg.norm(x.astype(float)) for x in (got - want, terms))
     assert err <= 64 * 2.0 ** -53 * scale, err / scale
+
+
+@pytest.mark.parametrize("points", [80, 700, 3000])
+@pytest.mark.parametrize("rhs", [1, 3])
+def test_eight_nodes_on_sparse_and_dense_leaves(ctx, oracle, points, rhs):
+    # the default leaf evaluation, which 8 nodes in 3-D have at every density
+    r = np.random.default_rng(points)
+    t, s, w = r.random((points, 3)), r.random((points, 3)), r.standard_normal((rhs, points))
+    ctx.set_kernel("inv_r_safe")
+    got, _ = ctx.solve(t, s, w, poly_ord=7, depth=3)
+    want, _ = oracle.fmm(3, 1, 0.0, 7, 3, 1, t, s, w[rhs - 1])
+    assert rel_l2(np.atleast_2d(got)[rhs - 1], want) <= TOL

@@ -26,3 +26,20 @@ def test_chunks(ctx, oracle, d, per_leaf, nrhs):
     for k in {0, nrhs - 1}:
         want = oracle.exact_rows(d, 5, 1e-2, np.arange(len(t)), t, s, w[k].copy())
         assert rel_l2(got[k], want) <= 1e-6
+
+
+@pytest.mark.parametrize("d", [1, 2, 3])
+@pytest.mark.parametrize("n", [49, 50, 63, 64, 81, 96, 113, 128, 145])
+def test_pairs_of_chunks_sum_as_chunks_alone(ctx, d, n):
+    """One rhs: chunks of 32 targets of a leaf go in pairs where the second holds at least 17.  A chunk's sums do not
+    depend on the company: the leaf's targets at once and 32 at a time give the same bits."""
+    r = np.random.default_rng(n + 1000 * d)
+    t = r.random((n, d)) * 0.49  # one leaf; its order is that of the targets
+    s = np.concatenate([r.random((500, d)), np.zeros((1, d)), np.ones((1, d))])
+    w = r.uniform(-1, 1, len(s))
+    ctx.set_kernel("multiquadric", 1e-2)
+
+    def solve(x):
+        return ctx.solve(np.ascontiguousarray(x), s, w, poly_ord=2, depth=2, precision="tf32x3")[0]
+    whole = solve(t)
+    np.testing.assert_array_equal(whole, np.concatenate([solve(t[i:i + 32]) for i in range(0, n, 32)]))

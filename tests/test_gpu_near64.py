@@ -68,6 +68,24 @@ def test_near_gradient_is_the_exact_one(ctx, kid):
     assert rel_l2(g, ge) <= 1e-12
 
 
+@pytest.mark.parametrize("d,kid", [(1, k) for k in range(7)] + [(2, k) for k in (0, 1, 3, 4, 5, 6)] + [(3, 1), (3, 6)])
+@pytest.mark.parametrize("coincident", [False, True])
+def test_near_gradient_in_every_dimension(ctx, d, kid, coincident):
+    # against the exact gradient, which another kernel sums pair by pair; coincident points take the guards
+    r = np.random.default_rng(20 * d + kid)
+    t, s, w = r.random((300, d)), r.random((280, d)), r.standard_normal((2, 280))
+    if coincident:
+        t[:40] = s[:40]
+    ctx.set_kernel(kid, P0.get(kid, 0.0))
+    c, g, _ = ctx.solve_grad(t, s, w, poly_ord=2, depth=2)
+    ce, ge, _ = ctx.solve_grad(t, s, w, solver="exact")
+    ok = np.isfinite(ce)  # at r = 0 the potential of 1/r is infinite and that of s/r^2 undefined
+    np.testing.assert_array_equal(np.isfinite(c), ok)
+    assert ok.all() == (not coincident or kid not in (0, 6))
+    assert rel_l2(c[ok], ce[ok]) <= 1e-13
+    assert np.isfinite(ge).all() and rel_l2(g, ge) <= 1e-12
+
+
 def test_inverse_square_root(ctx):
     r = np.random.default_rng(1)
     x = np.concatenate([r.uniform(1, 4, 20000), 10.0 ** r.uniform(-150, 150, 20000)])
