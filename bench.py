@@ -177,6 +177,23 @@ def tensor_peak(peaks, timed_s, precision):
     return bf16 / div, regime, burst / div
 
 
+RADIAL = ("inv_r", "inv_r_safe", "log_r", "gaussian", "multiquadric")
+
+
+def fp64_m2l_roof(wl, dense_flops, ms, note=""):
+    """Roofline of the plain FP64 M2L from its launches' time and the library's
+    flop count, 2 P^2 per (target box, source box) pair.  Radial kernels in 3-D
+    with 3 to 8 nodes run on the grid's reflection symmetry, which needs 39.5
+    P^2 multiply-adds where a target box's 189 far slots take 189 P^2."""
+    sym = wl["d"] == 3 and wl["kernel"] in RADIAL and 2 <= wl["poly_ord"] <= 7
+    flops = dense_flops * (39.5 / 189 if sym else 1.0)
+    achieved = flops / (ms / 1e3) / 1e12 if ms else None
+    return {"bound": "fp64", "kernel": ("k_m2l_sym" if sym else "k_m2l_f64") + " (FP64 DMMA)" + note,
+            "achieved": achieved, "peak": 37.0, "unit": "TFLOP/s", "frac": achieved / 37.0 if achieved else None,
+            "traffic": None, "peak_source": "nominal B200 FP64 tensor",
+            "flops_per_launch_note": ("2 x 39.5/189 P^2" if sym else "2 P^2") + " per (target box, source box) pair"}
+
+
 def add_peak_fields(roof, regime, burst):
     roof["peak_regime"] = regime
     if roof.get("achieved"):
@@ -595,11 +612,7 @@ def run_adjoint(args, wl):
         n_total = wl["n"] * world
         peaks, peak_src = measured_peaks()
         if args.precision == "fp64":
-            achieved = m2l_fl / (m2l_ms / 1e3) / 1e12 if m2l_ms else None
-            roof = {"bound": "fp64", "kernel": "k_m2l_f64 (FP64 DMMA), the three solves of a step",
-                    "achieved": achieved, "peak": 37.0, "unit": "TFLOP/s",
-                    "frac": achieved / 37.0 if achieved else None, "traffic": None,
-                    "peak_source": "nominal B200 FP64 tensor"}
+            roof = fp64_m2l_roof(wl, m2l_fl, m2l_ms, ", the three solves of a step")
         else:
             tpk, regime, burst = tensor_peak(peaks, ms * args.steps / 1e3, args.precision)
             achieved = 3 * m2l_fl / (m2l_ms / 1e3) / 1e12 if m2l_ms else None
@@ -1097,9 +1110,7 @@ def main():
         n_products = 3 if args.precision != "fp64" else 1
         achieved = (m2l_flops * n_products / (m2l_ms / 1e3)) / 1e12 if m2l_ms > 0 else None
         if args.precision == "fp64":
-            roof = {"bound": "fp64", "achieved": achieved, "peak": 37.0, "unit": "TFLOP/s",
-                    "frac": achieved / 37.0 if achieved else None, "traffic": None,
-                    "kernel": "k_m2l_f64 (FP64 DMMA)", "peak_source": "nominal B200 FP64"}
+            roof = fp64_m2l_roof(wl, m2l_flops, m2l_ms)
         else:
             roof = {"bound": "tensor", "achieved": achieved, "peak": tpk, "unit": "TFLOP/s",
                     "frac": achieved / tpk if achieved else None, "traffic": None,

@@ -308,7 +308,9 @@ void* fmma_ctx_stream(fmma_ctx* ctx);
  * blocking the host: for device buffers that another stream fills.         */
 fmma_status fmma_wait_stream(fmma_ctx* ctx, void* stream);
 /* M2L kernels of the last solve: summed CUDA-event time of the launches,
- * algorithmic flops (2 P^2 per target/source box pair and rhs), launches. */
+ * flops of the sum box pair by box pair (2 P^2 per target/source box pair and
+ * rhs, whichever kernel ran: the FP64 one on the grid's reflection symmetry
+ * needs 39.5 where this counts 189), launches.                             */
 fmma_status fmma_m2l_stats(fmma_ctx* ctx, double* kernel_ms, double* flops,
                            int64_t* launches);
 /* Tree of the last fmm solve: M2L pairs over all levels, P2P point pairs,
