@@ -139,8 +139,9 @@ class Context:
     def set_schedule_options(self, m2l_split=0, l2p_mode=0):
         """The plan autotuner's choices by hand: the slot split of small
         tensor-core M2L levels (0 fill the SMs, 1 none, 2 half, 3 double) and
-        the leaf evaluation (0 by targets per leaf, 1 lanes over targets,
-        2 lanes over coefficients)."""
+        the leaf evaluation (0 by default lanes over targets, with 1 or more
+        than 8 nodes lanes over coefficients below 16 targets per leaf; 1 lanes
+        over targets, 2 lanes over coefficients)."""
         with self.lock:
             check(self._L.fmma_set_schedule_options(self._h, int(m2l_split), int(l2p_mode)))
 

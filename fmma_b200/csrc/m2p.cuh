@@ -23,8 +23,9 @@ namespace fmma_b200 {
 // of 16 with rsqrt() and all differences per pair.  N nodes per dimension, at
 // compile time: a row's N evaluations are independent.  FP64 pipe bound.
 // Against the general loop: tree solver's far sums, 200k points in 3-D, 6 nodes
-// 29.9 -> 13.3 ms (20 warps an SM at 102 registers; 24 at 80 were 10 % slower),
-// nrnmm 100k points 51.1 -> 27.9 ms a call.
+// 29.9 -> 13.3 ms (16 warps an SM at 117 registers, 20 in blocks of 64; 24 at 80
+// were 10 % slower), nrnmm 100k points 51.1 -> 27.9 ms a call; the FP64 pipe is
+// 55 to 61 % busy.
 template <int KID, int D, int RB, int N>
 __device__ __forceinline__ void far_box_row(const double* x, const double* __restrict__ X,
                                             const double* __restrict__ W, int P, double p0, double ip, double* acc) {
