@@ -177,8 +177,10 @@ fmma_status fmma_forest_depths_d(fmma_ctx* ctx, int dim, int nprob,
  * this geometry; decisions kept in the context's tuner cache), and captures
  * the sweep P2M..P2P into a CUDA graph.  fmma_plan_execute_d replays it for
  * new weights [nrhs][n_src] (results [nrhs][n_tgt]).  The plan owns a private
- * context created on the parent's device with the parent's kernel.  No
- * counterpart in the reference (which rebuilds everything per solve).       */
+ * context created on the parent's device with the parent's kernel; device
+ * points are copied once the work is done that the parent's stream waits for
+ * (fmma_wait_stream).  No counterpart in the reference (which rebuilds
+ * everything per solve).                                                    */
 typedef struct fmma_plan fmma_plan;
 fmma_status fmma_plan_create_d(fmma_ctx* parent, int dim, int nprob,
                                const int64_t* toff, const double* tgt,
