@@ -201,32 +201,50 @@ __device__ __forceinline__ void two_sum(double a, double b, double& s, double& e
   s = t;
 }
 
-// f + c = the kernel at |x - y|^2 = r2 + rl, c the rounding error of f and of r2.
+// (len (x/2 - (o + y/2)))^2 with its rounding error.
+__device__ __forceinline__ void sym_square(double x, double y, int o, double len, double& s, double& e) {
+  double a, al, t, tl;
+  two_sum(x / 2, -y / 2, a, al);
+  two_sum(a, -(double)o, t, tl);
+  const double p = len * t, pl = fma(len, t, -p) + len * (tl + al);
+  s = p * p;
+  e = fma(p, p, -s) + 2.0 * p * pl;
+}
+
+// Kernel values at offset o (in box widths) between a source node y and the
+// target nodes x0 and x1, which differ in the last dimension only.  The
+// Gaussian's argument is formed and divided with its rounding error, which its
+// value takes r^2/p0 times over otherwise; the other kernels as everywhere.
 template <int KID>
-__device__ __forceinline__ void sym_value(double r2, double rl, double p0, double& f, double& c) {
-  switch (KID) {
-    case FMMA_KERNEL_LOG_R:
-      f = 0.5 * log(r2);
-      c = 0.5 * rl / r2;
-      break;
-    case FMMA_KERNEL_GAUSSIAN: {
-      const double a = r2 / p0;
-      f = exp(-a);
-      c = -f * ((fma(-a, p0, r2) + rl) / p0);
-      break;
+__device__ __forceinline__ void sym_values(const double* x0, const double* x1, const double* y, const int* o,
+                                           double len, double p0, double ip, double (&f)[2]) {
+  if constexpr (KID == FMMA_KERNEL_GAUSSIAN) {
+    double r, e, s0, e0, s1, e1;
+    sym_square(x0[0], y[0], o[0], len, s0, e0);
+    sym_square(x0[1], y[1], o[1], len, s1, e1);
+    two_sum(s0, s1, r, e);
+    e += e0 + e1;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      double s, es, r2, rl;
+      sym_square(u ? x1[2] : x0[2], y[2], o[2], len, s, es);
+      two_sum(r, s, r2, rl);
+      rl += e + es;
+      const double a = ip != 0.0 ? r2 * ip : r2 / p0;  // and what is left of r^2
+      const double d = fma(-a, p0, r2) + rl;
+      f[u] = exp(-a);
+      if (f[u] > 0.0) f[u] -= f[u] * (ip != 0.0 ? d * ip : d / p0);
     }
-    case FMMA_KERNEL_MULTIQUADRIC: {
-      double h, e;
-      two_sum(r2, p0, h, e);
-      f = sqrt(h);
-      c = (fma(-f, f, h) + e + rl) / (2.0 * f);
-      break;
-    }
-    default: {  // 1/r: f (1 + (1 - f^2 r^2) / 2)
-      f = 1.0 / sqrt(r2);
-      const double p = f * f, pe = fma(f, f, -p);
-      c = 0.5 * f * (fma(-p, r2, 1.0) - pe * r2 - p * rl);
-      break;
+  } else {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      double v[3], w[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        v[q] = len * ((u ? x1[q] : x0[q]) / 2);
+        w[q] = len * ((double)o[q] + y[q] / 2);
+      }
+      f[u] = keval<KID, 3>(v, w, p0);
     }
   }
 }
@@ -235,13 +253,11 @@ __device__ __forceinline__ void sym_value(double r2, double rl, double p0, doubl
 // half-indices: the 64 values of f over the reversals of i and j (two per
 // lane), transformed along both by shuffles, give the entry (i, j) of all 64
 // blocks.  The halves of the inverse transforms on both sides, 1/64 in all, are
-// in the folded sources.  Value, argument and the sums of 64 carry their
-// rounding errors along, so that an entry is rounded once (34 -> 54 us a level
-// at 6 nodes, once a geometry).  What that is for is the narrow Gaussian, whose
-// value takes the argument's error r^2/p0 times over: error of the M2L against
-// long double, p0 = 0.01 in the unit cube, over that of k_m2l_f64, 4 nodes 1.13
-// -> 0.16, 6 nodes 0.58 -> 0.20; over 3 to 8 nodes, four kernels and all levels
-// the median is 0.29 -> 0.25 (the sums are 39.5/189 as long).
+// in the folded sources.  Error of the M2L against long double over that of
+// k_m2l_f64, median over 3 to 8 nodes, four kernels and all levels: 0.25 (the
+// sums are 39.5/189 as long); what the care for the Gaussian's argument is for
+// (36 -> 41 us a level at 5 nodes, once a geometry): p0 = 0.01 in the unit cube,
+// level 2, 4 nodes, 1.13 -> 0.16.
 template <int KID>
 __global__ void __launch_bounds__(256) k_sym_table(const double* __restrict__ lens, int ntab,
                                                    const double* __restrict__ node_all,
@@ -250,6 +266,7 @@ __global__ void __launch_bounds__(256) k_sym_table(const double* __restrict__ le
   const SymGeom& g = *gp;
   const int n = g.n, he = g.he, ho = g.ho, NB = g.NB;
   const int nh = he * he * he, lane = threadIdx.x & 31;
+  const double ip = kinv<KID>(p0);
   const int64_t total = (int64_t)ntab * kOrbits * nh * nh;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < total; e += nw) {
@@ -257,40 +274,18 @@ __global__ void __launch_bounds__(256) k_sym_table(const double* __restrict__ le
     const int64_t t = e / ((int64_t)nh * nh * kOrbits);
     const double len = lens[t];
     const Half I(hi, he, ho), J(hj, he, ho);
-    double v[2], c[2];  // value and its error; index = row reversal * 8 + column reversal = lane + 32 u
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int kl = I.node((lane >> 3) + 4 * u, n), km = J.node(lane & 7, n);
-      double r2 = 0.0, rl = 0.0;
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {  // len (x_k / 2 - (o + x_m / 2))
-        double a, al, t, tl, e;
-        two_sum(node_all[kl * 3 + q] / 2, -node_all[km * 3 + q] / 2, a, al);
-        two_sum(a, -(double)g.rep[w][q], t, tl);
-        const double p = len * t, pl = fma(len, t, -p) + len * (tl + al);
-        const double s = p * p;
-        rl += fma(p, p, -s) + 2.0 * p * pl;
-        two_sum(r2, s, r2, e);
-        rl += e;
-      }
-      two_sum(r2, rl, r2, rl);
-      sym_value<KID>(r2, rl, p0, v[u], c[u]);
-    }
-    double s, d, es, ed;
-    two_sum(v[0], v[1], s, es);
-    two_sum(v[0], -v[1], d, ed);
-    es += c[0] + c[1];
-    ed += c[0] - c[1];
-    v[0] = s, c[0] = es;
-    v[1] = d, c[1] = ed;
+    double v[2];  // index = row reversal * 8 + column reversal = lane + 32 u
+    sym_values<KID>(node_all + 3 * I.node(lane >> 3, n), node_all + 3 * I.node((lane >> 3) + 4, n),
+                    node_all + 3 * J.node(lane & 7, n), g.rep[w], len, p0, ip, v);
+    const double s = v[0] + v[1], d = v[0] - v[1];
+    v[0] = s;
+    v[1] = d;
 #pragma unroll
     for (int q = 1; q < 32; q <<= 1)
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const double o = __shfl_xor_sync(0xffffffffu, v[u], q), oc = __shfl_xor_sync(0xffffffffu, c[u], q);
-        const bool up = lane & q;
-        two_sum(up ? -v[u] : v[u], o, v[u], s);
-        c[u] = (up ? oc - c[u] : c[u] + oc) + s;
+        const double o = __shfl_xor_sync(0xffffffffu, v[u], q);
+        v[u] = (lane & q) ? o - v[u] : v[u] + o;
       }
     const int z = g.zmask[w], b = lane & 7, b0 = b & ~z;
     if (b & J.mid) continue;
@@ -306,7 +301,7 @@ __global__ void __launch_bounds__(256) k_sym_table(const double* __restrict__ le
       const int col = I.in_block(a, he, ho);
       const int l = (col & 7) * 4 + (k & 3), nb = col >> 3;  // lane and column group of the fragment
       const int64_t at = ((int64_t)a * 2 + (step & 1)) * (32 * NB) + (NB == 1 ? l : (nb >> 1) * 64 + l * 2 + (nb & 1));
-      base[at] = v[u] + c[u];
+      base[at] = v[u];
     }
   }
 }

@@ -216,3 +216,13 @@ def test_eight_nodes_on_sparse_and_dense_leaves(ctx, oracle, points, rhs):
     got, _ = ctx.solve(t, s, w, poly_ord=7, depth=3)
     want, _ = oracle.fmm(3, 1, 0.0, 7, 3, 1, t, s, w[rhs - 1])
     assert rel_l2(np.atleast_2d(got)[rhs - 1], want) <= TOL
+
+
+def test_gaussian_of_points_beyond_its_range(ctx):
+    # far boxes at a distance whose square overflows: their operators are zero, not undefined
+    r = np.random.default_rng(2)
+    s = 1e160 * r.random((600, 3))
+    w = r.standard_normal(600)
+    ctx.set_kernel("gaussian", 0.01)
+    got, _ = ctx.solve(s, s, w, poly_ord=4, depth=4)
+    np.testing.assert_array_equal(got, w)  # only the coincident pair of every point counts
