@@ -111,3 +111,18 @@ def test_inverse_square_root(ctx):
         got, _ = ctx.solve(y[:, None].copy(), np.zeros((1, 1)), np.ones(1), solver="exact")
         with np.errstate(over="ignore", under="ignore"):
             np.testing.assert_allclose(got, np.exp(-(y * y) / p0), rtol=1e-13, atol=0)
+
+
+@pytest.mark.parametrize("d,depth,per,rhs", [(1, 8, 10, 1), (1, 8, 22, 1), (1, 8, 30, 4), (1, 13, 3, 1), (1, 13, 25, 2),
+                                             (2, 5, 5, 1), (2, 5, 8, 3), (2, 7, 2, 1), (2, 7, 31, 1), (2, 7, 60, 1),
+                                             (3, 3, 2, 1), (3, 3, 3, 8), (3, 5, 1, 1), (3, 5, 10, 1), (3, 5, 20, 1)])
+def test_units_of_one_and_of_four_warps(ctx, oracle, d, depth, per, rhs):
+    # lists and numbers of units on both sides of the rule that has four warps share a unit; the other stages are as
+    # in the parity tests: 1e-12
+    r = np.random.default_rng(100 * d + depth + per)
+    n = per * 2 ** (d * (depth - 1))
+    t, s, w = r.random((n, d)), r.random((n, d)), r.standard_normal((rhs, n))
+    ctx.set_kernel("inv_r_safe")
+    got, _ = ctx.solve(t, s, w if rhs > 1 else w[0].copy(), poly_ord=1, depth=depth)
+    want, _ = oracle.fmm(d, 1, 0.0, 1, depth, 1, t, s, w[rhs - 1].copy())
+    assert rel_l2(np.atleast_2d(got)[rhs - 1], want) <= 1e-12
