@@ -356,6 +356,7 @@ __global__ void __launch_bounds__(kTreeThreads) k_tree_emit(const uint64_t* __re
 // Sort keys of the rows of every level in one array: M2L rows of level v
 // (boxes with targets at real level >= 2) by (v, problem, class), then the
 // near-field rows (leaves with targets) as level V; boxes of neither kind last.
+// V: the levels that can have rows; the boxes of the coarser ones have none.
 // Entry i < total is box i - lo.o[v] of its level v, entry total + b leaf b.
 __global__ void k_row_keys(const uint64_t* __restrict__ key, const int* __restrict__ tb, const int* __restrict__ te,
                            const LevelOff lo, int V, int64_t total, int64_t nleaf, int d, int np,
@@ -371,7 +372,12 @@ __global__ void k_row_keys(const uint64_t* __restrict__ key, const int* __restri
       continue;
     }
     int v = 0;
-    while (i >= lo.o[v + 1]) ++v;
+    while (v < V && i >= lo.o[v + 1]) ++v;
+    if (v == V) {
+      ck[i] = none;
+      cv[i] = 0;
+      continue;
+    }
     const uint64_t k = key[i];
     const int p = key_pid(k);
     const bool row = te[i] > tb[i] && depth[p] - 1 - v >= 2;
@@ -548,17 +554,20 @@ void build_forest(fmma_ctx* ctx, int d, const std::vector<int64_t>& toff, const 
     const int64_t total = lo.o[V], nleaf = tr.lev[0].nbox, nkey = total + nleaf;
     const Level& first = tr.lev[0];  // the arrays of all levels start at the leaves
     // Rows of all levels and the near-field rows in one sort; the table of
-    // segment begins by (level, problem, class) is read back in one wait.
-    const int64_t ntable = ((int64_t)V * np + 2) << d;
+    // segment begins by (level, problem, class) is read back in one wait.  Real
+    // level >= 2 leaves the V - 2 finest levels (the table of 4000 problems of
+    // Depth 2 in 3-D: 64,016 entries with all levels, 16 without).
+    const int VR = std::max(0, V - 2);
+    const int64_t ntable = ((int64_t)VR * np + 2) << d;
     uint64_t* ck = ctx_buf_t<uint64_t>(ctx, "row_ck", (size_t)nkey);
     int* cv = ctx_buf_t<int>(ctx, "row_cv", (size_t)nkey);
     uint64_t* ck2 = ctx_buf_t<uint64_t>(ctx, "row_ck2", (size_t)nkey);
     int* cv2 = ctx_buf_t<int>(ctx, "row_cv2", (size_t)nkey);
     int* begin = ctx_buf_t<int>(ctx, "row_begin", (size_t)ntable);
     FMMA_CHECK_CUDA(cudaMemsetAsync(begin, 0xff, sizeof(int) * (size_t)ntable, ctx->stream));
-    FMMA_LAUNCH(ctx, k_row_keys, grid_for(nkey, blk), blk, 0, first.key, first.tb, first.te, lo, V, total, nleaf, d, np,
-                tr.d_depth, ck, cv);
-    radix_sort_swap(ctx, &ck, &cv, &ck2, &cv2, nkey, 0, d + bits_for(V * np + 2));
+    FMMA_LAUNCH(ctx, k_row_keys, grid_for(nkey, blk), blk, 0, first.key, first.tb, first.te, lo, VR, total, nleaf, d,
+                np, tr.d_depth, ck, cv);
+    radix_sort_swap(ctx, &ck, &cv, &ck2, &cv2, nkey, 0, d + bits_for(VR * np + 2));
     FMMA_LAUNCH(ctx, k_row_segs, grid_for(nkey, blk), blk, 0, ck, nkey, begin);
     std::vector<int> hb((size_t)ntable);
     read_ints(ctx, begin, hb.data(), (int)ntable);
@@ -583,7 +592,7 @@ void build_forest(fmma_ctx* ctx, int d, const std::vector<int64_t>& toff, const 
       Lv.segs.clear();
       const int64_t r0 = ro.o[v];
       int64_t r1 = r0;
-      for (int64_t k = ((int64_t)v * np) << d; k < ((int64_t)(v + 1) * np) << d; ++k) {
+      for (int64_t k = ((int64_t)v * np) << d; v < VR && k < ((int64_t)(v + 1) * np) << d; ++k) {
         if (hb[(size_t)k] < 0) continue;
         r1 = ends[(size_t)k];
         Lv.segs.push_back(make_int4((int)(k >> d) - v * np, (int)(k & ((1 << d) - 1)), (int)(hb[(size_t)k] - r0),
@@ -592,7 +601,7 @@ void build_forest(fmma_ctx* ctx, int d, const std::vector<int64_t>& toff, const 
       ro.o[v + 1] = r1;
       Lv.nrow = r1 - r0;
     }
-    const int64_t nrow = ro.o[V], knear = ((int64_t)V * np) << d;
+    const int64_t nrow = ro.o[V], knear = ((int64_t)VR * np) << d;
     tr.nnear_rows = hb[(size_t)knear] >= 0 ? ends[(size_t)knear] - hb[(size_t)knear] : 0;
     tr.near_row_box = cv + nrow;
     // neighbour lists of every level top-down, far lists of the rows on the way

@@ -128,3 +128,21 @@ def test_plan_engines_agree_on_a_large_level(ctx):
     plain, _ = ctx.solve(t, s, w, poly_ord=5, depth=6)
     assert rel_l2(got, direct) <= 1e-6, rel_l2(got, direct)
     assert rel_l2(got, plain) <= 1e-5
+
+
+@pytest.mark.parametrize("d", [1, 2, 3])
+@pytest.mark.parametrize("depths", [[1], [1, 1, 2], [2, 2, 2, 2], [2, 3, 1], [3, 3], [4, 1, 2, 3], [1, 5]])
+@pytest.mark.parametrize("precision", ["fp64", "tf32x3"])
+def test_shallow_problems(ctx, oracle, d, depths, precision):
+    # rows of the far field exist from real level 2 on: forests without any, with some and with all levels
+    r = np.random.default_rng(len(depths) + d)
+    sizes = [int(r.integers(5, 60)) * 2 ** (k - 1) for k in depths]
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    t, s, w = r.random((off[-1], d)), r.random((off[-1], d)), r.standard_normal(off[-1])
+    ctx.set_kernel("multiquadric", 1e-2)
+    got = ctx.forest_solve(t, off, s, off, w, depths, poly_ord=3, precision=precision)
+    for p, depth in enumerate(depths):
+        a, b = off[p], off[p + 1]
+        want, _ = oracle.fmm(d, 5, 1e-2, 3, depth, 1, t[a:b].copy(), s[a:b].copy(), w[a:b].copy())
+        # mixed: FP32 kernel values (2^-23) and split products (2^-20) of sums of both signs
+        assert rel_l2(got[a:b], want) <= (1e-12 if precision == "fp64" else 1e-5)
