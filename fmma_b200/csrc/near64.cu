@@ -231,9 +231,10 @@ __global__ void __launch_bounds__(kNearThreads, GRAD || RB > 2 ? 2 : 3) k_near64
 // The two cuts of the near field.  slots: a row's chunks of 32 targets, so
 // that every chunk of a mean row is a unit.  wpu: four warps share a unit's
 // sources, tile by tile, where the lists are long enough for the reduction over
-// them: from three tiles on when the units fill less than a quarter of the
-// warps the GPU holds (24 an SM), from nine when less than all, from seventeen
-// below eight waves.  us with one warp and with four, 1/r, uniform points, one
+// them: from 48 sources when the units fill less than a quarter of the warps
+// the GPU holds (24 an SM), from 192 when less than all, from 400 below eight
+// waves.  That is in pairs of 1/r; a pair of another kernel counts by what it
+// costs against it (log r 4, the Gaussian 3, a root or division 2.5).  us with one warp and with four, 1/r, uniform points, one
 // rhs: 96 units x 240 sources 23 and 13, 128 x 30 both 9; 2,048 x 360 40 and 36,
 // x 60 13 and 21; 8,192 x 1,080 284 and 232, x 60 30 and 56; 32,768 x 30 54 and
 // 150 (four rhs 118 and 365).  The list's length is estimated from the mean
@@ -246,8 +247,12 @@ NearArgs near_args(fmma_ctx* ctx, int nnear, const Tree& tr, const double* tx, c
   const int64_t mean = (tr.nt + tr.nnear_rows - 1) / tr.nnear_rows;
   a.slots = (int)std::max<int64_t>(1, std::min<int64_t>(64, (mean + 31) / 32));
   const int64_t units = a.nrow * a.slots, warps = (int64_t)ctx->sm_count * 24;
-  const int64_t list = tr.ns * nnear / std::max<int64_t>(1, Lf.nbox);  // sources of a unit
-  const int64_t most = list > 512 ? 8 * warps : (list > 256 ? warps : (list > 64 ? warps / 4 : 0));
+  const int k = ctx->kernel_id;
+  const int cost = k == FMMA_KERNEL_INV_R || k == FMMA_KERNEL_INV_R_SAFE
+                       ? 10
+                       : (k == FMMA_KERNEL_LOG_R ? 40 : (k == FMMA_KERNEL_GAUSSIAN ? 30 : 25));
+  const int64_t list = tr.ns * nnear * cost / (10 * std::max<int64_t>(1, Lf.nbox));  // a unit's sources
+  const int64_t most = list >= 400 ? 8 * warps : (list >= 192 ? warps : (list >= 48 ? warps / 4 : 0));
   a.wpu = units < most ? kNearWarps / 2 : 1;
   return a;
 }
