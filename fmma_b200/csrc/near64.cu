@@ -68,6 +68,24 @@ struct NearArgs {
   int slots, wpu;  // units per row; warps per unit (1 or kNearWarps / 2)
 };
 
+// The sums of sorted target t from right-hand side r0, and its gradient, with
+// the far field's added, to the caller's order.
+template <int D, int RB, bool GRAD, typename T>
+__device__ __forceinline__ void near_store(const NearArgs& a, const double* acc, int r0, int t, T* __restrict__ out,
+                                           double* __restrict__ grad) {
+  const int64_t ot = a.perm_t[t];
+#pragma unroll
+  for (int r = 0; r < RB; ++r)
+    if (r0 + r < a.R && out)
+      out[(int64_t)(r0 + r) * a.nt + ot] = (T)(acc[r] + (a.pot ? a.pot[(int64_t)(r0 + r) * a.nt + t] : 0.0));
+  if constexpr (GRAD) {
+#pragma unroll
+    for (int q = 0; q < D; ++q)
+      grad[((int64_t)r0 * a.nt + ot) * D + q] =
+          acc[RB + q] + (a.potg ? a.potg[((int64_t)r0 * a.nt + t) * D + q] : 0.0);
+  }
+}
+
 // A unit is every `slots`-th target chunk of a leaf row, taken by wpu warps
 // that share its sources tile by tile.  The 3^d neighbour leaves form one list
 // of sources (lane k holds neighbour k's range and the prefix sum of the
@@ -209,23 +227,79 @@ __global__ void __launch_bounds__(kNearThreads, GRAD || RB > 2 ? 2 : 3) k_near64
           }
           asm volatile("bar.sync %0, %1;" ::"r"(1 + unit_in), "r"(wpu * 32) : "memory");
         }
-        if (wu == 0 && g == 0 && tv) {
-          const int t = tc + ti;
-          const int64_t ot = a.perm_t[t];
-#pragma unroll
-          for (int r = 0; r < RB; ++r)
-            if (r0 + r < a.R && out)
-              out[(int64_t)(r0 + r) * a.nt + ot] = (T)(acc[r] + (a.pot ? a.pot[(int64_t)(r0 + r) * a.nt + t] : 0.0));
-          if constexpr (GRAD) {
-#pragma unroll
-            for (int q = 0; q < D; ++q)
-              grad[((int64_t)r0 * a.nt + ot) * D + q] =
-                  acc[RB + q] + (a.potg ? a.potg[((int64_t)r0 * a.nt + t) * D + q] : 0.0);
-          }
-        }
+        if (wu == 0 && g == 0 && tv) near_store<D, RB, GRAD>(a, acc, r0, tc + ti, out, grad);
       }
     }
   }
+}
+
+// Sparse leaves in 1-D and 2-D: a warp per leaf row, its lanes split as
+// (target, source subset), that walks the row's few neighbours in global
+// memory.  With a handful of sources in all, the latency of the row's loads is
+// what counts, and this form keeps twice the warps of k_near64 and has no list
+// to make: against it, us, 262,144 clustered points in 1-D 95 -> 46 (3 rhs 211
+// -> 117), in 2-D 158 -> 97 (gradient 291 -> 135), 20,000 uniform points in 2-D
+// 25 -> 19.  From about five points a leaf in 1-D and two in 2-D k_near64 is as
+// fast or faster (10 points, 1-D, 256 leaves x 4 rhs 15 against 27), and in 3-D,
+// with up to 27 neighbours, at one point a leaf already.
+template <int KID, int D, int RB, bool GRAD, typename T>
+__global__ void __launch_bounds__(kNearThreads) k_near64_sparse(const NearArgs a, T* __restrict__ out,
+                                                                double* __restrict__ grad) {
+  constexpr int NA = RB + (GRAD ? D : 0);
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * kNearThreads) >> 5;
+  for (int64_t row = ((int64_t)blockIdx.x * kNearThreads + threadIdx.x) >> 5; row < a.nrow; row += nw) {
+    const int b = a.row_box[row];
+    const int t0 = a.tb[b], t1 = a.te[b];
+    for (int tc = t0; tc < t1; tc += 32) {
+      const int cnt = min(32, t1 - tc);
+      int lanes = 1;
+      while (lanes < cnt) lanes <<= 1;
+      const int G = 32 / lanes, ti = lane & (lanes - 1), g = lane / lanes;
+      const bool tv = ti < cnt;
+      double x[D];
+#pragma unroll
+      for (int q = 0; q < D; ++q) x[q] = tv ? a.tx[(int64_t)q * a.nt + tc + ti] : 0.0;
+      for (int r0 = 0; r0 < a.R; r0 += RB) {
+        double acc[NA];
+#pragma unroll
+        for (int r = 0; r < NA; ++r) acc[r] = 0.0;
+        if (tv) {
+          for (int k = 0; k < a.nnear; ++k) {
+            const int s = a.near[row * a.nnear + k];
+            if (s < 0) continue;
+            const int j1 = a.se[s];
+            for (int j = a.sb[s] + g; j < j1; j += G) {
+              double y[D];
+#pragma unroll
+              for (int q = 0; q < D; ++q) y[q] = a.sx[(int64_t)q * a.ns + j];
+              const double f = keval<KID, D>(x, y, a.p0);
+#pragma unroll
+              for (int r = 0; r < RB; ++r)
+                if (r0 + r < a.R) acc[r] += a.ws[(int64_t)(r0 + r) * a.ns + j] * f;
+              if constexpr (GRAD) {
+                double gr[D];
+                kgrad_x<KID, D>(x, y, a.p0, gr);
+                const double w = a.ws[(int64_t)r0 * a.ns + j];
+#pragma unroll
+                for (int q = 0; q < D; ++q) acc[RB + q] += w * gr[q];
+              }
+            }
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < NA; ++r)
+          for (int o = lanes; o < 32; o <<= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+        if (g == 0 && tv) near_store<D, RB, GRAD>(a, acc, r0, tc + ti, out, grad);
+      }
+    }
+  }
+}
+
+// Where the sparse form runs: fewer than 16 sources in a mean row's list, all
+// of whose neighbours are taken to exist.
+bool near_sparse(const NearArgs& a, int d, int64_t nbox) {
+  return d < 3 && a.ns * a.nnear < 16 * nbox;
 }
 
 // The two cuts of the near field.  slots: a row's chunks of 32 targets, so
@@ -234,7 +308,8 @@ __global__ void __launch_bounds__(kNearThreads, GRAD || RB > 2 ? 2 : 3) k_near64
 // them: from 48 sources when the units fill less than a quarter of the warps
 // the GPU holds (24 an SM), from 192 when less than all, from 400 below eight
 // waves.  That is in pairs of 1/r; a pair of another kernel counts by what it
-// costs against it (log r 4, the Gaussian 3, a root or division 2.5).  us with one warp and with four, 1/r, uniform points, one
+// costs against it (log r 4, the Gaussian 3, a root or division 2.5), but the
+// last line takes 192 sources, six tiles, at least.  us with one warp and with four, 1/r, uniform points, one
 // rhs: 96 units x 240 sources 23 and 13, 128 x 30 both 9; 2,048 x 360 40 and 36,
 // x 60 13 and 21; 8,192 x 1,080 284 and 232, x 60 30 and 56; 32,768 x 30 54 and
 // 150 (four rhs 118 and 365).  The list's length is estimated from the mean
@@ -251,8 +326,8 @@ NearArgs near_args(fmma_ctx* ctx, int nnear, const Tree& tr, const double* tx, c
   const int cost = k == FMMA_KERNEL_INV_R || k == FMMA_KERNEL_INV_R_SAFE
                        ? 10
                        : (k == FMMA_KERNEL_LOG_R ? 40 : (k == FMMA_KERNEL_GAUSSIAN ? 30 : 25));
-  const int64_t list = tr.ns * nnear * cost / (10 * std::max<int64_t>(1, Lf.nbox));  // a unit's sources
-  const int64_t most = list >= 400 ? 8 * warps : (list >= 192 ? warps : (list >= 48 ? warps / 4 : 0));
+  const int64_t list = tr.ns * nnear / std::max<int64_t>(1, Lf.nbox), work = list * cost / 10;  // of a unit
+  const int64_t most = work >= 400 && list >= 192 ? 8 * warps : (work >= 192 ? warps : (work >= 48 ? warps / 4 : 0));
   a.wpu = units < most ? kNearWarps / 2 : 1;
   return a;
 }
@@ -269,6 +344,15 @@ struct NearLaunch {
   static void run(fmma_ctx* ctx, const Tree& tr, const double* tx, const double* sx, const double* ws, int R,
                   const double* pot, T* out) {
     const NearArgs a = near_args(ctx, D == 1 ? 3 : (D == 2 ? 9 : 27), tr, tx, sx, ws, R, pot, nullptr);
+    if constexpr (D < 3) {
+      if (near_sparse(a, D, tr.lev[0].nbox)) {
+        const unsigned g = grid_for(a.nrow * 32, kNearThreads, (int64_t)ctx->sm_count * 16);
+        if (R == 1) FMMA_LAUNCH(ctx, (k_near64_sparse<KID, D, 1, false, T>), g, kNearThreads, 0, a, out, nullptr);
+        else if (R <= 4) FMMA_LAUNCH(ctx, (k_near64_sparse<KID, D, 4, false, T>), g, kNearThreads, 0, a, out, nullptr);
+        else FMMA_LAUNCH(ctx, (k_near64_sparse<KID, D, 8, false, T>), g, kNearThreads, 0, a, out, nullptr);
+        return;
+      }
+    }
     const unsigned g = near_grid(ctx, a);
     if (R == 1) FMMA_LAUNCH(ctx, (k_near64<KID, D, 1, false, T>), g, kNearThreads, 0, a, out, nullptr);
     else if (R == 2) FMMA_LAUNCH(ctx, (k_near64<KID, D, 2, false, T>), g, kNearThreads, 0, a, out, nullptr);
@@ -282,6 +366,13 @@ struct NearGradLaunch {
   static void run(fmma_ctx* ctx, const Tree& tr, const double* tx, const double* sx, const double* ws, int R,
                   const double* pot, const double* potg, double* out, double* grad) {
     const NearArgs a = near_args(ctx, D == 1 ? 3 : (D == 2 ? 9 : 27), tr, tx, sx, ws, R, pot, potg);
+    if constexpr (D < 3) {
+      if (near_sparse(a, D, tr.lev[0].nbox)) {
+        FMMA_LAUNCH(ctx, (k_near64_sparse<KID, D, 1, true, double>),
+                    grid_for(a.nrow * 32, kNearThreads, (int64_t)ctx->sm_count * 16), kNearThreads, 0, a, out, grad);
+        return;
+      }
+    }
     FMMA_LAUNCH(ctx, (k_near64<KID, D, 1, true, double>), near_grid(ctx, a), kNearThreads, 0, a, out, grad);
   }
 };

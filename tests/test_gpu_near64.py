@@ -126,3 +126,33 @@ def test_units_of_one_and_of_four_warps(ctx, oracle, d, depth, per, rhs):
     got, _ = ctx.solve(t, s, w if rhs > 1 else w[0].copy(), poly_ord=1, depth=depth)
     want, _ = oracle.fmm(d, 1, 0.0, 1, depth, 1, t, s, w[rhs - 1].copy())
     assert rel_l2(np.atleast_2d(got)[rhs - 1], want) <= 1e-12
+
+
+@pytest.mark.parametrize("d,depth,per", [(1, 11, 1), (1, 11, 4), (1, 11, 5), (1, 11, 6), (2, 7, 1), (2, 7, 2)])
+@pytest.mark.parametrize("kid", [1, 4])
+def test_sparse_leaves(ctx, oracle, d, depth, per, kid):
+    # lists of fewer than 16 sources in 1-D and 2-D have a form of their own: both sides of the line, one to nine rhs
+    # the gradient is below, where the near field is all there is
+    r = np.random.default_rng(10 * d + per)
+    n = per * 2 ** (d * (depth - 1))
+    t, s, w = r.random((n, d)), r.random((n, d)), r.standard_normal((9, n))
+    ctx.set_kernel(kid, P0.get(kid, 0.0))
+    for rhs in (1, 3, 9):
+        got, _ = ctx.solve(t, s, w[:rhs] if rhs > 1 else w[0].copy(), poly_ord=1, depth=depth)
+        want, _ = oracle.fmm(d, kid, P0.get(kid, 0.0), 1, depth, 1, t, s, w[rhs - 1].copy())
+        assert rel_l2(np.atleast_2d(got)[rhs - 1], want) <= 1e-12
+
+
+@pytest.mark.parametrize("d", [1, 2])
+@pytest.mark.parametrize("kid", [1, 2, 4, 6])
+def test_gradient_on_sparse_leaves(ctx, d, kid):
+    # Depth 2 with a point or two a leaf: the direct sum, by the sparse form
+    if kid == 2 and d > 1:
+        pytest.skip("1/(x-y) is one-dimensional")
+    r = np.random.default_rng(kid)
+    ctx.set_kernel(kid, P0.get(kid, 0.0))
+    for n in (2, 3, 5):
+        t, s, w = r.random((n, d)), r.random((n, d)), r.standard_normal((2, n))
+        c, g, _ = ctx.solve_grad(t, s, w, poly_ord=2, depth=2)
+        ce, ge, _ = ctx.solve_grad(t, s, w, solver="exact")
+        assert rel_l2(c, ce) <= 1e-13 and rel_l2(g, ge) <= 1e-12
